@@ -43,7 +43,7 @@ struct trn_scene {
   float* light_cdf = nullptr;
   float* light_radiance = nullptr;
   float* light_integral_dev = nullptr;
-  float light_lum[64];
+  float* light_lum = nullptr;     // [64] luminance per light (device)
   std::vector<float> h_light_radiance;
   // materials
   trn::BsdfDesc* bsdfs = nullptr;
@@ -90,16 +90,12 @@ struct trn_scene {
   unsigned long long* keys_alt = nullptr; // [T]
   void* sort_tmp = nullptr;
   size_t sort_tmp_bytes = 0;
-  // PLOC build scratch (cluster node ids and boxes, current + merged copies)
-  int* ploc_node = nullptr;       // [2][T]
-  float* ploc_box = nullptr;      // [2][T][6]
-  int* ploc_nn = nullptr;         // [T]
-  int* ploc_flag = nullptr;       // [T]
-  int* ploc_pos = nullptr;        // [T]
-  int* ploc_count = nullptr;      // [3] merge counter, cluster count, rounds that merged
-  int ploc_rounds = 0;            // rounds the last build needed (0 = none yet)
-  void* scan_tmp = nullptr;
-  size_t scan_tmp_bytes = 0;
+  // clustering scratch: the clusters each node left, their boxes, where the two
+  // children of a node meet, merges so far
+  int* cluster_id = nullptr;      // [T]
+  float* cluster_box = nullptr;   // [2T][6]
+  int* cluster_meet = nullptr;    // [T]
+  int* cluster_count = nullptr;   // [1]
   float* bounds = nullptr;        // [6]
   trn::WNode* wnodes = nullptr;   // [<= T] 8-wide nodes
   float4* wtri = nullptr;         // [T][3]

@@ -1,0 +1,82 @@
+"""Ray queries against brute force at the sizes where the hierarchy's build and
+the traversal change form: one triangle (the root is a leaf), a few, the
+build's cluster size (16) and its double, one more or less than a warp; meshes
+in one plane, of equal triangles, with degenerate ones. The watertight test is
+individually rounded and ties go to the smaller triangle, so the results are
+those of the oracle bit for bit."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import tr_oracle as O
+from tensorray_b200 import api, scenes
+
+pytestmark = pytest.mark.gpu
+
+
+def _scene(P, F):
+    spec = scenes.SceneSpec()
+    spec.bsdfs = [scenes.BsdfSpec(scenes.DIFFUSE, (0.5, 0.5, 0.5))]
+    spec.meshes.append(scenes.MeshSpec(P.astype(np.float32), F.astype(np.int32), bsdf=0))
+    spec.cameras = [scenes.CameraSpec((0.0, 0.0, 4.0), (0.0, 0.0, 0.0), (0.0, 1.0, 0.0), 8, 8, 45.0)]
+    return api.Scene(spec)
+
+
+def _mesh(kind, n, rng):
+    c = rng.uniform(-1, 1, (n, 1, 3))
+    P = c + 0.4 * rng.normal(size=(n, 3, 3))
+    if kind == "plane":
+        P[:, :, 1] = -1.0
+    elif kind == "same":
+        P[:] = P[:1]
+    elif kind == "degenerate":
+        P[::2, 2] = P[::2, 1]
+    elif kind == "graded":  # a gradient of sizes, as at a sphere's pole
+        P = c * np.geomspace(1e-4, 1, n)[:, None, None] + 0.4 * np.geomspace(1e-4, 1, n)[:, None, None] * (P - c)
+    return P.reshape(-1, 3), np.arange(3 * n).reshape(n, 3)
+
+
+def _rays(n, rng):
+    org = rng.uniform(-2, 2, (n, 3))
+    d = rng.normal(size=(n, 3))
+    d[::7] = np.eye(3)[rng.integers(0, 3, len(d[::7]))] * rng.choice([-1.0, 1.0], (len(d[::7]), 1))  # along an axis
+    d /= np.linalg.norm(d, axis=1, keepdims=True)
+    tmin, tmax = np.full(n, 1e-2), np.full(n, 1e32)
+    tmin[::5], tmax[::5] = -3.0, 0.5     # an interval that starts behind the origin
+    f = lambda x: torch.as_tensor(np.ascontiguousarray(x, np.float32))
+    return f(org), f(d), f(tmin), f(tmax)
+
+
+@pytest.mark.parametrize("kind,n", [("soup", 1), ("soup", 2), ("soup", 3), ("soup", 5), ("soup", 16), ("soup", 17),
+                                    ("soup", 31), ("soup", 32), ("soup", 33), ("soup", 129), ("soup", 2000),
+                                    ("plane", 40), ("same", 40), ("degenerate", 40), ("graded", 300)])
+def test_queries_match_brute_force(built_lib, kind, n):
+    rng = np.random.default_rng(n)
+    P, F = _mesh(kind, n, rng)
+    scene = _scene(P, F)
+    pos = torch.as_tensor(P.astype(np.float32)).reshape(n, 3, 3)
+    for refit in (False, True):
+        scene.configure(refit=refit)
+        for count in (1, 31, 700):
+            org, d, tmin, tmax = _rays(count, rng)
+            ref = O.intersect_brute(pos[:, 0], pos[:, 1], pos[:, 2], org, d, tmin, tmax)
+            got = [x.cpu() for x in scene.intersect(*(x.cuda() for x in (org, d, tmin, tmax)))]
+            assert torch.equal(got[0].long(), ref[0])
+            hit = ref[0] >= 0
+            for a, b in zip(got[1:], ref[1:]):
+                assert torch.equal(a[hit], b[hit])
+            vis = scene.occluded(*(x.cuda() for x in (org, d, tmin, tmax))).cpu()
+            assert torch.equal(vis, (~hit).int())
+
+
+def test_rays_without_a_direction_hit_nothing(built_lib):
+    rng = np.random.default_rng(0)
+    scene = _scene(*_mesh("soup", 200, rng))
+    scene.configure()
+    org, d, tmin, tmax = _rays(64, rng)
+    d[::3] = 0.0
+    d[1::3, 1] = float("nan")
+    org[2::3, 0] = float("nan")
+    args = [x.cuda() for x in (org, d, tmin, tmax)]
+    assert bool((scene.intersect(*args)[0] == -1).all())
+    assert bool((scene.occluded(*args) == 1).all())
