@@ -15,6 +15,7 @@
 #include "../../include/trn.h"
 #include "scene_impl.cuh"
 #include "shading.cuh"
+#include "cdf.cuh"
 
 namespace trn {
 
@@ -2824,40 +2825,6 @@ __global__ void k_prim_edges_views(int ne, const int* edges, const float* pos, c
   func_all[(long long)v * ne + e] = valid ? length(make_f3(pos + 3 * v1) - p0) : 0.f;
 }
 
-// Distribution1D::SetFunction for one block per view (prefix sums in double)
-// Distribution1D::SetFunction over n weights by one block (see k_cdf).
-TRN_D void cdf_block(int n, const float* func, float* cdf, float* integral_out) {
-  __shared__ double part[1024];
-  __shared__ float integral;
-  const int T = blockDim.x, tid = threadIdx.x;
-  const int chunk = (n + T - 1) / T;
-  const int a = min(n, tid * chunk), b = min(n, a + chunk);
-  double sacc = 0.0;
-  for (int i = a; i < b; i++) sacc += (double)func[i];
-  part[tid] = sacc;
-  __syncthreads();
-  if (tid == 0) { double run = 0.0; for (int i = 0; i < T; i++) { double x = part[i]; part[i] = run; run += x; } }
-  __syncthreads();
-  const float inv_size = 1.0f / (float)n;
-  double run = part[tid];
-  for (int i = a; i < b; i++) { run += (double)func[i]; cdf[i] = (float)run * inv_size; }
-  __syncthreads();
-  if (tid == 0) { integral = n > 0 ? cdf[n - 1] : 0.f; *integral_out = integral; }
-  __syncthreads();
-  if (integral > 0.f) for (int i = a; i < b; i++) cdf[i] = cdf[i] / integral;
-}
-
-// one distribution per block: view v's n weights at func_all + v n
-__global__ void k_cdf_views(int n, const float* func_all, float* cdf_all, float* integral_all) {
-  const int v = blockIdx.x;
-  cdf_block(n, func_all + (long long)v * n, cdf_all + (long long)v * n, integral_all + v);
-}
-
-// one distribution whose length is in device memory (the guiding tree's leaves)
-__global__ void k_cdf_count(const int* count, const float* func, float* cdf, float* integral) {
-  cdf_block(__ldg(count), func, cdf, integral);
-}
-
 // 0.5 |I - T|^2 per view and dL/dI = I - T (pyTensorRay/loss.py:34-38)
 __global__ void k_view_loss(long long npix, const ViewDesc* views, const long long* pbegin, int nviews,
                             const float* img, const float* tgt, float* dLdI, float* loss) {
@@ -2933,6 +2900,7 @@ struct trn_viewset {
   float* pfunc = nullptr;         // device [nviews][E]
   float* pcdf = nullptr;          // device [nviews][E]
   float* pint = nullptr;          // device [nviews]
+  double* pint_part = nullptr;    // device [nviews][kCdfChunks]
   unsigned long long* work = nullptr;
   // queue of the split indirect boundary term: one round of at most
   // kIndirectRound slots at a time
@@ -3183,8 +3151,8 @@ int guide_setup(trn_scene* s, const trn_render_options* o, Params& P, cudaStream
   k_aq_poly<<<(unsigned)((limit + 255) / 256), 256, 0, st>>>(G, stream, o->g_direct_spp, s->aq_box, s->aq_edge,
                                                               s->aq_count, cap, s->aq_poly);
   k_aq_mix<<<1, 1024, 0, st>>>(s->aq_count, s->aq_poly, s->aq_box, cap, o->g_eps, s->aq_func, s->aq_int);
-  k_cdf_count<<<1, 1024, 0, st>>>(s->aq_count, s->aq_func, s->aq_cdf, s->aq_int);
-  count_launch(launches + 3);
+  count_launch(launches + 2 +
+               cdf_launch(1, (int)limit, s->aq_count, s->aq_func, s->aq_cdf, s->aq_int, s->cdf_part, st));
   TRN_CUDA_TRY(cudaGetLastError());
   P.aq_poly = s->aq_poly;
   P.aq_cdf = s->aq_cdf;
@@ -3655,8 +3623,7 @@ int render_views(trn_scene* s, trn_viewset* vs, const trn_render_options* o, int
     if (s->ne == 0) return 0;
     dim3 g((s->ne + 255) / 256, vs->nviews);
     k_prim_edges_views<<<g, 256, 0, st>>>(s->ne, s->edges, s->pos, s->fnormal, vs->views, vs->pfunc);
-    k_cdf_views<<<vs->nviews, 1024, 0, st>>>(s->ne, vs->pfunc, vs->pcdf, vs->pint);
-    count_launch(2);
+    count_launch(1 + cdf_launch(vs->nviews, s->ne, nullptr, vs->pfunc, vs->pcdf, vs->pint, vs->pint_part, st));
   } else if ((integrator == TRN_DIRECT_EDGE || integrator == TRN_INDIRECT_EDGE) && s->ne == 0) {
     return 0;
   }
@@ -3711,17 +3678,19 @@ int set_views(trn_viewset* vs, int nviews, const trn_view* views) {
   }
   if (nviews > vs->cap) {
     wait_stages(vs);
-    void* old[] = {vs->views, vs->vbegin, vs->pbegin, vs->pfunc, vs->pcdf, vs->pint};
+    void* old[] = {vs->views, vs->vbegin, vs->pbegin, vs->pfunc, vs->pcdf, vs->pint, vs->pint_part};
     for (void* q : old) if (q) cudaFree(q);
     if (vs->h_stage) cudaFreeHost(vs->h_stage);
     if (vs->h_stage_begin) cudaFreeHost(vs->h_stage_begin);
     vs->views = nullptr; vs->vbegin = vs->pbegin = nullptr; vs->pfunc = vs->pcdf = vs->pint = nullptr;
+    vs->pint_part = nullptr;
     vs->h_stage = nullptr; vs->h_stage_begin = nullptr;
     const int cap = std::max(nviews, 2 * vs->cap);
     bool ok = cudaMalloc(&vs->views, sizeof(ViewDesc) * cap) == cudaSuccess &&
               cudaMalloc(&vs->vbegin, sizeof(long long) * cap) == cudaSuccess &&
               cudaMalloc(&vs->pbegin, sizeof(long long) * cap) == cudaSuccess &&
               cudaMalloc(&vs->pint, sizeof(float) * cap) == cudaSuccess &&
+              cudaMalloc(&vs->pint_part, sizeof(double) * kCdfChunks * cap) == cudaSuccess &&
               cudaMallocHost(&vs->h_stage, sizeof(ViewDesc) * cap * kStageRing) == cudaSuccess &&
               cudaMallocHost(&vs->h_stage_begin, sizeof(long long) * 2 * cap * kStageRing) == cudaSuccess;
     if (ok && vs->ne > 0)
@@ -3805,7 +3774,7 @@ int trn_viewset_update(trn_viewset* vs, int nviews, const trn_view* views) {
 int trn_viewset_destroy(trn_viewset* vs) {
   if (!vs) return 0;
   wait_stages(vs);
-  void* ptrs[] = {vs->views, vs->vbegin, vs->pbegin, vs->pfunc, vs->pcdf, vs->pint, vs->work, vs->iq, vs->iq_count, vs->sq, vs->pc, vs->pc_count};
+  void* ptrs[] = {vs->views, vs->vbegin, vs->pbegin, vs->pfunc, vs->pcdf, vs->pint, vs->pint_part, vs->work, vs->iq, vs->iq_count, vs->sq, vs->pc, vs->pc_count};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (vs->h_stage) cudaFreeHost(vs->h_stage);
@@ -3914,13 +3883,14 @@ int trn_render_grad(trn_scene* s, const trn_camera* cam, const trn_render_option
 // Scratch layout (each part 256-byte aligned): the view table (one ViewDesc),
 // the first-sample index of that view, the work counter, the silhouette
 // integral, then the silhouette function and its CDF (kNoAllocMaxEdges floats
-// each). Every call rewrites all of it that it reads, so it keeps the last
+// each), then the CDF's chunk sums. Every call rewrites all of it that it reads, so it keeps the last
 // call's contents but never needs clearing from the outside. Two calls that
 // overlap in time on one device share this one array and race; such callers
 // must serialise them.
 constexpr int kNoAllocMaxEdges = 1 << 20;
 constexpr size_t kNoAllocHeader = 4096;  // ViewDesc, vbegin, work counter, integral
-constexpr size_t kNoAllocScratchBytes = kNoAllocHeader + 2 * sizeof(float) * (size_t)kNoAllocMaxEdges;
+constexpr size_t kNoAllocScratchBytes =
+    kNoAllocHeader + 2 * sizeof(float) * (size_t)kNoAllocMaxEdges + kCdfChunks * sizeof(double);
 static_assert(sizeof(ViewDesc) + 3 * 256 <= kNoAllocHeader, "view table does not fit the scratch header");
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratchBytes];
@@ -4007,6 +3977,7 @@ int trn_render_grad_noalloc(trn_scene* s, const trn_camera* cam, const trn_rende
   float* pint = (float*)(base + kNoAllocHeader - 256);
   float* pfunc = (float*)(base + kNoAllocHeader);
   float* pcdf = pfunc + kNoAllocMaxEdges;
+  double* part = (double*)(pcdf + kNoAllocMaxEdges);
 
   ViewDesc v;
   std::memset(&v, 0, sizeof(v));
@@ -4050,8 +4021,7 @@ int trn_render_grad_noalloc(trn_scene* s, const trn_camera* cam, const trn_rende
   if (integrator == TRN_PRIMARY_EDGE) {
     dim3 g((s->ne + 255) / 256, 1);
     k_prim_edges_views<<<g, 256, 0, st>>>(s->ne, s->edges, s->pos, s->fnormal, table, pfunc);
-    k_cdf_views<<<1, 1024, 0, st>>>(s->ne, pfunc, pcdf, pint);
-    count_launch(2);
+    count_launch(1 + cdf_launch(1, s->ne, nullptr, pfunc, pcdf, pint, part, st));
   }
   // the guiding distribution lives in buffers the scene allocated at creation
   // (a refined tree in those of an earlier allocating call)

@@ -22,6 +22,7 @@
 
 #include "../../include/trn.h"
 #include "scene_impl.cuh"
+#include "cdf.cuh"
 
 namespace trn {
 
@@ -97,37 +98,6 @@ __global__ void k_sec_edges(int ne, const int* edges, const float* pos, const fl
     valid = valid0 && valid1;
   }
   func[e] = valid ? length(p1 - p0) : 0.f;
-}
-
-// Distribution1D::SetFunction over n weights: cdf_i = (S_i / n) / (S_n / n),
-// prefix sums accumulated in double in a fixed order.
-__global__ void k_cdf(int n, const float* func, float* cdf, float* integral_out) {
-  __shared__ double part[1024];
-  const int T = blockDim.x;
-  const int tid = threadIdx.x;
-  const int chunk = (n + T - 1) / T;
-  const int a = min(n, tid * chunk), b = min(n, a + chunk);
-  double s = 0.0;
-  for (int i = a; i < b; i++) s += (double)func[i];
-  part[tid] = s;
-  __syncthreads();
-  if (tid == 0) {
-    double run = 0.0;
-    for (int i = 0; i < T; i++) { double x = part[i]; part[i] = run; run += x; }
-  }
-  __syncthreads();
-  const float inv_size = 1.0f / (float)n;
-  double run = part[tid];
-  for (int i = a; i < b; i++) {
-    run += (double)func[i];
-    cdf[i] = (float)run * inv_size;
-  }
-  __syncthreads();
-  __shared__ float integral;
-  if (tid == 0) { integral = n > 0 ? cdf[n - 1] : 0.f; if (integral_out) *integral_out = integral; }
-  __syncthreads();
-  if (integral > 0.f)
-    for (int i = a; i < b; i++) cdf[i] = cdf[i] / integral;
 }
 
 // ---------------------------------------------------------------------------
@@ -985,6 +955,7 @@ int trn_scene_create(const trn_scene_desc* d, trn_scene** out) {
       dev_alloc_copy(&s->light_radiance, s->h_light_radiance.data(), s->h_light_radiance.size()) ||
       dev_alloc_copy(&s->light_integral_dev, (const float*)nullptr, 1) ||
       dev_alloc_copy(&s->light_lum, lum.data(), lum.size()) ||
+      dev_alloc_copy(&s->cdf_part, (const double*)nullptr, kCdfChunks) ||
       dev_alloc_copy(&s->bsdfs, s->h_bsdfs.data(), s->h_bsdfs.size()) ||
       dev_alloc_copy(&s->texs, texs.data(), std::max<size_t>(texs.size(), 0)) ||
       dev_alloc_copy(&s->edges, edges.data(), edges.size()) ||
@@ -1057,7 +1028,7 @@ int trn_scene_destroy(trn_scene* s) {
   void* ptrs[] = {s->raw_pos, s->translation, s->texels, s->pos, s->idx, s->fnormal, s->area, s->vnormal,
                   s->smooth, s->uv, s->uvidx, s->bsdf_id, s->emitter_id, s->vert_mesh, s->vf_off, s->vf_list,
                   s->emit_tris, s->tri_to_emit, s->light_func, s->light_cdf, s->light_radiance,
-                  s->light_integral_dev, s->light_lum, s->bsdfs, s->texs, s->edges, s->sec_func, s->sec_cdf,
+                  s->light_integral_dev, s->light_lum, s->cdf_part, s->bsdfs, s->texs, s->edges, s->sec_func, s->sec_cdf,
                   s->sec_integral_dev, s->nodes, s->tri_verts, s->parent, s->flags, s->keys, s->keys_alt,
                   s->sort_tmp, s->bounds, s->g_pos, s->g_vnormal, s->g_texels, s->g_translation, s->err,
                   s->stats, s->wnodes, s->wtri, s->wqueue, s->wcount, s->aq_poly, s->aq_func, s->aq_cdf,
@@ -1084,14 +1055,12 @@ int configure_geometry(trn_scene* s, cudaStream_t st) {
   if (s->n_emit > 0) {
     k_light_func<<<nblk(s->n_emit), 256, 0, st>>>(s->n_emit, s->emit_tris, s->emitter_id, s->light_lum, s->area,
                                                    s->light_func);
-    k_cdf<<<1, 1024, 0, st>>>(s->n_emit, s->light_func, s->light_cdf, s->light_integral_dev);
-    count_launch(2);
+    count_launch(1 + cdf_launch(1, s->n_emit, nullptr, s->light_func, s->light_cdf, s->light_integral_dev, s->cdf_part, st));
   }
   // secondary edge list
   if (s->ne > 0) {
     k_sec_edges<<<nblk(s->ne), 256, 0, st>>>(s->ne, s->edges, s->pos, s->fnormal, s->sec_func);
-    k_cdf<<<1, 1024, 0, st>>>(s->ne, s->sec_func, s->sec_cdf, s->sec_integral_dev);
-    count_launch(2);
+    count_launch(1 + cdf_launch(1, s->ne, nullptr, s->sec_func, s->sec_cdf, s->sec_integral_dev, s->cdf_part, st));
   }
   return 0;
 }

@@ -44,6 +44,7 @@ struct trn_scene {
   float* light_radiance = nullptr;
   float* light_integral_dev = nullptr;
   float* light_lum = nullptr;     // [64] luminance per light (device)
+  double* cdf_part = nullptr;     // chunk sums of a distribution being built
   std::vector<float> h_light_radiance;
   // materials
   trn::BsdfDesc* bsdfs = nullptr;
