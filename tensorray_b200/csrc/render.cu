@@ -173,17 +173,14 @@ TRN_D void atomic_add3(float* a, const F3& g) {
   if (g.z != 0.f) atomicAdd(a + 2, g.z);
 }
 
-// Per-warp staging area for aggregated scatters (one per block, 8 warps max).
-TRN_D float* warp_scratch() {
-  __shared__ float buf[8 * 32 * 3];
-  return buf + (threadIdx.x >> 5) * 96;
-}
-
-// Warp-aggregated scatter-add of a float3 into base[3*idx]: lanes of the
-// converged warp that target the same index first sum in shared memory, then
-// one lane per distinct index issues the global atomics. Replaces the plain
-// per-element atomicAdd of IndexedWriteKernel (TensorKernels.cuh:177-209),
+// Warp-aggregated scatter-add of a float3 into base[3*idx]: the lanes of the
+// converged warp that target the same address first sum up by shuffles, in
+// log2 rounds (odd ranks of a group drop out after handing over their value),
+// then one lane per distinct address issues the global atomics. Replaces the
+// plain per-element atomicAdd of IndexedWriteKernel (TensorKernels.cuh:177-209),
 // which serialises when many paths hit the same few vertices (quads, lights).
+// (Summing in shared memory instead serialised such groups as well: a float
+// atomicAdd on shared memory is a compare-and-swap loop.)
 TRN_D void agg_add3(float* base, long long idx, const F3& g) {
   const unsigned active = __activemask();
   const int lane = threadIdx.x & 31;
@@ -191,16 +188,19 @@ TRN_D void agg_add3(float* base, long long idx, const F3& g) {
   // scatter into different views' gradient buffers
   float* const target = base + 3 * idx;
   const unsigned peers = __match_any_sync(active, reinterpret_cast<unsigned long long>(target));
-  const int leader = __ffs(peers) - 1;
-  float* w = warp_scratch();
-  if (lane == leader) { w[3 * lane] = g.x; w[3 * lane + 1] = g.y; w[3 * lane + 2] = g.z; }
-  __syncwarp(active);
-  if (lane != leader) {
-    atomicAdd(w + 3 * leader, g.x); atomicAdd(w + 3 * leader + 1, g.y); atomicAdd(w + 3 * leader + 2, g.z);
+  const unsigned lt = (1u << lane) - 1u;
+  unsigned rank = __popc(peers & lt);
+  const bool leader = rank == 0u;
+  unsigned rest = peers & ~lt & ~(1u << lane);
+  F3 x = g;
+  while (__any_sync(active, rest != 0u)) {
+    const int next = rest ? __ffs(rest) - 1 : lane;
+    const F3 t(__shfl_sync(active, x.x, next), __shfl_sync(active, x.y, next), __shfl_sync(active, x.z, next));
+    if (rest) x = x + t;
+    rest &= __ballot_sync(active, !(rank & 1u));
+    rank >>= 1;
   }
-  __syncwarp(active);
-  if (lane == leader) atomic_add3(target, F3(w[3 * lane], w[3 * lane + 1], w[3 * lane + 2]));
-  __syncwarp(active);
+  if (leader) atomic_add3(target, x);
 }
 TRN_D F3 g_at(const Params& P, const ViewDesc& V, int pix) {
   if (pix < 0) return F3z();
