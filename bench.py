@@ -6,7 +6,7 @@ value noise, GGX microfacet (roughness 0.3) with a 512x512 albedo texture,
 ground quad and quad light, 512x512 pixels, 64 spp per term, depth 5, all
 boundary terms (primary, direct, indirect, pixel), gradients w.r.t. every
 vertex position and the texture. One step = parameter upload to the scene +
-Scene::Configure (geometry chain + LBVH rebuild) + PathTracer.renderC +
+Scene::Configure (geometry chain + BVH rebuild) + PathTracer.renderC +
 dL/dI of 0.5*|I - I_target|^2 + renderD of all five integrators + the
 geometry adjoint. A grad path-sample is one sample slot processed forward +
 adjoint by one integrator: W*H*spp per enabled term.
@@ -302,15 +302,18 @@ def run_single(a):
     # span is the term's production kernels (set-up rounds, edge keys and
     # their radix sort, body stages)
     kernel_names = ["interior_fwd", "interior_adj", "primary", "direct", "indirect", "pixel"]
+    path_kernels = ["k_wf_camera", "k_trace", "k_wf_start", "k_wf_shade", "k_wf_pixels"]
     term_kernels = {
-        "interior_fwd": ["k_path_fwd_rec_regen"] if not a.no_path_cache else ["k_path_fwd"],
-        "interior_adj": (["k_path_reverse<8,true> (over the forward's path records)"] if not a.no_path_cache
-                         else ["k_path_replay", "k_path_reverse"]),
-        "primary": ["k_edge_keys", "cub radix sort", "k_primary_setup", "k_primary_body_regen"],
-        "direct": ["k_edge_keys", "cub radix sort", "k_direct_setup", "k_direct_body"],
-        "indirect": ["k_edge_keys", "cub radix sort", "k_indirect_setup", "k_indirect_sensor_regen",
-                     "k_indirect_emitter_regen"],
-        "pixel": ["k_pixel_setup", "k_primary_body_regen"],
+        "interior_fwd": path_kernels,
+        "interior_adj": (["k_path_reverse<true> (over the forward's path records)"] if not a.no_path_cache
+                         else path_kernels[:-1] + ["k_path_reverse<false>"]),
+        "primary": ["k_edge_keys", "cub radix sort", "k_setup_*", "k_trace", "k_wf_start", "k_wf_shade",
+                    "k_wf_body_scatter"],
+        "direct": ["k_edge_keys", "cub radix sort", "k_setup_*", "k_trace", "k_wi_start", "k_wi_step",
+                   "k_wi_direct_scatter"],
+        "indirect": ["k_edge_keys", "cub radix sort", "k_setup_*", "k_trace", "k_wi_*", "k_wf_start", "k_wf_shade",
+                     "k_wf_emit_scatter"],
+        "pixel": ["k_setup_*", "k_trace", "k_wf_start", "k_wf_shade", "k_wf_body_scatter"],
     }
     units_per_step = a.res * a.res * a.spp * 5
     V0 = scene._raw_positions.clone()
@@ -408,7 +411,7 @@ def run_single(a):
             dist.all_reduce(t, op=dist.ReduceOp.MAX)
         replay = {"value": units_per_step * world / (float(t) / 1e3), "unit": "grad path-samples/s",
                   "ms_per_step": float(t), "steps": rsteps,
-                  "kernels": {"interior_fwd": ["k_path_fwd"], "interior_adj": ["k_path_replay", "k_path_reverse"]}}
+                  "kernels": {"interior_fwd": path_kernels, "interior_adj": path_kernels[:-1] + ["k_path_reverse<false>"]}}
         scene.set_path_cache(16 << 30)
 
     # ---- e2e: through the autograd.Function with host buffers ----
@@ -866,7 +869,7 @@ def run_inverse(a):
             "data": "synthetic (seeded displaced sphere target, seeded vertex perturbation)",
             "config": {"workload": f"inverse rendering, {tris} tris target, {nviews} views {res}^2, {spp} spp x "
                                    f"3 terms (interior+primary+guided direct, guiding tree depth {a.guide_depth}), depth {D}, Adam lr 1e-3, "
-                                   "LBVH refit per step; inputs larger than L2",
+                                   "BVH refit per step; inputs larger than L2",
                        "samples_per_step": units,
                        "parallelism": f"views sharded by cost over {world} rank(s), gradient all-reduce"},
             "loss": {"first": losses[0], "last": losses[-1], "per_step": losses},

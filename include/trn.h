@@ -128,9 +128,10 @@ typedef struct {
 
 /* Launch shape of the persistent integrator kernels (0 = library default):
  * threads per block, resident blocks per SM, sample slots each lane takes
- * per fetch from the work queue, and the sample slots (boundary terms) or
- * paths (interior adjoint) per round of the split kernels, log2, at most the
- * default (boundary 24, interior 21), at least 16. Chosen by the autotuner
+ * per fetch from the work queue (fused kernels), and the sample slots
+ * (boundary terms, image) or paths (replaying adjoint) per round of the
+ * wavefront, log2, at most the default (24; replaying adjoint 22), at least 16.
+ * Chosen by the autotuner
  * (tensorray_b200/autotune.py). */
 typedef struct {
   int block;
@@ -188,11 +189,11 @@ long long trn_mesh_edges(int num_triangles, const int* indices, int* out, long l
 
 /* Scene lifetime. Replaces Scene::Configure (Scene.cpp:522-533): create
  * uploads the description; configure runs Primitive::Configure, face/vertex
- * normals, light distribution, secondary edge list and the LBVH build. */
+ * normals, light distribution, secondary edge list and the BVH build. */
 int trn_scene_create(const trn_scene_desc* desc, trn_scene** out);
 int trn_scene_configure(trn_scene* scene, cudaStream_t stream);
 int trn_scene_destroy(trn_scene* scene);
-/* Re-run the geometry chain for new parameters and refit the LBVH boxes
+/* Re-run the geometry chain for new parameters and refit the BVH boxes
  * without rebuilding its topology (Scene::Update / UpdateAccelerationStructure,
  * Scene.cpp:368-469, 535-546). Falls back to trn_scene_configure the first time. */
 int trn_scene_refit(trn_scene* scene, cudaStream_t stream);
@@ -210,7 +211,7 @@ int trn_scene_get_geometry(trn_scene* scene, float* pos, float* fnormal, float* 
 int trn_scene_counts(const trn_scene* scene, int* num_vertices, int* num_triangles, int* num_edges,
                      long long* num_texels, int* num_meshes);
 
-/* Closest-hit ray query over the LBVH. Replaces RayIntersectOptix
+/* Closest-hit ray query over the BVH. Replaces RayIntersectOptix
  * (Optix.h:149, Optix.cpp:252-305): out_tri = -1 on a miss. Device arrays of
  * n rays: org/dir [n*3], tmin/tmax [n]; outputs tri [n], u/v/t [n]. */
 int trn_intersect(trn_scene* scene, int n, const float* org, const float* dir, const float* tmin,
@@ -249,10 +250,9 @@ int trn_render_grad(trn_scene* scene, const trn_camera* camera, const trn_render
  * array compiled into the library (about 8 MiB, held on every GPU that loads
  * the library until the process exits), and the call does not synchronise
  * the stream.
- * - Speed: it runs each term as one fused kernel (no split stages, no queues,
- *   no edge-sorted set-up order, since those need scratch that grows with
- *   the launch), which is about 20-50 % slower per term than
- *   trn_render_grad.
+ * - Speed: it runs each term as one fused kernel (no wavefront, no edge-sorted
+ *   set-up order, since those need scratch that grows with the launch), which
+ *   is slower per term than trn_render_grad but for a few 100K samples.
  * - Limit: for TRN_PRIMARY_EDGE the scene may have at most 1048576 edges;
  *   larger scenes are rejected with an error.
  * - A guided direct term with g_direct_depth > 0 needs the refined tree's
@@ -287,14 +287,13 @@ int trn_viewset_destroy(trn_viewset* views);
  * on one set must use one stream (the table is rewritten in stream order). */
 int trn_viewset_update(trn_viewset* views, int nviews, const trn_view* view_array);
 int trn_viewset_num_pixels(const trn_viewset* views, long long* npix);
-/* Allocate the set's round buffers now: the queue of the split integrator
- * kernels (one full round of any term at up to max_bounces) and the buffers
- * of the edge-sorted run order of the boundary set-up. Without it the first
- * gradient call of each term allocates them, and a larger batch later grows
+/* Allocate the set's round buffers now: the wavefront's (one full round of any
+ * term at up to max_bounces) and those of the edge-sorted run order of the
+ * boundary set-up. Without it the first call of each term allocates them, and a larger batch later grows
  * them (each growth synchronises the stream and frees the old buffer). For a
  * serving loop, or before capturing render calls into a CUDA graph. No
  * counterpart in the reference (its tensor library allocates per call).
- * About 5.5 GB for max_bounces <= 8 (rounds of 16M boundary samples). */
+ * About 6 GB for max_bounces <= 8 (rounds of 16M boundary samples). */
 int trn_viewset_reserve(trn_viewset* views, int max_bounces, cudaStream_t stream);
 /* Path cache. A forward render of TRN_PATH_TRACER can keep the record of
  * every path it traced (hit points, light samples, throughputs: about 620

@@ -519,8 +519,8 @@ class Scene:
               "trn_scene_set_texels")
 
     def configure(self, refit: bool = False) -> None:
-        """Scene::Configure (Scene.cpp:522-533): geometry chain + LBVH build, or
-        with refit=True Scene::Update: geometry chain + LBVH refit."""
+        """Scene::Configure (Scene.cpp:522-533): geometry chain + BVH build, or
+        with refit=True Scene::Update: geometry chain + BVH refit."""
         st = C.c_void_p(_stream())
         check(self._lib.trn_scene_set_translation(self._h, C.c_void_p(self._translation.data_ptr()), st),
               "trn_scene_set_translation")
@@ -801,7 +801,7 @@ class ViewSet:
         self.spps = [int(x) for x in spps]
 
     def reserve(self, max_bounces: int = 8) -> None:
-        """Allocate the split kernels' round buffers now (about 5.5 GB at
+        """Allocate the wavefront's round buffers now (about 6 GB at
         max_bounces <= 8), so that no later render call of this set allocates
         device memory or synchronises to grow them."""
         check(self.scene._lib.trn_viewset_reserve(self._h, int(max_bounces), C.c_void_p(_stream())),

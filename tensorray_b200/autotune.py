@@ -3,7 +3,7 @@
 For one (view set, integrator) pair it times every candidate launch shape --
 threads per block, resident blocks per SM, and the number of sample slots a
 lane takes per work-queue fetch -- with CUDA events and keeps the fastest.
-For the gradient calls it then times the round size of the split kernels
+For the gradient calls it then times the round size of the wavefront
 (sample slots per set-up/body round of the boundary terms, paths per round
 of the interior adjoint: smaller rounds need smaller queues, larger ones give
 each edge more samples per sort and fewer kernel tails) with that shape.
@@ -60,7 +60,7 @@ def tune(vs: api.ViewSet, integrator: int, options: api.RenderOptions, dLdI: tor
         ms = e0.elapsed_time(e1) / reps
         if ms < best_ms:
             best, best_ms = ln, ms
-    # round size of the split kernels, with the best shape (only sizes below
+    # round size of the wavefront, with the best shape (only sizes below
     # the call's slot count change anything)
     slots = vs.slots(integrator)
     for r in ROUND_LOG2:

@@ -14,7 +14,7 @@ CSRC = os.path.join(HERE, "csrc")
 LIBDIR = os.path.join(HERE, "_lib")
 LIB = os.path.join(LIBDIR, "libtrn.so")
 SOURCES = ["scene.cu", "render.cu"]
-HEADERS = ["common.cuh", "dual.cuh", "scene_types.cuh", "scene_impl.cuh", "shading.cuh", "trace.cuh", "cdf.cuh"]
+HEADERS = ["common.cuh", "dual.cuh", "scene_types.cuh", "scene_impl.cuh", "shading.cuh", "trace.cuh", "cdf.cuh", "wavefront.cuh"]
 
 NVCC_FLAGS = [
     "-O3",

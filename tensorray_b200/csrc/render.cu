@@ -54,11 +54,9 @@ struct Params {
   const int* aq_edge;         // [leaves] the secondary edge a leaf lies on
   const int* aq_n;            // leaf count
   long long aq_cap;
-  // queues of the split kernels (nullptr = fused kernel): q_count[0] counts
-  // `queue`, q_count[1] counts `queue2` (the indirect term's second stage),
-  // q_count[2] hands out the items of `queue` to a regenerating stage
+  // samples of a boundary term's round that passed its set-up (items), or the
+  // interior term's path records, and their count
   void* queue;
-  void* queue2;
   unsigned long long* q_count;
   long long q_cap;
   // run order of a split set-up round (nullptr = slot order): the i-th slot
@@ -66,6 +64,20 @@ struct Params {
   const unsigned* order;
   long long order_first;
 };
+
+// The wavefront kernels are launched with programmatic stream serialisation:
+// a kernel's blocks may become resident while the last blocks of the kernel
+// before it still run. Each kernel starts with this: it lets its own successor
+// come in as early, and waits until its predecessor has ended and its writes
+// are visible. (Nothing a wavefront kernel writes is read through the
+// non-coherent path, which may serve a line from before the wait.) A stage of a
+// small call takes a few us, about as long as the launch it then hides.
+TRN_D void stage_begin() {
+#if defined(__CUDA_ARCH__) && __CUDA_ARCH__ >= 900
+  asm volatile("griddepcontrol.launch_dependents;");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+#endif
+}
 
 // Slot that runs at position i of the current round.
 TRN_D long long slot_at(const Params& P, long long i) {
@@ -100,46 +112,6 @@ constexpr int kMaxDepth = 16;
 #ifndef TRN_MINB_REVERSE
 #define TRN_MINB_REVERSE 2
 #endif
-#ifndef TRN_MINB_FWDREC
-#define TRN_MINB_FWDREC 4
-#endif
-#ifndef TRN_MINB_INDIRECT
-#define TRN_MINB_INDIRECT 4
-#endif
-// the split forms' set-up kernels are latency-bound with little state: four
-// blocks per SM (64 registers) hide more of it (measured)
-#ifndef TRN_MINB_SETUP
-#define TRN_MINB_SETUP 4
-#endif
-#ifndef TRN_MINB_BODY
-#define TRN_MINB_BODY 4
-#endif
-// the indirect set-up traces the sensor-side ray first (1) or the
-// emitter-side ray first (0); a miss of the first skips the second
-#ifndef TRN_INDIRECT_SENSOR_FIRST
-#define TRN_INDIRECT_SENSOR_FIRST 0
-#endif
-// the indirect kernel's two set-up rays use the shared traversal
-#ifndef TRN_INDIRECT_SETUP_SHARED
-#define TRN_INDIRECT_SETUP_SHARED 1
-#endif
-// set-up rays of the other kernels: shared or inlined traversal (measured)
-#ifndef TRN_SETUP_SHARED_FWD
-#define TRN_SETUP_SHARED_FWD 0
-#endif
-#ifndef TRN_SETUP_SHARED_PATHADJ
-#define TRN_SETUP_SHARED_PATHADJ 0
-#endif
-#ifndef TRN_SETUP_SHARED_PRIMARY
-#define TRN_SETUP_SHARED_PRIMARY 1
-#endif
-#ifndef TRN_SETUP_SHARED_DIRECT
-#define TRN_SETUP_SHARED_DIRECT 0
-#endif
-#ifndef TRN_SETUP_SHARED_PIXEL
-#define TRN_SETUP_SHARED_PIXEL 0
-#endif
-
 // Per-thread work counters behind the roofline's algorithmic-byte model:
 // ray queries, shading vertices, light samples, gradient scatters, pixels.
 enum { kCntClosest = 0, kCntShadow, kCntShade, kCntSmooth, kCntTex, kCntLight, kCntVScatter, kCntNScatter,
@@ -386,26 +358,37 @@ TRN_D void scatter_point(const Params& P, const ViewDesc& V, int tri, float u, f
 // ---------------------------------------------------------------------------
 struct BounceRec {
   // NEE
-  int ltri; float lu, lv, lpdf, lmis; int nee_ok; F3 lLe;
+  int ltri; float lu, lv, lpdf, lmis; int nee_ok;
   // continuation
   float prev_pdf; float emis; F3 eLe;  // MIS weight and radiance at the next vertex
   int next_ok;
   int scrubbed;                        // contribution was non-finite
 };
 
-// Returns the contribution of this bounce (already NaN-scrubbed). On return
-// x/rdir/T hold the next vertex; the return flag says whether it exists.
-template <bool NI = false>
-TRN_D bool radiance_step(const DeviceScene& s, SurfF& x, F3& rdir, F3& T, float l0, float l1, float b0, float b1,
-                         float b2, F3& contrib, BounceRec* rec, Cnt& cnt) {
+// One bounce in two halves, so that the wavefront kernels can run the ray
+// queries between them: radiance_gen decides the shadow ray and the
+// continuation ray of a vertex and evaluates the next-event estimate as if the
+// light were visible; radiance_resolve adds what the queries showed.
+struct RadianceGen {
+  F3 nee;       // contribution of the light sample if it is visible
+  F3 sdir;      // shadow ray from the vertex: direction and end
+  float stmax;
+  bool shadow;  // the light sample needs the shadow ray
+  F3 wi;        // continuation ray and its density
+  float pdf;
+  bool cont;
+};
+
+// rec (may be null) takes the light sample's record.
+TRN_D void radiance_gen(const DeviceScene& s, const SurfF& x, const F3& rdir, const F3& T, float l0, float l1, float b0,
+                        float b1, float b2, RadianceGen& g, BounceRec* rec, Cnt& cnt) {
   const BsdfDesc b = s.bsdfs[x.bsdf];
   count_shade(cnt, s, x);
   long long texel;
   const F3 kd = bsdf_albedo(s, b, x.tu, x.tv, texel);
   const Frame<float> fr = make_frame(x.ns);
   const F3 wo = -rdir;
-  F3 val = F3z();
-  if (rec) { rec->nee_ok = 0; rec->next_ok = 0; rec->scrubbed = 0; }
+  g.shadow = false;
   LightSample ls;
   if (light_sample(s, l0, l1, ls)) {
     cnt.v[kCntLight]++;
@@ -419,33 +402,45 @@ TRN_D bool radiance_step(const DeviceScene& s, SurfF& x, F3& rdir, F3& T, float 
     const float dotSh = dot(x.ns, wi), dotGeo = dot(x.ng, wi);
     const bool stable = d > kShadowEps && fabsf(dotSh) > kEdgeEps;
     const bool noleak = dotSh * dotGeo > 0.f;
-    if (stable && noleak) cnt.v[kCntShadow]++;
-    if (stable && noleak && !occluded_k<NI>(s, x.p, wi, kShadowEps, d - kShadowEps)) {
+    if (stable && noleak) {
+      cnt.v[kCntShadow]++;
       const F3 Le = dot(-wi, nl) > 0.f ? light_radiance(s, ls.light) : F3z();
       const float G = fabsf(dot(nl, -wi)) / d2;
       const float bpdf = bsdf_pdf_local(b, fr.to_local(wo), fr.to_local(wi)) * G;
       const float mis = ls.pdf * ls.pdf / (ls.pdf * ls.pdf + bpdf * bpdf);
       const F3 bv = bsdf_eval(b, fr, x.ng, kd, wo, wi, false) * fabsf(dotSh);
-      F3 v;
-      for (int c = 0; c < 3; c++) v[c] = T[c] * (bv[c] * 1.f * G * Le[c] / ls.pdf * mis);
-      val = val + v;
+      for (int c = 0; c < 3; c++) g.nee[c] = T[c] * (bv[c] * 1.f * G * Le[c] / ls.pdf * mis);
+      g.sdir = wi; g.stmax = d - kShadowEps; g.shadow = true;
       if (rec) {
-        rec->nee_ok = 1; rec->ltri = ls.tri; rec->lu = ls.bu; rec->lv = ls.bv; rec->lpdf = ls.pdf;
-        rec->lmis = mis; rec->lLe = Le;
+        rec->ltri = ls.tri; rec->lu = ls.bu; rec->lv = ls.bv; rec->lpdf = ls.pdf; rec->lmis = mis;
       }
     }
   }
   // continuation (BSDF sampling)
-  F3 wi; float pdf;
-  bsdf_sample_only(b, fr, wo, b0, b1, b2, wi, pdf);
-  Hit h;
-  bool ok = pdf > 0.f && out_dir_valid(b, x.ns, x.ng, wi);
-  if (ok) { cnt.v[kCntClosest]++; ok = trace_k<NI, false>(s, x.p, wi, kShadowEps, kRayMax, h); }
-  if (!ok) {
+  bsdf_sample_only(b, fr, wo, b0, b1, b2, g.wi, g.pdf);
+  g.cont = g.pdf > 0.f && out_dir_valid(b, x.ns, x.ng, g.wi);
+  if (g.cont) cnt.v[kCntClosest]++;
+}
+
+// nee_ok: the light sample is visible; hit: the continuation ray's hit (tri <
+// 0: none was cast or it missed). Returns the contribution of this bounce
+// (already NaN-scrubbed) in contrib; x/rdir/T move to the next vertex, and the
+// return value says whether it exists.
+TRN_D bool radiance_resolve(const DeviceScene& s, SurfF& x, F3& rdir, F3& T, bool nee_ok, const F3& nee, float pdf,
+                            const Hit& h, F3& contrib, BounceRec* rec) {
+  F3 val = F3z();
+  if (nee_ok) val = val + nee;
+  if (rec) { rec->nee_ok = nee_ok; rec->next_ok = 0; }
+  if (h.tri < 0) {
     contrib = scrub(val);
     if (rec) rec->scrubbed = !finite3(val);
     return false;
   }
+  const BsdfDesc b = s.bsdfs[x.bsdf];
+  long long texel;
+  const F3 kd = bsdf_albedo(s, b, x.tu, x.tv, texel);
+  const Frame<float> fr = make_frame(x.ns);
+  const F3 wo = -rdir;
   const SurfF xn = post_intersect(s, h.tri, h.u, h.v);
   F3 dir = xn.p - x.p;
   const float dist2 = dot(dir, dir);
@@ -473,48 +468,26 @@ TRN_D bool radiance_step(const DeviceScene& s, SurfF& x, F3& rdir, F3& T, float 
   return true;
 }
 
-// One shared (non-inlined) copy of each per-bounce step, with the traversal
-// inlined inside it. A shared copy keeps a kernel's code small (the fused
-// kernels are instruction-fetch bound), but every object it takes by
-// reference lives in local memory: about 0.6-1 KB of stack per thread, which
-// at 512-768 threads per SM spills out of L1 and L2 into DRAM. Each kernel
-// chooses (measured) between this and the inlined step; the split stage
-// kernels are small enough to inline.
-#ifndef TRN_SHARED_STEPS_PRIMARY
-#define TRN_SHARED_STEPS_PRIMARY 0
-#endif
-#ifndef TRN_SHARED_STEPS_PIXEL
-#define TRN_SHARED_STEPS_PIXEL 0
-#endif
-#ifndef TRN_SHARED_STEPS_FWD
-#define TRN_SHARED_STEPS_FWD 0
-#endif
-#ifndef TRN_SHARED_STEPS_DIRECT
-#define TRN_SHARED_STEPS_DIRECT 0
-#endif
-#ifndef TRN_SHARED_STEPS_PATHADJ
-#define TRN_SHARED_STEPS_PATHADJ 0
-#endif
-// path_replay (k_path_replay, the fused k_path_adj and the loop-form recording
-// forward); TRN_SHARED_STEPS_PATHADJ is the regenerating recording forward
-#ifndef TRN_SHARED_STEPS_REPLAY
-#define TRN_SHARED_STEPS_REPLAY 1
-#endif
-// the indirect term's regenerating sensor and emitter stages
-#ifndef TRN_SHARED_STEPS_INDIRECT
-#define TRN_SHARED_STEPS_INDIRECT 0
-#endif
-__device__ __noinline__ bool radiance_step_shared(const DeviceScene& s, SurfF& x, F3& rdir, F3& T, float l0, float l1,
-                                                  float b0, float b1, float b2, F3& contrib, BounceRec* rec, Cnt& cnt) {
-  return radiance_step<false>(s, x, rdir, T, l0, l1, b0, b1, b2, contrib, rec, cnt);
-}
-template <bool SHARED>
-TRN_D bool radiance_step_k(const DeviceScene& s, SurfF& x, F3& rdir, F3& T, float l0, float l1, float b0, float b1,
-                           float b2, F3& contrib, BounceRec* rec, Cnt& cnt) {
-  if constexpr (SHARED) return radiance_step_shared(s, x, rdir, T, l0, l1, b0, b1, b2, contrib, rec, cnt);
-  else return radiance_step<false>(s, x, rdir, T, l0, l1, b0, b1, b2, contrib, rec, cnt);
+// The whole bounce by one thread (the fused kernels).
+TRN_D bool radiance_step(const DeviceScene& s, SurfF& x, F3& rdir, F3& T, float l0, float l1, float b0, float b1,
+                         float b2, F3& contrib, BounceRec* rec, Cnt& cnt) {
+  RadianceGen g;
+  radiance_gen(s, x, rdir, T, l0, l1, b0, b1, b2, g, rec, cnt);
+  const bool nee_ok = g.shadow && !occluded(s, x.p, g.sdir, kShadowEps, g.stmax);
+  Hit h;
+  h.tri = -1;
+  if (g.cont && !trace<false>(s, x.p, g.wi, kShadowEps, kRayMax, h)) h.tri = -1;
+  return radiance_resolve(s, x, rdir, T, nee_ok, g.nee, g.pdf, h, contrib, rec);
 }
 
+// One shared (non-inlined) copy of the step, with the traversal inlined inside
+// it, for the fused kernels that run it at more than one place or beside an
+// adjoint (they are instruction-fetch bound). Every object it takes by
+// reference lives in local memory.
+__device__ __noinline__ bool radiance_step_shared(const DeviceScene& s, SurfF& x, F3& rdir, F3& T, float l0, float l1,
+                                                  float b0, float b1, float b2, F3& contrib, BounceRec* rec, Cnt& cnt) {
+  return radiance_step(s, x, rdir, T, l0, l1, b0, b1, b2, contrib, rec, cnt);
+}
 
 // Per-warp compaction of the work queue: lanes keep pulling sample slots (one
 // warp-aggregated atomic per round) until each holds a slot that survives the
@@ -579,7 +552,6 @@ struct FwdState {
 
 __global__ void __launch_bounds__(256, TRN_MINB) k_path_fwd(TRN_KPARAMS) {
   Cnt cnt;
-  stage_top(P.s);
   int vhint = 0;
   for_each_valid<FwdState>(P,
     [&](long long gslot, FwdState& st) -> bool {
@@ -593,7 +565,7 @@ __global__ void __launch_bounds__(256, TRN_MINB) k_path_fwd(TRN_KPARAMS) {
       const F3 dir = camera_ray_dir(cam, pix % W, pix / W, S(0), S(1));
       Hit h;
       cnt.v[kCntClosest]++;
-      if (!trace_k<TRN_SETUP_SHARED_FWD, false>(P.s, org, dir, kShadowEps, kRayMax, h, P.err)) return false;
+      if (!trace<false>(P.s, org, dir, kShadowEps, kRayMax, h, P.err)) return false;
       st.V = &V; st.gslot = gslot; st.p = p; st.pix = pix;
       st.x = post_intersect(P.s, h.tri, h.u, h.v);
       const float t1 = camera_factor<float>(cam, st.x.p, st.x.ng, 1.f);
@@ -610,7 +582,7 @@ __global__ void __launch_bounds__(256, TRN_MINB) k_path_fwd(TRN_KPARAMS) {
       for (int b = 0; b < V.D; b++) {
         const int o = 2 + 5 * b;
         F3 c;
-        const bool more = radiance_step_k<TRN_SHARED_STEPS_FWD>(P.s, x, rdir, T, S(o), S(o + 1), S(o + 2), S(o + 3), S(o + 4), c, nullptr,
+        const bool more = radiance_step(P.s, x, rdir, T, S(o), S(o + 1), S(o + 2), S(o + 3), S(o + 4), c, nullptr,
                                         cnt);
         L = L + c;
         if (!more || (T.x == 0.f && T.y == 0.f && T.z == 0.f)) break;
@@ -893,7 +865,7 @@ TRN_D bool path_adj_setup(const Params& P, long long gslot, AdjState& st, int& v
   if (need_g && g.x == 0.f && g.y == 0.f && g.z == 0.f) return false;
   const F3 dir = camera_ray_dir(cam, pix % W, pix / W, S(0), S(1));
   cnt.v[kCntClosest]++;
-  if (!trace_k<TRN_SETUP_SHARED_PATHADJ, false>(s, cam_pos(cam), dir, kShadowEps, kRayMax, st.h, P.err)) return false;
+  if (!trace<false>(s, cam_pos(cam), dir, kShadowEps, kRayMax, st.h, P.err)) return false;
   st.V = &V; st.gslot = gslot; st.p = p; st.pix = pix; st.g = g;
   return true;
 }
@@ -944,7 +916,7 @@ TRN_D F3 path_replay(const Params& P, const AdjState& st, Rec& r, Cnt& cnt) {
     const int o = 2 + 5 * b;
     F3 c;
     BounceRec R;
-    const bool more = radiance_step_k<TRN_SHARED_STEPS_REPLAY>(s, x, rdir, T, S(o), S(o + 1), S(o + 2),
+    const bool more = radiance_step_shared(s, x, rdir, T, S(o), S(o + 1), S(o + 2),
                                     S(o + 3), S(o + 4), c, &R, cnt);
     // a scrubbed (non-finite) bounce contributes nothing and carries no gradient
     if (R.nee_ok && !R.scrubbed) mask |= 1u << k;
@@ -1052,7 +1024,6 @@ TRN_D void path_reverse(const Params& P, const Rec& r, Cnt& cnt) {
 template <int MAXD>
 __global__ void __launch_bounds__(256, TRN_MINB_PATHADJ) k_path_adj(TRN_KPARAMS) {
   Cnt cnt;
-  stage_top(P.s);
   int vhint = 0;
   for_each_valid<AdjState>(P,
     [&](long long gslot, AdjState& st) -> bool { return path_adj_setup(P, gslot, st, vhint, cnt); },
@@ -1064,257 +1035,125 @@ __global__ void __launch_bounds__(256, TRN_MINB_PATHADJ) k_path_adj(TRN_KPARAMS)
   flush_cnt(cnt, P.stats);
 }
 
-// Path records of the split interior adjoint in structure-of-arrays layout:
-// field k of path i lives at k * cap + i, so the lanes of a warp (consecutive
-// queue slots) read and write consecutive addresses. PathRecSoA gives the same
-// member syntax as PathRec over that layout.
-template <class T>
-struct Strided {
-  T* b;
-  long long s;
-  TRN_D T& operator[](int k) const { return b[(long long)k * s]; }
+// Path records in structure-of-arrays layout, for up to `cap` paths of up to
+// `depth` bounces: field k of path i lives at k * cap + i, so the lanes of a
+// warp (consecutive paths) read and write consecutive addresses. (`br` has no
+// entry 0, and `vr`, `Tk`, `Mk` start at vertex 1; entry 0 is left out.)
+struct PathSoA {
+  long long cap;
+  long long* p_;
+  int *view_, *K_, *D_;
+  unsigned* nee_;
+  F3* g_;
+  VRec* vr_;
+  LRec* br_;
+  F3 *Tk_, *Mk_;
+  unsigned* order;            // [cap] the records in the order their paths ended
+  unsigned long long* n_end;  // paths ended
+  TRN_D long long& p(long long i) const { return p_[i]; }
+  TRN_D int& view(long long i) const { return view_[i]; }
+  TRN_D int& K(long long i) const { return K_[i]; }
+  TRN_D int& D(long long i) const { return D_[i]; }
+  TRN_D unsigned& nee(long long i) const { return nee_[i]; }
+  TRN_D F3& g(long long i) const { return g_[i]; }
+  TRN_D VRec& vr(long long i, int k) const { return vr_[(k - 1) * cap + i]; }
+  TRN_D LRec& br(long long i, int k) const { return br_[(k - 1) * cap + i]; }
+  TRN_D F3& Tk(long long i, int k) const { return Tk_[(k - 1) * cap + i]; }
+  TRN_D F3& Mk(long long i, int k) const { return Mk_[(k - 1) * cap + i]; }
 };
 
-template <int MAXD>
-struct PathRecSoA {
-  long long& gslot;
-  long long& p;
-  int& view;
-  int& K;
-  int& D;
-  unsigned& nee_mask;
-  F3& g;
-  Strided<VRec> vr;
-  Strided<LRec> br;
-  Strided<F3> Tk, Mk;
-};
-
-template <int MAXD>
-TRN_HD size_t path_soa_bytes(long long cap) {
-  return (size_t)cap * (2 * sizeof(long long) + 3 * sizeof(int) + sizeof(unsigned) + sizeof(F3) +
-                        (MAXD + 2) * sizeof(VRec) + (MAXD + 1) * sizeof(LRec) + 2 * (MAXD + 2) * sizeof(F3)) +
-         16 * 256;
-}
-
-template <int MAXD>
-TRN_D PathRecSoA<MAXD> path_soa(void* base, long long cap, long long i) {
+// Places the arrays from `base` on and returns the bytes they take.
+inline size_t path_soa(PathSoA& a, void* base, long long cap, int depth) {
   char* c = static_cast<char*>(base);
-  auto take = [&](size_t bytes) { char* r = c; c += (bytes + 255) / 256 * 256; return r; };
-  long long* gslot = reinterpret_cast<long long*>(take(sizeof(long long) * cap));
-  long long* pp = reinterpret_cast<long long*>(take(sizeof(long long) * cap));
-  int* view = reinterpret_cast<int*>(take(sizeof(int) * cap));
-  int* K = reinterpret_cast<int*>(take(sizeof(int) * cap));
-  int* D = reinterpret_cast<int*>(take(sizeof(int) * cap));
-  unsigned* nee = reinterpret_cast<unsigned*>(take(sizeof(unsigned) * cap));
-  F3* g = reinterpret_cast<F3*>(take(sizeof(F3) * cap));
-  VRec* vr = reinterpret_cast<VRec*>(take(sizeof(VRec) * (MAXD + 2) * cap));
-  LRec* br = reinterpret_cast<LRec*>(take(sizeof(LRec) * (MAXD + 1) * cap));
-  F3* Tk = reinterpret_cast<F3*>(take(sizeof(F3) * (MAXD + 2) * cap));
-  F3* Mk = reinterpret_cast<F3*>(take(sizeof(F3) * (MAXD + 2) * cap));
-  return PathRecSoA<MAXD>{gslot[i], pp[i], view[i], K[i], D[i], nee[i], g[i],
-                          Strided<VRec>{vr + i, cap}, Strided<LRec>{br + i, cap},
-                          Strided<F3>{Tk + i, cap}, Strided<F3>{Mk + i, cap}};
+  size_t off = 0;
+  auto take = [&](size_t bytes) { char* r = c + off; off += (bytes + 255) / 256 * 256; return r; };
+  const size_t n = (size_t)cap, v = (size_t)depth + 1;
+  a.cap = cap;
+  a.p_ = reinterpret_cast<long long*>(take(sizeof(long long) * n));
+  a.view_ = reinterpret_cast<int*>(take(sizeof(int) * n));
+  a.K_ = reinterpret_cast<int*>(take(sizeof(int) * n));
+  a.D_ = reinterpret_cast<int*>(take(sizeof(int) * n));
+  a.nee_ = reinterpret_cast<unsigned*>(take(sizeof(unsigned) * n));
+  a.g_ = reinterpret_cast<F3*>(take(sizeof(F3) * n));
+  a.vr_ = reinterpret_cast<VRec*>(take(sizeof(VRec) * n * v));
+  a.br_ = reinterpret_cast<LRec*>(take(sizeof(LRec) * n * std::max(depth, 1)));
+  a.Tk_ = reinterpret_cast<F3*>(take(sizeof(F3) * n * v));
+  a.Mk_ = reinterpret_cast<F3*>(take(sizeof(F3) * n * v));
+  a.order = reinterpret_cast<unsigned*>(take(sizeof(unsigned) * n));
+  return off;
 }
 
-// Split form: k_path_replay traces and records every path into the queue;
-// k_path_reverse runs the reverse sweep over the queue. Each kernel carries
-// half of the fused kernel's code (the fused kernel is instruction-fetch
-// bound).
-template <int MAXD>
-__global__ void __launch_bounds__(256, TRN_MINB_PATHADJ) k_path_replay(TRN_KPARAMS) {
-  Cnt cnt;
-  stage_top(P.s);
-  int vhint = 0;
-  for_each_valid<AdjState>(P,
-    [&](long long gslot, AdjState& st) -> bool { return path_adj_setup(P, gslot, st, vhint, cnt); },
-    [&](AdjState& st) {
-      const unsigned act = __activemask();
-      const int lane = threadIdx.x & 31;
-      const int leader = __ffs(act) - 1;
-      unsigned long long base = 0;
-      if (lane == leader) base = atomicAdd(P.q_count, (unsigned long long)__popc(act));
-      base = __shfl_sync(act, base, leader);
-      const unsigned long long k = base + __popc(act & ((1u << lane) - 1u));
-      if (k >= (unsigned long long)P.q_cap) { atomicExch(P.err, 2); return; }
-      PathRecSoA<MAXD> r = path_soa<MAXD>(P.queue, P.q_cap, (long long)k);
-      path_replay<MAXD>(P, st, r, cnt);
-    });
-  flush_cnt(cnt, P.stats);
-}
+// One path's records with the member syntax of PathRec (path_reverse).
+struct PathRef {
+  const PathSoA& a;
+  long long i;
+  int view, K, D;
+  unsigned nee_mask;
+  F3 g;
+  struct Vr { const PathSoA& a; long long i; TRN_D const VRec& operator[](int k) const { return a.vr(i, k); } } vr;
+  struct Br { const PathSoA& a; long long i; TRN_D const LRec& operator[](int k) const { return a.br(i, k); } } br;
+  struct T { const PathSoA& a; long long i; TRN_D const F3& operator[](int k) const { return a.Tk(i, k); } } Tk;
+  struct M { const PathSoA& a; long long i; TRN_D const F3& operator[](int k) const { return a.Mk(i, k); } } Mk;
+};
 
-// CACHED: the records come from the recording forward render (k_path_fwd_rec)
-// and carry no dL/dI yet; each path reads its pixel's now and is skipped when
-// that is zero, as path_adj_setup skips it in the replaying form.
-template <int MAXD, bool CACHED = false>
-__global__ void __launch_bounds__(256, TRN_MINB_REVERSE) k_path_reverse(TRN_KPARAMS) {
+// Reverse sweep over the records, in the order in which their paths ended: the
+// paths of one bounce ended together, so a warp's sweeps have the same length
+// (in slot order a warp ran as long as its longest path, with less than a third
+// of its lanes active: 23.5 ms for 16.8M paths of depth 5, 12.0 in this order).
+// The order matters to the sums: a few vertices get millions of 32-bit adds, and
+// small ones are lost in a large sum. Shortest paths first stays nearest to the
+// sums in slot order (5e-5 of the positions' gradient; longest first 1.5e-4). Bound by instruction fetch:
+// the sweep is one long body of inlined scatters, and the few warps that fit
+// its registers do not hide the misses. (Its six scatters in a loop, or one
+// shared function, take 5 to 10 times as long: lanes then enter them one group
+// at a time.)
+// CACHED: the records come from the recording forward render and carry no
+// dL/dI yet; each path reads its pixel's now and is skipped when that is zero,
+// as the replaying form skips it.
+template <bool CACHED>
+__global__ void __launch_bounds__(256, TRN_MINB_REVERSE) k_path_reverse(TRN_KPARAMS, const __grid_constant__ PathSoA R) {
+  stage_begin();
   Cnt cnt;
-  stage_top(P.s);
-  const unsigned long long n = min(*P.q_count, (unsigned long long)P.q_cap);
+  const unsigned long long n = *R.n_end;
   for (unsigned long long k = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; k < n;
        k += (unsigned long long)gridDim.x * blockDim.x) {
-    const PathRecSoA<MAXD> r = path_soa<MAXD>(P.queue, P.q_cap, (long long)k);
+    const long long i = (long long)__ldcs(R.order + k);
+    const int view = R.view(i);
+    F3 g;
     if (CACHED) {
-      const ViewDesc& V = P.views[r.view];
-      const F3 g = g_at(P, V, (int)(r.p % ((long long)V.cam.w * V.cam.h)));
+      const ViewDesc& V = P.views[view];
+      g = g_at(P, V, (int)(R.p(i) % ((long long)V.cam.w * V.cam.h)));
       if (g.x == 0.f && g.y == 0.f && g.z == 0.f) continue;
-      r.g = g;
+    } else {
+      g = R.g(i);
     }
-    path_reverse<MAXD>(P, r, cnt);
+    const PathRef r{R, i, view, R.K(i), R.D(i), R.nee(i), g, {R, i}, {R, i}, {R, i}, {R, i}};
+    path_reverse<0>(P, r, cnt);
   }
   flush_cnt(cnt, P.stats);
 }
-
-// Forward interior render that also keeps every path with a primary hit as a
-// record (the records k_path_replay writes for the gradient call). A gradient
-// call of the same paths then runs k_path_reverse<MAXD, true> over them
-// instead of tracing them again. Same image as k_path_fwd.
-template <int MAXD>
-__global__ void __launch_bounds__(256, TRN_MINB_FWDREC) k_path_fwd_rec(TRN_KPARAMS) {
-  Cnt cnt;
-  stage_top(P.s);
-  int vhint = 0;
-  for_each_valid<AdjState>(P,
-    [&](long long gslot, AdjState& st) -> bool { return path_adj_setup(P, gslot, st, vhint, cnt, false); },
-    [&](AdjState& st) {
-      const unsigned act = __activemask();
-      const int lane = threadIdx.x & 31;
-      const int leader = __ffs(act) - 1;
-      unsigned long long base = 0;
-      if (lane == leader) base = atomicAdd(P.q_count, (unsigned long long)__popc(act));
-      base = __shfl_sync(act, base, leader);
-      const unsigned long long k = base + __popc(act & ((1u << lane) - 1u));
-      if (k >= (unsigned long long)P.q_cap) { atomicExch(P.err, 2); return; }
-      PathRecSoA<MAXD> r = path_soa<MAXD>(P.queue, P.q_cap, (long long)k);
-      const ViewDesc& V = *st.V;
-      const F3 L = path_replay<MAXD>(P, st, r, cnt) * V.inv_spp;
-      cnt.v[kCntPixel]++;
-      atomic_add3((V.image ? V.image : P.image + 3 * V.pix_off) + 3 * st.pix, L);
-    });
-  flush_cnt(cnt, P.stats);
-}
-
-// k_path_fwd_rec with path regeneration: lanes fetch slots until at least
-// TRN_COMPACT_MIN hold a path (as for_each_valid), then every lane with a
-// path takes one bounce; a lane whose path has ended writes its record's
-// totals and its pixel and takes the next slot at once. Each path runs
-// exactly the steps of path_replay.
-#ifndef TRN_FWD_REGEN
-#define TRN_FWD_REGEN 1
-#endif
-
-template <int MAXD>
-__global__ void __launch_bounds__(256, TRN_MINB_FWDREC) k_path_fwd_rec_regen(TRN_KPARAMS) {
-  Cnt cnt;
-  stage_top(P.s);
-  const DeviceScene& s = P.s;
-  const int lane = threadIdx.x & 31;
-  const unsigned lt = (1u << lane) - 1u;
-  int vhint = 0;
-  bool active = false, done = false;
-  const ViewDesc* V = nullptr;
-  long long gslot = 0, p = 0, kr = 0;
-  int pix = 0, b = 0, K = 1, D = 0;
-  unsigned mask = 0u;
-  SurfF x;
-  F3 T, rdir, L;
-  for (;;) {
-    // refill: fetch slots until enough lanes hold a path with a primary hit
-    for (;;) {
-      const unsigned need = __ballot_sync(0xffffffffu, !active && !done);
-      if (!need || __popc(__ballot_sync(0xffffffffu, active)) >= TRN_COMPACT_MIN) break;
-      const int leader = __ffs(need) - 1;
-      unsigned long long base = 0;
-      if (lane == leader) base = atomicAdd(P.work, (unsigned long long)__popc(need));
-      base = __shfl_sync(0xffffffffu, base, leader);
-      AdjState st;
-      bool got = false;
-      if (!active && !done) {
-        const long long g = (long long)base + __popc(need & lt);
-        if (g >= P.total) done = true;
-        else got = path_adj_setup(P, g, st, vhint, cnt, false);
-      }
-      const unsigned gm = __ballot_sync(0xffffffffu, got);
-      if (!gm) continue;
-      const int gl = __ffs(gm) - 1;
-      unsigned long long rb = 0;
-      if (lane == gl) rb = atomicAdd(P.q_count, (unsigned long long)__popc(gm));
-      rb = __shfl_sync(0xffffffffu, rb, gl);
-      if (got) {
-        kr = (long long)(rb + __popc(gm & lt));
-        if (kr >= P.q_cap) {
-          atomicExch(P.err, 2);
-        } else {
-          V = st.V; gslot = st.gslot; p = st.p; pix = st.pix;
-          PathRecSoA<MAXD> r = path_soa<MAXD>(P.queue, P.q_cap, kr);
-          r.gslot = gslot; r.p = p; r.view = (int)(V - P.views); r.g = F3z();
-          x = post_intersect(s, st.h.tri, st.h.u, st.h.v);
-          r.vr[1] = {st.h.tri, st.h.u, st.h.v};
-          const F3 org = cam_pos(V->cam);
-          const float t1 = camera_factor<float>(V->cam, x.p, x.ng, 1.f);
-          T = F3(t1, t1, t1);
-          rdir = normalize(x.p - org);
-          r.Tk[1] = T;
-          F3 m1 = emitted(s, x, -rdir);
-          if (!finite3(T * m1)) m1 = F3z();
-          r.Mk[1] = m1;
-          L = T * m1;
-          K = 1;
-          D = min(V->D, MAXD);
-          mask = 0u;
-          b = 0;
-          active = true;
-        }
-      }
-    }
-    if (!__any_sync(0xffffffffu, active)) break;
-    if (active) {
-      PathRecSoA<MAXD> r = path_soa<MAXD>(P.queue, P.q_cap, kr);
-      bool fin = b >= D;
-      if (!fin) {
-        const PathSmp S{&P, V->seed, gslot, p + V->slot_off};
-        const int k = b + 1;
-        const int o = 2 + 5 * b;
-        F3 c;
-        BounceRec R;
-        const bool more = radiance_step_k<TRN_SHARED_STEPS_PATHADJ>(s, x, rdir, T, S(o), S(o + 1), S(o + 2),
-                                                                   S(o + 3), S(o + 4), c, &R, cnt);
-        if (R.nee_ok && !R.scrubbed) mask |= 1u << k;
-        L = L + c;
-        r.br[k] = {R.ltri, R.lu, R.lv, R.lpdf, R.lmis, R.prev_pdf};
-        if (!more) {
-          fin = true;
-        } else {
-          r.vr[k + 1] = {x.tri, x.u, x.v};
-          r.Tk[k + 1] = T;
-          r.Mk[k + 1] = (R.scrubbed || R.emis == 0.f) ? F3z() : R.eLe * R.emis;
-          K = k + 1;
-          if (T.x == 0.f && T.y == 0.f && T.z == 0.f) fin = true;
-        }
-        b++;
-        if (b >= D) fin = true;
-      }
-      if (fin) {
-        r.K = K;
-        r.D = D;
-        r.nee_mask = mask;
-        cnt.v[kCntPixel]++;
-        atomic_add3((V->image ? V->image : P.image + 3 * V->pix_off) + 3 * pix, L * V->inv_spp);
-        active = false;
-      }
-    }
-  }
-  flush_cnt(cnt, P.stats);
-}
-
 
 // ---------------------------------------------------------------------------
 // EvalImportance for one ray (Integrator.cpp:75-176)
 // ---------------------------------------------------------------------------
-template <bool NI = false>
-TRN_D bool importance_step(const DeviceScene& s, const CameraDesc& cam, SurfF& x, F3& rdir, F3& T, float b0,
-                           float b1, float b2, F3& contrib, int& pix, Cnt& cnt) {
-  contrib = F3z();
-  pix = -1;
+// In two halves like a radiance bounce: importance_gen decides the ray from the
+// sensor to the vertex (with the contribution it would carry and its pixel)
+// and the continuation.
+struct ImportanceGen {
+  F3 c;         // contribution if the vertex is visible from the sensor
+  int pix;      // its pixel (-1: none)
+  F3 sdir;      // ray from the camera position: direction and end
+  float stmax;
+  bool shadow;
+  F3 wi, Tn;    // continuation ray and the throughput behind it
+  bool cont;
+};
+
+TRN_D void importance_gen(const DeviceScene& s, const CameraDesc& cam, const SurfF& x, const F3& rdir, const F3& T,
+                          float b0, float b1, float b2, ImportanceGen& g, Cnt& cnt) {
+  g.c = F3z();
+  g.pix = -1;
+  g.shadow = g.cont = false;
   const BsdfDesc b = s.bsdfs[x.bsdf];
   count_shade(cnt, s, x);
   long long texel;
@@ -1324,45 +1163,49 @@ TRN_D bool importance_step(const DeviceScene& s, const CameraDesc& cam, SurfF& x
   const F3 cpos = cam_pos(cam);
   const SensorSample sds = sample_direct(cam, x.p);
   if (sds.valid) {
-    const F3 dirc = sensor_ray_dir(cam, sds.qx, sds.qy);
-    const float dist2cam = length(x.p - cpos);
+    g.sdir = sensor_ray_dir(cam, sds.qx, sds.qy);
+    g.stmax = length(x.p - cpos) - kShadowEps;
+    g.shadow = true;
     cnt.v[kCntShadow]++;
-    if (!occluded_k<NI>(s, cpos, dirc, kShadowEps, dist2cam - kShadowEps)) {
-      F3 val = F3z();
-      if (out_dir_valid(b, x.ns, x.ng, wo)) {
-        const F3 wi = normalize(cpos - x.p);
-        if (out_dir_valid(b, x.ns, x.ng, wi))
-          val = bsdf_eval(b, fr, x.ng, kd, wo, wi, true) * fabsf(dot(x.ns, wi));
-      }
-      contrib = scrub(T * sds.sensor_val * val);
-      pix = image_pixel(cam, sds.qx, sds.qy);
+    F3 val = F3z();
+    if (out_dir_valid(b, x.ns, x.ng, wo)) {
+      const F3 wi = normalize(cpos - x.p);
+      if (out_dir_valid(b, x.ns, x.ng, wi))
+        val = bsdf_eval(b, fr, x.ng, kd, wo, wi, true) * fabsf(dot(x.ns, wi));
     }
+    g.c = scrub(T * sds.sensor_val * val);
+    g.pix = image_pixel(cam, sds.qx, sds.qy);
   }
-  if (!out_dir_valid(b, x.ns, x.ng, wo)) return false;
-  F3 wi; float pdf;
-  bsdf_sample_only(b, fr, wo, b0, b1, b2, wi, pdf);
-  const F3 bv = bsdf_eval(b, fr, x.ng, kd, wo, wi, true) * fabsf(dot(x.ns, wi));
-  const F3 Tn = T * bv / pdf;
-  if (!(pdf > 0.f) || !out_dir_valid(b, x.ns, x.ng, wi)) return false;
+  if (!out_dir_valid(b, x.ns, x.ng, wo)) return;
+  float pdf;
+  bsdf_sample_only(b, fr, wo, b0, b1, b2, g.wi, pdf);
+  const F3 bv = bsdf_eval(b, fr, x.ng, kd, wo, g.wi, true) * fabsf(dot(x.ns, g.wi));
+  g.Tn = T * bv / pdf;
+  g.cont = pdf > 0.f && out_dir_valid(b, x.ns, x.ng, g.wi);
+}
+
+// The whole step by one thread (the fused kernels).
+TRN_D bool importance_step(const DeviceScene& s, const CameraDesc& cam, SurfF& x, F3& rdir, F3& T, float b0,
+                           float b1, float b2, F3& contrib, int& pix, Cnt& cnt) {
+  ImportanceGen g;
+  importance_gen(s, cam, x, rdir, T, b0, b1, b2, g, cnt);
+  contrib = F3z();
+  pix = -1;
+  if (g.shadow && !occluded(s, cam_pos(cam), g.sdir, kShadowEps, g.stmax)) { contrib = g.c; pix = g.pix; }
+  if (!g.cont) return false;
   Hit h;
   cnt.v[kCntClosest]++;
-  if (!trace_k<NI, false>(s, x.p, wi, kShadowEps, kRayMax, h)) return false;
+  if (!trace<false>(s, x.p, g.wi, kShadowEps, kRayMax, h)) return false;
   x = post_intersect(s, h.tri, h.u, h.v);
-  rdir = wi;
-  T = Tn;
+  rdir = g.wi;
+  T = g.Tn;
   return true;
 }
 
 __device__ __noinline__ bool importance_step_shared(const DeviceScene& s, const CameraDesc& cam, SurfF& x, F3& rdir,
                                                     F3& T, float b0, float b1, float b2, F3& contrib, int& pix,
                                                     Cnt& cnt) {
-  return importance_step<false>(s, cam, x, rdir, T, b0, b1, b2, contrib, pix, cnt);
-}
-template <bool SHARED>
-TRN_D bool importance_step_k(const DeviceScene& s, const CameraDesc& cam, SurfF& x, F3& rdir, F3& T, float b0,
-                             float b1, float b2, F3& contrib, int& pix, Cnt& cnt) {
-  if constexpr (SHARED) return importance_step_shared(s, cam, x, rdir, T, b0, b1, b2, contrib, pix, cnt);
-  else return importance_step<false>(s, cam, x, rdir, T, b0, b1, b2, contrib, pix, cnt);
+  return importance_step(s, cam, x, rdir, T, b0, b1, b2, contrib, pix, cnt);
 }
 
 // scatter W * d xDotN / d(edge vertices, receiver point, far triangle)
@@ -1475,54 +1318,93 @@ struct EdgeState {
 };
 
 // Primary boundary set-up (SampleFromPrimEdges, Edge.cpp:350-367;
-// BoundaryPrimary.cpp:60-130): silhouette edge point, camera ray through it,
-// visibility, boundary geometry. Returns false for a rejected sample.
-TRN_D bool primary_setup(const Params& P, long long gslot, EdgeState& st, int& vhint, Cnt& cnt) {
+// BoundaryPrimary.cpp:60-130) in three parts around its two ray queries:
+// silhouette edge point and the ray that continues the camera's line behind
+// it; the sensor sample of the point hit there, with the ray that tests its
+// visibility; boundary geometry. Each returns false for a rejected sample.
+struct EdgePoint {
+  const ViewDesc* V;
+  long long p;
+  int v0, v1;
+  float s;            // position on the edge
+  float pdf;
+  F3 p0, edge, edge2;
+  F3 dir;             // first set-up ray, from p0
+};
+
+TRN_D bool primary_point(const Params& P, long long gslot, EdgePoint& q, int& vhint) {
   const DeviceScene& s = P.s;
   const ViewDesc& V = view_of(P, gslot, vhint);
-  const long long p = gslot - V.begin;
-  const CameraDesc& cam = V.cam;
-  const PathSmp S{&P, V.seed, gslot, p + V.slot_off};
-  const F3 cpos = cam_pos(cam);
+  q.V = &V;
+  q.p = gslot - V.begin;
+  const PathSmp S{&P, V.seed, gslot, q.p + V.slot_off};
   const float r0 = S(0), r1 = S(1);
   float reuse;
   const float integral = __ldg(V.pint);
   if (!(integral > 0.f)) return false;
   const int e = sample_discrete(V.pcdf, P.ne, r0, reuse);
-  const int v0 = P.edges[5 * e], v1 = P.edges[5 * e + 1], v2 = P.edges[5 * e + 4];
+  const int v2 = P.edges[5 * e + 4];
+  q.v0 = P.edges[5 * e]; q.v1 = P.edges[5 * e + 1];
   const float len_e = V.pfunc[e];
   if (!(len_e > 0.f)) return false;
   const float pmf = len_e / (integral * (float)P.ne);
-  const float pdf = pmf / len_e;
-  const F3 Pa = load3(s.pos, v0), Pb = load3(s.pos, v1), Pc = load3(s.pos, v2);
+  q.pdf = pmf / len_e;
+  const F3 Pa = load3(s.pos, q.v0), Pb = load3(s.pos, q.v1), Pc = load3(s.pos, v2);
   const F3 e1 = Pb - Pa;
-  const F3 p0 = Pa + e1 * r1;
-  const F3 edge = normalize(e1), edge2 = normalize(Pc - Pa);
-  const F3 dir = normalize(p0 - cpos);
-  Hit h;
-  cnt.v[kCntClosest]++;
-  if (!trace_k<TRN_SETUP_SHARED_PRIMARY, false>(s, p0, dir, kShadowEps, kRayMax, h, P.err)) return false;
-  const F3 hitP = p0 + dir * h.t;
-  const SensorSample sds = sample_direct(cam, hitP);
+  q.s = r1;
+  q.p0 = Pa + e1 * r1;
+  q.edge = normalize(e1); q.edge2 = normalize(Pc - Pa);
+  q.dir = normalize(q.p0 - cam_pos(V.cam));
+  return true;
+}
+
+// Sensor sample of the point that the first ray (p0, dir) hit at distance t.
+TRN_D bool primary_sensor(const CameraDesc& cam, const F3& p0, const F3& dir, float t, SensorSample& sds, F3& dirc,
+                          float& tmax) {
+  const F3 hitP = p0 + dir * t;
+  sds = sample_direct(cam, hitP);
   if (!sds.valid) return false;
-  const F3 dirc = sensor_ray_dir(cam, sds.qx, sds.qy);
-  const float dist2cam = length(p0 - cpos);
-  cnt.v[kCntShadow]++;
-  if (occluded_k<TRN_SETUP_SHARED_PRIMARY>(s, cpos, dirc, kShadowEps, dist2cam - kShadowEps)) return false;
-  const SurfF x = post_intersect(s, h.tri, h.u, h.v);
+  dirc = sensor_ray_dir(cam, sds.qx, sds.qy);
+  tmax = length(p0 - cam_pos(cam)) - kShadowEps;
+  return true;
+}
+
+TRN_D bool primary_finish(const Params& P, long long gslot, const EdgePoint& q, const Hit& h, const SensorSample& sds,
+                          const F3& dirc, EdgeState& st) {
+  const ViewDesc& V = *q.V;
+  const CameraDesc& cam = V.cam;
+  const F3 cpos = cam_pos(cam);
+  const SurfF x = post_intersect(P.s, h.tri, h.u, h.v);
   const float dist = length(x.p - cpos);
-  const float dist1 = length(p0 - cpos);
+  const float dist1 = length(q.p0 - cpos);
   const float cos2 = fabsf(dot(x.ng, -dirc));
   F3 n;
-  const float bval = base_val((dist / dist1), edge, dirc, x.ng, edge2, n) * cos2;
+  const float bval = base_val((dist / dist1), q.edge, dirc, x.ng, q.edge2, n) * cos2;
   const int pix = image_pixel(cam, sds.qx, sds.qy);
   const F3 g = g_at(P, V, pix);
   if (bval == 0.f || (g.x == 0.f && g.y == 0.f && g.z == 0.f)) return false;
-  st.V = &V; st.gslot = gslot; st.p = p; st.x = x; st.rdir = dirc;
+  st.V = &V; st.gslot = gslot; st.p = q.p; st.x = x; st.rdir = dirc;
   st.T0 = F3(sds.sensor_val, sds.sensor_val, sds.sensor_val);
-  st.p0 = p0; st.n = n; st.w0 = bval / pdf; st.sedge = r1; st.v0 = v0; st.v1 = v1; st.far_tri = h.tri;
+  st.p0 = q.p0; st.n = n; st.w0 = bval / q.pdf; st.sedge = q.s; st.v0 = q.v0; st.v1 = q.v1; st.far_tri = h.tri;
   st.pix = pix; st.g = g;
   return true;
+}
+
+// The whole set-up by one thread (the fused kernel).
+TRN_D bool primary_setup(const Params& P, long long gslot, EdgeState& st, int& vhint, Cnt& cnt) {
+  EdgePoint q;
+  if (!primary_point(P, gslot, q, vhint)) return false;
+  Hit h;
+  cnt.v[kCntClosest]++;
+  if (!trace_shared<false>(P.s, q.p0, q.dir, kShadowEps, kRayMax, h, P.err)) return false;
+  SensorSample sds;
+  F3 dirc;
+  float tmax;
+  if (!primary_sensor(q.V->cam, q.p0, q.dir, h.t, sds, dirc, tmax)) return false;
+  cnt.v[kCntShadow]++;
+  Hit hv;
+  if (trace_shared<true>(P.s, cam_pos(q.V->cam), dirc, kShadowEps, tmax, hv, nullptr)) return false;
+  return primary_finish(P, gslot, q, h, sds, dirc, st);
 }
 
 // Primary boundary body: detached radiance along the camera ray through the
@@ -1538,7 +1420,7 @@ TRN_D void primary_body(const Params& P, const ViewDesc& V, long long gslot, lon
   for (int b = 0; b < V.D; b++) {
     const int o = dim0 + 5 * b;
     F3 c;
-    const bool more = radiance_step_k<TRN_SHARED_STEPS_PRIMARY>(s, x, rdir, T, S(o), S(o + 1), S(o + 2), S(o + 3),
+    const bool more = radiance_step(s, x, rdir, T, S(o), S(o + 1), S(o + 2), S(o + 3),
                                                                 S(o + 4), c, nullptr, cnt);
     L = L + c;
     if (!more || (T.x == 0.f && T.y == 0.f && T.z == 0.f)) break;
@@ -1550,7 +1432,6 @@ TRN_D void primary_body(const Params& P, const ViewDesc& V, long long gslot, lon
 
 __global__ void __launch_bounds__(256, TRN_MINB) k_primary_adj(TRN_KPARAMS) {
   Cnt cnt;
-  stage_top(P.s);
   int vhint = 0;
   for_each_valid<EdgeState>(P,
     [&](long long gslot, EdgeState& st) -> bool { return primary_setup(P, gslot, st, vhint, cnt); },
@@ -1561,140 +1442,15 @@ __global__ void __launch_bounds__(256, TRN_MINB) k_primary_adj(TRN_KPARAMS) {
   flush_cnt(cnt, P.stats);
 }
 
-// Split form: k_primary_setup tests every slot once (no lane waits for the
-// others to find an accepted sample, which matters at the ~4 % acceptance of
-// silhouette samples) and queues the accepted ones; k_primary_body runs the
-// radiance path and the scatter for the queue.
+// A sample that passed the set-up of the primary (or pixel) term; its radiance
+// path and scatter follow.
 struct PrimaryItem {
-  long long gslot, p;
-  int view, x_tri, dim0, pad_;
+  long long p;
+  int view, x_tri;
   float x_u, x_v, T0, w0, sedge;
   int v0, v1, far_tri;
   F3 rdir, p0, n, g;
 };
-
-__global__ void __launch_bounds__(256, TRN_MINB_SETUP) k_primary_setup(TRN_KPARAMS) {
-  Cnt cnt;
-  stage_top(P.s);
-  int vhint = 0;
-  PrimaryItem* q = reinterpret_cast<PrimaryItem*>(P.queue);
-  const int lane = threadIdx.x & 31;
-  const unsigned lt = (1u << lane) - 1u;
-  for (;;) {
-    unsigned long long start = 0;
-    if (lane == 0) start = atomicAdd(P.work, 32ull);
-    start = __shfl_sync(0xffffffffu, start, 0);
-    if ((long long)start >= P.total) break;
-    const long long g = slot_at(P, (long long)start + lane);
-    EdgeState st;
-    const bool ok = g < P.total && primary_setup(P, g, st, vhint, cnt);
-    const unsigned m = __ballot_sync(0xffffffffu, ok);
-    if (!m) continue;
-    const int leader = __ffs(m) - 1;
-    unsigned long long base = 0;
-    if (lane == leader) base = atomicAdd(P.q_count, (unsigned long long)__popc(m));
-    base = __shfl_sync(0xffffffffu, base, leader);
-    const unsigned long long k = base + __popc(m & lt);
-    if (ok && k >= (unsigned long long)P.q_cap) atomicExch(P.err, 2);
-    if (ok && k < (unsigned long long)P.q_cap) {
-      PrimaryItem& it = q[k];
-      it.gslot = st.gslot; it.p = st.p; it.view = (int)(st.V - P.views); it.dim0 = 2;
-      it.x_tri = st.x.tri; it.x_u = st.x.u; it.x_v = st.x.v; it.T0 = st.T0.x; it.w0 = st.w0; it.sedge = st.sedge;
-      it.v0 = st.v0; it.v1 = st.v1; it.far_tri = st.far_tri;
-      it.rdir = st.rdir; it.p0 = st.p0; it.n = st.n; it.g = st.g;
-    }
-  }
-  flush_cnt(cnt, P.stats);
-}
-
-__global__ void __launch_bounds__(256, TRN_MINB_BODY) k_primary_body(TRN_KPARAMS) {
-  Cnt cnt;
-  stage_top(P.s);
-  const PrimaryItem* q = reinterpret_cast<const PrimaryItem*>(P.queue);
-  const unsigned long long n = min(*P.q_count, (unsigned long long)P.q_cap);
-  for (unsigned long long k = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; k < n;
-       k += (unsigned long long)gridDim.x * blockDim.x) {
-    const PrimaryItem& it = q[k];
-    const SurfF x = post_intersect(P.s, it.x_tri, it.x_u, it.x_v);
-    primary_body(P, P.views[it.view], it.gslot, it.p, x, it.rdir, F3(it.T0, it.T0, it.T0), it.w0, it.g, it.v0, it.v1,
-                 it.sedge, it.p0, it.far_tri, it.n, cnt, it.dim0);
-  }
-  flush_cnt(cnt, P.stats);
-}
-
-// Path regeneration for the queue's bodies: a lane whose radiance path has
-// ended takes the next queue item at once instead of idling until the warp's
-// longest path ends (the boundary paths end after one or two bounces on
-// average, at most D). Each item runs exactly the steps of primary_body.
-#ifndef TRN_BODY_REGEN
-#define TRN_BODY_REGEN 1
-#endif
-
-__global__ void __launch_bounds__(256, TRN_MINB_BODY) k_primary_body_regen(TRN_KPARAMS) {
-  Cnt cnt;
-  stage_top(P.s);
-  const DeviceScene& s = P.s;
-  const PrimaryItem* q = reinterpret_cast<const PrimaryItem*>(P.queue);
-  const unsigned long long n = min(*P.q_count, (unsigned long long)P.q_cap);
-  unsigned long long* next = P.q_count + 1;  // items handed out (zeroed with the round)
-  const int lane = threadIdx.x & 31;
-  const unsigned lt = (1u << lane) - 1u;
-  bool active = false, done = false;
-  unsigned long long k = 0;
-  const ViewDesc* V = nullptr;
-  SurfF x;
-  F3 T, rdir, L;
-  int b = 0, D = 0;
-  for (;;) {
-    const unsigned need = __ballot_sync(0xffffffffu, !active && !done);
-    if (need) {
-      const int leader = __ffs(need) - 1;
-      unsigned long long base = 0;
-      if (lane == leader) base = atomicAdd(next, (unsigned long long)__popc(need));
-      base = __shfl_sync(0xffffffffu, base, leader);
-      if (!active && !done) {
-        k = base + __popc(need & lt);
-        if (k >= n) {
-          done = true;
-        } else {
-          const PrimaryItem& it = q[k];
-          V = P.views + it.view;
-          D = V->D;
-          x = post_intersect(s, it.x_tri, it.x_u, it.x_v);
-          T = F3(it.T0, it.T0, it.T0);
-          rdir = it.rdir;
-          L = scrub(T * emitted(s, x, -rdir));
-          b = 0;
-          active = true;
-        }
-      }
-    }
-    if (!__any_sync(0xffffffffu, active)) break;
-    if (active) {
-      bool fin = b >= D;
-      if (!fin) {
-        const PrimaryItem& it = q[k];
-        const PathSmp S{&P, V->seed, it.gslot, it.p + V->slot_off};
-        const int o = it.dim0 + 5 * b;
-        F3 c;
-        const bool more = radiance_step_k<TRN_SHARED_STEPS_PRIMARY>(s, x, rdir, T, S(o), S(o + 1), S(o + 2),
-                                                                    S(o + 3), S(o + 4), c, nullptr, cnt);
-        L = L + c;
-        b++;
-        fin = !more || (T.x == 0.f && T.y == 0.f && T.z == 0.f) || b >= D;
-      }
-      if (fin) {
-        const PrimaryItem& it = q[k];
-        const float W = dot(it.g, L * it.w0);
-        if (W != 0.f && isfinite(W))
-          xdotn_vjp(P, *V, W, cam_pos(V->cam), false, -1, 0.f, 0.f, it.v0, it.v1, it.sedge, it.p0, it.far_tri, it.n,
-                    cnt);
-        active = false;
-      }
-    }
-  }
-  flush_cnt(cnt, P.stats);
-}
 
 // ---------------------------------------------------------------------------
 // direct boundary (BoundaryDirect.cpp:38-143, Edge.cpp:90-144, 201-309)
@@ -1707,12 +1463,20 @@ TRN_D float aq_lerp(const float* box, long long cap, int leaf, int axis, float r
 
 // Direct boundary set-up (SampleBoundarySegmentDirect, Edge.cpp:108-144, with
 // AQ guiding when enabled; EvalBoundarySegmentDirect's geometry,
-// Edge.cpp:201-291). Returns false for a rejected sample.
-TRN_D bool direct_setup(const Params& P, long long gslot, EdgeState& st, int& vhint, Cnt& cnt) {
+// Edge.cpp:201-291): edge and light points with the ray to the light; whether
+// that ray met the light point; the receiver behind the edge and the boundary
+// geometry. Each part returns false for a rejected sample.
+struct DirectPoint {
+  EdgePoint e;        // dir: from the edge point to the light
+  F3 p2, nL;          // light point and normal
+};
+
+TRN_D bool direct_point(const Params& P, long long gslot, DirectPoint& q, int& vhint, Cnt& cnt) {
   const DeviceScene& s = P.s;
   const ViewDesc& V = view_of(P, gslot, vhint);
-  const long long p = gslot - V.begin;
-  const PathSmp S{&P, V.seed, gslot, p + V.slot_off};
+  q.e.V = &V;
+  q.e.p = gslot - V.begin;
+  const PathSmp S{&P, V.seed, gslot, q.e.p + V.slot_off};
   float r0 = S(0), r1 = S(1), r2 = S(2);
   float reuse;
   const float integral = __ldg(P.eint);
@@ -1731,25 +1495,26 @@ TRN_D bool direct_setup(const Params& P, long long gslot, EdgeState& st, int& vh
     pdf_b = __fdiv_rn(__ldg(P.aq_poly + leaf), __ldg(P.aq_int + 1));
   }
   const int e = sample_discrete(P.ecdf, P.ne, r0, reuse);
-  const int v0 = P.edges[5 * e], v1 = P.edges[5 * e + 1], f0 = P.edges[5 * e + 2], f1 = P.edges[5 * e + 3],
-            v2 = P.edges[5 * e + 4];
+  const int f0 = P.edges[5 * e + 2], f1 = P.edges[5 * e + 3], v2 = P.edges[5 * e + 4];
+  q.e.v0 = P.edges[5 * e]; q.e.v1 = P.edges[5 * e + 1];
   const float len_e = P.efunc[e];
   if (!(len_e > 0.f)) return false;
   const float pdf_e = (len_e / (integral * (float)P.ne)) / len_e;
-  const F3 Pa = load3(s.pos, v0), Pb = load3(s.pos, v1), Pc = load3(s.pos, v2);
+  const F3 Pa = load3(s.pos, q.e.v0), Pb = load3(s.pos, q.e.v1), Pc = load3(s.pos, v2);
   const F3 e1 = Pb - Pa;
-  const F3 p0 = Pa + e1 * reuse;
-  const F3 edge = normalize(e1), edge2 = normalize(Pc - Pa);
+  q.e.s = reuse;
+  q.e.p0 = Pa + e1 * reuse;
+  q.e.edge = normalize(e1); q.e.edge2 = normalize(Pc - Pa);
   LightSample ls;
   if (!light_sample(s, r1, r2, ls)) return false;
   int j0, j1, j2; tri_vertices(s, ls.tri, j0, j1, j2);
-  const F3 p2 = bary3(ls.bu, ls.bv, load3(s.pos, j0), load3(s.pos, j1), load3(s.pos, j2));
-  const F3 nL = load3(s.fnormal, ls.tri);
-  const F3 ev = p2 - p0;
+  q.p2 = bary3(ls.bu, ls.bv, load3(s.pos, j0), load3(s.pos, j1), load3(s.pos, j2));
+  q.nL = load3(s.fnormal, ls.tri);
+  const F3 ev = q.p2 - q.e.p0;
   const float dist_sqr = dot(ev, ev);
   const float dist = sqrtf(dist_sqr);
   const F3 en = ev / dist;
-  const float cos_t = dot(nL, -en);
+  const float cos_t = dot(q.nL, -en);
   const F3 n0 = load3(s.fnormal, f0);
   const F3 n1 = f1 >= 0 ? load3(s.fnormal, f1) : F3z();
   const bool is_b = f1 < 0;
@@ -1758,27 +1523,47 @@ TRN_D bool direct_setup(const Params& P, long long gslot, EdgeState& st, int& vh
   const bool valid1 = (c0 > kEdgeEps && c1 < -kEdgeEps) || (c0 < -kEdgeEps && c1 > kEdgeEps);
   const bool right = (is_b && valid0) || (!is_b && valid1);
   if (!(right && cos_t > kEps && dist > kShadowEps)) return false;
-  const float pdf = pdf_e * ls.pdf * dist_sqr / cos_t * pdf_b;
-  const F3 rdir = normalize(p0 - p2);
-  Hit h0, h;
+  q.e.pdf = pdf_e * ls.pdf * dist_sqr / cos_t * pdf_b;
+  const F3 rdir = normalize(q.e.p0 - q.p2);
+  q.e.dir = -rdir;
   cnt.v[kCntClosest] += 2;
   cnt.v[kCntLight]++;
-  if (!trace_k<TRN_SETUP_SHARED_DIRECT, false>(s, p0, -rdir, kShadowEps, kRayMax, h0, P.err)) return false;
-  if (!trace_k<TRN_SETUP_SHARED_DIRECT, false>(s, p0, rdir, kShadowEps, kRayMax, h, P.err)) return false;
-  const F3 hp = p0 + (-rdir) * h0.t;
-  if (!(length(hp - p2) < kShadowEps)) return false;
+  return true;
+}
+
+// The first ray, from the edge point to the light, met the light point.
+TRN_D bool direct_lit(const DirectPoint& q, float t) {
+  const F3 hp = q.e.p0 + q.e.dir * t;
+  return length(hp - q.p2) < kShadowEps;
+}
+
+// h0: the light-side hit, h: the receiver behind the edge.
+TRN_D bool direct_finish(const Params& P, long long gslot, const DirectPoint& q, const Hit& h0, const Hit& h,
+                         EdgeState& st) {
+  const DeviceScene& s = P.s;
+  const F3 rdir = -q.e.dir;
   const SurfF xl = post_intersect(s, h0.tri, h0.u, h0.v);
   const F3 E = emitted(s, xl, rdir);
   const SurfF x = post_intersect(s, h.tri, h.u, h.v);
-  const float dl = length(p2 - x.p);
-  const float cos2 = fabsf(dot(nL, rdir));
-  const float its_t = length(x.p - p0);
+  const float dl = length(q.p2 - x.p);
+  const float cos2 = fabsf(dot(q.nL, rdir));
+  const float its_t = length(x.p - q.e.p0);
   F3 n;
-  const float bval = base_val(its_t / dl, edge, -rdir, nL, edge2, n) * cos2;
+  const float bval = base_val(its_t / dl, q.e.edge, q.e.dir, q.nL, q.e.edge2, n) * cos2;
   if (bval == 0.f || (E.x == 0.f && E.y == 0.f && E.z == 0.f)) return false;
-  st.V = &V; st.gslot = gslot; st.p = p; st.x = x; st.rdir = rdir; st.T0 = E; st.p0 = p0; st.n = n;
-  st.w0 = bval / pdf; st.sedge = reuse; st.v0 = v0; st.v1 = v1; st.far_tri = h0.tri;
+  st.V = q.e.V; st.gslot = gslot; st.p = q.e.p; st.x = x; st.rdir = rdir; st.T0 = E; st.p0 = q.e.p0; st.n = n;
+  st.w0 = bval / q.e.pdf; st.sedge = q.e.s; st.v0 = q.e.v0; st.v1 = q.e.v1; st.far_tri = h0.tri;
   return true;
+}
+
+TRN_D bool direct_setup(const Params& P, long long gslot, EdgeState& st, int& vhint, Cnt& cnt) {
+  DirectPoint q;
+  if (!direct_point(P, gslot, q, vhint, cnt)) return false;
+  Hit h0, h;
+  if (!trace<false>(P.s, q.e.p0, q.e.dir, kShadowEps, kRayMax, h0, P.err)) return false;
+  if (!trace<false>(P.s, q.e.p0, -q.e.dir, kShadowEps, kRayMax, h, P.err)) return false;
+  if (!direct_lit(q, h0.t)) return false;
+  return direct_finish(P, gslot, q, h0, h, st);
 }
 
 // Direct boundary body: trace towards the sensor (EvalImportance per bounce,
@@ -1794,7 +1579,7 @@ TRN_D void direct_body(const Params& P, const ViewDesc& V, long long gslot, long
   for (int b = 0; b < V.D; b++) {
     const int o = 3 + 3 * b;
     F3 c; int pix;
-    const bool more = importance_step_k<TRN_SHARED_STEPS_DIRECT>(s, V.cam, xs, dirs, T, S(o), S(o + 1), S(o + 2), c,
+    const bool more = importance_step(s, V.cam, xs, dirs, T, S(o), S(o + 1), S(o + 2), c,
                                                                  pix, cnt);
     if (pix >= 0) W += dot(g_at(P, V, pix), ev0 * c);
     if (!more) break;
@@ -1805,7 +1590,6 @@ TRN_D void direct_body(const Params& P, const ViewDesc& V, long long gslot, long
 
 __global__ void __launch_bounds__(256, TRN_MINB) k_direct_adj(TRN_KPARAMS) {
   Cnt cnt;
-  stage_top(P.s);
   int vhint = 0;
   for_each_valid<EdgeState>(P,
     [&](long long gslot, EdgeState& st) -> bool { return direct_setup(P, gslot, st, vhint, cnt); },
@@ -1816,62 +1600,13 @@ __global__ void __launch_bounds__(256, TRN_MINB) k_direct_adj(TRN_KPARAMS) {
   flush_cnt(cnt, P.stats);
 }
 
-// Split form: k_direct_setup tests every slot once and queues the accepted
-// samples; k_direct_body runs their importance paths and scatters.
+// A sample that passed the direct set-up; its importance path and scatter follow.
 struct DirectItem {
-  long long gslot, p;
+  long long p;
   int view, x_tri, v0, v1, far_tri, pad_;
   float x_u, x_v, sedge, pad2_;
   F3 rdir, ev0, p0, n;
 };
-
-__global__ void __launch_bounds__(256, TRN_MINB_SETUP) k_direct_setup(TRN_KPARAMS) {
-  Cnt cnt;
-  stage_top(P.s);
-  int vhint = 0;
-  DirectItem* q = reinterpret_cast<DirectItem*>(P.queue);
-  const int lane = threadIdx.x & 31;
-  const unsigned lt = (1u << lane) - 1u;
-  for (;;) {
-    unsigned long long start = 0;
-    if (lane == 0) start = atomicAdd(P.work, 32ull);
-    start = __shfl_sync(0xffffffffu, start, 0);
-    if ((long long)start >= P.total) break;
-    const long long g = slot_at(P, (long long)start + lane);
-    EdgeState st;
-    const bool ok = g < P.total && direct_setup(P, g, st, vhint, cnt);
-    const unsigned m = __ballot_sync(0xffffffffu, ok);
-    if (!m) continue;
-    const int leader = __ffs(m) - 1;
-    unsigned long long base = 0;
-    if (lane == leader) base = atomicAdd(P.q_count, (unsigned long long)__popc(m));
-    base = __shfl_sync(0xffffffffu, base, leader);
-    const unsigned long long k = base + __popc(m & lt);
-    if (ok && k >= (unsigned long long)P.q_cap) atomicExch(P.err, 2);
-    if (ok && k < (unsigned long long)P.q_cap) {
-      DirectItem& it = q[k];
-      it.gslot = st.gslot; it.p = st.p; it.view = (int)(st.V - P.views);
-      it.x_tri = st.x.tri; it.x_u = st.x.u; it.x_v = st.x.v; it.v0 = st.v0; it.v1 = st.v1; it.far_tri = st.far_tri;
-      it.sedge = st.sedge; it.rdir = st.rdir; it.ev0 = st.T0 * st.w0; it.p0 = st.p0; it.n = st.n;
-    }
-  }
-  flush_cnt(cnt, P.stats);
-}
-
-__global__ void __launch_bounds__(256, TRN_MINB_BODY) k_direct_body(TRN_KPARAMS) {
-  Cnt cnt;
-  stage_top(P.s);
-  const DirectItem* q = reinterpret_cast<const DirectItem*>(P.queue);
-  const unsigned long long n = min(*P.q_count, (unsigned long long)P.q_cap);
-  for (unsigned long long k = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; k < n;
-       k += (unsigned long long)gridDim.x * blockDim.x) {
-    const DirectItem& it = q[k];
-    const SurfF x = post_intersect(P.s, it.x_tri, it.x_u, it.x_v);
-    direct_body(P, P.views[it.view], it.gslot, it.p, x, it.rdir, it.ev0, it.v0, it.v1, it.sedge, it.p0, it.far_tri,
-                it.n, cnt);
-  }
-  flush_cnt(cnt, P.stats);
-}
 
 // ---------------------------------------------------------------------------
 // AQ guiding of the direct boundary term (AdaptiveQuadratureDistribution::setup,
@@ -1882,33 +1617,45 @@ constexpr uint32_t kGuideTerm = 5;  // hash-sampler term of the set-up samples
 // |baseVal| of one (edge, light) sample in guiding mode (Edge.cpp:201-259 with
 // guiding_mode=true): only the evaluation mask (same point, both rays hit)
 // applies, and neither radiance nor pdf enters. Invalid samples give 0.
-TRN_D float guide_base_val(const Params& P, float x, float y, float z) {
+// e.dir: from the edge point to the light point.
+TRN_D bool guide_point(const Params& P, float x, float y, float z, DirectPoint& q) {
   const DeviceScene& s = P.s;
   float reuse;
   const int e = sample_discrete(P.ecdf, P.ne, x, reuse);
   const int v0 = P.edges[5 * e], v1 = P.edges[5 * e + 1], v2 = P.edges[5 * e + 4];
   const F3 Pa = load3(s.pos, v0), Pb = load3(s.pos, v1), Pc = load3(s.pos, v2);
   const F3 e1 = Pb - Pa;
-  const F3 p0 = Pa + e1 * reuse;
-  const F3 edge = normalize(e1), edge2 = normalize(Pc - Pa);
+  q.e.p0 = Pa + e1 * reuse;
+  q.e.edge = normalize(e1); q.e.edge2 = normalize(Pc - Pa);
   LightSample ls;
-  if (!light_sample(s, y, z, ls)) return 0.f;
+  if (!light_sample(s, y, z, ls)) return false;
   int j0, j1, j2; tri_vertices(s, ls.tri, j0, j1, j2);
-  const F3 p2 = bary3(ls.bu, ls.bv, load3(s.pos, j0), load3(s.pos, j1), load3(s.pos, j2));
-  const F3 nL = load3(s.fnormal, ls.tri);
-  const F3 rdir = normalize(p0 - p2);
-  Hit h0, h;
-  if (!trace<false>(s, p0, -rdir, kShadowEps, kRayMax, h0, P.err)) return 0.f;
-  if (!trace<false>(s, p0, rdir, kShadowEps, kRayMax, h, P.err)) return 0.f;
-  const F3 hp = p0 + (-rdir) * h0.t;
-  if (!(length(hp - p2) < kShadowEps)) return 0.f;
-  const SurfF xs = post_intersect(s, h.tri, h.u, h.v);
-  const float dl = length(p2 - xs.p);
-  const float cos2 = fabsf(dot(nL, rdir));
-  const float its_t = length(xs.p - p0);
+  q.p2 = bary3(ls.bu, ls.bv, load3(s.pos, j0), load3(s.pos, j1), load3(s.pos, j2));
+  q.nL = load3(s.fnormal, ls.tri);
+  q.e.dir = -normalize(q.e.p0 - q.p2);
+  return true;
+}
+
+// h: the receiver behind the edge; the ray to the light met the light point.
+TRN_D float guide_value(const Params& P, const DirectPoint& q, const Hit& h) {
+  const SurfF xs = post_intersect(P.s, h.tri, h.u, h.v);
+  const float dl = length(q.p2 - xs.p);
+  const float cos2 = fabsf(dot(q.nL, -q.e.dir));
+  const float its_t = length(xs.p - q.e.p0);
   F3 n;
-  const float bv = fabsf(base_val(its_t / dl, edge, -rdir, nL, edge2, n) * cos2);
+  const float bv = fabsf(base_val(its_t / dl, q.e.edge, q.e.dir, q.nL, q.e.edge2, n) * cos2);
   return isfinite(bv) ? bv : 0.f;
+}
+
+// The whole sample by one thread (the allocation-free entry point).
+TRN_D float guide_base_val(const Params& P, float x, float y, float z) {
+  DirectPoint q;
+  if (!guide_point(P, x, y, z, q)) return 0.f;
+  Hit h0, h;
+  if (!trace<false>(P.s, q.e.p0, q.e.dir, kShadowEps, kRayMax, h0, P.err)) return 0.f;
+  if (!trace<false>(P.s, q.e.p0, -q.e.dir, kShadowEps, kRayMax, h, P.err)) return 0.f;
+  if (!direct_lit(q, h0.t)) return 0.f;
+  return guide_value(P, q, h);
 }
 
 constexpr uint32_t kRefineTerm = 6;  // hash-sampler term of the refinement's random points
@@ -2141,40 +1888,43 @@ __global__ void k_aq_mix(const int* count, float* poly, const float* box, long l
 // indirect boundary (BoundaryIndirect.cpp:38-192, Edge.cpp:146-199)
 // ---------------------------------------------------------------------------
 // Indirect boundary set-up (SampleBoundarySegmentIndirect, Edge.cpp:146-199,
-// BoundaryIndirect.cpp:58-130): edge point, direction in the edge wedge, both
-// rays, boundary geometry. Returns false for a rejected sample.
-TRN_D bool indirect_setup(const Params& P, long long gslot, EdgeState& st, int& vhint, Cnt& cnt) {
+// BoundaryIndirect.cpp:58-130): edge point and direction in the edge wedge;
+// with the hits of the two rays that leave the point along -dir (emitter side)
+// and dir (sensor side), the boundary geometry. Both return false for a
+// rejected sample.
+TRN_D bool indirect_point(const Params& P, long long gslot, EdgePoint& q, int& vhint) {
   const DeviceScene& s = P.s;
   const ViewDesc& V = view_of(P, gslot, vhint);
-  const long long p = gslot - V.begin;
+  q.V = &V;
+  q.p = gslot - V.begin;
   if (V.D < 2) return false;
-  const PathSmp S{&P, V.seed, gslot, p + V.slot_off};
+  const PathSmp S{&P, V.seed, gslot, q.p + V.slot_off};
   const float r0 = S(0), r1 = S(1), r2 = S(2);
   float reuse;
   const float integral = __ldg(P.eint);
   if (!(integral > 0.f)) return false;
   const int e = sample_discrete(P.ecdf, P.ne, r0, reuse);
-  const int v0 = P.edges[5 * e], v1 = P.edges[5 * e + 1], f0 = P.edges[5 * e + 2], f1 = P.edges[5 * e + 3],
-            v2 = P.edges[5 * e + 4];
+  const int f0 = P.edges[5 * e + 2], f1 = P.edges[5 * e + 3], v2 = P.edges[5 * e + 4];
+  q.v0 = P.edges[5 * e]; q.v1 = P.edges[5 * e + 1];
   const float len_e = P.efunc[e];
   if (!(len_e > 0.f)) return false;
   const float pdf_e = (len_e / (integral * (float)P.ne)) / len_e;
-  const F3 Pa = load3(s.pos, v0), Pb = load3(s.pos, v1), Pc = load3(s.pos, v2);
+  const F3 Pa = load3(s.pos, q.v0), Pb = load3(s.pos, q.v1), Pc = load3(s.pos, v2);
   const F3 e1 = Pb - Pa;
-  const F3 p0 = Pa + e1 * reuse;
-  const F3 edge = normalize(e1), edge2 = normalize(Pc - Pa);
+  q.s = reuse;
+  q.p0 = Pa + e1 * reuse;
+  q.edge = normalize(e1); q.edge2 = normalize(Pc - Pa);
   const F3 n0 = load3(s.fnormal, f0);
-  F3 dir;
   float pdf_d;
   if (f1 < 0) {
-    const F3 nrm = cross(n0, edge);
+    const F3 nrm = cross(n0, q.edge);
     F3 tg, bt; coordinate_system(nrm, tg, bt);
     const float z = fminf(1.f - 2.f * r1, 1.f - kEdgeEps);
     const float r = sqrtf(fmaxf(0.f, 1.f - z * z));
     const float phi = 2.f * kPi * r2;
     float sp, cp;
     sincos_det(phi, sp, cp);
-    dir = tg * (r * cp) + bt * (r * sp) + nrm * z;
+    q.dir = tg * (r * cp) + bt * (r * sp) + nrm * z;
     pdf_d = 0.25f / kPi;
   } else {
     const F3 n1 = load3(s.fnormal, f1);
@@ -2191,29 +1941,37 @@ TRN_D bool indirect_setup(const Params& P, long long gslot, EdgeState& st, int& 
     const bool m0 = r2 > 0.5f;
     const float bq = 4.f * r2 - (m0 ? 3.f : 1.f);
     const float aq = sqrtf(1.f - bq * bq) * (1.f - (m0 ? 1.f : 0.f) * 2.f);
-    dir = x1 * aq + yy * bq;
+    q.dir = x1 * aq + yy * bq;
   }
-  const float pdf = pdf_e * pdf_d;
-  Hit he, hs;
-  cnt.v[kCntClosest] += 2;
-#if TRN_INDIRECT_SENSOR_FIRST
-  if (!trace_k<TRN_INDIRECT_SETUP_SHARED, false>(s, p0, dir, kShadowEps, kRayMax, hs, P.err)) return false;
-  if (!trace_k<TRN_INDIRECT_SETUP_SHARED, false>(s, p0, -dir, kShadowEps, kRayMax, he, P.err)) return false;
-#else
-  if (!trace_k<TRN_INDIRECT_SETUP_SHARED, false>(s, p0, -dir, kShadowEps, kRayMax, he, P.err)) return false;
-  if (!trace_k<TRN_INDIRECT_SETUP_SHARED, false>(s, p0, dir, kShadowEps, kRayMax, hs, P.err)) return false;
-#endif
+  q.pdf = pdf_e * pdf_d;
+  return true;
+}
+
+// he: emitter-side hit, hs: sensor-side hit.
+TRN_D bool indirect_finish(const Params& P, long long gslot, const EdgePoint& q, const Hit& he, const Hit& hs,
+                           EdgeState& st) {
+  const DeviceScene& s = P.s;
   const SurfF xe = post_intersect(s, he.tri, he.u, he.v);
   const SurfF xs = post_intersect(s, hs.tri, hs.u, hs.v);
   const float dl = length(xe.p - xs.p);
-  const float cos2 = fabsf(dot(xe.ng, dir));
-  const float its_t = length(xs.p - p0);
+  const float cos2 = fabsf(dot(xe.ng, q.dir));
+  const float its_t = length(xs.p - q.p0);
   F3 n;
-  const float bval = base_val(its_t / dl, edge, -dir, xe.ng, edge2, n) * cos2;
+  const float bval = base_val(its_t / dl, q.edge, -q.dir, xe.ng, q.edge2, n) * cos2;
   if (bval == 0.f) return false;
-  st.V = &V; st.gslot = gslot; st.p = p; st.x = xs; st.xe = xe; st.rdir = dir; st.p0 = p0; st.n = n;
-  st.w0 = bval / pdf; st.sedge = reuse; st.v0 = v0; st.v1 = v1; st.far_tri = he.tri;
+  st.V = q.V; st.gslot = gslot; st.p = q.p; st.x = xs; st.xe = xe; st.rdir = q.dir; st.p0 = q.p0; st.n = n;
+  st.w0 = bval / q.pdf; st.sedge = q.s; st.v0 = q.v0; st.v1 = q.v1; st.far_tri = he.tri;
   return true;
+}
+
+TRN_D bool indirect_setup(const Params& P, long long gslot, EdgeState& st, int& vhint, Cnt& cnt) {
+  EdgePoint q;
+  if (!indirect_point(P, gslot, q, vhint)) return false;
+  Hit he, hs;
+  cnt.v[kCntClosest] += 2;
+  if (!trace_shared<false>(P.s, q.p0, -q.dir, kShadowEps, kRayMax, he, P.err)) return false;
+  if (!trace_shared<false>(P.s, q.p0, q.dir, kShadowEps, kRayMax, hs, P.err)) return false;
+  return indirect_finish(P, gslot, q, he, hs, st);
 }
 
 // Indirect boundary sensor side (BoundaryIndirect.cpp:158-175 pairs sensor
@@ -2272,9 +2030,8 @@ TRN_D float indirect_emitter(const Params& P, const ViewDesc& V, long long gslot
 }
 
 template <int MAXD>
-__global__ void __launch_bounds__(256, TRN_MINB_INDIRECT) k_indirect_adj(TRN_KPARAMS) {
+__global__ void __launch_bounds__(256, TRN_MINB) k_indirect_adj(TRN_KPARAMS) {
   Cnt cnt;
-  stage_top(P.s);
   int vhint = 0;
   for_each_valid<EdgeState>(P,
     [&](long long gslot, EdgeState& st) -> bool { return indirect_setup(P, gslot, st, vhint, cnt); },
@@ -2295,345 +2052,16 @@ __global__ void __launch_bounds__(256, TRN_MINB_INDIRECT) k_indirect_adj(TRN_KPA
   flush_cnt(cnt, P.stats);
 }
 
-// Split form of the same term: k_indirect_sensor runs the set-up and the
-// sensor side and queues the samples whose sensor side reached the image;
-// k_indirect_emitter runs the emitter side and the scatter for the queue.
-// Each kernel carries half of the fused kernel's code (the fused kernel is
-// instruction-fetch bound), and the emitter pass runs on survivors only.
-template <int MAXD>
+// A sample that passed the indirect set-up; its sensor side, emitter side and
+// scatter follow.
 struct IndirectItem {
-  long long gslot, p;
-  int view, jmax, D;
-  int xe_tri, xs_tri;
-  float xe_u, xe_v, xs_u, xs_v;
-  F3 rdir, p0, n;
-  float w0, sedge;
-  int v0, v1, far_tri;
-  F3 sc[MAXD];
-};
-
-template <int MAXD>
-__global__ void __launch_bounds__(256, TRN_MINB_INDIRECT) k_indirect_sensor(TRN_KPARAMS) {
-  Cnt cnt;
-  stage_top(P.s);
-  int vhint = 0;
-  IndirectItem<MAXD>* q = reinterpret_cast<IndirectItem<MAXD>*>(P.queue);
-  for_each_valid<EdgeState>(P,
-    [&](long long gslot, EdgeState& st) -> bool { return indirect_setup(P, gslot, st, vhint, cnt); },
-    [&](EdgeState& st) {
-      const int D = min(st.V->D, MAXD);
-      F3 sc[MAXD];
-      const int bmin = indirect_sensor<MAXD>(P, st, D, sc, cnt);
-      if (bmin >= D - 1) return;
-      const unsigned long long k = atomicAdd(P.q_count, 1ull);
-      if (k >= (unsigned long long)P.q_cap) { atomicExch(P.err, 2); return; }
-      IndirectItem<MAXD>& it = q[k];
-      it.gslot = st.gslot; it.p = st.p;
-      it.view = (int)(st.V - P.views); it.jmax = D - 2 - bmin; it.D = D;
-      it.xe_tri = st.xe.tri; it.xe_u = st.xe.u; it.xe_v = st.xe.v;
-      it.xs_tri = st.x.tri; it.xs_u = st.x.u; it.xs_v = st.x.v;
-      it.rdir = st.rdir; it.p0 = st.p0; it.n = st.n; it.w0 = st.w0; it.sedge = st.sedge;
-      it.v0 = st.v0; it.v1 = st.v1; it.far_tri = st.far_tri;
-      for (int b = 0; b < D - 1; b++) it.sc[b] = sc[b];
-    });
-  flush_cnt(cnt, P.stats);
-}
-
-template <int MAXD>
-__global__ void __launch_bounds__(256, TRN_MINB_INDIRECT) k_indirect_emitter(TRN_KPARAMS) {
-  Cnt cnt;
-  stage_top(P.s);
-  // two-stage form: the queue and its count; three-stage form: the second queue
-  const IndirectItem<MAXD>* q = reinterpret_cast<const IndirectItem<MAXD>*>(P.queue2 ? P.queue2 : P.queue);
-  const unsigned long long n = min(P.q_count[P.queue2 ? 1 : 0], (unsigned long long)P.q_cap);
-  for (unsigned long long k = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; k < n;
-       k += (unsigned long long)gridDim.x * blockDim.x) {
-    const IndirectItem<MAXD>& it = q[k];
-    const ViewDesc& V = P.views[it.view];
-    const SurfF xe = post_intersect(P.s, it.xe_tri, it.xe_u, it.xe_v);
-    const float W = indirect_emitter<MAXD>(P, V, it.gslot, it.p, xe, it.rdir, it.w0, it.D, it.jmax, it.sc, cnt);
-    if (W == 0.f || !isfinite(W)) continue;
-    const SurfF xs = post_intersect(P.s, it.xs_tri, it.xs_u, it.xs_v);
-    xdotn_vjp(P, V, W, xs.p, true, it.xs_tri, it.xs_u, it.xs_v, it.v0, it.v1, it.sedge, it.p0, it.far_tri, it.n,
-              cnt);
-  }
-  flush_cnt(cnt, P.stats);
-}
-
-// Three-stage form of the indirect term: k_indirect_setup tests every slot
-// once (the two set-up rays are most of the term's rays) and queues the
-// accepted samples; k_indirect_sensor_q runs the sensor side over that queue
-// and queues survivors for k_indirect_emitter.
-struct IndirectSetupItem {
-  long long gslot, p;
+  unsigned p_lo;  // view-local sample index in two halves: 92 bytes without padding
+  int p_hi;
   int view, xe_tri, xs_tri, v0, v1, far_tri;
   float xe_u, xe_v, xs_u, xs_v, w0, sedge;
   F3 rdir, p0, n;
+  TRN_D long long p() const { return (long long)p_hi << 32 | p_lo; }
 };
-
-__global__ void __launch_bounds__(256, TRN_MINB_SETUP) k_indirect_setup(TRN_KPARAMS) {
-  Cnt cnt;
-  stage_top(P.s);
-  int vhint = 0;
-  IndirectSetupItem* q = reinterpret_cast<IndirectSetupItem*>(P.queue);
-  const int lane = threadIdx.x & 31;
-  const unsigned lt = (1u << lane) - 1u;
-  for (;;) {
-    unsigned long long start = 0;
-    if (lane == 0) start = atomicAdd(P.work, 32ull);
-    start = __shfl_sync(0xffffffffu, start, 0);
-    if ((long long)start >= P.total) break;
-    const long long g = slot_at(P, (long long)start + lane);
-    EdgeState st;
-    const bool ok = g < P.total && indirect_setup(P, g, st, vhint, cnt);
-    const unsigned m = __ballot_sync(0xffffffffu, ok);
-    if (!m) continue;
-    const int leader = __ffs(m) - 1;
-    unsigned long long base = 0;
-    if (lane == leader) base = atomicAdd(P.q_count, (unsigned long long)__popc(m));
-    base = __shfl_sync(0xffffffffu, base, leader);
-    const unsigned long long k = base + __popc(m & lt);
-    if (ok && k >= (unsigned long long)P.q_cap) atomicExch(P.err, 2);
-    if (ok && k < (unsigned long long)P.q_cap) {
-      IndirectSetupItem& it = q[k];
-      it.gslot = st.gslot; it.p = st.p; it.view = (int)(st.V - P.views);
-      it.xe_tri = st.xe.tri; it.xe_u = st.xe.u; it.xe_v = st.xe.v;
-      it.xs_tri = st.x.tri; it.xs_u = st.x.u; it.xs_v = st.x.v;
-      it.v0 = st.v0; it.v1 = st.v1; it.far_tri = st.far_tri; it.w0 = st.w0; it.sedge = st.sedge;
-      it.rdir = st.rdir; it.p0 = st.p0; it.n = st.n;
-    }
-  }
-  flush_cnt(cnt, P.stats);
-}
-
-template <int MAXD>
-__global__ void __launch_bounds__(256, TRN_MINB_INDIRECT) k_indirect_sensor_q(TRN_KPARAMS) {
-  Cnt cnt;
-  stage_top(P.s);
-  const IndirectSetupItem* qa = reinterpret_cast<const IndirectSetupItem*>(P.queue);
-  IndirectItem<MAXD>* qb = reinterpret_cast<IndirectItem<MAXD>*>(P.queue2);
-  const unsigned long long n = min(P.q_count[0], (unsigned long long)P.q_cap);
-  const int lane = threadIdx.x & 31;
-  for (unsigned long long k0 = (blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x) & ~31ull; k0 < n;
-       k0 += (unsigned long long)gridDim.x * blockDim.x) {
-    const unsigned long long k = k0 + lane;
-    bool push = false;
-    EdgeState st;
-    F3 sc[MAXD];
-    int D = 0, bmin = 0;
-    if (k < n) {
-      const IndirectSetupItem& a = qa[k];
-      st.V = P.views + a.view; st.gslot = a.gslot; st.p = a.p;
-      st.x = post_intersect(P.s, a.xs_tri, a.xs_u, a.xs_v);
-      st.rdir = a.rdir;
-      D = min(st.V->D, MAXD);
-      bmin = indirect_sensor<MAXD>(P, st, D, sc, cnt);
-      push = bmin < D - 1;
-    }
-    const unsigned m = __ballot_sync(0xffffffffu, push);
-    if (!m) continue;
-    const int leader = __ffs(m) - 1;
-    unsigned long long base = 0;
-    if (lane == leader) base = atomicAdd(P.q_count + 1, (unsigned long long)__popc(m));
-    base = __shfl_sync(0xffffffffu, base, leader);
-    const unsigned long long j = base + __popc(m & ((1u << lane) - 1u));
-    if (push && j >= (unsigned long long)P.q_cap) atomicExch(P.err, 2);
-    if (push && j < (unsigned long long)P.q_cap) {
-      const IndirectSetupItem& a = qa[k];
-      IndirectItem<MAXD>& it = qb[j];
-      it.gslot = a.gslot; it.p = a.p; it.view = a.view; it.jmax = D - 2 - bmin; it.D = D;
-      it.xe_tri = a.xe_tri; it.xe_u = a.xe_u; it.xe_v = a.xe_v;
-      it.xs_tri = a.xs_tri; it.xs_u = a.xs_u; it.xs_v = a.xs_v;
-      it.rdir = a.rdir; it.p0 = a.p0; it.n = a.n; it.w0 = a.w0; it.sedge = a.sedge;
-      it.v0 = a.v0; it.v1 = a.v1; it.far_tri = a.far_tri;
-      for (int b = 0; b < D - 1; b++) it.sc[b] = sc[b];
-    }
-  }
-  flush_cnt(cnt, P.stats);
-}
-
-// k_indirect_sensor_q with path regeneration: a lane whose importance path
-// has ended queues its item (when a depth reached the image) and takes the
-// next set-up item at once. Each item runs exactly the steps of
-// indirect_sensor.
-#ifndef TRN_SENSOR_REGEN
-#define TRN_SENSOR_REGEN 1
-#endif
-
-template <int MAXD>
-__global__ void __launch_bounds__(256, TRN_MINB_INDIRECT) k_indirect_sensor_regen(TRN_KPARAMS) {
-  Cnt cnt;
-  stage_top(P.s);
-  const DeviceScene& s = P.s;
-  const IndirectSetupItem* qa = reinterpret_cast<const IndirectSetupItem*>(P.queue);
-  IndirectItem<MAXD>* qb = reinterpret_cast<IndirectItem<MAXD>*>(P.queue2);
-  const unsigned long long n = min(P.q_count[0], (unsigned long long)P.q_cap);
-  unsigned long long* next = P.q_count + 2;
-  const int lane = threadIdx.x & 31;
-  const unsigned lt = (1u << lane) - 1u;
-  bool active = false, done = false;
-  unsigned long long k = 0;
-  const ViewDesc* V = nullptr;
-  SurfF xx;
-  F3 T, rd;
-  F3 sc[MAXD];
-  int b = 0, D = 0, bmin = 0;
-  for (;;) {
-    const unsigned need = __ballot_sync(0xffffffffu, !active && !done);
-    if (need) {
-      const int leader = __ffs(need) - 1;
-      unsigned long long base = 0;
-      if (lane == leader) base = atomicAdd(next, (unsigned long long)__popc(need));
-      base = __shfl_sync(0xffffffffu, base, leader);
-      if (!active && !done) {
-        k = base + __popc(need & lt);
-        if (k >= n) {
-          done = true;
-        } else {
-          const IndirectSetupItem& a = qa[k];
-          V = P.views + a.view;
-          D = min(V->D, MAXD);
-          xx = post_intersect(s, a.xs_tri, a.xs_u, a.xs_v);
-          rd = a.rdir;
-          T = F3(1.f, 1.f, 1.f);
-          for (int j = 0; j < D - 1; j++) sc[j] = F3z();
-          bmin = D;
-          b = 0;
-          active = true;
-        }
-      }
-    }
-    if (!__any_sync(0xffffffffu, active)) break;
-    bool fin = false;
-    if (active) {
-      fin = b >= D - 1;
-      if (!fin) {
-        const IndirectSetupItem& a = qa[k];
-        const PathSmp S{&P, V->seed, a.gslot, a.p + V->slot_off};
-        const int o = 3 + 5 * (D - 1) + 3 * b;
-        F3 c;
-        int pix;
-        const bool more = importance_step_k<TRN_SHARED_STEPS_INDIRECT>(s, V->cam, xx, rd, T, S(o), S(o + 1),
-                                                                        S(o + 2), c, pix, cnt);
-        if (pix >= 0) {
-          sc[b] = g_at(P, *V, pix) * c;
-          if (sc[b].x != 0.f || sc[b].y != 0.f || sc[b].z != 0.f) bmin = min(bmin, b);
-        }
-        b++;
-        fin = !more || b >= D - 1;
-      }
-    }
-    const bool push = fin && bmin < D - 1;
-    const unsigned m = __ballot_sync(0xffffffffu, push);
-    if (m) {
-      const int leader = __ffs(m) - 1;
-      unsigned long long base = 0;
-      if (lane == leader) base = atomicAdd(P.q_count + 1, (unsigned long long)__popc(m));
-      base = __shfl_sync(0xffffffffu, base, leader);
-      const unsigned long long j = base + __popc(m & lt);
-      if (push && j >= (unsigned long long)P.q_cap) atomicExch(P.err, 2);
-      if (push && j < (unsigned long long)P.q_cap) {
-        const IndirectSetupItem& a = qa[k];
-        IndirectItem<MAXD>& it = qb[j];
-        it.gslot = a.gslot; it.p = a.p; it.view = a.view; it.jmax = D - 2 - bmin; it.D = D;
-        it.xe_tri = a.xe_tri; it.xe_u = a.xe_u; it.xe_v = a.xe_v;
-        it.xs_tri = a.xs_tri; it.xs_u = a.xs_u; it.xs_v = a.xs_v;
-        it.rdir = a.rdir; it.p0 = a.p0; it.n = a.n; it.w0 = a.w0; it.sedge = a.sedge;
-        it.v0 = a.v0; it.v1 = a.v1; it.far_tri = a.far_tri;
-        for (int q = 0; q < D - 1; q++) it.sc[q] = sc[q];
-      }
-    }
-    if (fin) active = false;
-  }
-  flush_cnt(cnt, P.stats);
-}
-
-// k_indirect_emitter with path regeneration (three-stage form): a lane whose
-// emitter-side path has ended adds the remaining depths' terms with its last
-// radiance, as the loop form does after the path dies, scatters, and takes
-// the next item at once. Each item runs exactly the steps and the
-// additions of indirect_emitter.
-#ifndef TRN_EMITTER_REGEN
-#define TRN_EMITTER_REGEN 1
-#endif
-
-template <int MAXD>
-__global__ void __launch_bounds__(256, TRN_MINB_INDIRECT) k_indirect_emitter_regen(TRN_KPARAMS) {
-  Cnt cnt;
-  stage_top(P.s);
-  const DeviceScene& s = P.s;
-  const IndirectItem<MAXD>* q = reinterpret_cast<const IndirectItem<MAXD>*>(P.queue2);
-  const unsigned long long n = min(P.q_count[1], (unsigned long long)P.q_cap);
-  unsigned long long* next = P.q_count + 3;
-  const int lane = threadIdx.x & 31;
-  const unsigned lt = (1u << lane) - 1u;
-  bool active = false, done = false;
-  unsigned long long k = 0;
-  const ViewDesc* V = nullptr;
-  SurfF xx;
-  F3 T, rd, cur;
-  float W = 0.f;
-  int j = 0;
-  for (;;) {
-    const unsigned need = __ballot_sync(0xffffffffu, !active && !done);
-    if (need) {
-      const int leader = __ffs(need) - 1;
-      unsigned long long base = 0;
-      if (lane == leader) base = atomicAdd(next, (unsigned long long)__popc(need));
-      base = __shfl_sync(0xffffffffu, base, leader);
-      if (!active && !done) {
-        k = base + __popc(need & lt);
-        if (k >= n) {
-          done = true;
-        } else {
-          const IndirectItem<MAXD>& it = q[k];
-          V = P.views + it.view;
-          xx = post_intersect(s, it.xe_tri, it.xe_u, it.xe_v);
-          rd = -it.rdir;
-          T = F3(1.f, 1.f, 1.f);
-          cur = F3z();
-          W = 0.f;
-          j = 0;
-          active = true;
-        }
-      }
-    }
-    if (!__any_sync(0xffffffffu, active)) break;
-    if (active) {
-      const IndirectItem<MAXD>& it = q[k];
-      const int D = it.D, jmax = it.jmax;
-      bool alive = false;
-      if (j <= jmax) {
-        const PathSmp S{&P, V->seed, it.gslot, it.p + V->slot_off};
-        const int o = 3 + 5 * j;
-        F3 c;
-        alive = radiance_step_k<TRN_SHARED_STEPS_INDIRECT>(s, xx, rd, T, S(o), S(o + 1), S(o + 2), S(o + 3),
-                                                           S(o + 4), c, nullptr, cnt);
-        cur = cur + c;
-        if (T.x == 0.f && T.y == 0.f && T.z == 0.f) alive = false;
-        W += dot(it.sc[D - 2 - j], cur) * it.w0;
-        j++;
-      }
-      if (!alive || j > jmax) {
-        // the path has ended: the remaining depths pair with the last radiance
-        for (; j <= jmax; j++) W += dot(it.sc[D - 2 - j], cur) * it.w0;
-        if (W != 0.f && isfinite(W)) {
-          const SurfF xs = post_intersect(s, it.xs_tri, it.xs_u, it.xs_v);
-          xdotn_vjp(P, *V, W, xs.p, true, it.xs_tri, it.xs_u, it.xs_v, it.v0, it.v1, it.sedge, it.p0, it.far_tri,
-                    it.n, cnt);
-        }
-        active = false;
-      }
-    }
-  }
-  flush_cnt(cnt, P.stats);
-}
-
-// Slot range of one split round: the work counter starts at `first`, the
-// queue is empty.
-__global__ void k_indirect_round(unsigned long long* work, unsigned long long first, unsigned long long* q_count) {
-  if (threadIdx.x == 0) { *work = first; q_count[0] = 0ull; q_count[1] = 0ull; q_count[2] = 0ull; q_count[3] = 0ull; }
-}
 
 // Sort keys of one round of a split boundary set-up: view x (E + 1) + the
 // edge that the slot's edge sample picks (E when it picks none), value = the
@@ -2679,38 +2107,37 @@ __global__ void k_edge_keys(TRN_KPARAMS, int term, int bits_r1, int bits_r2, uns
 }
 
 
-#ifndef TRN_PIXEL_INTERLEAVE
-#define TRN_PIXEL_INTERLEAVE 1
-#endif
-
 // ---------------------------------------------------------------------------
 // pixel boundary (BoundaryPixel.cpp:36-159, Edge.cpp:377-409, Camera.cpp:433-467)
 // ---------------------------------------------------------------------------
 // Pixel boundary set-up (SampleBoundarySegmentPixel, Edge.cpp:377-409;
 // GeneratePixelBoundarySamples, Camera.cpp:433-467): a point on the pixel's
-// boundary from the antithetic copy's sample, the camera ray through it, the
-// boundary geometry. Returns false for a rejected sample.
-TRN_D bool pixel_setup(const Params& P, long long gslot, EdgeState& st, int& vhint, Cnt& cnt) {
-  const DeviceScene& s = P.s;
+// boundary from the antithetic copy's sample and the camera ray through it;
+// with that ray's hit, the boundary geometry.
+struct PixelPoint {
+  const ViewDesc* V;
+  long long slot;     // of the view's slots, shared by the 4 antithetic copies
+  int pixel;
+  float pdf;
+  F3 p0, dir, edge, edge2;
+};
+
+TRN_D void pixel_point(const Params& P, long long gslot, PixelPoint& q, int& vhint) {
   const ViewDesc& V = view_of(P, gslot, vhint);
+  q.V = &V;
   const CameraDesc& cam = V.cam;
   const int W_ = cam.w, WH = cam.w * cam.h;
-  const F3 cpos = cam_pos(cam);
   const long long nanti = V.n / 4;
-#if TRN_PIXEL_INTERLEAVE
   // Run order: the 4 antithetic copies of a slot take adjacent lanes. Their
   // camera rays leave one pixel's border and share every later sample, so
   // their paths stay close together (coherent traversal). Sample index p
-  // (copy * nanti + slot) and everything derived from it are unchanged.
+  // (copy * nanti + slot) and everything derived from it do not depend on it.
   const long long i = gslot - V.begin;
   const long long p = (i & 3) * nanti + (i >> 2);
-#else
-  const long long p = gslot - V.begin;
-#endif
-  const long long slot = p % nanti;
+  q.slot = p % nanti;
   const int anti = (int)(p / nanti);
   // the 4 antithetic copies of a slot share its samples (BoundaryPixel.cpp:135-138)
-  const PathSmp S{&P, V.seed, V.begin / 4 + slot, slot + V.slot_off};
+  const PathSmp S{&P, V.seed, V.begin / 4 + q.slot, q.slot + V.slot_off};
   const float r = S(0);
   float rr;
   if (anti == 0) rr = r;
@@ -2725,39 +2152,50 @@ TRN_D bool pixel_setup(const Params& P, long long gslot, EdgeState& st, int& vhi
   else if (bi == 2) { ox = 1.f; oy = 3.f - r4; }
   else { ox = 4.f - r4; oy = 0.f; }
   const int bsel = bi < 0 ? 0 : (bi > 3 ? 3 : bi);
-  const float pdf = (bsel & 1) ? 0.25f / (cam.plane_len_x * (float)cam.h) : 0.25f / (cam.plane_len_y * (float)cam.w);
+  q.pdf = (bsel & 1) ? 0.25f / (cam.plane_len_x * (float)cam.h) : 0.25f / (cam.plane_len_y * (float)cam.w);
   const F3 dedge = (bsel & 1) ? F3(1.f, 0.f, 0.f) : F3(0.f, 1.f, 0.f);
   const F3 dvis = bsel == 0 ? F3(1.f, 0.f, 0.f) : (bsel == 1 ? F3(0.f, -1.f, 0.f)
                                                 : (bsel == 2 ? F3(-1.f, 0.f, 0.f) : F3(0.f, 1.f, 0.f)));
-  const F3 edge = normalize(xform_vector(cam.raster_to_world, dedge));
-  const F3 edge2 = normalize(xform_vector(cam.raster_to_world, dvis));
-  const int pixel = (int)(p % WH);
-  const F3 p0 = xform_point(cam.raster_to_world, F3((float)(pixel % W_) + ox, (float)(pixel / W_) + oy, 0.f));
-  const F3 dir = normalize(p0 - cpos);
-  Hit h;
-  cnt.v[kCntClosest]++;
-  if (!trace_k<TRN_SETUP_SHARED_PIXEL, false>(s, p0, dir, kShadowEps, kRayMax, h, P.err)) return false;
-  const F3 hitP = p0 + dir * h.t;
+  q.edge = normalize(xform_vector(cam.raster_to_world, dedge));
+  q.edge2 = normalize(xform_vector(cam.raster_to_world, dvis));
+  q.pixel = (int)(p % WH);
+  q.p0 = xform_point(cam.raster_to_world, F3((float)(q.pixel % W_) + ox, (float)(q.pixel / W_) + oy, 0.f));
+  q.dir = normalize(q.p0 - cam_pos(cam));
+}
+
+TRN_D bool pixel_finish(const Params& P, const PixelPoint& q, const Hit& h, EdgeState& st) {
+  const ViewDesc& V = *q.V;
+  const CameraDesc& cam = V.cam;
+  const F3 cpos = cam_pos(cam);
+  const F3 hitP = q.p0 + q.dir * h.t;
   const SensorSample sds = sample_direct(cam, hitP);
   const F3 dirc = sensor_ray_dir(cam, sds.qx, sds.qy);
-  const SurfF x = post_intersect(s, h.tri, h.u, h.v);
+  const SurfF x = post_intersect(P.s, h.tri, h.u, h.v);
   const float dist = length(x.p - cpos);
-  const float dist1 = length(p0 - cpos);
+  const float dist1 = length(q.p0 - cpos);
   const float cos2 = fabsf(dot(x.ng, -dirc));
   F3 n;
   // BoundaryPixel.cpp:92 reverses the sign convention
-  const float bval = -base_val(dist / dist1, edge, dirc, x.ng, edge2, n) * cos2;
-  const F3 g = g_at(P, V, pixel);
+  const float bval = -base_val(dist / dist1, q.edge, dirc, x.ng, q.edge2, n) * cos2;
+  const F3 g = g_at(P, V, q.pixel);
   if (bval == 0.f || (g.x == 0.f && g.y == 0.f && g.z == 0.f)) return false;
-  st.V = &V; st.gslot = V.begin / 4 + slot; st.p = slot; st.x = x; st.rdir = dirc;
+  st.V = &V; st.gslot = V.begin / 4 + q.slot; st.p = q.slot; st.x = x; st.rdir = dirc;
   st.T0 = F3(sds.sensor_val, sds.sensor_val, sds.sensor_val);
-  st.p0 = p0; st.n = n; st.w0 = bval / pdf; st.far_tri = h.tri; st.g = g;
+  st.p0 = q.p0; st.n = n; st.w0 = bval / q.pdf; st.far_tri = h.tri; st.g = g;
   return true;
+}
+
+TRN_D bool pixel_setup(const Params& P, long long gslot, EdgeState& st, int& vhint, Cnt& cnt) {
+  PixelPoint q;
+  pixel_point(P, gslot, q, vhint);
+  Hit h;
+  cnt.v[kCntClosest]++;
+  if (!trace<false>(P.s, q.p0, q.dir, kShadowEps, kRayMax, h, P.err)) return false;
+  return pixel_finish(P, q, h, st);
 }
 
 __global__ void __launch_bounds__(256, TRN_MINB) k_pixel_adj(TRN_KPARAMS) {
   Cnt cnt;
-  stage_top(P.s);
   int vhint = 0;
   for_each_valid<EdgeState>(P,
     [&](long long gslot, EdgeState& st) -> bool { return pixel_setup(P, gslot, st, vhint, cnt); },
@@ -2769,41 +2207,7 @@ __global__ void __launch_bounds__(256, TRN_MINB) k_pixel_adj(TRN_KPARAMS) {
   flush_cnt(cnt, P.stats);
 }
 
-// Split form: k_pixel_setup queues the accepted samples as PrimaryItem
-// (dimension 1 onwards, no edge vertices); k_primary_body runs them.
-__global__ void __launch_bounds__(256, TRN_MINB_SETUP) k_pixel_setup(TRN_KPARAMS) {
-  Cnt cnt;
-  stage_top(P.s);
-  int vhint = 0;
-  PrimaryItem* q = reinterpret_cast<PrimaryItem*>(P.queue);
-  const int lane = threadIdx.x & 31;
-  const unsigned lt = (1u << lane) - 1u;
-  for (;;) {
-    unsigned long long start = 0;
-    if (lane == 0) start = atomicAdd(P.work, 32ull);
-    start = __shfl_sync(0xffffffffu, start, 0);
-    if ((long long)start >= P.total) break;
-    const long long g = (long long)start + lane;
-    EdgeState st;
-    const bool ok = g < P.total && pixel_setup(P, g, st, vhint, cnt);
-    const unsigned m = __ballot_sync(0xffffffffu, ok);
-    if (!m) continue;
-    const int leader = __ffs(m) - 1;
-    unsigned long long base = 0;
-    if (lane == leader) base = atomicAdd(P.q_count, (unsigned long long)__popc(m));
-    base = __shfl_sync(0xffffffffu, base, leader);
-    const unsigned long long k = base + __popc(m & lt);
-    if (ok && k >= (unsigned long long)P.q_cap) atomicExch(P.err, 2);
-    if (ok && k < (unsigned long long)P.q_cap) {
-      PrimaryItem& it = q[k];
-      it.gslot = st.gslot; it.p = st.p; it.view = (int)(st.V - P.views); it.dim0 = 1;
-      it.x_tri = st.x.tri; it.x_u = st.x.u; it.x_v = st.x.v; it.T0 = st.T0.x; it.w0 = st.w0; it.sedge = 0.f;
-      it.v0 = -1; it.v1 = -1; it.far_tri = st.far_tri;
-      it.rdir = st.rdir; it.p0 = st.p0; it.n = st.n; it.g = st.g;
-    }
-  }
-  flush_cnt(cnt, P.stats);
-}
+#include "wavefront.cuh"
 
 // ---------------------------------------------------------------------------
 // primary edge list for one camera (ConstructPrimEdgeList, Edge.cpp:313-348)
@@ -2851,21 +2255,34 @@ __global__ void k_view_loss(long long npix, const ViewDesc* views, const long lo
   if (v >= 0 && (int)(threadIdx.x & 31) == __ffs(m) - 1 && loss) atomicAdd(loss + v, sum);
 }
 
-__global__ void k_intersect(DeviceScene s, int n, const float* org, const float* dir, const float* tmin,
-                            const float* tmax, int* tri, float* u, float* v, float* t, int* err) {
-  stage_top(s);
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  Hit h;
-  trace<false>(s, make_f3(org + 3 * i), make_f3(dir + 3 * i), tmin[i], tmax[i], h, err);
-  tri[i] = h.tri; u[i] = h.u; v[i] = h.v; t[i] = h.t;
-}
-__global__ void k_occluded(DeviceScene s, int n, const float* org, const float* dir, const float* tmin,
-                           const float* tmax, int* vis) {
-  stage_top(s);
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  vis[i] = occluded(s, make_f3(org + 3 * i), make_f3(dir + 3 * i), tmin[i], tmax[i]) ? 0 : 1;
+// Ray queries of a program's own rays. Each warp streams through tiles of
+// `chunk` rays, every warp of the grid in turn, so that a run of costly rays (a
+// program's rays often come in image order) is spread over all of them. Few
+// rays are spread over all warps of the GPU as well, since a query is then as
+// long as its longest ray.
+template <bool ANY>
+__global__ void __launch_bounds__(TRN_TRACE_BLOCK, TRN_TRACE_MINB)
+    k_query(const __grid_constant__ DeviceScene s, int n, int chunk, const float* org, const float* dir,
+            const float* tmin_, const float* tmax_, int* tri_, float* u_, float* v_, float* t_, int* err) {
+  const long long step = (long long)gridDim.x * (blockDim.x >> 5) * chunk;
+  long long tile = (blockIdx.x * (long long)(blockDim.x >> 5) + (threadIdx.x >> 5)) * chunk, pos = tile;
+  trace_stream(s,
+    [&](int k, int& lim, bool& more) {
+      const int base = (int)min((long long)n, pos);
+      lim = (int)min((long long)n, tile + chunk);
+      pos += k;
+      if (pos >= lim) pos = tile += step;
+      more = pos < n;
+      return base;
+    },
+    [&](int i, F3& o, F3& d, float& tmin, float& tmax, bool& any) {
+      o = make_f3(org + 3ll * i); d = make_f3(dir + 3ll * i);
+      tmin = tmin_[i]; tmax = tmax_[i]; any = ANY;
+    },
+    [&](int i, bool, int tri, float u, float v, float t) {
+      if (ANY) tri_[i] = tri >= 0 ? 0 : 1;
+      else { tri_[i] = tri; u_[i] = u; v_[i] = v; t_[i] = t; }
+    }, err);
 }
 
 }  // namespace trn
@@ -2902,11 +2319,14 @@ struct trn_viewset {
   float* pint = nullptr;          // device [nviews]
   double* pint_part = nullptr;    // device [nviews][kCdfChunks]
   unsigned long long* work = nullptr;
-  // queue of the split indirect boundary term: one round of at most
-  // kIndirectRound slots at a time
+  // buffers of one wavefront round (items, rays, path state) and its counters
   void* iq = nullptr;
   size_t iq_bytes = 0;
   unsigned long long* iq_count = nullptr;
+  // a captured launch holds the address of iq: from then on a growth keeps the
+  // old buffer (each at least doubles, so they sum to less than the last)
+  bool iq_captured = false;
+  std::vector<void*> iq_old;
   // run order of the split set-up rounds: keys and values double-buffered for
   // one round, then the radix sort's temporary storage
   void* sq = nullptr;
@@ -2917,7 +2337,7 @@ struct trn_viewset {
   // depth; hash samples only)
   void* pc = nullptr;
   size_t pc_bytes = 0;
-  unsigned long long* pc_count = nullptr;
+  unsigned long long* pc_count = nullptr;  // [2] records, paths ended
   long long pc_limit = 0;  // bytes the records may take (0 = off)
   bool pc_valid = false;
   std::vector<char> pc_key;
@@ -3061,7 +2481,6 @@ Params base_params(trn_scene* s, trn_viewset* vs, const trn_render_options* o, i
   P.aq_edge = P.aq_n = nullptr;
   P.aq_cap = 0;
   P.queue = nullptr;
-  P.queue2 = nullptr;
   P.q_count = nullptr;
   P.q_cap = 0;
   P.order = nullptr;
@@ -3099,6 +2518,325 @@ int aq_reserve(trn_scene* s, long long cap) {
   return 0;
 }
 
+void launch_dims(const trn_launch* ln, long long total, int& grid, int& block) {
+  block = (ln && ln->block > 0) ? ln->block : 128;
+  const int per_sm = (ln && ln->blocks_per_sm > 0) ? ln->blocks_per_sm : 1024 / block;
+  const long long chunk = (ln && ln->chunk > 0) ? ln->chunk : 1;
+  long long want = (long long)sms() * per_sm;
+  const long long need = (total + 32 * chunk - 1) / (32 * chunk) * 32 / block + 1;
+  grid = (int)std::max<long long>(1, std::min(want, need));
+}
+
+// Rays per tile of a query: down to 4 while all warps that fit the GPU get one,
+// up to 32.
+void query_dims(int n, int& grid, int& chunk) {
+  const long long blocks = (long long)sms() * TRN_TRACE_MINB, warps = blocks * (TRN_TRACE_BLOCK / 32);
+  chunk = (int)std::min<long long>(32, std::max<long long>(4, (n + warps - 1) / warps));
+  const long long per_block = (long long)chunk * (TRN_TRACE_BLOCK / 32);
+  grid = (int)std::min(blocks, (n + per_block - 1) / per_block);
+}
+
+int validate_launch(const trn_launch* ln) {
+  if (!ln) return 0;
+  if (ln->block != 0 && (ln->block < 32 || ln->block > 256 || ln->block % 32 != 0)) {
+    set_error("launch block must be a multiple of 32 in [32, 256]");
+    return -1;
+  }
+  if (ln->blocks_per_sm < 0 || ln->blocks_per_sm > 64 || ln->chunk < 0 || ln->chunk > 64) {
+    set_error("launch blocks_per_sm must be in [0, 64] and chunk in [0, 64]");
+    return -1;
+  }
+  if (ln->round_log2 != 0 && (ln->round_log2 < 16 || ln->round_log2 > 40)) {
+    set_error("launch round_log2 must be 0 (default) or in [16, 40]");
+    return -1;
+  }
+  return 0;
+}
+
+template <class K>
+void launch(K kernel, const trn_launch* ln, long long total, const Params& P, cudaStream_t st) {
+  int grid, block;
+  launch_dims(ln, total, grid, block);
+  kernel<<<grid, block, 0, st>>>(P);
+  count_launch(1);
+}
+
+// Slots per round of the boundary terms and the image, and paths per round of
+// the replaying adjoint. Larger rounds give each edge more samples per sort and
+// the terms fewer kernel tails, at up to 341 bytes per slot (indirect term,
+// depth 8): 2^24 against 2^23 slots, indirect 30.4 -> 28.2 ms, direct 3.2 ->
+// 2.4, primary 12.1 -> 11.2 (16.8M samples on 102,400 triangles). The replay
+// keeps 2^22 (0.7 kB of records and state per path at depth 8).
+#ifndef TRN_ROUND_LOG2
+#define TRN_ROUND_LOG2 24
+#endif
+#ifndef TRN_PATH_ROUND_LOG2
+#define TRN_PATH_ROUND_LOG2 22
+#endif
+constexpr long long kRound = 1LL << TRN_ROUND_LOG2;
+constexpr long long kReplayRound = 1LL << TRN_PATH_ROUND_LOG2;
+constexpr int kWaveCounters = 256;
+
+// Slots (or paths) per round: the launch's round_log2 when set, never above
+// the default that the buffers are sized for.
+long long round_cap(const trn_launch* ln, long long dflt) {
+  if (ln && ln->round_log2 > 0) return std::min(dflt, 1LL << ln->round_log2);
+  return dflt;
+}
+
+size_t item_bytes(int integrator) {
+  switch (integrator) {
+    case TRN_PATH_TRACER: return 0;
+    case TRN_DIRECT_EDGE: return sizeof(DirectItem);
+    case TRN_INDIRECT_EDGE: return sizeof(IndirectItem);
+    default: return sizeof(PrimaryItem);
+  }
+}
+
+// Places a round's buffers for `cap` samples from `base` on (the term's items
+// first) and returns the bytes they take.
+size_t wave_layout(Wave& W, void** items, void* base, long long cap, int integrator, int depth) {
+  char* c = static_cast<char*>(base);
+  size_t off = 0;
+  const size_t n = (size_t)cap;
+  auto take = [&](size_t bytes) { char* r = c + off; off += (bytes + 255) / 256 * 256; return static_cast<void*>(r); };
+  const bool edge = integrator != TRN_PATH_TRACER;
+  *items = take(item_bytes(integrator) * n);
+  W.cap = cap;
+  W.ro = static_cast<float4*>(take(2 * n * sizeof(float4)));
+  W.rd = static_cast<float4*>(take(2 * n * sizeof(float4)));
+  W.hit[0] = static_cast<float4*>(take(n * sizeof(float4)));
+  W.occ = static_cast<unsigned char*>(take(n));
+  W.list[0] = static_cast<unsigned*>(take(n * sizeof(unsigned)));
+  W.list[1] = static_cast<unsigned*>(take(n * sizeof(unsigned)));
+  for (float4*& s : W.st) s = static_cast<float4*>(take(n * sizeof(float4)));
+  W.hit[1] = W.st[0];  // of a set-up's second rays, before any path has state
+  W.p = static_cast<long long*>(take(edge ? 0 : n * sizeof(long long)));
+  W.view = static_cast<int*>(take(edge ? 0 : n * sizeof(int)));
+  W.rec = static_cast<unsigned*>(take(n * sizeof(unsigned)));
+  W.L = static_cast<F3*>(take(edge ? 0 : n * sizeof(F3)));
+  W.W = static_cast<float*>(take(edge ? n * sizeof(float) : 0));
+  const bool ind = integrator == TRN_INDIRECT_EDGE;
+  W.list2 = static_cast<unsigned*>(take(ind ? n * sizeof(unsigned) : 0));
+  W.sc = static_cast<float*>(take(ind ? 3 * sizeof(float) * n * (size_t)std::max(depth - 1, 0) : 0));
+  return off;
+}
+
+// Bytes of the interior term's round: wavefront buffers and, for the replaying
+// adjoint, its records.
+size_t path_round_bytes(long long cap, int depth, bool records) {
+  Wave W;
+  PathSoA R;
+  void* items;
+  return wave_layout(W, &items, nullptr, cap, TRN_PATH_TRACER, depth) + (records ? path_soa(R, nullptr, cap, depth) : 0);
+}
+
+// Largest round any term needs (depth <= 8 when shallow, else up to kMaxDepth).
+size_t full_queue_bytes(bool shallow) {
+  const int depth = shallow ? 8 : kMaxDepth;
+  size_t most = std::max(path_round_bytes(kReplayRound, depth, true), path_round_bytes(kRound, depth, false));
+  for (int t = 1; t < 5; t++) {
+    Wave W;
+    void* items;
+    most = std::max(most, wave_layout(W, &items, nullptr, kRound, t, depth));
+  }
+  return most;
+}
+
+bool capturing(cudaStream_t st) {
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  return cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone;
+}
+
+// The view set's round buffers, grown on first use to at least `need` bytes
+// (not inside stream capture: run the integrator once before capturing it, or
+// reserve with trn_viewset_reserve). A growth at least doubles them, up to `most`
+// (one full round), so that a set whose batches grow (a serving loop) reallocates a
+// few times at most. Returns 1, with the error text set, when the call cannot
+// have them: inside a capture, or out of memory.
+int ensure_queue(trn_viewset* vs, size_t need, size_t most, cudaStream_t st) {
+  const bool cap = capturing(st);
+  if (vs->iq_bytes >= need && vs->iq_count) {
+    vs->iq_captured |= cap;
+    return 0;
+  }
+  if (cap) {
+    set_error("boundary term: its queue must be allocated before stream capture (run it once first)");
+    return 1;
+  }
+  TRN_CUDA_TRY(cudaStreamSynchronize(st));
+  if (vs->iq_bytes < need) {
+    const size_t bytes = std::max(need, std::min(2 * vs->iq_bytes, most));
+    if (vs->iq && vs->iq_captured) vs->iq_old.push_back(vs->iq);
+    else if (vs->iq) cudaFree(vs->iq);
+    vs->iq_captured = false;
+    vs->iq = nullptr;
+    vs->iq_bytes = 0;
+    if (cudaMalloc(&vs->iq, bytes) != cudaSuccess) {
+      cudaGetLastError();
+      vs->iq = nullptr;
+      set_error("boundary term: out of memory for its queue");
+      return 1;
+    }
+    vs->iq_bytes = bytes;
+  }
+  if (!vs->iq_count && cudaMalloc(&vs->iq_count, kWaveCounters * sizeof(unsigned long long)) != cudaSuccess) {
+    set_error("boundary term: out of memory");
+    return -1;
+  }
+  return 0;
+}
+
+// One round's launches. Counters are handed out in launch order and zeroed
+// together at the start of the round.
+struct WaveRun {
+  trn_viewset* vs;
+  Params P;
+  Wave W;
+  PathSoA R;
+  const trn_launch* ln;
+  cudaStream_t st;
+  int used;
+
+  // Launches K over the round: as many blocks as fit the GPU at once (the
+  // kernels stride over a count they read on the device), or the shape the
+  // caller asked for; fewer when the round is small.
+  template <auto K, class... A>
+  void go(A... args) const {
+    const int block = ln && ln->block > 0 ? ln->block : 128;
+    int per_sm = ln && ln->blocks_per_sm > 0 ? ln->blocks_per_sm : 0;
+    if (!per_sm) {
+      static const int fit = [] {
+        int n = 0;
+        return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, K, 128, 0) == cudaSuccess && n > 0 ? n : 4;
+      }();
+      per_sm = std::max(1, fit * 128 / block);
+    }
+    launch<K>(std::min<long long>((long long)sms() * per_sm, (W.cap + block - 1) / block), block, args...);
+  }
+  template <auto K, class... A>
+  void launch(long long grid, int block, A... args) const {
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3((unsigned)std::max(1LL, grid));
+    c.blockDim = dim3(block);
+    c.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = attr;
+    c.numAttrs = 1;
+    cudaLaunchKernelEx(&c, K, args...);
+    count_launch(1);
+  }
+
+  unsigned long long* ctr() { return vs->iq_count + used++; }
+  int begin() {
+    used = 0;
+    TRN_CUDA_TRY(cudaMemsetAsync(vs->iq_count, 0, kWaveCounters * sizeof(unsigned long long), st));
+    return 0;
+  }
+  // rays [r0, r0 + *n): hits to W.hit[which], occlusion to W.occ
+  void trace(long long r0, const unsigned long long* n, int which) {
+    constexpr int kFew = 4;  // rays per warp below which more warps would not help
+    const long long need = (2 * W.cap + kFew * (TRN_TRACE_BLOCK / 32) - 1) / (kFew * (TRN_TRACE_BLOCK / 32));
+    launch<k_trace>(std::min((long long)sms() * TRN_TRACE_MINB, need), TRN_TRACE_BLOCK, P.s, W, r0, n, ctr(),
+                    W.hit[which], P.err);
+  }
+  // bounces of the entries that a start kernel left in list[0]
+  template <int MODE>
+  void bounces(const unsigned long long* n, unsigned long long* n_ray, int depth) {
+    for (int b = 0; b < depth; b++) {
+      trace(0, n_ray, 0);
+      Stage S{n, W.list[b & 1], ctr(), W.list[(b + 1) & 1], ctr(), nullptr, b};
+      go<k_wf_shade<MODE>>(P, W, S, R);
+      n = S.n_out; n_ray = S.n_ray;
+    }
+  }
+  template <bool SENSOR>
+  void importance(int depth) {
+    Stage S{P.q_count, nullptr, ctr(), W.list[0], ctr(), nullptr, 0};
+    go<k_wi_start<SENSOR>>(P, W, S);
+    const unsigned long long *n = S.n_out, *n_ray = S.n_ray;
+    for (int b = 0; b < depth; b++) {
+      trace(0, n_ray, 0);
+      Stage B{n, W.list[b & 1], ctr(), W.list[(b + 1) & 1], ctr(), nullptr, b};
+      go<k_wi_step<SENSOR>>(P, W, B);
+      n = B.n_out; n_ray = B.n_ray;
+    }
+  }
+  // set-up rays and geometry of a boundary term: items to P.queue
+  template <int TERM>
+  void setup(long long first) {
+    unsigned long long* n = ctr();
+    go<k_setup_rays<TERM>>(P, W, first, n);
+    trace(0, n, 0);
+    if constexpr (TERM != TRN_PIXEL_EDGE) {
+      unsigned long long* n2 = ctr();
+      go<k_setup_rays2<TERM>>(P, W, first, n, n2);
+      trace(W.cap, n2, 1);
+      n = n2;
+    }
+    go<k_setup_finish<TERM>>(P, W, first, n);
+  }
+};
+
+WaveRun wave_run(trn_viewset* vs, const Params& P, const trn_launch* ln, long long cap, cudaStream_t st) {
+  WaveRun r;
+  std::memset(&r.W, 0, sizeof(r.W));
+  std::memset(&r.R, 0, sizeof(r.R));
+  r.vs = vs;
+  r.P = P;
+  r.st = st;
+  r.used = 0;
+  r.ln = ln;
+  return r;
+}
+
+// Interior term over all slots, in rounds: forward image (kWfFwd), with records
+// into P.queue (kWfRec, records given by `cache`), or replayed records and the
+// reverse sweep of each round (kWfReplay). Returns 1 when there are no buffers
+// for it (ensure_queue).
+template <int MODE>
+int path_wave(trn_viewset* vs, const Params& P0, const trn_launch* ln, long long total, const PathSoA* cache,
+              cudaStream_t st) {
+  const int depth = vs->max_depth;
+  const long long cap = std::min(total, round_cap(ln, MODE == kWfReplay ? kReplayRound : kRound));
+  // an image-only set stays at an image's round
+  const size_t most = MODE == kWfReplay ? full_queue_bytes(depth <= 8) : path_round_bytes(kRound, depth, false);
+  const int rc = ensure_queue(vs, path_round_bytes(cap, depth, MODE == kWfReplay), most, st);
+  if (rc) return rc;
+  WaveRun r = wave_run(vs, P0, ln, cap, st);
+  void* items;
+  const size_t wb = wave_layout(r.W, &items, vs->iq, cap, TRN_PATH_TRACER, depth);
+  if (MODE == kWfRec) {
+    r.R = *cache;
+    r.R.n_end = vs->pc_count + 1;
+  }
+  if (MODE == kWfReplay) {
+    path_soa(r.R, static_cast<char*>(vs->iq) + wb, cap, depth);
+    r.P.q_cap = cap;
+  }
+  for (long long first = 0; first < total; first += cap) {
+    const long long n = std::min(cap, total - first);
+    if (r.begin()) return -1;
+    r.W.first = first;
+    if (MODE == kWfReplay) {
+      r.P.q_count = r.ctr();
+      r.R.n_end = r.ctr();
+    }
+    unsigned long long* rays = r.ctr();
+    r.go<k_wf_camera>(r.P, r.W, n, MODE == kWfReplay, rays);
+    r.trace(0, rays, 0);
+    Stage S{rays, r.W.list[1], r.ctr(), r.W.list[0], r.ctr(), r.ctr(), 0};
+    r.go<k_wf_start<MODE>>(r.P, r.W, S, r.R);
+    r.bounces<MODE>(S.n_out, S.n_ray, depth);
+    if (MODE == kWfReplay) r.go<k_path_reverse<false>>(r.P, r.R);
+    else r.go<k_wf_pixels>(r.P, r.W, n);
+  }
+  TRN_CUDA_TRY(cudaGetLastError());
+  return 0;
+}
+
 // AdaptiveQuadratureDistribution::setup (AQ_distrb.h:83-173) for one
 // direct-boundary call: the depth-0 tree, g_direct_depth refinement passes
 // (the loop the reference keeps commented out, AQ_distrb.h:121-136, with
@@ -3106,8 +2844,8 @@ int aq_reserve(trn_scene* s, long long cap) {
 // g_direct_spp samples per leaf, eps mixing, leaf distribution. The tree
 // holds at most max(E, g_direct_max_size) leaves. The set-up samples come
 // from the counter hash (their own terms), also when the call's samples come
-// from a table. may_alloc = false (the allocation-free entry point) refuses
-// a refinement that would need larger arrays than the scene holds.
+// from a table. The allocation-free entry point refuses a refinement that would
+// need larger arrays than the scene holds.
 int guide_setup(trn_scene* s, const trn_render_options* o, Params& P, cudaStream_t st, bool may_alloc = true) {
   if (!o->g_direct || s->ne == 0) return 0;
   if (o->g_direct_spp <= 0) { set_error("g_direct_spp must be positive when g_direct is set"); return -1; }
@@ -3164,162 +2902,6 @@ int guide_setup(trn_scene* s, const trn_render_options* o, Params& P, cudaStream
   return 0;
 }
 
-void launch_dims(const trn_launch* ln, long long total, int& grid, int& block) {
-  block = (ln && ln->block > 0) ? ln->block : 128;
-  const int per_sm = (ln && ln->blocks_per_sm > 0) ? ln->blocks_per_sm : 1024 / block;
-  const long long chunk = (ln && ln->chunk > 0) ? ln->chunk : 1;
-  long long want = (long long)sms() * per_sm;
-  const long long need = (total + 32 * chunk - 1) / (32 * chunk) * 32 / block + 1;
-  grid = (int)std::max<long long>(1, std::min(want, need));
-}
-
-int validate_launch(const trn_launch* ln) {
-  if (!ln) return 0;
-  if (ln->block != 0 && (ln->block < 32 || ln->block > 256 || ln->block % 32 != 0)) {
-    set_error("launch block must be a multiple of 32 in [32, 256]");
-    return -1;
-  }
-  if (ln->blocks_per_sm < 0 || ln->blocks_per_sm > 64 || ln->chunk < 0 || ln->chunk > 64) {
-    set_error("launch blocks_per_sm must be in [0, 64] and chunk in [0, 64]");
-    return -1;
-  }
-  if (ln->round_log2 != 0 && (ln->round_log2 < 16 || ln->round_log2 > 40)) {
-    set_error("launch round_log2 must be 0 (default) or in [16, 40]");
-    return -1;
-  }
-  return 0;
-}
-
-template <class K>
-void launch(K kernel, const trn_launch* ln, long long total, const Params& P, cudaStream_t st) {
-  int grid, block;
-  launch_dims(ln, total, grid, block);
-  kernel<<<grid, block, 0, st>>>(P);
-  count_launch(1);
-}
-
-#ifndef TRN_INDIRECT_SPLIT
-#define TRN_INDIRECT_SPLIT 1
-#endif
-// slots per round of the split boundary terms: 16M (one round for a 512² x
-// 64 spp term). Larger rounds give each edge more samples per sort and the
-// terms fewer kernel tails (measured: 4M 195.6, 8M 189.5, 16M 186.2 ms/step
-// on that workload), at about 5.5 GB of queue per view set.
-#ifndef TRN_ROUND_LOG2
-#define TRN_ROUND_LOG2 24
-#endif
-constexpr long long kIndirectRound = 1LL << TRN_ROUND_LOG2;
-constexpr long long kPathRound = 1LL << 21;  // paths per split round of the interior adjoint
-
-// Slots (or paths) per round: the launch's round_log2 when set, never above
-// the default that the queues are sized for.
-long long round_cap(const trn_launch* ln, long long dflt) {
-  if (ln && ln->round_log2 > 0) return std::min(dflt, 1LL << ln->round_log2);
-  return dflt;
-}
-
-// Largest queue that any split term needs for one full round (depth <= 8
-// when shallow, else up to kMaxDepth).
-size_t full_queue_bytes(bool shallow) {
-  const size_t c = (size_t)kIndirectRound;
-  const size_t ind = (sizeof(IndirectSetupItem) * c + 255) / 256 * 256 +
-                     (shallow ? sizeof(IndirectItem<8>) : sizeof(IndirectItem<kMaxDepth>)) * c;
-  const size_t path = shallow ? path_soa_bytes<8>(kPathRound) : path_soa_bytes<kMaxDepth>(kPathRound);
-  return std::max(std::max(ind, path), std::max(sizeof(PrimaryItem) * c, sizeof(DirectItem) * c));
-}
-
-#ifndef TRN_PRIMARY_SPLIT
-#define TRN_PRIMARY_SPLIT 1
-#endif
-
-// The view set's queue of the split terms, grown on first use to at least
-// `need` bytes (not inside stream capture: run the integrator once before
-// capturing it, or reserve with trn_viewset_reserve). A growth at least
-// doubles the queue, up to one full round, so that a set whose batches grow
-// (a serving loop) reallocates a few times at most.
-int ensure_queue(trn_viewset* vs, size_t need, cudaStream_t st) {
-  if (vs->iq_bytes >= need && vs->iq_count) return 0;
-  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  TRN_CUDA_TRY(cudaStreamIsCapturing(st, &cs));
-  if (cs != cudaStreamCaptureStatusNone) {
-    set_error("boundary term: its queue must be allocated before stream capture (run it once first)");
-    return -1;
-  }
-  TRN_CUDA_TRY(cudaStreamSynchronize(st));
-  if (vs->iq_bytes < need) {
-    const size_t bytes = std::max(need, std::min(2 * vs->iq_bytes, full_queue_bytes(vs->max_depth <= 8)));
-    if (vs->iq) cudaFree(vs->iq);
-    vs->iq = nullptr;
-    vs->iq_bytes = 0;
-    if (cudaMalloc(&vs->iq, bytes) != cudaSuccess) { set_error("boundary term: out of memory for its queue"); return -1; }
-    vs->iq_bytes = bytes;
-  }
-  if (!vs->iq_count && cudaMalloc(&vs->iq_count, 4 * sizeof(unsigned long long)) != cudaSuccess) {
-    set_error("boundary term: out of memory");
-    return -1;
-  }
-  return 0;
-}
-
-#ifndef TRN_PATHADJ_SPLIT
-#define TRN_PATHADJ_SPLIT 1
-#endif
-
-// The split interior adjoint in rounds of at most kPathRound paths (a queue
-// of about 1.3 GB at depth <= 8).
-int path_adj_split(trn_viewset* vs, Params P, const trn_launch* ln, long long total, bool shallow, cudaStream_t st) {
-  const long long cap = std::min(total, round_cap(ln, kPathRound));
-  if (ensure_queue(vs, shallow ? path_soa_bytes<8>(cap) : path_soa_bytes<kMaxDepth>(cap), st)) return -1;
-  P.queue = vs->iq;
-  P.q_count = vs->iq_count;
-  P.q_cap = cap;
-  int grid, block;
-  launch_dims(ln, cap, grid, block);
-  for (long long first = 0; first < total; first += cap) {
-    P.total = std::min(total, first + cap);
-    k_indirect_round<<<1, 32, 0, st>>>(P.work, (unsigned long long)first, P.q_count);
-    if (shallow) {
-      k_path_replay<8><<<grid, block, 0, st>>>(P);
-      k_path_reverse<8><<<grid, block, 0, st>>>(P);
-    } else {
-      k_path_replay<kMaxDepth><<<grid, block, 0, st>>>(P);
-      k_path_reverse<kMaxDepth><<<grid, block, 0, st>>>(P);
-    }
-    count_launch(3);
-  }
-  TRN_CUDA_TRY(cudaGetLastError());
-  return 0;
-}
-
-#ifndef TRN_PIXEL_SPLIT
-#define TRN_PIXEL_SPLIT 1
-#endif
-
-// The split pixel boundary term in rounds of at most kIndirectRound samples.
-int pixel_split(trn_viewset* vs, Params P, const trn_launch* ln, long long total, cudaStream_t st) {
-  const long long cap = std::min(total, round_cap(ln, kIndirectRound));
-  if (ensure_queue(vs, sizeof(PrimaryItem) * (size_t)cap, st)) return -1;
-  P.queue = vs->iq;
-  P.q_count = vs->iq_count;
-  P.q_cap = cap;
-  int grid, block;
-  launch_dims(ln, cap, grid, block);
-  for (long long first = 0; first < total; first += cap) {
-    P.total = std::min(total, first + cap);
-    k_indirect_round<<<1, 32, 0, st>>>(P.work, (unsigned long long)first, P.q_count);
-    k_pixel_setup<<<grid, block, 0, st>>>(P);
-    if (TRN_BODY_REGEN) k_primary_body_regen<<<grid, block, 0, st>>>(P);
-    else k_primary_body<<<grid, block, 0, st>>>(P);
-    count_launch(3);
-  }
-  TRN_CUDA_TRY(cudaGetLastError());
-  return 0;
-}
-
-#ifndef TRN_DIRECT_SPLIT
-#define TRN_DIRECT_SPLIT 1
-#endif
-
 #ifndef TRN_EDGE_ORDER
 #define TRN_EDGE_ORDER 1
 #endif
@@ -3346,7 +2928,7 @@ int alloc_order(trn_viewset* vs, long long cap, cudaStream_t st) {
     set_error("boundary term: its sort buffers must be allocated before stream capture (run it once first)");
     return -1;
   }
-  const long long n = std::max(cap, std::min(2 * vs->sq_cap, kIndirectRound));
+  const long long n = std::max(cap, std::min(2 * vs->sq_cap, kRound));
   cub::DoubleBuffer<unsigned> k(nullptr, nullptr), v(nullptr, nullptr);
   size_t tmp = 0;
   TRN_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, tmp, k, v, (int)n, 0, 32, st));
@@ -3397,104 +2979,45 @@ int order_round(trn_viewset* vs, Params& P, int term, cudaStream_t st) {
   return 0;
 }
 
-// The split direct term in rounds of at most kIndirectRound slots.
-int direct_split(trn_viewset* vs, Params P, const trn_launch* ln, long long total, cudaStream_t st) {
-  const long long cap = std::min(total, round_cap(ln, kIndirectRound));
-  if (ensure_queue(vs, sizeof(DirectItem) * (size_t)cap, st)) return -1;
-  P.queue = vs->iq;
-  P.q_count = vs->iq_count;
-  P.q_cap = cap;
-  int grid, block;
-  launch_dims(ln, cap, grid, block);
-  const int ordered = TRN_EDGE_ORDER ? ensure_order(vs, P, cap, st) : 1;
+// A boundary term over all slots, in rounds: run order, set-up, the paths of
+// the samples that passed, scatter.
+template <int TERM>
+int edge_wave(trn_viewset* vs, const Params& P0, const trn_launch* ln, long long total, cudaStream_t st) {
+  const int depth = vs->max_depth;
+  const long long cap = std::min(total, round_cap(ln, kRound));
+  WaveRun r = wave_run(vs, P0, ln, cap, st);
+  void* items;
+  if (ensure_queue(vs, wave_layout(r.W, &items, nullptr, cap, TERM, depth), full_queue_bytes(depth <= 8), st))
+    return -1;
+  wave_layout(r.W, &items, vs->iq, cap, TERM, depth);
+  r.P.queue = items;
+  r.P.q_cap = cap;
+  const int ordered = TRN_EDGE_ORDER && TERM != TRN_PIXEL_EDGE ? ensure_order(vs, r.P, cap, st) : 1;
   if (ordered < 0) return -1;
   for (long long first = 0; first < total; first += cap) {
-    P.total = std::min(total, first + cap);
-    P.order_first = first;
-    if (!ordered && order_round(vs, P, TRN_DIRECT_EDGE, st)) return -1;
-    k_indirect_round<<<1, 32, 0, st>>>(P.work, (unsigned long long)first, P.q_count);
-    k_direct_setup<<<grid, block, 0, st>>>(P);
-    k_direct_body<<<grid, block, 0, st>>>(P);
-    count_launch(3);
-  }
-  TRN_CUDA_TRY(cudaGetLastError());
-  return 0;
-}
-
-// The split primary term in rounds of at most kIndirectRound slots.
-int primary_split(trn_viewset* vs, Params P, const trn_launch* ln, long long total, cudaStream_t st) {
-  const long long cap = std::min(total, round_cap(ln, kIndirectRound));
-  if (ensure_queue(vs, sizeof(PrimaryItem) * (size_t)cap, st)) return -1;
-  P.queue = vs->iq;
-  P.q_count = vs->iq_count;
-  P.q_cap = cap;
-  int grid, block;
-  launch_dims(ln, cap, grid, block);
-  const int ordered = TRN_EDGE_ORDER ? ensure_order(vs, P, cap, st) : 1;
-  if (ordered < 0) return -1;
-  for (long long first = 0; first < total; first += cap) {
-    P.total = std::min(total, first + cap);
-    P.order_first = first;
-    if (!ordered && order_round(vs, P, TRN_PRIMARY_EDGE, st)) return -1;
-    k_indirect_round<<<1, 32, 0, st>>>(P.work, (unsigned long long)first, P.q_count);
-    k_primary_setup<<<grid, block, 0, st>>>(P);
-    if (TRN_BODY_REGEN) k_primary_body_regen<<<grid, block, 0, st>>>(P);
-    else k_primary_body<<<grid, block, 0, st>>>(P);
-    count_launch(3);
-  }
-  TRN_CUDA_TRY(cudaGetLastError());
-  return 0;
-}
-
-#ifndef TRN_INDIRECT_STAGES
-#define TRN_INDIRECT_STAGES 3
-#endif
-
-// The split indirect term in rounds of at most kIndirectRound slots: two
-// stages (set-up + sensor side, emitter side) or three (set-up, sensor side,
-// emitter side; the default).
-int indirect_split(trn_viewset* vs, Params P, const trn_launch* ln, long long total, bool shallow, cudaStream_t st) {
-  const long long cap = std::min(total, round_cap(ln, kIndirectRound));
-  const size_t item = shallow ? sizeof(IndirectItem<8>) : sizeof(IndirectItem<kMaxDepth>);
-  const size_t item_a = TRN_INDIRECT_STAGES == 3 ? sizeof(IndirectSetupItem) : 0;
-  const size_t bytes_a = (item_a * (size_t)cap + 255) / 256 * 256;
-  if (ensure_queue(vs, bytes_a + item * (size_t)cap, st)) return -1;
-  P.queue = vs->iq;
-  P.queue2 = TRN_INDIRECT_STAGES == 3 ? static_cast<char*>(vs->iq) + bytes_a : nullptr;
-  P.q_count = vs->iq_count;
-  P.q_cap = cap;
-  int grid, block;
-  launch_dims(ln, cap, grid, block);
-  const int ordered = TRN_EDGE_ORDER && TRN_INDIRECT_STAGES == 3 ? ensure_order(vs, P, cap, st) : 1;
-  if (ordered < 0) return -1;
-  for (long long first = 0; first < total; first += cap) {
-    P.total = std::min(total, first + cap);
-    P.order_first = first;
-    if (!ordered && order_round(vs, P, TRN_INDIRECT_EDGE, st)) return -1;
-    k_indirect_round<<<1, 32, 0, st>>>(P.work, (unsigned long long)first, P.q_count);
-    if (TRN_INDIRECT_STAGES == 3) {
-      k_indirect_setup<<<grid, block, 0, st>>>(P);
-      if (shallow) {
-        if (TRN_SENSOR_REGEN) k_indirect_sensor_regen<8><<<grid, block, 0, st>>>(P);
-        else k_indirect_sensor_q<8><<<grid, block, 0, st>>>(P);
-        if (TRN_EMITTER_REGEN) k_indirect_emitter_regen<8><<<grid, block, 0, st>>>(P);
-        else k_indirect_emitter<8><<<grid, block, 0, st>>>(P);
-      } else {
-        if (TRN_SENSOR_REGEN) k_indirect_sensor_regen<kMaxDepth><<<grid, block, 0, st>>>(P);
-        else k_indirect_sensor_q<kMaxDepth><<<grid, block, 0, st>>>(P);
-        if (TRN_EMITTER_REGEN) k_indirect_emitter_regen<kMaxDepth><<<grid, block, 0, st>>>(P);
-        else k_indirect_emitter<kMaxDepth><<<grid, block, 0, st>>>(P);
-      }
-      count_launch(4);
+    r.P.total = std::min(total, first + cap);
+    r.P.order_first = first;
+    if (!ordered && order_round(vs, r.P, TERM, st)) return -1;
+    if (r.begin()) return -1;
+    r.P.q_count = r.ctr();
+    r.setup<TERM>(first);
+    if constexpr (TERM == TRN_DIRECT_EDGE) {
+      r.importance<false>(depth);
+      r.go<k_wi_direct_scatter>(r.P, r.W);
+    } else if constexpr (TERM == TRN_INDIRECT_EDGE) {
+      const int d = std::min(depth, (int)kMaxDepth) - 1;
+      r.importance<true>(d);
+      unsigned long long* n_emit = r.ctr();
+      r.go<k_wi_collect>(r.P, r.W, n_emit);
+      Stage S{n_emit, r.W.list2, r.ctr(), r.W.list[0], r.ctr(), nullptr, 0};
+      r.go<k_wf_start<kWfEmit>>(r.P, r.W, S, r.R);
+      r.bounces<kWfEmit>(S.n_out, S.n_ray, d);
+      r.go<k_wf_emit_scatter>(r.P, r.W, n_emit);
     } else {
-      if (shallow) {
-        k_indirect_sensor<8><<<grid, block, 0, st>>>(P);
-        k_indirect_emitter<8><<<grid, block, 0, st>>>(P);
-      } else {
-        k_indirect_sensor<kMaxDepth><<<grid, block, 0, st>>>(P);
-        k_indirect_emitter<kMaxDepth><<<grid, block, 0, st>>>(P);
-      }
-      count_launch(3);
+      Stage S{r.P.q_count, nullptr, r.ctr(), r.W.list[0], r.ctr(), nullptr, 0};
+      r.go<k_wf_start<kWfBody>>(r.P, r.W, S, r.R);
+      r.bounces<kWfBody>(S.n_out, S.n_ray, depth);
+      r.go<k_wf_body_scatter>(r.P, r.W);
     }
   }
   TRN_CUDA_TRY(cudaGetLastError());
@@ -3529,11 +3052,6 @@ std::vector<char> path_key(const trn_viewset* vs, const trn_render_options* o, i
   return k;
 }
 
-bool capturing(cudaStream_t st) {
-  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  return cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone;
-}
-
 // Recording forward render of the interior term into the view set's path
 // cache. Returns 1 when the cache is not used (off, a sample table, stream
 // capture, above the limit, or no memory for it): the caller then renders
@@ -3542,8 +3060,8 @@ int path_cache_fwd(trn_viewset* vs, Params P, const trn_launch* ln, const trn_re
                    long long total, cudaStream_t st) {
   vs->pc_valid = false;
   if (!TRN_PATH_CACHE || vs->pc_limit <= 0 || P.table || capturing(st)) return 1;
-  const bool shallow = vs->max_depth <= 8;
-  const size_t bytes = shallow ? path_soa_bytes<8>(total) : path_soa_bytes<kMaxDepth>(total);
+  PathSoA R;
+  const size_t bytes = path_soa(R, nullptr, total, vs->max_depth);
   if (bytes > (size_t)vs->pc_limit) return 1;
   if (vs->pc_bytes < bytes || !vs->pc_count) {
     TRN_CUDA_TRY(cudaStreamSynchronize(st));
@@ -3551,7 +3069,7 @@ int path_cache_fwd(trn_viewset* vs, Params P, const trn_launch* ln, const trn_re
     vs->pc = nullptr;
     vs->pc_bytes = 0;
     if (cudaMalloc(&vs->pc, bytes) != cudaSuccess ||
-        (!vs->pc_count && cudaMalloc(&vs->pc_count, sizeof(unsigned long long)) != cudaSuccess)) {
+        (!vs->pc_count && cudaMalloc(&vs->pc_count, 2 * sizeof(unsigned long long)) != cudaSuccess)) {
       cudaGetLastError();  // out of memory: render without records
       if (vs->pc) cudaFree(vs->pc);
       vs->pc = nullptr;
@@ -3559,17 +3077,12 @@ int path_cache_fwd(trn_viewset* vs, Params P, const trn_launch* ln, const trn_re
     }
     vs->pc_bytes = bytes;
   }
-  TRN_CUDA_TRY(cudaMemsetAsync(vs->pc_count, 0, sizeof(unsigned long long), st));
-  P.queue = vs->pc;
+  TRN_CUDA_TRY(cudaMemsetAsync(vs->pc_count, 0, 2 * sizeof(unsigned long long), st));
   P.q_count = vs->pc_count;
   P.q_cap = total;
-  if (TRN_FWD_REGEN) {
-    if (shallow) launch(k_path_fwd_rec_regen<8>, ln, total, P, st);
-    else launch(k_path_fwd_rec_regen<kMaxDepth>, ln, total, P, st);
-  } else {
-    if (shallow) launch(k_path_fwd_rec<8>, ln, total, P, st); else launch(k_path_fwd_rec<kMaxDepth>, ln, total, P, st);
-  }
-  TRN_CUDA_TRY(cudaGetLastError());
+  path_soa(R, vs->pc, total, vs->max_depth);
+  const int rc = path_wave<kWfRec>(vs, P, ln, total, &R, st);
+  if (rc) return rc;
   vs->pc_key = path_key(vs, o, spp_override, total);
   vs->pc_valid = true;
   return 0;
@@ -3581,13 +3094,14 @@ int path_cache_grad(trn_viewset* vs, Params P, const trn_launch* ln, const trn_r
                     long long total, cudaStream_t st) {
   if (!vs->pc_valid || P.table || capturing(st)) return 1;
   if (vs->pc_key != path_key(vs, o, spp_override, total)) return 1;
-  P.queue = vs->pc;
   P.q_count = vs->pc_count;
   P.q_cap = total;
+  PathSoA R;
+  path_soa(R, vs->pc, total, vs->max_depth);
+  R.n_end = vs->pc_count + 1;
   int grid, block;
   launch_dims(ln, total, grid, block);
-  if (vs->max_depth <= 8) k_path_reverse<8, true><<<grid, block, 0, st>>>(P);
-  else k_path_reverse<kMaxDepth, true><<<grid, block, 0, st>>>(P);
+  k_path_reverse<true><<<grid, block, 0, st>>>(P, R);
   count_launch(1);
   TRN_CUDA_TRY(cudaGetLastError());
   return 0;
@@ -3613,6 +3127,9 @@ int render_views(trn_scene* s, trn_viewset* vs, const trn_render_options* o, int
     TRN_CUDA_TRY(cudaMemsetAsync(vs->work, 0, sizeof(unsigned long long), st));
     const int cached = path_cache_fwd(vs, P, ln, o, spp_override, total, st);
     if (cached <= 0) return cached;
+    const int rc = path_wave<kWfFwd>(vs, P, ln, total, nullptr, st);
+    if (rc <= 0) return rc;
+    // without round buffers: one thread per path
     launch(k_path_fwd, ln, total, P, st);
     TRN_CUDA_TRY(cudaGetLastError());
     return 0;
@@ -3629,34 +3146,17 @@ int render_views(trn_scene* s, trn_viewset* vs, const trn_render_options* o, int
   }
   if (integrator == TRN_DIRECT_EDGE && guide_setup(s, o, P, st)) return -1;
   TRN_CUDA_TRY(cudaMemsetAsync(vs->work, 0, sizeof(unsigned long long), st));
-  const bool shallow = vs->max_depth <= 8;  // smaller per-thread path records
   switch (integrator) {
     case TRN_PATH_TRACER: {
       const int cached = path_cache_grad(vs, P, ln, o, spp_override, total, st);
       if (cached <= 0) return cached;
-      if (TRN_PATHADJ_SPLIT) return path_adj_split(vs, P, ln, total, shallow, st);
-      if (shallow) launch(k_path_adj<8>, ln, total, P, st); else launch(k_path_adj<kMaxDepth>, ln, total, P, st);
-      break;
+      return path_wave<kWfReplay>(vs, P, ln, total, nullptr, st) ? -1 : 0;
     }
-    case TRN_PRIMARY_EDGE:
-      if (TRN_PRIMARY_SPLIT) return primary_split(vs, P, ln, total, st);
-      launch(k_primary_adj, ln, total, P, st);
-      break;
-    case TRN_DIRECT_EDGE:
-      if (TRN_DIRECT_SPLIT) return direct_split(vs, P, ln, total, st);
-      launch(k_direct_adj, ln, total, P, st);
-      break;
-    case TRN_INDIRECT_EDGE:
-      if (TRN_INDIRECT_SPLIT) return indirect_split(vs, P, ln, total, shallow, st);
-      if (shallow) launch(k_indirect_adj<8>, ln, total, P, st); else launch(k_indirect_adj<kMaxDepth>, ln, total, P, st);
-      break;
-    default:
-      if (TRN_PIXEL_SPLIT) return pixel_split(vs, P, ln, total, st);
-      launch(k_pixel_adj, ln, total, P, st);
-      break;
+    case TRN_PRIMARY_EDGE: return edge_wave<TRN_PRIMARY_EDGE>(vs, P, ln, total, st);
+    case TRN_DIRECT_EDGE: return edge_wave<TRN_DIRECT_EDGE>(vs, P, ln, total, st);
+    case TRN_INDIRECT_EDGE: return edge_wave<TRN_INDIRECT_EDGE>(vs, P, ln, total, st);
+    default: return edge_wave<TRN_PIXEL_EDGE>(vs, P, ln, total, st);
   }
-  TRN_CUDA_TRY(cudaGetLastError());
-  return 0;
 }
 
 // (Re)define the views of a set. Device arrays grow to the largest view count
@@ -3777,6 +3277,7 @@ int trn_viewset_destroy(trn_viewset* vs) {
   void* ptrs[] = {vs->views, vs->vbegin, vs->pbegin, vs->pfunc, vs->pcdf, vs->pint, vs->pint_part, vs->work, vs->iq, vs->iq_count, vs->sq, vs->pc, vs->pc_count};
   for (void* p : ptrs)
     if (p) cudaFree(p);
+  for (void* p : vs->iq_old) cudaFree(p);
   if (vs->h_stage) cudaFreeHost(vs->h_stage);
   if (vs->h_stage_begin) cudaFreeHost(vs->h_stage_begin);
   for (cudaEvent_t e : vs->stage_done)
@@ -3794,8 +3295,9 @@ int trn_viewset_num_pixels(const trn_viewset* vs, long long* npix) {
 int trn_viewset_reserve(trn_viewset* vs, int max_bounces, cudaStream_t st) {
   if (!vs) { set_error("trn_viewset_reserve: null view set"); return -1; }
   if (max_bounces < 0 || max_bounces > kMaxDepth) { set_error("trn_viewset_reserve: max_bounces must be in [0, 16]"); return -1; }
-  if (ensure_queue(vs, full_queue_bytes(max_bounces <= 8), st)) return -1;
-  if (TRN_EDGE_ORDER && alloc_order(vs, kIndirectRound, st)) return -1;
+  const size_t most = full_queue_bytes(max_bounces <= 8);
+  if (ensure_queue(vs, most, most, st)) return -1;
+  if (TRN_EDGE_ORDER && alloc_order(vs, kRound, st)) return -1;
   return 0;
 }
 
@@ -4048,7 +3550,9 @@ int trn_intersect(trn_scene* s, int n, const float* org, const float* dir, const
   if (!s || !s->configured) { set_error("trn_intersect: scene not configured"); return -1; }
   if (n <= 0) return 0;
   if (!org || !dir || !tmin || !tmax || !tri || !u || !v || !t) { set_error("trn_intersect: null argument"); return -1; }
-  k_intersect<<<(n + 127) / 128, 128, 0, st>>>(s->view(), n, org, dir, tmin, tmax, tri, u, v, t, s->err);
+  int grid, chunk;
+  query_dims(n, grid, chunk);
+  k_query<false><<<grid, TRN_TRACE_BLOCK, 0, st>>>(s->view(), n, chunk, org, dir, tmin, tmax, tri, u, v, t, s->err);
   count_launch(1);
   TRN_CUDA_TRY(cudaGetLastError());
   return 0;
@@ -4059,7 +3563,10 @@ int trn_occluded(trn_scene* s, int n, const float* org, const float* dir, const 
   if (!s || !s->configured) { set_error("trn_occluded: scene not configured"); return -1; }
   if (n <= 0) return 0;
   if (!org || !dir || !tmin || !tmax || !vis) { set_error("trn_occluded: null argument"); return -1; }
-  k_occluded<<<(n + 127) / 128, 128, 0, st>>>(s->view(), n, org, dir, tmin, tmax, vis);
+  int grid, chunk;
+  query_dims(n, grid, chunk);
+  k_query<true><<<grid, TRN_TRACE_BLOCK, 0, st>>>(s->view(), n, chunk, org, dir, tmin, tmax, vis, nullptr, nullptr,
+                                                  nullptr, s->err);
   count_launch(1);
   TRN_CUDA_TRY(cudaGetLastError());
   return 0;

@@ -354,26 +354,23 @@ __global__ void __launch_bounds__(128) k_cluster(int n, const unsigned long long
 }
 
 __device__ __forceinline__ void write_child_box(BvhNode* nd, int side, const float lo[3], const float hi[3]) {
-  float* a = reinterpret_cast<float*>(nd);
-  if (side == 0) {
-    a[0] = lo[0]; a[1] = lo[1]; a[2] = lo[2]; a[3] = hi[0]; a[4] = hi[1]; a[5] = hi[2];
-  } else {
-    a[6] = lo[0]; a[7] = lo[1]; a[8] = lo[2]; a[9] = hi[0]; a[10] = hi[1]; a[11] = hi[2];
-  }
+  float* a = reinterpret_cast<float*>(nd) + 6 * side;
+  for (int k = 0; k < 3; k++) { a[2 * k] = lo[k]; a[2 * k + 1] = hi[k]; }
 }
 
 // Leaves write their (padded) boxes into the parent; the second thread to
 // arrive at an internal node merges both child boxes and moves up.
 __global__ void k_refit(int n, const unsigned long long* keys, const float* pos, const int* idx,
-                        BvhNode* nodes, const int* parent, int* flags, float4* tri_verts) {
+                        BvhNode* nodes, const int* parent, int* flags, LeafTri* tri_verts) {
   int leaf = blockIdx.x * blockDim.x + threadIdx.x;
   if (leaf >= n) return;
   const int f = (int)(keys[leaf] & 0xffffffffull);
   const F3 p0 = make_f3(pos + 3 * idx[3 * f]), p1 = make_f3(pos + 3 * idx[3 * f + 1]),
            p2 = make_f3(pos + 3 * idx[3 * f + 2]);
-  tri_verts[3 * leaf + 0] = make_float4(p0.x, p0.y, p0.z, __int_as_float(f));
-  tri_verts[3 * leaf + 1] = make_float4(p1.x, p1.y, p1.z, 0.f);
-  tri_verts[3 * leaf + 2] = make_float4(p2.x, p2.y, p2.z, 0.f);
+  float4* tv = reinterpret_cast<float4*>(tri_verts + leaf);
+  tv[0] = make_float4(p0.x, p0.y, p0.z, __int_as_float(f));
+  tv[1] = make_float4(p1.x, p1.y, p1.z, p2.x);
+  tv[2] = make_float4(p2.y, p2.z, 0.f, 0.f);
   float lo[3], hi[3];
   for (int k = 0; k < 3; k++) {
     lo[k] = fminf(fminf(p0[k], p1[k]), p2[k]);
@@ -398,213 +395,14 @@ __global__ void k_refit(int n, const unsigned long long* keys, const float* pos,
     // read both child boxes (volatile: the sibling wrote one of them)
     const volatile float* va = a;
     for (int k = 0; k < 3; k++) {
-      lo[k] = fminf(va[k], va[6 + k]);
-      hi[k] = fmaxf(va[3 + k], va[9 + k]);
+      lo[k] = fminf(va[2 * k], va[6 + 2 * k]);
+      hi[k] = fmaxf(va[2 * k + 1], va[7 + 2 * k]);
     }
     child = p;
     p = parent[p];
   }
 }
 
-
-// ---------------------------------------------------------------------------
-// Multi-triangle leaves: every subtree of the binary LBVH with at most
-// TRN_LEAF_MAX triangles becomes one leaf whose triangles are contiguous in
-// ctri. cnodes keeps the binary nodes (same indices and child boxes) with
-// such children re-encoded as leaves: ~(first | (count - 1) << 29). Nodes
-// inside a collapsed subtree are not reached. A ray meets the same triangles
-// or fewer node boxes; its result (closest (t, triangle id), or any hit)
-// does not depend on the tree.
-// ---------------------------------------------------------------------------
-__host__ __device__ constexpr int leaf_code(int first, int count) { return ~(first | ((count - 1) << 29)); }
-
-// subtree triangle counts, bottom-up from the leaves (the second child to
-// arrive at a node continues, as in k_refit)
-__global__ void k_leaf_counts(int n, const BvhNode* nodes, const int* parent, int* flags, int* cnt) {
-  const int leaf = blockIdx.x * blockDim.x + threadIdx.x;
-  if (leaf >= n) return;
-  int p = parent[n - 1 + leaf];
-  while (p >= 0) {
-    __threadfence();
-    if (atomicAdd(&flags[p], 1) == 0) return;
-    __threadfence();
-    const int4 d = nodes[p].d;
-    const volatile int* vc = cnt;
-    const int c = (d.x < 0 ? 1 : vc[d.x]) + (d.y < 0 ? 1 : vc[d.y]);
-    cnt[p] = c;
-    p = parent[p];
-  }
-}
-
-// triangles each reachable node's leaf children hold (0 inside a collapsed
-// subtree): the scan of this gives each node its first ctri slot
-__global__ void k_leaf_slots(int ninner, const BvhNode* nodes, const int* cnt, int* slots) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= ninner) return;
-  if (cnt[i] <= TRN_LEAF_MAX) { slots[i] = 0; return; }
-  const int4 d = nodes[i].d;
-  int k = 0;
-  for (int side = 0; side < 2; side++) {
-    const int c = side ? d.y : d.x;
-    k += c < 0 ? 1 : (cnt[c] <= TRN_LEAF_MAX ? cnt[c] : 0);
-  }
-  slots[i] = k;
-}
-
-__device__ __forceinline__ void copy_tri(const float4* src, int leaf, float4* dst, int slot) {
-  dst[3 * slot + 0] = src[3 * leaf + 0];
-  dst[3 * slot + 1] = src[3 * leaf + 1];
-  dst[3 * slot + 2] = src[3 * leaf + 2];
-}
-
-__global__ void k_leaf_collapse(int ninner, const BvhNode* nodes, const int* cnt, const int* base,
-                                const float4* tri_verts, BvhNode* cnodes, float4* ctri) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= ninner || cnt[i] <= TRN_LEAF_MAX) return;
-  BvhNode o = nodes[i];
-  int slot = base[i];
-  int child[2];
-  for (int side = 0; side < 2; side++) {
-    const int c = side ? o.d.y : o.d.x;
-    if (c < 0) {
-      copy_tri(tri_verts, ~c, ctri, slot);
-      child[side] = leaf_code(slot, 1);
-      slot += 1;
-    } else if (cnt[c] <= TRN_LEAF_MAX) {
-      // gather the subtree's triangles (at most TRN_LEAF_MAX leaves)
-      const int first = slot;
-      int stack[TRN_LEAF_MAX];
-      int sp = 0;
-      stack[sp++] = c;
-      while (sp > 0) {
-        const int4 d = nodes[stack[--sp]].d;
-        for (int k = 0; k < 2; k++) {  // (the order within a leaf is immaterial)
-          const int g = k ? d.y : d.x;
-          if (g < 0) {
-            copy_tri(tri_verts, ~g, ctri, slot++);
-          } else if (sp < TRN_LEAF_MAX) {
-            stack[sp++] = g;
-          }
-        }
-      }
-      child[side] = leaf_code(first, cnt[c]);
-    } else {
-      child[side] = c;
-    }
-  }
-  o.d = make_int4(child[0], child[1], 0, 0);
-  cnodes[i] = o;
-}
-
-// ---------------------------------------------------------------------------
-// collapse the binary LBVH into the 8-wide quantised BVH (top-down, one
-// level of wide nodes per launch). Each wide node takes the two children of
-// its binary node and repeatedly opens the internal child with the largest
-// surface area until it holds 8 children or only leaves.
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ float box_area(const float* lo, const float* hi) {
-  const float dx = fmaxf(hi[0] - lo[0], 0.f), dy = fmaxf(hi[1] - lo[1], 0.f), dz = fmaxf(hi[2] - lo[2], 0.f);
-  return dx * dy + dy * dz + dz * dx;
-}
-
-__device__ __forceinline__ void child_box(const BvhNode& n, int side, float* lo, float* hi) {
-  const float* a = reinterpret_cast<const float*>(&n);
-  const int o = side ? 6 : 0;
-  lo[0] = a[o]; lo[1] = a[o + 1]; lo[2] = a[o + 2];
-  hi[0] = a[o + 3]; hi[1] = a[o + 4]; hi[2] = a[o + 5];
-}
-
-__device__ __forceinline__ float qdecode(int q, float scale, float origin) {
-  return __fmaf_rn((float)q, scale, origin);
-}
-
-__global__ void k_collapse(int n_in, const int2* in, int2* out, int* counters, const BvhNode* nodes,
-                           const float4* tri_verts, WNode* wnodes, float4* wtri) {
-  const int item = blockIdx.x * blockDim.x + threadIdx.x;
-  if (item >= n_in) return;
-  const int b = in[item].x, w = in[item].y;
-  int cid[8];
-  float clo[8][3], chi[8][3];
-  const BvhNode nb = nodes[b];
-  cid[0] = nb.d.x; child_box(nb, 0, clo[0], chi[0]);
-  cid[1] = nb.d.y; child_box(nb, 1, clo[1], chi[1]);
-  int n = 2;
-  while (n < 8) {
-    int best = -1;
-    float best_a = -1.f;
-    for (int i = 0; i < n; i++)
-      if (cid[i] >= 0) {
-        const float a = box_area(clo[i], chi[i]);
-        if (a > best_a) { best_a = a; best = i; }
-      }
-    if (best < 0) break;
-    const BvhNode c = nodes[cid[best]];
-    cid[best] = c.d.x; child_box(c, 0, clo[best], chi[best]);
-    cid[n] = c.d.y; child_box(c, 1, clo[n], chi[n]);
-    n++;
-  }
-  int ni = 0, nl = 0;
-  for (int i = 0; i < n; i++) (cid[i] >= 0 ? ni : nl)++;
-  const int child_base = ni ? atomicAdd(&counters[0], ni) : 0;
-  const int tri_base = nl ? atomicAdd(&counters[1], nl) : 0;
-  const int qbase = ni ? atomicAdd(&counters[2], ni) : 0;
-  WNode wn;
-  float lo[3] = {3.4e38f, 3.4e38f, 3.4e38f}, hi[3] = {-3.4e38f, -3.4e38f, -3.4e38f};
-  for (int i = 0; i < n; i++)
-    for (int k = 0; k < 3; k++) { lo[k] = fminf(lo[k], clo[i][k]); hi[k] = fmaxf(hi[k], chi[i][k]); }
-  float scale[3];
-  unsigned char ebias[3];
-  for (int k = 0; k < 3; k++) {
-    const float ext = hi[k] - lo[k];
-    int e = -100;
-    if (ext > 0.f) {
-      int ee;
-      const float m = frexpf(ext / 255.f, &ee);
-      e = (m == 0.5f) ? ee - 1 : ee;
-      while (ldexpf(255.f, e) < ext) e++;
-    }
-    e = max(-126, min(127, e));
-    ebias[k] = (unsigned char)(e + 127);
-    scale[k] = __uint_as_float((unsigned)(e + 127) << 23);
-  }
-  wn.ox = lo[0]; wn.oy = lo[1]; wn.oz = lo[2];
-  wn.ex = ebias[0]; wn.ey = ebias[1]; wn.ez = ebias[2];
-  wn.nchild = (unsigned char)n;
-  wn.child_base = child_base;
-  wn.tri_base = tri_base;
-  int ii = 0, il = 0;
-  for (int i = 0; i < 8; i++) {
-    if (i >= n) {
-      wn.meta[i] = 0;
-      for (int k = 0; k < 3; k++) { wn.qlo[k][i] = 255; wn.qhi[k][i] = 0; }
-      continue;
-    }
-    for (int k = 0; k < 3; k++) {
-      int ql = (int)floorf((clo[i][k] - lo[k]) / scale[k]);
-      int qh = (int)ceilf((chi[i][k] - lo[k]) / scale[k]);
-      ql = max(0, min(255, ql));
-      qh = max(0, min(255, qh));
-      while (ql > 0 && qdecode(ql, scale[k], lo[k]) > clo[i][k]) ql--;
-      while (qh < 255 && qdecode(qh, scale[k], lo[k]) < chi[i][k]) qh++;
-      wn.qlo[k][i] = (unsigned char)ql;
-      wn.qhi[k][i] = (unsigned char)qh;
-    }
-    if (cid[i] >= 0) {
-      wn.meta[i] = (unsigned char)(0x80 | ii);
-      out[qbase + ii] = make_int2(cid[i], child_base + ii);
-      ii++;
-    } else {
-      const int leaf = ~cid[i];
-      wn.meta[i] = (unsigned char)(0xC0 | il);
-      const int slot = tri_base + il;
-      wtri[3 * slot + 0] = tri_verts[3 * leaf + 0];
-      wtri[3 * slot + 1] = tri_verts[3 * leaf + 1];
-      wtri[3 * slot + 2] = tri_verts[3 * leaf + 2];
-      il++;
-    }
-  }
-  wnodes[w] = wn;
-}
 
 // ---------------------------------------------------------------------------
 // geometry-chain adjoint
@@ -970,20 +768,12 @@ int trn_scene_create(const trn_scene_desc* d, trn_scene** out) {
       dev_alloc_copy(&s->aq_edge, (const int*)nullptr, std::max<size_t>(1, (size_t)s->ne)) ||
       dev_alloc_copy(&s->aq_count, (const int*)nullptr, 4) ||
       dev_alloc_copy(&s->nodes, (const BvhNode*)nullptr, std::max(1, nt - 1)) ||
-      dev_alloc_copy(&s->tri_verts, (const float4*)nullptr, 3 * (size_t)nt) ||
+      dev_alloc_copy(&s->tri_verts, (const LeafTri*)nullptr, (size_t)nt) ||
       dev_alloc_copy(&s->parent, (const int*)nullptr, 2 * (size_t)nt) ||
       dev_alloc_copy(&s->flags, (const int*)nullptr, std::max(1, nt - 1)) ||
-      (TRN_LEAF_MAX > 1 && nt > TRN_LEAF_MAX &&
-       (dev_alloc_copy(&s->cnodes, (const BvhNode*)nullptr, (size_t)nt - 1) ||
-        dev_alloc_copy(&s->ctri, (const float4*)nullptr, 3 * (size_t)nt) ||
-        dev_alloc_copy(&s->leaf_cnt, (const int*)nullptr, 3 * ((size_t)nt - 1)))) ||
       dev_alloc_copy(&s->keys, (const unsigned long long*)nullptr, (size_t)nt) ||
       dev_alloc_copy(&s->keys_alt, (const unsigned long long*)nullptr, (size_t)nt) ||
       dev_alloc_copy(&s->bounds, (const float*)nullptr, 6) ||
-      dev_alloc_copy(&s->wnodes, (const WNode*)nullptr, std::max(1, nt)) ||
-      dev_alloc_copy(&s->wtri, (const float4*)nullptr, 3 * (size_t)nt) ||
-      dev_alloc_copy(&s->wqueue, (const int*)nullptr, 4 * (size_t)std::max(1, nt)) ||
-      dev_alloc_copy(&s->wcount, (const int*)nullptr, 4) ||
       dev_alloc_copy(&s->g_pos, (const float*)nullptr, 3 * (size_t)nv) ||
       dev_alloc_copy(&s->g_vnormal, (const float*)nullptr, 3 * (size_t)nv) ||
       dev_alloc_copy(&s->g_texels, (const float*)nullptr, std::max<size_t>(3, 3 * (size_t)ntexel)) ||
@@ -1003,15 +793,6 @@ int trn_scene_create(const trn_scene_desc* d, trn_scene** out) {
   cub::DeviceRadixSort::SortKeys(nullptr, bytes, s->keys, s->keys_alt, nt, 32, 63);
   s->sort_tmp_bytes = bytes;
   if (cudaMalloc(&s->sort_tmp, bytes) != cudaSuccess) { set_error("trn_scene_create: out of memory"); return fail(); }
-  if (s->cnodes) {
-    size_t sb = 0;
-    cub::DeviceScan::ExclusiveSum(nullptr, sb, s->leaf_cnt, s->leaf_cnt, nt - 1);
-    s->leaf_scan_bytes = std::max<size_t>(sb, 16);
-    if (cudaMalloc(&s->leaf_scan_tmp, s->leaf_scan_bytes) != cudaSuccess) {
-      set_error("trn_scene_create: out of memory");
-      return fail();
-    }
-  }
   if (dev_alloc_copy(&s->cluster_id, (const int*)nullptr, (size_t)nt) ||
       dev_alloc_copy(&s->cluster_box, (const float*)nullptr, 12 * (size_t)nt) ||
       dev_alloc_copy(&s->cluster_meet, (const int*)nullptr, (size_t)nt) ||
@@ -1031,9 +812,9 @@ int trn_scene_destroy(trn_scene* s) {
                   s->light_integral_dev, s->light_lum, s->cdf_part, s->bsdfs, s->texs, s->edges, s->sec_func, s->sec_cdf,
                   s->sec_integral_dev, s->nodes, s->tri_verts, s->parent, s->flags, s->keys, s->keys_alt,
                   s->sort_tmp, s->bounds, s->g_pos, s->g_vnormal, s->g_texels, s->g_translation, s->err,
-                  s->stats, s->wnodes, s->wtri, s->wqueue, s->wcount, s->aq_poly, s->aq_func, s->aq_cdf,
+                  s->stats, s->aq_poly, s->aq_func, s->aq_cdf,
                   s->aq_int, s->aq_box, s->aq_edge, s->aq_count, s->aq_eval, s->aq_flag, s->aq_prefix, s->cluster_id,
-                  s->cluster_box, s->cluster_meet, s->cluster_count, s->cnodes, s->ctri, s->leaf_cnt, s->leaf_scan_tmp};
+                  s->cluster_box, s->cluster_meet, s->cluster_count};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   delete s;
@@ -1064,29 +845,6 @@ int configure_geometry(trn_scene* s, cudaStream_t st) {
   }
   return 0;
 }
-// Rebuild the collapsed arrays from the binary LBVH (after a build or refit).
-int leaf_collapse(trn_scene* s, cudaStream_t st) {
-  s->collapsed = false;
-  if (!s->cnodes) return 0;
-  const int nt = s->nt, ninner = nt - 1;
-  int* cnt = s->leaf_cnt;
-  int* slots = s->leaf_cnt + ninner;
-  int* base = s->leaf_cnt + 2 * ninner;
-  TRN_CUDA_TRY(cudaMemsetAsync(s->flags, 0, sizeof(int) * ninner, st));
-  k_leaf_counts<<<nblk(nt), 256, 0, st>>>(nt, s->nodes, s->parent, s->flags, cnt);
-  k_leaf_slots<<<nblk(ninner), 256, 0, st>>>(ninner, s->nodes, cnt, slots);
-  size_t sb = s->leaf_scan_bytes;
-  if (cub::DeviceScan::ExclusiveSum(s->leaf_scan_tmp, sb, slots, base, ninner, st) != cudaSuccess) {
-    set_error("trn_scene_configure: leaf scan failed");
-    return -1;
-  }
-  k_leaf_collapse<<<nblk(ninner), 256, 0, st>>>(ninner, s->nodes, cnt, base, s->tri_verts, s->cnodes, s->ctri);
-  count_launch(4);
-  TRN_CUDA_TRY(cudaGetLastError());
-  s->collapsed = true;
-  return 0;
-}
-
 }  // namespace
 
 extern "C" {
@@ -1115,31 +873,6 @@ int trn_scene_configure(trn_scene* s, cudaStream_t st) {
   }
   k_refit<<<nblk(nt), 256, 0, st>>>(nt, s->keys_alt, s->pos, s->idx, s->nodes, s->parent, s->flags, s->tri_verts);
   count_launch(1);
-  if (!TRN_WIDE_BVH && leaf_collapse(s, st)) return -1;
-  // 8-wide quantised BVH
-  s->n_wnodes = 0;
-  if (TRN_WIDE_BVH && nt > 1) {
-    int2* qa = reinterpret_cast<int2*>(s->wqueue);
-    int2* qb = qa + nt;
-    const int init[4] = {1, 0, 0, 0};
-    const int2 root = make_int2(0, 0);
-    TRN_CUDA_TRY(cudaMemcpyAsync(s->wcount, init, sizeof(init), cudaMemcpyHostToDevice, st));
-    TRN_CUDA_TRY(cudaMemcpyAsync(qa, &root, sizeof(int2), cudaMemcpyHostToDevice, st));
-    int n_in = 1;
-    int levels = 0;
-    while (n_in > 0) {
-      TRN_CUDA_TRY(cudaMemsetAsync(s->wcount + 2, 0, sizeof(int), st));
-      k_collapse<<<nblk(n_in, 128), 128, 0, st>>>(n_in, qa, qb, s->wcount, s->nodes, s->tri_verts, s->wnodes, s->wtri);
-      count_launch(1);
-      int c[4];
-      TRN_CUDA_TRY(cudaMemcpyAsync(c, s->wcount, sizeof(c), cudaMemcpyDeviceToHost, st));
-      TRN_CUDA_TRY(cudaStreamSynchronize(st));
-      n_in = c[2];
-      s->n_wnodes = c[0];
-      std::swap(qa, qb);
-      if (++levels > 64) { set_error("trn_scene_configure: wide BVH collapse did not terminate"); return -1; }
-    }
-  }
   TRN_CUDA_TRY(cudaGetLastError());
   s->configured = true;
   s->built = true;
@@ -1151,13 +884,12 @@ int trn_scene_configure(trn_scene* s, cudaStream_t st) {
 // BVH topology; leaf boxes and node boxes are recomputed bottom-up.
 int trn_scene_refit(trn_scene* s, cudaStream_t st) {
   if (!s) { set_error("trn_scene_refit: null scene"); return -1; }
-  if (!s->built || TRN_WIDE_BVH) return trn_scene_configure(s, st);  // the wide BVH is re-collapsed
+  if (!s->built) return trn_scene_configure(s, st);
   const int nt = s->nt;
   if (configure_geometry(s, st)) return -1;
   if (nt > 1) TRN_CUDA_TRY(cudaMemsetAsync(s->flags, 0, sizeof(int) * (nt - 1), st));
   k_refit<<<nblk(nt), 256, 0, st>>>(nt, s->keys_alt, s->pos, s->idx, s->nodes, s->parent, s->flags, s->tri_verts);
   count_launch(1);
-  if (leaf_collapse(s, st)) return -1;
   TRN_CUDA_TRY(cudaGetLastError());
   s->configured = true;
   s->version++;

@@ -11,8 +11,7 @@
 //   uv/uvidx   [NUV][2], [T][3]  texture coordinates (Scene.cpp:687-697)
 //   bsdf_id    [T]    i32  material per triangle (mSbtIndexBuffer)
 //   emitter_id [T]    i32  area-light id or -1 (mEmitterIDBuffer)
-//   tri_verts  [T][12] f32 leaf-ordered triangle vertices for traversal:
-//                          (P0.xyz, tri_id) (P1.xyz, 0) (P2.xyz, 0)
+//   tri_verts  [T]    LeafTri  leaf-ordered triangles for traversal
 //   nodes      [T-1]  BvhNode  binary LBVH, child boxes stored in the parent
 #pragma once
 #include "common.cuh"
@@ -34,44 +33,22 @@ struct TexDesc {
   long long offset;  // texel offset into the texel array (RGB triples)
 };
 
-struct alignas(16) BvhNode {
-  // child 0 box (lo, hi), child 1 box (lo, hi), children (>=0 node, <0 ~leaf)
-  float4 a;  // l0x l0y l0z h0x
-  float4 b;  // h0y h0z l1x l1y
-  float4 c;  // l1z h1x h1y h1z
+struct alignas(64) BvhNode {
+  // child boxes as (lo, hi) per axis, children (>= 0 node, < 0 ~leaf)
+  float4 a;  // l0x h0x l0y h0y
+  float4 b;  // l0z h0z l1x h1x
+  float4 c;  // l1y h1y l1z h1z
   int4 d;    // c0 c1 - -
 };
 
-// 8-wide BVH node with quantised child boxes (80 bytes). Child boxes are
-// stored as 8-bit offsets from `origin` in units of a per-axis power of two,
-// rounded outwards, so decoding is conservative. Internal children of a node
-// are stored contiguously from child_base, leaf triangles from tri_base;
-// meta[i]: bit 7 = slot used, bit 6 = leaf, bits 0-5 = offset from the base.
-struct alignas(16) WNode {
-  float ox, oy, oz;
-  unsigned char ex, ey, ez, nchild;  // biased exponents (IEEE bias 127)
-  int child_base;
-  int tri_base;
-  unsigned char meta[8];
-  unsigned char qlo[3][8];
-  unsigned char qhi[3][8];
+// A leaf's triangle, two sectors: 40 bytes used.
+struct alignas(64) LeafTri {
+  float p0[3];
+  int tri;
+  float p1[3], p2[3];
+  float pad_[6];
 };
-static_assert(sizeof(WNode) == 80, "WNode must be 80 bytes");
-
-constexpr int kTopNodes = 73;  // root + 8 + 64 wide nodes staged in shared memory
-
-// Traversal structure: the binary LBVH with child boxes in the parent (default;
-// measured faster on B200 for the scenes here) or the 8-wide quantised BVH.
-// most triangles in one leaf of the traversed LBVH (1 = the binary tree's
-// one-triangle leaves, the default: leaves of up to 2 measured the same, up
-// to 4 slower, because a leaf's box admits more rays than its triangles'
-// boxes did and each costs exact watertight tests)
-#ifndef TRN_LEAF_MAX
-#define TRN_LEAF_MAX 1
-#endif
-#ifndef TRN_WIDE_BVH
-#define TRN_WIDE_BVH 0
-#endif
+static_assert(sizeof(LeafTri) == 64, "LeafTri must be two 32-byte sectors");
 
 struct DeviceScene {
   int nv, nt;
@@ -100,11 +77,7 @@ struct DeviceScene {
   const float* texels;        // [sum w*h][3]
   // acceleration structure
   const BvhNode* nodes;
-  const float4* tri_verts;    // [T][3] float4 (binary-leaf order)
-  const WNode* wnodes;        // 8-wide quantised BVH
-  const float4* wtri;         // [T][3] float4 in wide-leaf order
-  int n_wnodes;
-  int root_is_leaf;
+  const LeafTri* tri_verts;   // [T] leaf order
 };
 
 // Pinhole camera (Camera.cpp:89-137, BaseCamera.cpp:45-88). Matrices are

@@ -21,15 +21,39 @@ struct Hit {
   float u, v, t;  // u weights P1, v weights P2 (Scene.cpp:677-684)
 };
 
+// Two floats for the packed multiply-add (one instruction for both).
+struct Pair { float a, b; };
+TRN_D Pair fma2(const Pair& x, const Pair& y, const Pair& z) {
+  Pair r;
+#if defined(__CUDA_ARCH__) && __CUDA_ARCH__ >= 1000
+  asm("{\n\t.reg .b64 x, y, z, r;\n\t"
+      "mov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmov.b64 z, {%6, %7};\n\t"
+      "fma.rn.f32x2 r, x, y, z;\n\tmov.b64 {%0, %1}, r;\n\t}"
+      : "=f"(r.a), "=f"(r.b) : "f"(x.a), "f"(x.b), "f"(y.a), "f"(y.b), "f"(z.a), "f"(z.b));
+#else
+  r.a = fmaf(x.a, y.a, z.a);
+  r.b = fmaf(x.b, y.b, z.b);
+#endif
+  return r;
+}
+
+// A ray as the traversal uses it: the shear of the watertight triangle test
+// (kx, ky, kz, sx, sy, sz) and, for the box slabs, the reciprocal direction
+// with the origin folded in: the distances of an axis' two planes are one
+// packed multiply-add, (lo, hi) * inv + c. c holds -o * inv, moved by
+// |o * inv| 2^-22 away from the box (down for the plane that is entered, up for
+// the one that is left): more than the rounding of o * inv and of its product,
+// so that a box is never missed (see `slab`).
 struct RayPre {
-  F3 o, d, inv;
+  F3 o;
+  Pair ix, iy, iz, cx, cy, cz;
   int kx, ky, kz;
   float sx, sy, sz;
 };
 
 TRN_D RayPre ray_setup(const F3& o, const F3& d) {
   RayPre r;
-  r.o = o; r.d = d;
+  r.o = o;
   float ax = fabsf(d.x), ay = fabsf(d.y), az = fabsf(d.z);
   int kz = 0; float m = ax;
   if (ay > m) { kz = 1; m = ay; }
@@ -43,7 +67,15 @@ TRN_D RayPre ray_setup(const F3& o, const F3& d) {
   r.sz = __fdiv_rn(1.f, d[kz]);
   // reciprocal direction for the box slabs (culling only)
   auto safe = [](float x) { return fabsf(x) < 1e-20f ? copysignf(1e-20f, x) : x; };
-  r.inv = F3(1.f / safe(d.x), 1.f / safe(d.y), 1.f / safe(d.z));
+  auto axis = [&](float o, float d, Pair& inv, Pair& c) {
+    inv.a = inv.b = 1.f / safe(d);
+    const float k = -(o * inv.a), e = fabsf(k) * 2.384185791015625e-7f;  // 2^-22
+    c.a = inv.a < 0.f ? k + e : k - e;
+    c.b = inv.a < 0.f ? k - e : k + e;
+  };
+  axis(o.x, d.x, r.ix, r.cx);
+  axis(o.y, d.y, r.iy, r.cy);
+  axis(o.z, d.z, r.iz, r.cz);
   return r;
 }
 
@@ -85,255 +117,190 @@ TRN_D bool intersect_tri(const RayPre& r, const F3& p0, const F3& p1, const F3& 
   return true;
 }
 
-// Slab test of one child box; boxes are padded at build time and the far
-// distance gets a relative slack so culling stays conservative w.r.t. the
-// exactly rounded triangle test.
-TRN_D bool slab(const RayPre& r, float lx, float ly, float lz, float hx, float hy, float hz,
-                float tmin, float tmax, float& tnear) {
-  float tx0 = (lx - r.o.x) * r.inv.x, tx1 = (hx - r.o.x) * r.inv.x;
-  float ty0 = (ly - r.o.y) * r.inv.y, ty1 = (hy - r.o.y) * r.inv.y;
-  float tz0 = (lz - r.o.z) * r.inv.z, tz1 = (hz - r.o.z) * r.inv.z;
-  float tn = fmaxf(fmaxf(fminf(tx0, tx1), fminf(ty0, ty1)), fmaxf(fminf(tz0, tz1), tmin));
-  float tf = fminf(fminf(fmaxf(tx0, tx1), fmaxf(ty0, ty1)), fminf(fmaxf(tz0, tz1), tmax));
-  tnear = tn;
-  return tn <= tf * 1.0000004f;
+// ---- box steps ---------------------------------------------------------------
+// What bounds traversal here is instruction issue and the L1's data path (one
+// lane's line per cycle and SM). A node is fetched in two 32-byte loads, a
+// triangle in two; plane distances are one multiply-add each and the slab's
+// extremes three-input min/max.
+TRN_D float max3(float a, float b, float c) {
+#if defined(__CUDA_ARCH__) && __CUDA_ARCH__ >= 1000
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+#else
+  return fmaxf(fmaxf(a, b), c);
+#endif
+}
+TRN_D float min3(float a, float b, float c) {
+#if defined(__CUDA_ARCH__) && __CUDA_ARCH__ >= 1000
+  float r;
+  asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+#else
+  return fminf(fminf(a, b), c);
+#endif
 }
 
-constexpr int kStackSize = 64;
+// 32 bytes at a 32-byte aligned address, WIDE in one load (the stream
+// traversal; ptxas 12.9 crashes on the wide load in the fused kernels, which
+// spill).
+template <bool WIDE>
+TRN_D void load8(const void* p, float4& a, float4& b) {
+  if (!WIDE) {
+    a = __ldg(static_cast<const float4*>(p));
+    b = __ldg(static_cast<const float4*>(p) + 1);
+    return;
+  }
+#if defined(__CUDA_ARCH__) && __CUDA_ARCH__ >= 1000
+  asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+      : "l"(p));
+#else
+  a = static_cast<const float4*>(p)[0];
+  b = static_cast<const float4*>(p)[1];
+#endif
+}
 
+constexpr int kStackSize = 72;          // one entry per level at most, and one to spare
+// traversal states beside the node to visit next (>= 0 inner, < 0 leaf)
+constexpr int kTraceDone = 0x7fffffff;  // nothing left
+constexpr int kTracePop = 0x7ffffffe;   // the stack's next entry
+
+// One box (lo, hi per axis) against the ray's interval [tmin, tmax]. Culling is
+// conservative: the ray's c covers the origin's share of the rounding, boxes
+// are padded at build time, and for the relative error of at most 2^-23 per
+// distance (reciprocal and final rounding) the far distance gets a slack of
+// 4e-7.
+TRN_D bool slab(const RayPre& r, const Pair& bx, const Pair& by, const Pair& bz, float tmin, float tmax, float& tnear) {
+  const Pair x = fma2(bx, r.ix, r.cx), y = fma2(by, r.iy, r.cy), z = fma2(bz, r.iz, r.cz);
+  tnear = fmaxf(max3(fminf(x.a, x.b), fminf(y.a, y.b), fminf(z.a, z.b)), tmin);
+  const float tf = fminf(min3(fmaxf(x.a, x.b), fmaxf(y.a, y.b), fmaxf(z.a, z.b)), tmax);
+  return tnear <= tf * 1.0000004f;
+}
+
+// Traversal stacks: entries are (child, bits of its box's entry distance).
+struct LocalStack {
+  int2 e[kStackSize];
+  TRN_D void set(int i, int2 v) { e[i] = v; }
+  TRN_D int2 get(int i) const { return e[i]; }
+};
+// The stream traversal's first entries lie in shared memory: the lanes of a
+// warp stand at different depths, and an access to local memory then takes a
+// pass through the L1 for every depth among them, where here each lane has its
+// own banks (672 -> 580 us for 2^20 rays). Deeper entries are rare.
+#ifndef TRN_SHARED_STACK
+#define TRN_SHARED_STACK 12
+#endif
+#ifndef TRN_TRACE_BLOCK
+#define TRN_TRACE_BLOCK 128
+#endif
+struct SharedStack {
+  int2* top;                                 // this thread's column
+  int2 e[kStackSize - TRN_SHARED_STACK];
+  TRN_D void set(int i, int2 v) {
+    if (i < TRN_SHARED_STACK) top[i * TRN_TRACE_BLOCK] = v;
+    else e[i - TRN_SHARED_STACK] = v;
+  }
+  TRN_D int2 get(int i) const { return i < TRN_SHARED_STACK ? top[i * TRN_TRACE_BLOCK] : e[i - TRN_SHARED_STACK]; }
+};
+TRN_D int2* shared_stack() {
+  __shared__ int2 s[TRN_SHARED_STACK * TRN_TRACE_BLOCK];
+  return s + threadIdx.x;
+}
+
+// Farthest entry distance that can still matter. (A popped entry whose box
+// starts behind the closest hit is dropped without a fetch.)
+TRN_D float pop_limit(float best_t) { return best_t + fabsf(best_t) * 4e-7f; }
+
+// One box step. Returns the nearer child that is hit (inner node >= 0, leaf <
+// 0) or kTracePop; the farther one goes to the stack as (child, bits of its
+// entry distance). Straight-line code: lanes of a warp differ in which children
+// they hit, and every branch would run once more per warp.
+template <bool WIDE, class Stack>
+TRN_D int visit_node(const DeviceScene& s, const RayPre& r, int node, float tmin, float best_t, Stack& stack, int& sp,
+                     int* err) {
+  const char* n = reinterpret_cast<const char*>(s.nodes) + ((size_t)(unsigned)node << 6);
+  float4 a, b, c, d;
+  load8<WIDE>(n, a, b);
+  load8<WIDE>(n + 32, c, d);
+  float t0, t1;
+  const bool h0 = slab(r, {a.x, a.y}, {a.z, a.w}, {b.x, b.y}, tmin, best_t, t0);
+  const bool h1 = slab(r, {b.z, b.w}, {c.x, c.y}, {c.z, c.w}, tmin, best_t, t1);
+  const int c0 = __float_as_int(d.x), c1 = __float_as_int(d.y);
+  const bool both = h0 && h1;
+  const bool second = h1 && (!h0 || t1 < t0);   // the nearer one is child 1
+  if (both) {
+    stack.set(sp, make_int2(second ? c0 : c1, __float_as_int(second ? t0 : t1)));
+    sp++;
+    if (sp >= kStackSize) {
+      sp = kStackSize - 1;
+      if (err) atomicExch(err, 1);
+    }
+  }
+  return h0 || h1 ? (second ? c1 : c0) : kTracePop;
+}
+
+// One attempt to take the next entry.
+template <class Stack>
+TRN_D void pop_entry(const Stack& stack, int& sp, float limit, int& cur) {
+  if (cur == kTracePop) {
+    sp--;
+    const int2 e = stack.get(max(sp, 0));
+    cur = sp < 0 ? kTraceDone : (__int_as_float(e.y) <= limit ? e.x : kTracePop);
+  }
+}
+
+template <bool WIDE>
 TRN_D void leaf_tri(const DeviceScene& s, int leaf, F3& p0, F3& p1, F3& p2, int& tri) {
-  const float4 a = __ldg(&s.tri_verts[3 * leaf + 0]);
-  const float4 b = __ldg(&s.tri_verts[3 * leaf + 1]);
-  const float4 c = __ldg(&s.tri_verts[3 * leaf + 2]);
-  p0 = F3(a.x, a.y, a.z); p1 = F3(b.x, b.y, b.z); p2 = F3(c.x, c.y, c.z);
-  tri = __float_as_int(a.w);
+  const char* q = reinterpret_cast<const char*>(s.tri_verts) + ((size_t)(unsigned)leaf << 6);
+  float4 a, b;
+  load8<WIDE>(q, a, b);
+  const float2 c = __ldg(reinterpret_cast<const float2*>(q + 32));
+  p0 = F3(a.x, a.y, a.z); tri = __float_as_int(a.w);
+  p1 = F3(b.x, b.y, b.z); p2 = F3(b.w, c.x, c.y);
 }
 
-
-// ---- 8-wide quantised BVH -------------------------------------------------
-// Top levels (root, its children, grandchildren: kTopNodes nodes) are staged
-// in shared memory once per block by stage_top(); deeper nodes are read with
-// 16-byte read-only loads.
-TRN_D WNode* top_nodes() {
-  __shared__ WNode top[kTopNodes];
-  return top;
-}
-
-// every kernel that traces rays calls this once before its work loop
-TRN_D void stage_top(const DeviceScene& s) {
-  if (!TRN_WIDE_BVH) return;
-  const int n = min(s.n_wnodes, kTopNodes);
-  const uint4* src = reinterpret_cast<const uint4*>(s.wnodes);
-  uint4* dst = reinterpret_cast<uint4*>(top_nodes());
-  for (int i = threadIdx.x; i < n * 5; i += blockDim.x) dst[i] = __ldg(src + i);
-  __syncthreads();
-}
-
-TRN_D void load_wnode(const DeviceScene& s, int idx, WNode& n) {
-  uint4* d = reinterpret_cast<uint4*>(&n);
-  if (idx < kTopNodes) {
-    const uint4* src = reinterpret_cast<const uint4*>(top_nodes() + idx);
-#pragma unroll
-    for (int i = 0; i < 5; i++) d[i] = src[i];
-  } else {
-    const uint4* src = reinterpret_cast<const uint4*>(s.wnodes + idx);
-#pragma unroll
-    for (int i = 0; i < 5; i++) d[i] = __ldg(src + i);
-  }
-}
-
-template <bool ANY>
-__device__ __noinline__ bool trace_wide(const DeviceScene& s, const RayPre& r, float tmin, float tmax, Hit& hit,
-                                        int* err) {
-  float best_t = tmax;
-  int best_tri = 0x7fffffff;
-  bool found = false;
-  int2 stack[kStackSize];  // (node, tnear bits)
-  int sp = 0;
-  int cur = 0;
-  for (;;) {
-    WNode n;
-    load_wnode(s, cur, n);
-    const float sx = __uint_as_float((unsigned)n.ex << 23);
-    const float sy = __uint_as_float((unsigned)n.ey << 23);
-    const float sz = __uint_as_float((unsigned)n.ez << 23);
-    // box tests of all children first; hits go to two bit masks
-    unsigned leaf_mask = 0u, node_mask = 0u;
-    float tnear[8];
-#pragma unroll
-    for (int i = 0; i < 8; i++) {
-      const unsigned m = n.meta[i];
-      tnear[i] = 0.f;
-      if (!(m & 0x80u)) continue;
-      const float lx = __fmaf_rn((float)n.qlo[0][i], sx, n.ox), hx = __fmaf_rn((float)n.qhi[0][i], sx, n.ox);
-      const float ly = __fmaf_rn((float)n.qlo[1][i], sy, n.oy), hy = __fmaf_rn((float)n.qhi[1][i], sy, n.oy);
-      const float lz = __fmaf_rn((float)n.qlo[2][i], sz, n.oz), hz = __fmaf_rn((float)n.qhi[2][i], sz, n.oz);
-      float tn;
-      if (slab(r, lx, ly, lz, hx, hy, hz, tmin, best_t, tn)) {
-        tnear[i] = tn;
-        if (m & 0x40u) leaf_mask |= 1u << i; else node_mask |= 1u << i;
-      }
-    }
-    // leaf triangles
-    while (leaf_mask) {
-      const int i = __ffs(leaf_mask) - 1;
-      leaf_mask &= leaf_mask - 1u;
-      const int slot = n.tri_base + (int)(n.meta[i] & 0x3fu);
-      const float4 a = __ldg(&s.wtri[3 * slot + 0]);
-      const float4 b = __ldg(&s.wtri[3 * slot + 1]);
-      const float4 c = __ldg(&s.wtri[3 * slot + 2]);
-      const int tri = __float_as_int(a.w);
-      float t, u, v;
-      if (intersect_tri(r, F3(a.x, a.y, a.z), F3(b.x, b.y, b.z), F3(c.x, c.y, c.z), tmin, tmax, t, u, v)) {
-        if (ANY) { hit.tri = tri; hit.t = t; hit.u = u; hit.v = v; return true; }
-        if (t < best_t || (t == best_t && tri < best_tri)) {
-          best_t = t; best_tri = tri; hit.u = u; hit.v = v; found = true;
-        }
-      }
-    }
-    // internal children: descend into the nearest, push the rest far-to-near
-    int next = -1;
-    if (node_mask) {
-      float nt = 3.4e38f;
-      int ni = 0;
-      for (unsigned mm = node_mask; mm; mm &= mm - 1u) {
-        const int i = __ffs(mm) - 1;
-        if (tnear[i] < nt) { nt = tnear[i]; ni = i; }
-      }
-      node_mask &= ~(1u << ni);
-      next = n.child_base + (int)(n.meta[ni] & 0x3fu);
-      while (node_mask) {
-        // push the farthest remaining first so nearer ones pop earlier
-        float ft = -1.f;
-        int fi = 0;
-        for (unsigned mm = node_mask; mm; mm &= mm - 1u) {
-          const int i = __ffs(mm) - 1;
-          if (tnear[i] >= ft) { ft = tnear[i]; fi = i; }
-        }
-        node_mask &= ~(1u << fi);
-        if (sp < kStackSize) stack[sp++] = make_int2(n.child_base + (int)(n.meta[fi] & 0x3fu), __float_as_int(ft));
-        else if (err) atomicExch(err, 1);
-      }
-    }
-    if (next >= 0) { cur = next; continue; }
-    // pop the next node whose box is still in front of the closest hit
-    bool got = false;
-    while (sp > 0) {
-      const int2 e = stack[--sp];
-      if (__int_as_float(e.y) <= best_t * 1.0000004f) { cur = e.x; got = true; break; }
-    }
-    if (!got) break;
-  }
-  if (ANY) return false;
-  if (found) { hit.tri = best_tri; hit.t = best_t; }
-  return found;
+// A ray that can meet no triangle: any NaN makes every edge function NaN, and
+// a zero direction has no largest axis. (The box tests above would let such a
+// ray into every node.)
+TRN_D bool ray_is_void(const F3& o, const F3& d) {
+  return isnan(o.x) || isnan(o.y) || isnan(o.z) || isnan(d.x) || isnan(d.y) || isnan(d.z) ||
+         (d.x == 0.f && d.y == 0.f && d.z == 0.f);
 }
 
 // Closest hit (ANY == false) or occlusion (ANY == true). Returns true on hit.
-#ifndef TRN_ONE_LEAF_SITE
-#define TRN_ONE_LEAF_SITE 1
-#endif
-static_assert(TRN_ONE_LEAF_SITE || TRN_LEAF_MAX == 1, "multi-triangle leaves need the one-leaf-site traversal");
-
 template <bool ANY>
 TRN_D bool trace(const DeviceScene& s, const F3& o, const F3& d, float tmin, float tmax, Hit& hit,
                  int* err = nullptr) {
   hit.tri = -1; hit.u = 0.f; hit.v = 0.f; hit.t = -1.f;
-  if (s.nt <= 0) return false;
+  if (s.nt <= 0 || ray_is_void(o, d)) return false;
   const RayPre r = ray_setup(o, d);
-  if (TRN_WIDE_BVH && s.n_wnodes > 0) return trace_wide<ANY>(s, r, tmin, tmax, hit, err);
   float best_t = tmax;
-  int best_tri = 0x7fffffff;
-  bool found = false;
-  auto test_leaf = [&](int leaf) -> bool {
+  int best_tri = -1;
+  LocalStack stack;
+  int sp = 0, cur = s.nt == 1 ? ~0 : 0;
+  // leaves are visited through the loop like inner nodes, so the triangle
+  // test is instantiated once per traversal (smaller code)
+  for (;;) {
+    while (cur == kTracePop) pop_entry(stack, sp, pop_limit(best_t), cur);
+    if (cur == kTraceDone) break;
+    if (cur >= 0) {
+      cur = visit_node<false>(s, r, cur, tmin, best_t, stack, sp, err);
+      continue;
+    }
     F3 p0, p1, p2; int tri;
-    leaf_tri(s, leaf, p0, p1, p2, tri);
+    leaf_tri<false>(s, ~cur, p0, p1, p2, tri);
+    cur = kTracePop;
     float t, u, v;
-    if (intersect_tri(r, p0, p1, p2, tmin, tmax, t, u, v)) {
-      if (ANY) { hit.tri = tri; hit.t = t; hit.u = u; hit.v = v; return true; }
-      if (t < best_t || (t == best_t && tri < best_tri)) {
-        best_t = t; best_tri = tri; hit.u = u; hit.v = v; found = true;
-      }
-    }
-    return false;
-  };
-  if (s.root_is_leaf) {
-    if (test_leaf(0)) return true;
-  } else if (TRN_ONE_LEAF_SITE) {
-    // leaves are visited through the loop like inner nodes, so the triangle
-    // test is instantiated once per traversal (smaller code)
-    int stack[kStackSize];
-    int sp = 0;
-    int cur = 0;
-    for (;;) {
-      if (cur < 0) {
-        if (TRN_LEAF_MAX == 1) {
-          if (test_leaf(~cur)) return true;
-        } else {
-          // leaf: ~(first | (count - 1) << 29), count triangles from first
-          const int v = ~cur;
-          const int first = v & 0x1fffffff, count = (v >> 29) + 1;
-          for (int k = 0; k < count; k++)
-            if (test_leaf(first + k)) return true;
-        }
-        if (sp == 0) break;
-        cur = stack[--sp];
-        continue;
-      }
-      const BvhNode* n = &s.nodes[cur];
-      const float4 a = __ldg(&n->a), b = __ldg(&n->b), c = __ldg(&n->c);
-      const int4 dd = __ldg(&n->d);
-      float tn0, tn1;
-      const bool h0 = slab(r, a.x, a.y, a.z, a.w, b.x, b.y, tmin, best_t, tn0);
-      const bool h1 = slab(r, b.z, b.w, c.x, c.y, c.z, c.w, tmin, best_t, tn1);
-      if (h0 && h1) {
-        int nearc = dd.x, farc = dd.y;
-        if (tn1 < tn0) { nearc = dd.y; farc = dd.x; }
-        if (sp < kStackSize) stack[sp++] = farc;
-        else if (err) atomicExch(err, 1);
-        cur = nearc;
-      } else if (h0) {
-        cur = dd.x;
-      } else if (h1) {
-        cur = dd.y;
-      } else {
-        if (sp == 0) break;
-        cur = stack[--sp];
-      }
-    }
-  } else {
-    int stack[kStackSize];
-    int sp = 0;
-    int cur = 0;
-    for (;;) {
-      const BvhNode* n = &s.nodes[cur];
-      const float4 a = __ldg(&n->a), b = __ldg(&n->b), c = __ldg(&n->c);
-      const int4 dd = __ldg(&n->d);
-      float tn0, tn1;
-      bool h0 = slab(r, a.x, a.y, a.z, a.w, b.x, b.y, tmin, best_t, tn0);
-      bool h1 = slab(r, b.z, b.w, c.x, c.y, c.z, c.w, tmin, best_t, tn1);
-      int c0 = dd.x, c1 = dd.y;
-      if (h0 && c0 < 0) { if (test_leaf(~c0)) return true; h0 = false; }
-      if (h1 && c1 < 0) { if (test_leaf(~c1)) return true; h1 = false; }
-      if (h0 && h1) {
-        int nearc = c0, farc = c1;
-        if (tn1 < tn0) { nearc = c1; farc = c0; }
-        if (sp < kStackSize) stack[sp++] = farc;
-        else if (err) atomicExch(err, 1);
-        cur = nearc;
-      } else if (h0) {
-        cur = c0;
-      } else if (h1) {
-        cur = c1;
-      } else {
-        if (sp == 0) break;
-        cur = stack[--sp];
-      }
+    // best_tri = -1 before the first hit: a hit at exactly the ray's end is none
+    if (intersect_tri(r, p0, p1, p2, tmin, INFINITY, t, u, v) && (t < best_t || (t == best_t && tri < best_tri))) {
+      best_t = t; best_tri = tri; hit.u = u; hit.v = v;
+      if (ANY) break;
     }
   }
-  if (ANY) return false;
-  if (found) { hit.tri = best_tri; hit.t = best_t; }
-  return found;
+  if (best_tri < 0) return false;
+  hit.tri = best_tri; hit.t = best_t;
+  return true;
 }
 
 TRN_D bool occluded(const DeviceScene& s, const F3& o, const F3& d, float tmin, float tmax) {
@@ -341,28 +308,106 @@ TRN_D bool occluded(const DeviceScene& s, const F3& o, const F3& d, float tmin, 
   return trace<true>(s, o, d, tmin, tmax, h);
 }
 
-// One shared, non-inlined copy of the traversal. Kernels with many ray-query
-// sites (the indirect boundary term traces on both sides of the edge, with
-// NEE and importance rays on each) call this one (NI = true): inlined copies
-// would inflate them past the instruction cache. Kernels with few sites keep
-// the inlined form (NI = false), which avoids the call's register traffic.
+// ---- many rays by one warp ---------------------------------------------------
+// Traversal of a stream of rays by a whole warp. A lane whose ray has ended
+// takes the next ray as soon as TRN_REFILL lanes are free, instead of waiting
+// for the warp's longest ray. A ray visits about ten nodes for each triangle
+// it tests, so a lane that meets a leaf puts it aside and goes on with its
+// nodes until it meets a second one; the warp turns to the triangles when
+// TRN_LEAF_SHARE / 4 of its busy lanes have one. Between those decisions lie
+// TRN_NODE_STEPS box steps of straight-line code.
+//
+// Bound by instruction issue and the L1 (62 % each of their peaks, 14 of 32
+// lanes active; one ray per thread left 5 to 8). 2^20 rays against 102,400
+// triangles: closest hit 814 us with one ray per thread, 564 here; occlusion
+// 587 and 502. Of the steps on the way: one step per turn and a vote between
+// nodes and triangles 672, stacks in shared memory 580, four steps a turn 564
+// (six 589); stacks of 8 and 16 shared entries are no better than 12.
+//   fetch(k, lim, more)  warp-uniform: the first of k new rays; rays at or above
+//                        lim are not among them; more: a later fetch has rays
+//   load(i, o, d, tmin, tmax, any)   ray i
+//   store(i, any, tri, u, v, t)      its result (tri < 0: no hit)
+#ifndef TRN_REFILL
+#define TRN_REFILL 8
+#endif
+#ifndef TRN_LEAF_SHARE
+#define TRN_LEAF_SHARE 1
+#endif
+#ifndef TRN_NODE_STEPS
+#define TRN_NODE_STEPS 4
+#endif
+
+template <class Fetch, class Load, class Store>
+TRN_D void trace_stream(const DeviceScene& s, Fetch&& fetch, Load&& load, Store&& store, int* err) {
+  const unsigned lt = (1u << (threadIdx.x & 31)) - 1u;
+  RayPre r;
+  float tmin = 0.f, best_t = 0.f, bu = 0.f, bv = 0.f;
+  // leaf: the leaf put aside (< 0), else 0
+  int best_tri = -1, cur = kTraceDone, leaf = 0, sp = 0;
+  int id = -1;  // -1: no result to store
+  bool any = false, more = s.nt > 0;
+  SharedStack stack;
+  stack.top = shared_stack();
+  for (;;) {
+    const bool free_ = cur == kTraceDone && leaf == 0;
+    const unsigned idle = __ballot_sync(0xffffffffu, free_);
+    if (idle == 0xffffffffu || (more && __popc(idle) >= TRN_REFILL)) {
+      // results are stored when their lanes get new rays: together
+      if (free_ && id >= 0) {
+        store(id, any, best_tri, bu, bv, best_tri < 0 ? -1.f : best_t);
+        id = -1;
+      }
+      if (!more) break;
+      int lim;
+      const int base = fetch(__popc(idle), lim, more);
+      if (free_ && base + __popc(idle & lt) < lim) {
+        id = base + __popc(idle & lt);
+        F3 o, d;
+        load(id, o, d, tmin, best_t, any);
+        best_tri = -1; bu = bv = 0.f;
+        if (!ray_is_void(o, d)) {
+          r = ray_setup(o, d);
+          sp = 0;
+          cur = s.nt == 1 ? ~0 : 0;
+        }
+      }
+      continue;
+    }
+    const float limit = pop_limit(best_t);
+#pragma unroll
+    for (int k = 0; k < TRN_NODE_STEPS; k++) {
+      pop_entry(stack, sp, limit, cur);
+      if (cur < 0 && leaf == 0) {
+        leaf = cur;
+        cur = kTracePop;
+      }
+      if (cur >= 0 && cur < kTracePop) cur = visit_node<true>(s, r, cur, tmin, best_t, stack, sp, err);
+    }
+    const unsigned leaves = __ballot_sync(0xffffffffu, leaf < 0);
+    if (4 * __popc(leaves) < TRN_LEAF_SHARE * (32 - __popc(idle)) &&
+        __any_sync(0xffffffffu, (cur >= 0 && cur != kTraceDone) || (cur < 0 && leaf == 0)))
+      continue;
+    if (leaf < 0) {
+      F3 p0, p1, p2;
+      int tri;
+      leaf_tri<true>(s, ~leaf, p0, p1, p2, tri);
+      leaf = 0;
+      float t, u, v;
+      // best_tri = -1 before the first hit: a hit at exactly the ray's end is none
+      if (intersect_tri(r, p0, p1, p2, tmin, INFINITY, t, u, v) && (t < best_t || (t == best_t && tri < best_tri))) {
+        best_t = t; best_tri = tri; bu = u; bv = v;
+        if (any) cur = kTraceDone;
+      }
+    }
+  }
+}
+
+// One shared, non-inlined copy of the traversal, for fused kernels that trace
+// at several places.
 template <bool ANY>
 __device__ __noinline__ bool trace_shared(const DeviceScene& s, const F3& o, const F3& d, float tmin, float tmax,
                                           Hit& hit, int* err) {
   return trace<ANY>(s, o, d, tmin, tmax, hit, err);
-}
-
-template <bool NI, bool ANY>
-TRN_D bool trace_k(const DeviceScene& s, const F3& o, const F3& d, float tmin, float tmax, Hit& hit,
-                   int* err = nullptr) {
-  if constexpr (NI) return trace_shared<ANY>(s, o, d, tmin, tmax, hit, err);
-  else return trace<ANY>(s, o, d, tmin, tmax, hit, err);
-}
-
-template <bool NI>
-TRN_D bool occluded_k(const DeviceScene& s, const F3& o, const F3& d, float tmin, float tmax) {
-  Hit h;
-  return trace_k<NI, true>(s, o, d, tmin, tmax, h);
 }
 
 }  // namespace trn

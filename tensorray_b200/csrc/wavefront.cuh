@@ -1,0 +1,810 @@
+// Wavefront form of the integrators: paths of one round advance together, one
+// bounce per pair of launches. A shading kernel ends the previous bounce
+// with its ray results and decides the next bounce's rays; k_trace runs all of
+// them. Between them only the rays, their results and 64 bytes of path state
+// pass through memory (an L2's worth at a time).
+//
+// Why: with one thread per path, traversal and shading of 32 unrelated paths
+// shared a warp, with 6 to 8 of 32 lanes active per instruction. Here a
+// traversal warp refills its free lanes with rays of any path (trace_stream),
+// and a shading warp holds 32 paths at the same bounce. 16.8M samples of depth
+// 5 on 102,400 triangles, one thread per path and here, in ms: image 27.6 and
+// 15.8, primary 14.8 and 11.2, direct 2.8 and 2.4, indirect 37.3 and 28.8,
+// pixel 20.6 and 16.0. k_trace takes 65 % of that.
+//
+// The price is a launch pair per bounce, each as long as its longest ray: at
+// 0.5M samples of depth 12 the image is even (1.92 and 1.93 ms) and the
+// boundary terms are behind (direct 0.64 and 0.94, indirect 3.5 and 3.8, pixel
+// 1.6 and 1.9), less than the interior adjoint's records from the same kernels
+// give back (1.1 and 0.4, primary 2.3 and 1.9). One form serves all sizes.
+//
+// Included by render.cu (uses its parameter block and path functions).
+#pragma once
+
+// Buffers of one round of up to `cap` samples.
+struct Wave {
+  long long cap;
+  float4 *ro, *rd;          // [2 cap] rays: origin + id bits, direction + end
+  float4* hit[2];           // [cap] closest-hit results by ray id: tri, u, v, t
+  unsigned char* occ;       // [cap] occlusion results by ray id
+  unsigned* list[2];        // [cap] active samples of a stage, ping-pong
+  unsigned* list2;          // [cap] samples that go on to the emitter side
+  float4* st[4];            // [cap] path state
+  long long* p;             // [cap] view-local sample index (interior term;
+  int* view;                // [cap]  the other terms' items hold theirs)
+  unsigned* rec;            // [cap] record index (recording modes) / sensor depths seen
+  float* W;                 // [cap] weight of the sample's scatter
+  F3* L;                    // [cap] radiance by slot of the round (forward modes)
+  long long first;          // first slot of the round (interior term)
+  float* sc;                // [max depth - 1][cap][3] sensor-side weights (indirect term)
+};
+
+// ray ids: bit 31 marks an occlusion query
+constexpr unsigned kAnyRay = 0x80000000u;
+// list entries: the sample, and which rays its current bounce has cast
+constexpr unsigned kCastShadow = 0x80000000u, kCastCont = 0x40000000u, kEntryMask = 0x3fffffffu;
+
+// One stage: its input list with the count, its output list with the count,
+// and the ray counter. All counts are device counters zeroed with the round.
+struct Stage {
+  const unsigned long long* n;
+  const unsigned* in;
+  unsigned long long* n_out;
+  unsigned* out;
+  unsigned long long* n_ray;
+  unsigned long long* n_state;  // path states handed out (first stage of the camera modes)
+  int b;                    // bounce
+};
+
+// Position of each wanting lane behind `counter` (one atomic per warp; all
+// lanes of the warp call it).
+TRN_D unsigned long long warp_append(unsigned long long* counter, bool want) {
+  const unsigned m = __ballot_sync(0xffffffffu, want);
+  if (!m) return 0;
+  const int lane = threadIdx.x & 31, leader = __ffs(m) - 1;
+  unsigned long long base = 0;
+  if (lane == leader) base = atomicAdd(counter, (unsigned long long)__popc(m));
+  base = __shfl_sync(0xffffffffu, base, leader);
+  return base + __popc(m & ((1u << lane) - 1u));
+}
+
+TRN_D void put_ray(const Wave& W, unsigned long long k, const F3& o, const F3& d, float tmax, unsigned id) {
+  __stcs(W.ro + k, make_float4(o.x, o.y, o.z, __uint_as_float(id)));
+  __stcs(W.rd + k, make_float4(d.x, d.y, d.z, tmax));
+}
+TRN_D void push_ray(const Wave& W, unsigned long long* n_ray, bool want, const F3& o, const F3& d, float tmax,
+                    unsigned id) {
+  const unsigned long long k = warp_append(n_ray, want);
+  if (want) put_ray(W, k, o, d, tmax, id);
+}
+TRN_D Hit get_hit(const float4* h, unsigned long long i) {
+  const float4 a = __ldcs(h + i);
+  Hit r;
+  r.tri = __float_as_int(a.x); r.u = a.y; r.v = a.z; r.t = a.w;
+  return r;
+}
+
+// Warp-uniform loop over [0, n): body(index, exists).
+template <class F>
+TRN_D void for_each_entry(unsigned long long n, F&& body) {
+  const int lane = threadIdx.x & 31;
+  for (unsigned long long k0 = (blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x) & ~31ull; k0 < n;
+       k0 += (unsigned long long)gridDim.x * blockDim.x)
+    body(k0 + lane, k0 + lane < n);
+}
+
+// ---------------------------------------------------------------------------
+// ray queries of a stage: rays [r0, r0 + *n_ray) of the queue
+// ---------------------------------------------------------------------------
+#ifndef TRN_TRACE_MINB
+#define TRN_TRACE_MINB 8
+#endif
+
+// Each warp starts on rays of its own and then fetches from `next`; few rays
+// are spread over all warps (a query is as long as its longest ray, and a warp
+// of few rays takes fewer turns).
+__global__ void __launch_bounds__(TRN_TRACE_BLOCK, TRN_TRACE_MINB)
+    k_trace(const __grid_constant__ DeviceScene s, const __grid_constant__ Wave W, long long r0, const unsigned long long* n_ray,
+            unsigned long long* next, float4* hits, int* err) {
+  stage_begin();
+  const int n = (int)*n_ray;
+  const int warps = gridDim.x * (blockDim.x >> 5);
+  const int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const float4* ro = W.ro + r0;
+  const float4* rd = W.rd + r0;
+  const int own = min(32, max(1, (n + warps - 1) / warps));
+  bool first = true;
+  trace_stream(s,
+    [&](int k, int& lim, bool& more) -> int {
+      if (first) {
+        first = false;
+        lim = min(n, own * (w + 1));
+        more = own * warps < n;
+        return min(n, own * w);
+      }
+      unsigned long long base = 0;
+      if ((threadIdx.x & 31) == 0) base = atomicAdd(next, (unsigned long long)k);
+      lim = n;
+      const int r = (int)min((unsigned long long)n, (unsigned long long)(own * warps) + __shfl_sync(0xffffffffu, base, 0));
+      more = r + k < n;
+      return r;
+    },
+    [&](int i, F3& o, F3& d, float& tmin, float& tmax, bool& any) {
+      const float4 a = __ldcs(ro + i), b = __ldcs(rd + i);
+      o = F3(a.x, a.y, a.z); d = F3(b.x, b.y, b.z);
+      tmin = kShadowEps; tmax = b.w;
+      any = (__float_as_uint(a.w) & kAnyRay) != 0u;
+    },
+    [&](int i, bool any, int tri, float u, float v, float t) {
+      const unsigned id = __float_as_uint(ro[i].w) & ~kAnyRay;
+      if (any) W.occ[id] = tri >= 0;
+      else __stcs(hits + id, make_float4(__int_as_float(tri), u, v, t));
+    }, err);
+}
+
+// ---------------------------------------------------------------------------
+// radiance paths: interior term (image, records, replay), primary / pixel
+// bodies, indirect emitter side
+// ---------------------------------------------------------------------------
+// kWfFwd: forward image; kWfRec: forward image and path records; kWfReplay:
+// path records for the adjoint; kWfBody: detached radiance of a queued primary
+// or pixel sample; kWfEmit: emitter side of a queued indirect sample.
+enum WfMode { kWfFwd = 0, kWfRec, kWfReplay, kWfBody, kWfEmit };
+
+// first sample dimension of bounce b
+template <int MODE>
+TRN_D int wf_dim(const Params& P, int b) {
+  if (MODE == kWfBody) return (P.term == TRN_PIXEL_EDGE ? 1 : 2) + 5 * b;
+  return (MODE == kWfEmit ? 3 : 2) + 5 * b;
+}
+// launch-global slot of a sample, which indexes a caller's sample table
+TRN_D long long wf_gslot(const Params& P, const ViewDesc& V, long long p) {
+  return p + (P.term == TRN_PIXEL_EDGE ? V.begin / 4 : V.begin);
+}
+
+struct WfPath {
+  SurfF x;
+  F3 rdir, T, L;
+};
+
+// Decides the rays of bounce b for the lanes that go on, appends them and the
+// lanes' list entries, and stores the path state. All lanes of the warp call it.
+template <int MODE>
+TRN_D void wf_advance(const Params& P, const Wave& W, const Stage& S, int b, bool go, unsigned i, const ViewDesc* V,
+                      long long p, const WfPath& q, const PathSoA& R, Cnt& cnt) {
+  RadianceGen g;
+  g.shadow = g.cont = false;
+  if (go) {
+    const PathSmp smp{&P, V->seed, wf_gslot(P, *V, p), p + V->slot_off};
+    const int o = wf_dim<MODE>(P, b);
+    BounceRec br;
+    constexpr bool rec = MODE == kWfRec || MODE == kWfReplay;
+    radiance_gen(P.s, q.x, q.rdir, q.T, smp(o), smp(o + 1), smp(o + 2), smp(o + 3), smp(o + 4), g, rec ? &br : nullptr,
+                 cnt);
+    W.st[0][i] = make_float4(__int_as_float(q.x.tri), q.x.u, q.x.v, g.pdf);
+    W.st[1][i] = make_float4(q.rdir.x, q.rdir.y, q.rdir.z, q.T.x);
+    W.st[2][i] = make_float4(q.T.y, q.T.z, q.L.x, q.L.y);
+    W.st[3][i] = make_float4(q.L.z, g.nee.x, g.nee.y, g.nee.z);
+    if (rec && g.shadow) {
+      LRec& l = R.br(W.rec[i], b + 1);
+      l.ltri = br.ltri; l.lu = br.lu; l.lv = br.lv; l.lpdf = br.lpdf; l.lmis = br.lmis;
+    }
+  }
+  const unsigned long long j = warp_append(S.n_out, go);
+  push_ray(W, S.n_ray, g.shadow, q.x.p, g.sdir, g.stmax, (unsigned)j | kAnyRay);
+  push_ray(W, S.n_ray, g.cont, q.x.p, g.wi, kRayMax, (unsigned)j);
+  if (go) S.out[j] = i | (g.shadow ? kCastShadow : 0u) | (g.cont ? kCastCont : 0u);
+}
+
+// Ends the path of sample i.
+template <int MODE>
+TRN_D void wf_finish(const Params& P, const Wave& W, unsigned i, const ViewDesc& V, long long p, const F3& L, Cnt& cnt) {
+  if (MODE == kWfFwd || MODE == kWfRec) {
+    cnt.v[kCntPixel]++;
+    W.L[p + V.begin - W.first] = L;
+  } else if (MODE == kWfBody) {
+    const PrimaryItem& it = reinterpret_cast<const PrimaryItem*>(P.queue)[i];
+    W.W[i] = dot(it.g, L * it.w0);
+  }
+}
+
+// Lists the records of the paths that end here (all lanes of the warp call it).
+template <int MODE>
+TRN_D void wf_record_end(const Wave& W, const PathSoA& R, bool ends, unsigned i) {
+  if constexpr (MODE == kWfRec || MODE == kWfReplay) {
+    const unsigned long long j = warp_append(R.n_end, ends);
+    if (ends) R.order[j] = W.rec[i];
+  }
+}
+
+// Camera rays of the round's n slots. For the adjoint (grad), slots whose pixel
+// has a zero dL/dI are left out (they carry no gradient); for an image, the
+// radiance of slots that end without a path is zero.
+__global__ void __launch_bounds__(256, 4) k_wf_camera(TRN_KPARAMS, const __grid_constant__ Wave W, long long n, bool grad,
+                            unsigned long long* n_out) {
+  stage_begin();
+  Cnt cnt;
+  int vhint = 0;
+  for_each_entry((unsigned long long)n, [&](unsigned long long k, bool in) {
+    F3 org, dir;
+    if (in) {
+      const long long slot = W.first + (long long)k;
+      const ViewDesc& V = view_of(P, slot, vhint);
+      const long long p = slot - V.begin;
+      const int pix = (int)(p % ((long long)V.cam.w * V.cam.h));
+      if (grad) {
+        cnt.v[kCntPixel]++;
+        const F3 g = g_at(P, V, pix);
+        in = !(g.x == 0.f && g.y == 0.f && g.z == 0.f);
+      } else {
+        W.L[k] = F3z();
+      }
+      if (in) {
+        cnt.v[kCntClosest]++;
+        const PathSmp S{&P, V.seed, slot, p + V.slot_off};
+        org = cam_pos(V.cam);
+        dir = camera_ray_dir(V.cam, pix % V.cam.w, pix / V.cam.w, S(0), S(1));
+      }
+    }
+    const unsigned long long j = warp_append(n_out, in);
+    if (in) {
+      put_ray(W, j, org, dir, kRayMax, (unsigned)j);
+      W.list[1][j] = (unsigned)k;
+    }
+  });
+  flush_cnt(cnt, P.stats);
+}
+
+// Adds the round's radiance to the image: one thread per pixel sums its samples
+// of this round in slot order (a view's samples of one pixel lie W * H slots
+// apart). The image does not depend on the order in which paths end.
+__global__ void __launch_bounds__(256) k_wf_pixels(TRN_KPARAMS, const __grid_constant__ Wave W, long long n) {
+  stage_begin();
+  int vhint = 0;
+  const long long end = W.first + n;
+  for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x) {
+    const long long slot = W.first + k;
+    const ViewDesc& V = view_of(P, slot, vhint);
+    const long long WH = (long long)V.cam.w * V.cam.h;
+    // the view's first W * H slots of the round stand for its pixels
+    if (slot - max(W.first, V.begin) >= WH) continue;
+    const long long last = min(end, V.begin + V.n);
+    F3 acc = F3z();
+    for (long long q = slot; q < last; q += WH) acc = acc + W.L[q - W.first] * V.inv_spp;
+    atomic_add3((V.image ? V.image : P.image + 3 * V.pix_off) + 3 * ((slot - V.begin) % WH), acc);
+  }
+}
+
+// First vertex of every path.
+template <int MODE>
+__global__ void __launch_bounds__(256, 3) k_wf_start(TRN_KPARAMS, const __grid_constant__ Wave W, const __grid_constant__ Stage S,
+                           const __grid_constant__ PathSoA R) {
+  stage_begin();
+  Cnt cnt;
+  const DeviceScene& s = P.s;
+  int vhint = 0;
+  for_each_entry(*S.n, [&](unsigned long long k, bool in) {
+    WfPath q;
+    unsigned i = 0;
+    const ViewDesc* V = nullptr;
+    long long p = 0;
+    Hit h;
+    h.tri = -1;
+    int D = 0;
+    if constexpr (MODE <= kWfReplay) {
+      if (in) h = get_hit(W.hit[0], k);
+      in = h.tri >= 0;
+      // a state and, in the recording modes, a record for the path
+      const unsigned long long j = warp_append(S.n_state, in);
+      unsigned long long kr = 0;
+      if (MODE != kWfFwd) {
+        kr = warp_append(P.q_count, in);
+        if (in && kr >= (unsigned long long)P.q_cap) { atomicExch(P.err, 2); in = false; }
+      }
+      if (in) {
+        i = (unsigned)j;
+        const long long slot = W.first + (long long)S.in[k];
+        V = &view_of(P, slot, vhint);
+        p = slot - V->begin;
+        W.p[i] = p;
+        W.view[i] = (int)(V - P.views);
+        D = V->D;
+        const CameraDesc& cam = V->cam;
+        const F3 org = cam_pos(cam);
+        q.x = post_intersect(s, h.tri, h.u, h.v);
+        const float t1 = camera_factor<float>(cam, q.x.p, q.x.ng, 1.f);
+        q.T = F3(t1, t1, t1);
+        q.rdir = normalize(q.x.p - org);
+        const F3 m1 = emitted(s, q.x, -q.rdir);
+        if (MODE == kWfFwd) {
+          q.L = scrub(q.T * m1);
+        } else {
+          W.rec[i] = (unsigned)kr;
+          const F3 m = finite3(q.T * m1) ? m1 : F3z();
+          q.L = q.T * m;
+          R.p(kr) = p; R.view(kr) = (int)(V - P.views);
+          R.g(kr) = MODE == kWfReplay ? g_at(P, *V, (int)(p % ((long long)cam.w * cam.h))) : F3z();
+          R.vr(kr, 1) = {h.tri, h.u, h.v};
+          R.Tk(kr, 1) = q.T;
+          R.Mk(kr, 1) = m;
+          R.K(kr) = 1; R.D(kr) = D; R.nee(kr) = 0u;
+        }
+      }
+    } else if (in) {
+      F3 T0(1.f, 1.f, 1.f);
+      if constexpr (MODE == kWfBody) {
+        i = (unsigned)k;
+        const PrimaryItem& it = reinterpret_cast<const PrimaryItem*>(P.queue)[i];
+        V = P.views + it.view;
+        p = it.p;
+        q.x = post_intersect(s, it.x_tri, it.x_u, it.x_v);
+        q.rdir = it.rdir;
+        T0 = F3(it.T0, it.T0, it.T0);
+        q.L = scrub(T0 * emitted(s, q.x, -q.rdir));
+        D = V->D;
+      } else {
+        i = S.in[k];
+        const IndirectItem& it = reinterpret_cast<const IndirectItem*>(P.queue)[i];
+        V = P.views + it.view;
+        p = it.p();
+        q.x = post_intersect(s, it.xe_tri, it.xe_u, it.xe_v);
+        q.rdir = -it.rdir;
+        q.L = F3z();
+        W.W[i] = 0.f;
+        D = 1;  // queued only when it pairs with a sensor depth
+      }
+      q.T = T0;
+    }
+    const bool go = in && D > 0;
+    if (in && !go) wf_finish<MODE>(P, W, i, *V, p, q.L, cnt);
+    wf_record_end<MODE>(W, R, in && !go, i);
+    wf_advance<MODE>(P, W, S, 0, go, i, V, p, q, R, cnt);
+  });
+  flush_cnt(cnt, P.stats);
+}
+
+// One bounce: ends bounce S.b with its ray results, and decides the rays of the
+// next for the paths that go on. Bound by the gathers of the two vertices
+// (latency) and the state traffic; 32 paths of a warp take the same branches
+// but for material and light.
+template <int MODE>
+__global__ void __launch_bounds__(256, 3) k_wf_shade(TRN_KPARAMS, const __grid_constant__ Wave W, const __grid_constant__ Stage S,
+                           const __grid_constant__ PathSoA R) {
+  stage_begin();
+  Cnt cnt;
+  const DeviceScene& s = P.s;
+  constexpr bool rec = MODE == kWfRec || MODE == kWfReplay;
+  const int b = S.b, k = b + 1;
+  for_each_entry(*S.n, [&](unsigned long long idx, bool in) {
+    WfPath q;
+    unsigned i = 0;
+    const ViewDesc* V = nullptr;
+    long long p = 0;
+    bool go = false;
+    if (in) {
+      const unsigned e = __ldcs(S.in + idx);
+      i = e & kEntryMask;
+      const bool nee_ok = (e & kCastShadow) && !W.occ[idx];
+      Hit h;
+      h.tri = -1;
+      if (e & kCastCont) h = get_hit(W.hit[0], idx);
+      const float4 a = W.st[0][i], c1 = W.st[1][i], c2 = W.st[2][i], c3 = W.st[3][i];
+      if constexpr (MODE <= kWfReplay) {
+        p = W.p[i];
+        V = P.views + W.view[i];
+      } else if constexpr (MODE == kWfBody) {
+        const PrimaryItem& it = reinterpret_cast<const PrimaryItem*>(P.queue)[i];
+        p = it.p;
+        V = P.views + it.view;
+      } else {
+        const IndirectItem& it = reinterpret_cast<const IndirectItem*>(P.queue)[i];
+        p = it.p();
+        V = P.views + it.view;
+      }
+      q.rdir = F3(c1.x, c1.y, c1.z);
+      q.T = F3(c1.w, c2.x, c2.y);
+      q.L = F3(c2.z, c2.w, c3.x);
+      q.x = post_intersect(s, __float_as_int(a.x), a.y, a.z);
+      F3 c;
+      BounceRec br;
+      const bool more = radiance_resolve(s, q.x, q.rdir, q.T, nee_ok, F3(c3.y, c3.z, c3.w), a.w, h, c, rec ? &br : nullptr);
+      q.L = q.L + c;
+      const bool dark = q.T.x == 0.f && q.T.y == 0.f && q.T.z == 0.f;
+      int D = V->D;
+      if constexpr (rec) {
+        const unsigned kr = W.rec[i];
+        // a scrubbed (non-finite) bounce contributes nothing and carries no gradient
+        if (br.nee_ok && !br.scrubbed) R.nee(kr) |= 1u << k;
+        if (more) {
+          R.br(kr, k).ppdf = br.prev_pdf;
+          R.vr(kr, k + 1) = {q.x.tri, q.x.u, q.x.v};
+          R.Tk(kr, k + 1) = q.T;
+          R.Mk(kr, k + 1) = (br.scrubbed || br.emis == 0.f) ? F3z() : br.eLe * br.emis;
+          R.K(kr) = k + 1;
+        }
+      }
+      go = more && !dark;
+      if constexpr (MODE == kWfEmit) {
+        // the radiance accumulated over b + 1 bounces pairs with sensor depth
+        // D - 2 - b (BoundaryIndirect.cpp:158-175); when the path has ended, the
+        // remaining depths pair with its last radiance
+        const float w0 = reinterpret_cast<const IndirectItem*>(P.queue)[i].w0;
+        const unsigned seen = W.rec[i];
+        D = min(D, kMaxDepth);
+        const int jmax = D - 2 - (int)(seen >> 16);
+        float w = W.W[i];
+        go = go && b < jmax;
+        for (int j = b; j <= (go ? b : jmax); j++) {
+          const int d = D - 2 - j;
+          const float* sc = W.sc + 3 * ((long long)d * W.cap + i);
+          const F3 v = (seen >> d) & 1u ? F3(sc[0], sc[1], sc[2]) : F3z();
+          w += dot(v, q.L) * w0;
+        }
+        W.W[i] = w;
+      } else {
+        go = go && b + 1 < D;
+        if (!go) wf_finish<MODE>(P, W, i, *V, p, q.L, cnt);
+      }
+    }
+    wf_record_end<MODE>(W, R, in && !go, i);
+    wf_advance<MODE>(P, W, S, b + 1, go, i, V, p, q, R, cnt);
+  });
+  flush_cnt(cnt, P.stats);
+}
+
+// xDotN scatter of the bodies' samples (all of the queue).
+__global__ void __launch_bounds__(256, 3) k_wf_body_scatter(TRN_KPARAMS, const __grid_constant__ Wave W) {
+  stage_begin();
+  Cnt cnt;
+  const PrimaryItem* q = reinterpret_cast<const PrimaryItem*>(P.queue);
+  const unsigned long long n = min(*P.q_count, (unsigned long long)P.q_cap);
+  for (unsigned long long k = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; k < n;
+       k += (unsigned long long)gridDim.x * blockDim.x) {
+    const float w = W.W[k];
+    if (w == 0.f || !isfinite(w)) continue;
+    const PrimaryItem& it = q[k];
+    const ViewDesc& V = P.views[it.view];
+    xdotn_vjp(P, V, w, cam_pos(V.cam), false, -1, 0.f, 0.f, it.v0, it.v1, it.sedge, it.p0, it.far_tri, it.n, cnt);
+  }
+  flush_cnt(cnt, P.stats);
+}
+
+// Scatter of the indirect samples that reached the emitter side (list2).
+__global__ void __launch_bounds__(256, 3) k_wf_emit_scatter(TRN_KPARAMS, const __grid_constant__ Wave W, const unsigned long long* n_emit) {
+  stage_begin();
+  Cnt cnt;
+  const IndirectItem* q = reinterpret_cast<const IndirectItem*>(P.queue);
+  const unsigned long long n = *n_emit;
+  for (unsigned long long k = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; k < n;
+       k += (unsigned long long)gridDim.x * blockDim.x) {
+    const unsigned i = W.list2[k];
+    const float w = W.W[i];
+    if (w == 0.f || !isfinite(w)) continue;
+    const IndirectItem& it = q[i];
+    const SurfF xs = post_intersect(P.s, it.xs_tri, it.xs_u, it.xs_v);
+    xdotn_vjp(P, P.views[it.view], w, xs.p, true, it.xs_tri, it.xs_u, it.xs_v, it.v0, it.v1, it.sedge, it.p0,
+              it.far_tri, it.n, cnt);
+  }
+  flush_cnt(cnt, P.stats);
+}
+
+// ---------------------------------------------------------------------------
+// importance paths: direct body, indirect sensor side
+// ---------------------------------------------------------------------------
+// State: st[0] = contribution of the current depth and its pixel, st[1] =
+// continuation direction and throughput x, st[2] = throughput y, z.
+TRN_D int wi_depths(const ViewDesc& V, bool sensor) { return sensor ? min(V.D, kMaxDepth) - 1 : V.D; }
+
+template <bool SENSOR>
+TRN_D void wi_advance(const Params& P, const Wave& W, const Stage& S, int b, bool go, unsigned i, const ViewDesc* V,
+                      long long p, const SurfF& x, const F3& rdir, const F3& T, Cnt& cnt) {
+  ImportanceGen g;
+  g.shadow = g.cont = false;
+  F3 cpos;
+  if (go) {
+    const PathSmp smp{&P, V->seed, p + V->begin, p + V->slot_off};
+    const int D = wi_depths(*V, SENSOR);
+    const int o = 3 + 3 * b + (SENSOR ? 5 * D : 0);
+    cpos = cam_pos(V->cam);
+    importance_gen(P.s, V->cam, x, rdir, T, smp(o), smp(o + 1), smp(o + 2), g, cnt);
+    // nothing reads the hit behind the last depth
+    g.cont = g.cont && b + 1 < D;
+    if (g.cont) cnt.v[kCntClosest]++;
+    go = g.shadow || g.cont;
+    if (go) {
+      W.st[0][i] = make_float4(g.c.x, g.c.y, g.c.z, __int_as_float(g.pix));
+      W.st[1][i] = make_float4(g.wi.x, g.wi.y, g.wi.z, g.Tn.x);
+      W.st[2][i] = make_float4(g.Tn.y, g.Tn.z, 0.f, 0.f);
+    }
+  }
+  const unsigned long long j = warp_append(S.n_out, go);
+  push_ray(W, S.n_ray, g.shadow, cpos, g.sdir, g.stmax, (unsigned)j | kAnyRay);
+  push_ray(W, S.n_ray, g.cont, x.p, g.wi, kRayMax, (unsigned)j);
+  if (go) S.out[j] = i | (g.shadow ? kCastShadow : 0u) | (g.cont ? kCastCont : 0u);
+}
+
+template <bool SENSOR>
+__global__ void __launch_bounds__(256, 3) k_wi_start(TRN_KPARAMS, const __grid_constant__ Wave W, const __grid_constant__ Stage S) {
+  stage_begin();
+  Cnt cnt;
+  for_each_entry(min(*P.q_count, (unsigned long long)P.q_cap), [&](unsigned long long k, bool in) {
+    const unsigned i = (unsigned)k;
+    SurfF x;
+    F3 rdir;
+    const ViewDesc* V = nullptr;
+    long long p = 0;
+    bool go = false;
+    if (in) {
+      if constexpr (SENSOR) {
+        const IndirectItem& it = reinterpret_cast<const IndirectItem*>(P.queue)[i];
+        V = P.views + it.view; p = it.p(); rdir = it.rdir;
+        x = post_intersect(P.s, it.xs_tri, it.xs_u, it.xs_v);
+        W.rec[i] = 0u;
+      } else {
+        const DirectItem& it = reinterpret_cast<const DirectItem*>(P.queue)[i];
+        V = P.views + it.view; p = it.p; rdir = it.rdir;
+        x = post_intersect(P.s, it.x_tri, it.x_u, it.x_v);
+      }
+      W.W[i] = 0.f;
+      go = wi_depths(*V, SENSOR) > 0;
+    }
+    wi_advance<SENSOR>(P, W, S, 0, go, i, V, p, x, rdir, F3(1.f, 1.f, 1.f), cnt);
+  });
+  flush_cnt(cnt, P.stats);
+}
+
+// Sensor side: W.rec collects the depths whose weight is kept (bits 0-15);
+// a path that ends with a nonzero weight at some depth goes on to the emitter
+// side, with the shallowest such depth in bits 16 and up (BoundaryIndirect.cpp:
+// 158-175 pairs sensor depth b with the radiance over D - 1 - b bounces).
+template <bool SENSOR>
+__global__ void __launch_bounds__(256, 3) k_wi_step(TRN_KPARAMS, const __grid_constant__ Wave W, const __grid_constant__ Stage S) {
+  stage_begin();
+  Cnt cnt;
+  const int b = S.b;
+  for_each_entry(*S.n, [&](unsigned long long idx, bool in) {
+    unsigned i = 0;
+    SurfF x;
+    F3 rdir, T;
+    const ViewDesc* V = nullptr;
+    long long p = 0;
+    bool go = false;
+    if (in) {
+      const unsigned e = __ldcs(S.in + idx);
+      i = e & kEntryMask;
+      if constexpr (SENSOR) {
+        const IndirectItem& it = reinterpret_cast<const IndirectItem*>(P.queue)[i];
+        V = P.views + it.view; p = it.p();
+      } else {
+        const DirectItem& it = reinterpret_cast<const DirectItem*>(P.queue)[i];
+        V = P.views + it.view; p = it.p;
+      }
+      if ((e & kCastShadow) && !W.occ[idx]) {
+        const float4 a = W.st[0][i];
+        const int pix = __float_as_int(a.w);
+        if (pix >= 0) {
+          const F3 c(a.x, a.y, a.z);
+          if constexpr (SENSOR) {
+            const F3 v = g_at(P, *V, pix) * c;
+            float* sc = W.sc + 3 * ((long long)b * W.cap + i);
+            sc[0] = v.x; sc[1] = v.y; sc[2] = v.z;
+            const unsigned seen = W.rec[i];
+            const bool lit = v.x != 0.f || v.y != 0.f || v.z != 0.f;
+            // bits 16 and up hold 1 + the shallowest lit depth until the path ends
+            W.rec[i] = seen | (1u << b) | (lit && !(seen >> 16) ? (unsigned)(b + 1) << 16 : 0u);
+          } else {
+            W.W[i] += dot(g_at(P, *V, pix), reinterpret_cast<const DirectItem*>(P.queue)[i].ev0 * c);
+          }
+        }
+      }
+      if (e & kCastCont) {
+        const Hit h = get_hit(W.hit[0], idx);
+        if (h.tri >= 0) {
+          const float4 c1 = W.st[1][i], c2 = W.st[2][i];
+          x = post_intersect(P.s, h.tri, h.u, h.v);
+          rdir = F3(c1.x, c1.y, c1.z);
+          T = F3(c1.w, c2.x, c2.y);
+          go = true;  // a continuation is cast only before the last depth
+        }
+      }
+    }
+    wi_advance<SENSOR>(P, W, S, b + 1, go, i, V, p, x, rdir, T, cnt);
+  });
+  flush_cnt(cnt, P.stats);
+}
+
+// Samples whose sensor side reached the image: to list2.
+__global__ void __launch_bounds__(256) k_wi_collect(TRN_KPARAMS, const __grid_constant__ Wave W, unsigned long long* n_emit) {
+  stage_begin();
+  for_each_entry(min(*P.q_count, (unsigned long long)P.q_cap), [&](unsigned long long k, bool in) {
+    unsigned seen = 0;
+    if (in) seen = W.rec[k];
+    const bool lit = (seen >> 16) != 0u;
+    const unsigned long long j = warp_append(n_emit, lit);
+    if (lit) {
+      W.list2[j] = (unsigned)k;
+      W.rec[k] = seen - (1u << 16);
+    }
+  });
+}
+
+__global__ void __launch_bounds__(256, 3) k_wi_direct_scatter(TRN_KPARAMS, const __grid_constant__ Wave W) {
+  stage_begin();
+  Cnt cnt;
+  const DirectItem* q = reinterpret_cast<const DirectItem*>(P.queue);
+  const unsigned long long n = min(*P.q_count, (unsigned long long)P.q_cap);
+  for (unsigned long long k = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; k < n;
+       k += (unsigned long long)gridDim.x * blockDim.x) {
+    const float w = W.W[k];
+    if (w == 0.f || !isfinite(w)) continue;
+    const DirectItem& it = q[k];
+    const SurfF x = post_intersect(P.s, it.x_tri, it.x_u, it.x_v);
+    xdotn_vjp(P, P.views[it.view], w, x.p, true, it.x_tri, it.x_u, it.x_v, it.v0, it.v1, it.sedge, it.p0, it.far_tri,
+              it.n, cnt);
+  }
+  flush_cnt(cnt, P.stats);
+}
+
+// ---------------------------------------------------------------------------
+// boundary set-ups: a ray per sample, a second ray for the samples whose first
+// one hit, and the boundary geometry for those that are left
+// ---------------------------------------------------------------------------
+// First rays of the round's samples in run order (slot_at); list[0][ray id] is
+// the sample's offset in the round.
+template <int TERM>
+__global__ void __launch_bounds__(256, 4) k_setup_rays(TRN_KPARAMS, const __grid_constant__ Wave W, long long first, unsigned long long* n_ray) {
+  stage_begin();
+  Cnt cnt;
+  int vhint = 0;
+  for_each_entry((unsigned long long)(P.total - first), [&](unsigned long long k, bool in) {
+    long long slot = 0;
+    F3 o, d;
+    if (in) {
+      slot = slot_at(P, first + (long long)k);
+      if constexpr (TERM == TRN_PRIMARY_EDGE) {
+        EdgePoint q;
+        in = primary_point(P, slot, q, vhint);
+        if (in) { cnt.v[kCntClosest]++; o = q.p0; d = q.dir; }
+      } else if constexpr (TERM == TRN_DIRECT_EDGE) {
+        DirectPoint q;
+        in = direct_point(P, slot, q, vhint, cnt);
+        if (in) { o = q.e.p0; d = q.e.dir; }
+      } else if constexpr (TERM == TRN_INDIRECT_EDGE) {
+        EdgePoint q;
+        in = indirect_point(P, slot, q, vhint);
+        if (in) { cnt.v[kCntClosest] += 2; o = q.p0; d = -q.dir; }
+      } else {
+        PixelPoint q;
+        pixel_point(P, slot, q, vhint);
+        cnt.v[kCntClosest]++;
+        o = q.p0; d = q.dir;
+      }
+    }
+    const unsigned long long j = warp_append(n_ray, in);
+    if (in) {
+      put_ray(W, j, o, d, kRayMax, (unsigned)j);
+      W.list[0][j] = (unsigned)(slot - first);
+    }
+  });
+  flush_cnt(cnt, P.stats);
+}
+
+// Second rays, behind the first ones in the ray queue; list[1][second ray id]
+// is the first ray's id.
+template <int TERM>
+__global__ void __launch_bounds__(256, 4) k_setup_rays2(TRN_KPARAMS, const __grid_constant__ Wave W, long long first, const unsigned long long* n_ray,
+                              unsigned long long* n_ray2) {
+  stage_begin();
+  Cnt cnt;
+  int vhint = 0;
+  for_each_entry(*n_ray, [&](unsigned long long k, bool in) {
+    F3 o, d;
+    float tmax = kRayMax;
+    if (in) {
+      const Hit h = get_hit(W.hit[0], k);
+      in = h.tri >= 0;
+      if (in) {
+        if constexpr (TERM == TRN_DIRECT_EDGE) {
+          DirectPoint q;
+          Cnt again;  // counted by the first pass
+          direct_point(P, first + W.list[0][k], q, vhint, again);
+          in = direct_lit(q, h.t);
+          o = q.e.p0; d = -q.e.dir;
+        } else {
+          const float4 a = __ldcs(W.ro + k), b = __ldcs(W.rd + k);
+          o = F3(a.x, a.y, a.z); d = F3(b.x, b.y, b.z);
+          if constexpr (TERM == TRN_PRIMARY_EDGE) {
+            const CameraDesc& cam = view_of(P, first + W.list[0][k], vhint).cam;
+            SensorSample sds;
+            F3 dirc;
+            in = primary_sensor(cam, o, d, h.t, sds, dirc, tmax);
+            o = cam_pos(cam); d = dirc;
+            if (in) cnt.v[kCntShadow]++;
+          } else {
+            d = -d;
+          }
+        }
+      }
+    }
+    const unsigned long long j = warp_append(n_ray2, in);
+    if (in) {
+      put_ray(W, (unsigned long long)W.cap + j, o, d, tmax, (unsigned)j | (TERM == TRN_PRIMARY_EDGE ? kAnyRay : 0u));
+      W.list[1][j] = (unsigned)k;
+    }
+  });
+  flush_cnt(cnt, P.stats);
+}
+
+// Boundary geometry of the samples whose rays allow one, queued as the term's
+// items. n: the rays of the last query (the pixel term has only one).
+template <int TERM>
+__global__ void __launch_bounds__(256, 3) k_setup_finish(TRN_KPARAMS, const __grid_constant__ Wave W, long long first, const unsigned long long* n) {
+  stage_begin();
+  int vhint = 0;
+  for_each_entry(*n, [&](unsigned long long k2, bool in) {
+    EdgeState st;
+    if (in) {
+      const unsigned long long k = TERM == TRN_PIXEL_EDGE ? k2 : W.list[1][k2];
+      if constexpr (TERM == TRN_PRIMARY_EDGE) in = !W.occ[k2];
+      Hit h2;
+      if constexpr (TERM == TRN_DIRECT_EDGE || TERM == TRN_INDIRECT_EDGE) {
+        h2 = get_hit(W.hit[1], k2);
+        in = h2.tri >= 0;
+      }
+      if (in) {
+        const Hit h = get_hit(W.hit[0], k);
+        in = h.tri >= 0;
+        const long long slot = first + W.list[0][k];
+        if (in) {
+          if constexpr (TERM == TRN_PRIMARY_EDGE) {
+            EdgePoint q;
+            primary_point(P, slot, q, vhint);
+            SensorSample sds;
+            F3 dirc;
+            float tmax;
+            primary_sensor(q.V->cam, q.p0, q.dir, h.t, sds, dirc, tmax);
+            in = primary_finish(P, slot, q, h, sds, dirc, st);
+          } else if constexpr (TERM == TRN_DIRECT_EDGE) {
+            DirectPoint q;
+            Cnt again;
+            direct_point(P, slot, q, vhint, again);
+            in = direct_finish(P, slot, q, h, h2, st);
+          } else if constexpr (TERM == TRN_INDIRECT_EDGE) {
+            EdgePoint q;
+            indirect_point(P, slot, q, vhint);
+            in = indirect_finish(P, slot, q, h, h2, st);
+          } else {
+            PixelPoint q;
+            pixel_point(P, slot, q, vhint);
+            in = pixel_finish(P, q, h, st);
+          }
+        }
+      }
+    }
+    const unsigned long long j = warp_append(P.q_count, in);
+    if (in && j >= (unsigned long long)P.q_cap) { atomicExch(P.err, 2); in = false; }
+    if (!in) return;
+    if constexpr (TERM == TRN_DIRECT_EDGE) {
+      DirectItem& it = reinterpret_cast<DirectItem*>(P.queue)[j];
+      it.p = st.p; it.view = (int)(st.V - P.views);
+      it.x_tri = st.x.tri; it.x_u = st.x.u; it.x_v = st.x.v; it.v0 = st.v0; it.v1 = st.v1; it.far_tri = st.far_tri;
+      it.sedge = st.sedge; it.rdir = st.rdir; it.ev0 = st.T0 * st.w0; it.p0 = st.p0; it.n = st.n;
+    } else if constexpr (TERM == TRN_INDIRECT_EDGE) {
+      IndirectItem& it = reinterpret_cast<IndirectItem*>(P.queue)[j];
+      it.p_lo = (unsigned)st.p; it.p_hi = (int)(st.p >> 32); it.view = (int)(st.V - P.views);
+      it.xe_tri = st.xe.tri; it.xe_u = st.xe.u; it.xe_v = st.xe.v;
+      it.xs_tri = st.x.tri; it.xs_u = st.x.u; it.xs_v = st.x.v;
+      it.v0 = st.v0; it.v1 = st.v1; it.far_tri = st.far_tri; it.w0 = st.w0; it.sedge = st.sedge;
+      it.rdir = st.rdir; it.p0 = st.p0; it.n = st.n;
+    } else {
+      constexpr bool pixel = TERM == TRN_PIXEL_EDGE;
+      PrimaryItem& it = reinterpret_cast<PrimaryItem*>(P.queue)[j];
+      it.p = st.p; it.view = (int)(st.V - P.views);
+      it.x_tri = st.x.tri; it.x_u = st.x.u; it.x_v = st.x.v; it.T0 = st.T0.x; it.w0 = st.w0;
+      it.sedge = pixel ? 0.f : st.sedge;
+      it.v0 = pixel ? -1 : st.v0; it.v1 = pixel ? -1 : st.v1;  // a pixel-edge point is no scene parameter
+      it.far_tri = st.far_tri;
+      it.rdir = st.rdir; it.p0 = st.p0; it.n = st.n; it.g = st.g;
+    }
+  });
+}

@@ -4,7 +4,7 @@ The reference optimises scene parameters from Python: per view it calls
 RenderFunction (forward renderC, backward renderD of every integrator,
 pyTensorRay/renderer_multi_view.py:40-98), reads the gradients through the
 parameter manager (pyTensorRay/parameter_manager.py:36-101) and steps a torch
-optimiser. Here one step is: new vertex positions -> geometry chain + LBVH
+optimiser. Here one step is: new vertex positions -> geometry chain + BVH
 refit (Scene::Update, Scene.cpp:535-546) -> one batched forward launch over
 all views -> per-view loss and dL/dI in one launch -> one batched adjoint
 launch per integrator -> geometry adjoint -> Adam on the device. Nothing

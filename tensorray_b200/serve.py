@@ -38,11 +38,10 @@ PHASE_FWD, PHASE_GRAD, PHASE_FINISH, PHASE_DONE = 0, 1, 2, 3
 # interior path tracer and the four boundary terms
 ALL_TERMS = (TRN_PATH_TRACER, TRN_PRIMARY_EDGE, TRN_DIRECT_EDGE, TRN_INDIRECT_EDGE, TRN_PIXEL_EDGE)
 
-# Device bytes a gradient view set holds for the queues of the split
-# integrator kernels (one round: 16M boundary samples, at most about 312 bytes
-# each at depth <= 8) and for the boundary set-up's run order (16 bytes per
-# slot plus the sort's temporary storage). Forward view sets hold none.
-VIEWSET_QUEUE_BYTES = 5_600_000_000
+# Device bytes a view set holds for the wavefront's round buffers (one round: 16M
+# samples, at most 341 bytes each at depth <= 8) and for the boundary set-up's
+# run order (16 bytes per slot plus the sort's temporary storage).
+VIEWSET_QUEUE_BYTES = 6_000_000_000
 
 
 @dataclass
@@ -88,10 +87,10 @@ class Server:
     def __init__(self, scenes: dict, hbm_budget_bytes: float = 120e9, chunk_spp: int = 8, max_active: int = 256,
                  clock=time.perf_counter, iter_samples: int = 1 << 25, max_depth: int = 8):
         self.scenes = scenes
-        # gradient view sets reserve their round buffers for this depth when
+        # view sets reserve their round buffers for this depth when
         # created (deeper requests still run; their first batch grows them)
         self.max_depth = int(max_depth)
-        # the gradient view set of every scene holds one round of queues
+        # the view set of every scene holds one round of buffers
         self.reserve = len(scenes) * VIEWSET_QUEUE_BYTES
         self.budget = int(hbm_budget_bytes) - self.reserve
         self.chunk_spp = chunk_spp
@@ -248,14 +247,16 @@ class Server:
                              C.c_void_p(r.dLdI.data_ptr()) if grad else None)
         return arr, spps
 
-    def _viewset(self, name: str, phase: int, reqs: list, arr, spps):
-        key = (name, phase)
+    def _viewset(self, name: str, group: int, reqs: list, arr, spps):
+        """The scene's view set for this group of requests. The forward chunks
+        run on the first gradient group's set, whose round buffers they share
+        (one stream per scene orders them)."""
+        key = (name, group)
         cams = [r.camera for r in reqs]
         vs = self.vsets.get(key)
         if vs is None:
             vs = api.ViewSet(self.scenes[name], cams, spps, views=arr)
-            if phase != PHASE_FWD:
-                vs.reserve(self.max_depth)
+            vs.reserve(self.max_depth)
             self.vsets[key] = vs
         else:
             vs.update(cams, spps, arr)
@@ -265,7 +266,7 @@ class Server:
         if not reqs:
             return
         arr, spps = self._views(reqs, grad=False)
-        vs = self._viewset(name, PHASE_FWD, reqs, arr, spps)
+        vs = self._viewset(name, 0, reqs, arr, spps)
         vs.render(TRN_PATH_TRACER, api.RenderOptions(0, 0, 0, 0, 0, 0, 0), out=False)
         for r in reqs:
             r.chunk += 1
@@ -283,7 +284,7 @@ class Server:
             groups.setdefault(tuple(r.terms), []).append(r)
         for gi, (terms, grp) in enumerate(sorted(groups.items())):
             arr, spps = self._views(grp, grad=True)
-            vs = self._viewset(name, (PHASE_GRAD, gi), grp, arr, spps)
+            vs = self._viewset(name, gi, grp, arr, spps)
             for t in terms:
                 vs.render_grad(t, api.RenderOptions(0, 0, 0, 0, 0, 0, 0), None)
         for r in reqs:

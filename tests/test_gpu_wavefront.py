@@ -1,0 +1,88 @@
+"""The wavefront's own edges: rounds, stream capture and growth of its buffers,
+paths without a bounce, views that end inside a round."""
+import pytest
+import torch
+
+from tensorray_b200 import api, scenes
+from tests.helpers import rel_l2
+
+pytestmark = pytest.mark.gpu
+
+TERMS = (api.TRN_PATH_TRACER, api.TRN_PRIMARY_EDGE, api.TRN_DIRECT_EDGE, api.TRN_INDIRECT_EDGE, api.TRN_PIXEL_EDGE)
+
+
+def _scene(w=40, h=28):
+    sc = api.Scene(scenes.config1_scene(w, h))
+    sc.configure()
+    return sc
+
+
+def _views(sc, n=3, spp=(8, 21, 4)):
+    cams = [api.Camera(c.pos, c.target, c.up, c.width, c.height, c.fov)
+            for c in scenes.fibonacci_cameras(n, 4.0, [48], seed=2)]
+    cams[1] = api.Camera(cams[1].pos, (0.0, 0.0, 0.0), (0.0, 1.0, 0.0), 60, 33, 45.0)
+    return api.ViewSet(sc, cams, list(spp[:n]))
+
+
+def test_image_does_not_depend_on_rounds_or_runs(built_lib):
+    """Samples of a pixel are summed in slot order within a round, so an image
+    repeats bit for bit; rounds only regroup the sum."""
+    sc = _scene(128, 96)
+    o = api.RenderOptions(5, 4, 40, 0, 0, 0, 0)
+    a = api.PathTracer().renderC(sc, o).clone()
+    assert torch.equal(a, api.PathTracer().renderC(sc, o))
+    vs = _views(sc, 3, (64, 70, 50))
+    opts = api.RenderOptions(5, 4, 0, 0, 0, 0, 0)
+    ref = vs.render(api.TRN_PATH_TRACER, opts).clone()
+    for cache in (0, 1 << 30):
+        vs.set_path_cache(cache)
+        img = vs.render(api.TRN_PATH_TRACER, opts, launch=api.launch_config(round_log2=16))
+        # up to 70 additions of 32-bit values in another grouping
+        torch.testing.assert_close(img, ref, rtol=70 * 2 ** -24, atol=1e-7)
+
+
+@pytest.mark.parametrize("depth", [0, 1, 2, 9, 16])
+def test_view_set_equals_single_views(built_lib, depth):
+    """All terms of a view set, in rounds that end inside views, against one
+    view at a time in one round."""
+    sc = _scene()
+    vs = _views(sc)
+    opts = api.RenderOptions(3, depth, 0, 0, 0, 0, 0)
+    d = torch.rand(vs.npix, 3, device=sc.device) - 0.3
+    small = api.launch_config(round_log2=16)
+    for term in TERMS:
+        vs.render_grad(term, opts, d, launch=small)
+        g = sc.get_grads()["positions"]
+        for i, (c, s) in enumerate(zip(vs.cameras, vs.spps)):
+            one = api.ViewSet(sc, [c], [s], seeds=[i])
+            one.render_grad(term, opts, d[vs.offsets[i]:vs.offsets[i] + c.width * c.height])
+        ref = sc.get_grads()["positions"]
+        assert rel_l2(g, ref) <= 1e-5 if float(ref.abs().sum()) > 0 else float(g.abs().sum()) == 0
+
+
+def test_capture_without_buffers_and_replay_after_growth(built_lib):
+    """A forward render captured before any buffers exist runs one thread per
+    path; one captured with buffers still replays after the set's buffers grew."""
+    sc = _scene()
+    opts = api.RenderOptions(3, 3, 0, 0, 0, 0, 0)
+    vs, bare = _views(sc), _views(sc)
+    out = torch.empty(vs.npix, 3, device=sc.device)
+    ref = vs.render(api.TRN_PATH_TRACER, opts).clone()   # vs has its round buffers now
+    bare.render(api.TRN_PRIMARY_EDGE, opts)              # uploads the view table, allocates none
+    graphs = []
+    for v in (bare, vs):
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            v.render(api.TRN_PATH_TRACER, opts, out=out)
+        graphs.append(g)
+    for g in graphs:
+        out.zero_()
+        g.replay()
+        torch.testing.assert_close(out, ref, rtol=1e-5, atol=1e-6)
+    vs.reserve(8)  # the buffers that the second graph holds grow
+    d = torch.rand(vs.npix, 3, device=sc.device) - 0.3
+    for term in TERMS:
+        vs.render_grad(term, opts, d)
+    out.zero_()
+    graphs[1].replay()
+    torch.testing.assert_close(out, ref, rtol=1e-5, atol=1e-6)
