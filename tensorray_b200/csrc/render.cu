@@ -2837,6 +2837,39 @@ int path_wave(trn_viewset* vs, const Params& P0, const trn_launch* ln, long long
   return 0;
 }
 
+// |baseVal| of the guiding tree's samples, in rounds of whole leaves: to value
+// (EVAL: tree.per per leaf) or as leaf means to poly. Returns 1 when there are
+// no buffers for it (ensure_queue).
+template <bool EVAL>
+int guide_wave(trn_viewset* vs, const Params& P, const trn_launch* ln, const GuideTree& tree, long long limit,
+               float* value, float* poly, cudaStream_t st) {
+  const long long leaves = std::min(limit, std::max(1LL, round_cap(ln, kRound) / tree.per));
+  const long long cap = leaves * tree.per;
+  WaveRun r = wave_run(vs, P, ln, cap, st);
+  void* items;
+  const int rc = ensure_queue(vs, wave_layout(r.W, &items, nullptr, cap, TRN_DIRECT_EDGE, vs->max_depth),
+                              full_queue_bytes(vs->max_depth <= 8), st);
+  if (rc) return rc;
+  wave_layout(r.W, &items, vs->iq, cap, TRN_DIRECT_EDGE, vs->max_depth);
+  for (long long leaf = 0; leaf < limit; leaf += leaves) {
+    const long long nl = std::min(leaves, limit - leaf), n = nl * tree.per, first = leaf * tree.per;
+    float* v = EVAL ? value + first : r.W.W;
+    if (r.begin()) return -1;
+    unsigned long long *a = r.ctr(), *b = r.ctr();
+    r.go<k_guide_rays<EVAL>>(r.P, r.W, tree, first, n, v, a);
+    r.trace(0, a, 0);
+    r.go<k_guide_rays2<EVAL>>(r.P, r.W, tree, first, a, b);
+    r.trace(r.W.cap, b, 1);
+    r.go<k_guide_values<EVAL>>(r.P, r.W, tree, first, b, v);
+    if (!EVAL) {
+      k_guide_mean<<<(unsigned)((nl + 255) / 256), 256, 0, st>>>(tree.count, tree.per, leaf, nl, v, poly);
+      count_launch(1);
+    }
+  }
+  TRN_CUDA_TRY(cudaGetLastError());
+  return 0;
+}
+
 // AdaptiveQuadratureDistribution::setup (AQ_distrb.h:83-173) for one
 // direct-boundary call: the depth-0 tree, g_direct_depth refinement passes
 // (the loop the reference keeps commented out, AQ_distrb.h:121-136, with
@@ -2846,7 +2879,11 @@ int path_wave(trn_viewset* vs, const Params& P0, const trn_launch* ln, long long
 // from the counter hash (their own terms), also when the call's samples come
 // from a table. The allocation-free entry point refuses a refinement that would
 // need larger arrays than the scene holds.
-int guide_setup(trn_scene* s, const trn_render_options* o, Params& P, cudaStream_t st, bool may_alloc = true) {
+// With a view set (vs), the samples' ray queries run as a wavefront in its
+// round buffers; without one (allocation-free), or without room for them, each
+// thread traces its own.
+int guide_setup(trn_scene* s, trn_viewset* vs, const trn_render_options* o, const trn_launch* ln, Params& P,
+                cudaStream_t st) {
   if (!o->g_direct || s->ne == 0) return 0;
   if (o->g_direct_spp <= 0) { set_error("g_direct_spp must be positive when g_direct is set"); return -1; }
   if (!(o->g_eps >= 0.f && o->g_eps <= 1.f)) { set_error("g_eps must be in [0, 1]"); return -1; }
@@ -2860,7 +2897,7 @@ int guide_setup(trn_scene* s, const trn_render_options* o, Params& P, cudaStream
   }
   if (depth > 0) {
     if (!(o->g_direct_thold >= 0.f)) { set_error("g_direct_thold must be >= 0"); return -1; }
-    if ((limit > s->aq_cap || !s->aq_eval) && !may_alloc) {
+    if ((limit > s->aq_cap || !s->aq_eval) && !vs) {
       set_error("refining the guiding tree (g_direct_depth > 0) allocates its arrays on first use; call "
                 "trn_render_grad once with the same options first");
       return -1;
@@ -2876,8 +2913,12 @@ int guide_setup(trn_scene* s, const trn_render_options* o, Params& P, cudaStream
   int launches = 1;
   for (int pass = 0; pass < depth; pass++) {
     const uint32_t ps = stream + (uint32_t)pass;
-    k_aq_eval<<<(unsigned)((limit * kAqPoints + 255) / 256), 256, 0, st>>>(G, ps, s->aq_box, s->aq_edge, s->aq_count,
-                                                                           cap, s->aq_eval);
+    const GuideTree tree{s->aq_box, s->aq_edge, s->aq_count, cap, ps, kAqPoints};
+    const int rc = vs ? guide_wave<true>(vs, G, ln, tree, limit, s->aq_eval, nullptr, st) : 1;
+    if (rc < 0) return -1;
+    if (rc)
+      k_aq_eval<<<(unsigned)((limit * kAqPoints + 255) / 256), 256, 0, st>>>(G, ps, s->aq_box, s->aq_edge, s->aq_count,
+                                                                             cap, s->aq_eval);
     k_aq_flag<<<(unsigned)((limit + 255) / 256), 256, 0, st>>>(s->aq_box, s->aq_count, cap, s->aq_eval,
                                                                o->g_direct_thold, ps, s->aq_flag);
     k_aq_scan<<<1, 1024, 0, st>>>(s->aq_count, s->aq_flag, s->aq_prefix, s->aq_count, (int)limit);
@@ -2886,8 +2927,12 @@ int guide_setup(trn_scene* s, const trn_render_options* o, Params& P, cudaStream
     k_aq_commit<<<1, 1, 0, st>>>(s->aq_count);
     launches += 5;
   }
-  k_aq_poly<<<(unsigned)((limit + 255) / 256), 256, 0, st>>>(G, stream, o->g_direct_spp, s->aq_box, s->aq_edge,
-                                                              s->aq_count, cap, s->aq_poly);
+  const GuideTree tree{s->aq_box, s->aq_edge, s->aq_count, cap, stream, o->g_direct_spp};
+  const int rc = vs ? guide_wave<false>(vs, G, ln, tree, limit, nullptr, s->aq_poly, st) : 1;
+  if (rc < 0) return -1;
+  if (rc)
+    k_aq_poly<<<(unsigned)((limit + 255) / 256), 256, 0, st>>>(G, stream, o->g_direct_spp, s->aq_box, s->aq_edge,
+                                                                s->aq_count, cap, s->aq_poly);
   k_aq_mix<<<1, 1024, 0, st>>>(s->aq_count, s->aq_poly, s->aq_box, cap, o->g_eps, s->aq_func, s->aq_int);
   count_launch(launches + 2 +
                cdf_launch(1, (int)limit, s->aq_count, s->aq_func, s->aq_cdf, s->aq_int, s->cdf_part, st));
@@ -3144,7 +3189,7 @@ int render_views(trn_scene* s, trn_viewset* vs, const trn_render_options* o, int
   } else if ((integrator == TRN_DIRECT_EDGE || integrator == TRN_INDIRECT_EDGE) && s->ne == 0) {
     return 0;
   }
-  if (integrator == TRN_DIRECT_EDGE && guide_setup(s, o, P, st)) return -1;
+  if (integrator == TRN_DIRECT_EDGE && guide_setup(s, vs, o, ln, P, st)) return -1;
   TRN_CUDA_TRY(cudaMemsetAsync(vs->work, 0, sizeof(unsigned long long), st));
   switch (integrator) {
     case TRN_PATH_TRACER: {
@@ -3527,7 +3572,7 @@ int trn_render_grad_noalloc(trn_scene* s, const trn_camera* cam, const trn_rende
   }
   // the guiding distribution lives in buffers the scene allocated at creation
   // (a refined tree in those of an earlier allocating call)
-  if (integrator == TRN_DIRECT_EDGE && guide_setup(s, o, P, st, false)) return -1;
+  if (integrator == TRN_DIRECT_EDGE && guide_setup(s, nullptr, o, nullptr, P, st)) return -1;
   const bool shallow = o->max_bounces <= 8;
   switch (integrator) {
     case TRN_PATH_TRACER:

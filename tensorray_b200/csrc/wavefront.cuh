@@ -808,3 +808,104 @@ __global__ void __launch_bounds__(256, 3) k_setup_finish(TRN_KPARAMS, const __gr
     }
   });
 }
+
+// ---------------------------------------------------------------------------
+// guiding samples of the direct boundary term: |baseVal| of `per` samples in
+// each leaf of the guiding tree (guide_base_val, one ray query per launch).
+// One thread per leaf traced all of its samples' rays one after the other, with
+// a few thousand threads in all: an inverse-rendering step of three views with
+// guiding took 43 ms and takes 19 with a slot per sample.
+// ---------------------------------------------------------------------------
+struct GuideTree {
+  const float* box;       // [6][cap]
+  const int* edge;
+  const int* count;       // leaves
+  long long cap;
+  uint32_t stream;
+  int per;                // samples per leaf
+};
+
+// Sample point of (leaf, k): uniform in the leaf's box, or (EVAL) the
+// refinement's evaluation point.
+template <bool EVAL>
+TRN_D bool guide_sample(const Params& P, const GuideTree& g, long long t, DirectPoint& q) {
+  const int leaf = (int)(t / g.per), k = (int)(t % g.per);
+  if (leaf >= __ldg(g.count) || !(P.efunc[g.edge[leaf]] > 0.f) || !(__ldg(P.eint) > 0.f)) return false;
+  float x[3];
+  if (EVAL) {
+    aq_point(g.box, g.cap, leaf, k, g.stream, x);
+  } else {
+    for (int a = 0; a < 3; a++)
+      x[a] = aq_lerp(g.box, g.cap, leaf, a, hash_uniform(g.stream, kGuideTerm, (uint32_t)a, (uint32_t)t));
+  }
+  return guide_point(P, x[0], x[1], x[2], q);
+}
+
+// Rays from the edge points to the light points of samples [first, first + n);
+// value[] of the round starts at 0.
+template <bool EVAL>
+__global__ void __launch_bounds__(256, 4) k_guide_rays(TRN_KPARAMS, const __grid_constant__ Wave W, const __grid_constant__ GuideTree g,
+                             long long first, long long n, float* value, unsigned long long* n_ray) {
+  stage_begin();
+  for_each_entry((unsigned long long)n, [&](unsigned long long k, bool in) {
+    DirectPoint q;
+    if (in) {
+      value[k] = 0.f;
+      in = guide_sample<EVAL>(P, g, first + (long long)k, q);
+    }
+    const unsigned long long j = warp_append(n_ray, in);
+    if (in) {
+      put_ray(W, j, q.e.p0, q.e.dir, kRayMax, (unsigned)j);
+      W.list[0][j] = (unsigned)k;
+    }
+  });
+}
+
+// Rays away from the light, for the samples whose first ray met the light point.
+template <bool EVAL>
+__global__ void __launch_bounds__(256, 4) k_guide_rays2(TRN_KPARAMS, const __grid_constant__ Wave W, const __grid_constant__ GuideTree g,
+                              long long first, const unsigned long long* n_ray, unsigned long long* n_ray2) {
+  stage_begin();
+  for_each_entry(*n_ray, [&](unsigned long long k, bool in) {
+    DirectPoint q;
+    if (in) {
+      const Hit h = get_hit(W.hit[0], k);
+      in = h.tri >= 0;
+      if (in) {
+        guide_sample<EVAL>(P, g, first + W.list[0][k], q);
+        in = direct_lit(q, h.t);
+      }
+    }
+    const unsigned long long j = warp_append(n_ray2, in);
+    if (in) {
+      put_ray(W, (unsigned long long)W.cap + j, q.e.p0, -q.e.dir, kRayMax, (unsigned)j);
+      W.list[1][j] = W.list[0][k];
+    }
+  });
+}
+
+template <bool EVAL>
+__global__ void __launch_bounds__(256, 4) k_guide_values(TRN_KPARAMS, const __grid_constant__ Wave W, const __grid_constant__ GuideTree g,
+                               long long first, const unsigned long long* n_ray2, float* value) {
+  stage_begin();
+  const unsigned long long n = *n_ray2;
+  for (unsigned long long j = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; j < n;
+       j += (unsigned long long)gridDim.x * blockDim.x) {
+    const Hit h = get_hit(W.hit[1], j);
+    if (h.tri < 0) continue;
+    DirectPoint q;
+    guide_sample<EVAL>(P, g, first + W.list[1][j], q);
+    value[W.list[1][j]] = guide_value(P, q, h);
+  }
+}
+
+// Leaf weights of the round's leaves: the mean of their values, added in order.
+__global__ void k_guide_mean(const int* count, int per, long long leaf0, long long n_leaf, const float* value, float* poly) {
+  stage_begin();
+  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (i >= n_leaf || leaf0 + i >= __ldg(count)) return;
+  const float fs = (float)per;
+  float acc = 0.f;
+  for (int k = 0; k < per; k++) acc = __fadd_rn(acc, __fdiv_rn(value[i * per + k], fs));
+  poly[leaf0 + i] = acc;
+}
