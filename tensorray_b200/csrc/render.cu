@@ -1099,20 +1099,17 @@ struct PathRef {
 // Reverse sweep over the records, in the order in which their paths ended: the
 // paths of one bounce ended together, so a warp's sweeps have the same length
 // (in slot order a warp ran as long as its longest path, with less than a third
-// of its lanes active: 1.00 ms for 1M paths on 1,284 triangles, 0.60 in this
-// order). Above kEndOrder records the sweep goes in slot order (16.8M paths:
-// 23.5 ms; 12.0 in ending order). The order matters to the sums: the ground's few
-// vertices get an add from almost every path, in 32 bits, and small ones are
-// lost in a large sum. Which ones depends on the order, and at 16.8M paths single
-// components of the gradient then move by 0.7 % of its RMS (at 1M paths by 2e-5).
-// Bound by instruction fetch: the sweep is one long body of inlined scatters, and
-// the few warps that fit its registers do not hide the misses. (Its six scatters
-// in a loop, or one shared function, take 5 to 10 times as long: lanes then enter
-// them one group at a time.)
+// of its lanes active: 23.5 ms for 16.8M paths of depth 5, 12.0 in this order).
+// The order matters to the sums: a few vertices get millions of 32-bit adds, and
+// small ones are lost in a large sum. Shortest paths first stays nearest to the
+// sums in slot order (5e-5 of the positions' gradient; longest first 1.5e-4). Bound by instruction fetch:
+// the sweep is one long body of inlined scatters, and the few warps that fit
+// its registers do not hide the misses. (Its six scatters in a loop, or one
+// shared function, take 5 to 10 times as long: lanes then enter them one group
+// at a time.)
 // CACHED: the records come from the recording forward render and carry no
 // dL/dI yet; each path reads its pixel's now and is skipped when that is zero,
 // as the replaying form skips it.
-constexpr unsigned long long kEndOrder = 1ull << 22;
 template <bool CACHED>
 __global__ void __launch_bounds__(256, TRN_MINB_REVERSE) k_path_reverse(TRN_KPARAMS, const __grid_constant__ PathSoA R) {
   stage_begin();
@@ -1120,7 +1117,7 @@ __global__ void __launch_bounds__(256, TRN_MINB_REVERSE) k_path_reverse(TRN_KPAR
   const unsigned long long n = *R.n_end;
   for (unsigned long long k = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; k < n;
        k += (unsigned long long)gridDim.x * blockDim.x) {
-    const long long i = n <= kEndOrder ? (long long)__ldcs(R.order + k) : (long long)k;
+    const long long i = (long long)__ldcs(R.order + k);
     const int view = R.view(i);
     F3 g;
     if (CACHED) {
@@ -2264,10 +2261,6 @@ __global__ void k_view_loss(long long npix, const ViewDesc* views, const long lo
 // rays are spread over all warps of the GPU as well, down to one each, since a
 // query is then as long as its longest ray (1,000 rays on 7,000 triangles: 56 us
 // with four per warp, 46 with one).
-// Against one ray per thread (the traversal before), on 102,400 triangles, closest
-// hit: 1,000 rays 123 -> 83 us, 4,099 111 -> 93, 2^20 1.44x as fast. In between
-// one slow ray decides, and a box step takes a lone ray a fifth longer here:
-// 32,000 rays 206 -> 250 us, 300,000 340 -> 323.
 template <bool ANY>
 __global__ void __launch_bounds__(TRN_TRACE_BLOCK, TRN_TRACE_MINB)
     k_query(const __grid_constant__ DeviceScene s, int n, int chunk, const float* org, const float* dir,
