@@ -2261,6 +2261,10 @@ __global__ void k_view_loss(long long npix, const ViewDesc* views, const long lo
 // rays are spread over all warps of the GPU as well, down to one each, since a
 // query is then as long as its longest ray (1,000 rays on 7,000 triangles: 56 us
 // with four per warp, 46 with one).
+// Against one ray per thread (the traversal before), on 102,400 triangles, closest
+// hit: 1,000 rays 123 -> 83 us, 4,099 111 -> 93, 2^20 1.44x as fast. In between
+// one slow ray decides, and a box step takes a lone ray a fifth longer here:
+// 32,000 rays 206 -> 250 us, 300,000 340 -> 323.
 template <bool ANY>
 __global__ void __launch_bounds__(TRN_TRACE_BLOCK, TRN_TRACE_MINB)
     k_query(const __grid_constant__ DeviceScene s, int n, int chunk, const float* org, const float* dir,

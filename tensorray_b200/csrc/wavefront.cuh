@@ -813,8 +813,8 @@ __global__ void __launch_bounds__(256, 3) k_setup_finish(TRN_KPARAMS, const __gr
 // guiding samples of the direct boundary term: |baseVal| of `per` samples in
 // each leaf of the guiding tree (guide_base_val, one ray query per launch).
 // One thread per leaf traced all of its samples' rays one after the other, with
-// a few thousand threads in all: an inverse-rendering step of three views with
-// guiding took 43 ms and takes 19 with a slot per sample.
+// a few thousand threads in all: an inverse-rendering step of four views with
+// guiding took 43 ms and takes 17 with a slot per sample.
 // ---------------------------------------------------------------------------
 struct GuideTree {
   const float* box;       // [6][cap]
