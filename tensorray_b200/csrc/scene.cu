@@ -361,6 +361,7 @@ __global__ void __launch_bounds__(128) k_cluster(int n, const unsigned long long
       if (other < 0) active = false;  // the sibling's thread goes on
       else __threadfence();           // what the sibling wrote before it arrived
     }
+    __syncwarp();  // all lanes read it below (a vote orders no memory)
     const bool root = active && right - left + 1 == n;
     unsigned todo = __ballot_sync(0xffffffffu, root || (active && right - left + 1 > kClusters));
     while (todo) {
@@ -371,6 +372,7 @@ __global__ void __launch_bounds__(128) k_cluster(int n, const unsigned long long
       cluster_merge(n, l, sp, r, r - l + 1 == n ? 1 : kClusters, cid, cbox, nodes, parent, counter,
                     perm[threadIdx.x >> 5]);
       __threadfence();
+      __syncwarp();  // all lanes' writes before the one lane that arrives at the parent
     }
     if (root) active = false;
   }
