@@ -1048,8 +1048,6 @@ struct PathSoA {
   VRec* vr_;
   LRec* br_;
   F3 *Tk_, *Mk_;
-  unsigned* order;            // [cap] the records in the order their paths ended
-  unsigned long long* n_end;  // paths ended
   TRN_D long long& p(long long i) const { return p_[i]; }
   TRN_D int& view(long long i) const { return view_[i]; }
   TRN_D int& K(long long i) const { return K_[i]; }
@@ -1079,7 +1077,6 @@ inline size_t path_soa(PathSoA& a, void* base, long long cap, int depth) {
   a.br_ = reinterpret_cast<LRec*>(take(sizeof(LRec) * n * std::max(depth, 1)));
   a.Tk_ = reinterpret_cast<F3*>(take(sizeof(F3) * n * v));
   a.Mk_ = reinterpret_cast<F3*>(take(sizeof(F3) * n * v));
-  a.order = reinterpret_cast<unsigned*>(take(sizeof(unsigned) * n));
   return off;
 }
 
@@ -1096,17 +1093,16 @@ struct PathRef {
   struct M { const PathSoA& a; long long i; TRN_D const F3& operator[](int k) const { return a.Mk(i, k); } } Mk;
 };
 
-// Reverse sweep over the records, in the order in which their paths ended: the
-// paths of one bounce ended together, so a warp's sweeps have the same length
-// (in slot order a warp ran as long as its longest path, with less than a third
-// of its lanes active: 23.5 ms for 16.8M paths of depth 5, 12.0 in this order).
-// The order matters to the sums: a few vertices get millions of 32-bit adds, and
-// small ones are lost in a large sum. Shortest paths first stays nearest to the
-// sums in slot order (5e-5 of the positions' gradient; longest first 1.5e-4). Bound by instruction fetch:
-// the sweep is one long body of inlined scatters, and the few warps that fit
-// its registers do not hide the misses. (Its six scatters in a loop, or one
-// shared function, take 5 to 10 times as long: lanes then enter them one group
-// at a time.)
+// Reverse sweep over the records, in their own order (the paths' slots, but for
+// the order in which warps start). The order matters to the sums: a few vertices
+// get millions of 32-bit adds, and small ones are lost in a large sum. In the
+// order in which paths ended a warp's sweeps have the same length, and the sweep
+// takes half the time (16.8M paths of depth 5: 11.8 ms, in this order 23.7), but
+// the lanes that add together are others, and the position gradient moves by
+// 6e-5, where two runs differ by 1.5e-5. Bound by instruction fetch: the sweep is
+// one long body of inlined scatters, and the few warps that fit its registers do
+// not hide the misses. (Its six scatters in a loop, or one shared function, take
+// 5 to 10 times as long: lanes then enter them one group at a time.)
 // CACHED: the records come from the recording forward render and carry no
 // dL/dI yet; each path reads its pixel's now and is skipped when that is zero,
 // as the replaying form skips it.
@@ -1114,10 +1110,10 @@ template <bool CACHED>
 __global__ void __launch_bounds__(256, TRN_MINB_REVERSE) k_path_reverse(TRN_KPARAMS, const __grid_constant__ PathSoA R) {
   stage_begin();
   Cnt cnt;
-  const unsigned long long n = *R.n_end;
+  const unsigned long long n = min(*P.q_count, (unsigned long long)P.q_cap);
   for (unsigned long long k = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; k < n;
        k += (unsigned long long)gridDim.x * blockDim.x) {
-    const long long i = (long long)__ldcs(R.order + k);
+    const long long i = (long long)k;
     const int view = R.view(i);
     F3 g;
     if (CACHED) {
@@ -1136,24 +1132,10 @@ __global__ void __launch_bounds__(256, TRN_MINB_REVERSE) k_path_reverse(TRN_KPAR
 // ---------------------------------------------------------------------------
 // EvalImportance for one ray (Integrator.cpp:75-176)
 // ---------------------------------------------------------------------------
-// In two halves like a radiance bounce: importance_gen decides the ray from the
-// sensor to the vertex (with the contribution it would carry and its pixel)
-// and the continuation.
-struct ImportanceGen {
-  F3 c;         // contribution if the vertex is visible from the sensor
-  int pix;      // its pixel (-1: none)
-  F3 sdir;      // ray from the camera position: direction and end
-  float stmax;
-  bool shadow;
-  F3 wi, Tn;    // continuation ray and the throughput behind it
-  bool cont;
-};
-
-TRN_D void importance_gen(const DeviceScene& s, const CameraDesc& cam, const SurfF& x, const F3& rdir, const F3& T,
-                          float b0, float b1, float b2, ImportanceGen& g, Cnt& cnt) {
-  g.c = F3z();
-  g.pix = -1;
-  g.shadow = g.cont = false;
+TRN_D bool importance_step(const DeviceScene& s, const CameraDesc& cam, SurfF& x, F3& rdir, F3& T, float b0,
+                           float b1, float b2, F3& contrib, int& pix, Cnt& cnt) {
+  contrib = F3z();
+  pix = -1;
   const BsdfDesc b = s.bsdfs[x.bsdf];
   count_shade(cnt, s, x);
   long long texel;
@@ -1163,42 +1145,32 @@ TRN_D void importance_gen(const DeviceScene& s, const CameraDesc& cam, const Sur
   const F3 cpos = cam_pos(cam);
   const SensorSample sds = sample_direct(cam, x.p);
   if (sds.valid) {
-    g.sdir = sensor_ray_dir(cam, sds.qx, sds.qy);
-    g.stmax = length(x.p - cpos) - kShadowEps;
-    g.shadow = true;
+    const F3 dirc = sensor_ray_dir(cam, sds.qx, sds.qy);
+    const float dist2cam = length(x.p - cpos);
     cnt.v[kCntShadow]++;
-    F3 val = F3z();
-    if (out_dir_valid(b, x.ns, x.ng, wo)) {
-      const F3 wi = normalize(cpos - x.p);
-      if (out_dir_valid(b, x.ns, x.ng, wi))
-        val = bsdf_eval(b, fr, x.ng, kd, wo, wi, true) * fabsf(dot(x.ns, wi));
+    if (!occluded(s, cpos, dirc, kShadowEps, dist2cam - kShadowEps)) {
+      F3 val = F3z();
+      if (out_dir_valid(b, x.ns, x.ng, wo)) {
+        const F3 wi = normalize(cpos - x.p);
+        if (out_dir_valid(b, x.ns, x.ng, wi))
+          val = bsdf_eval(b, fr, x.ng, kd, wo, wi, true) * fabsf(dot(x.ns, wi));
+      }
+      contrib = scrub(T * sds.sensor_val * val);
+      pix = image_pixel(cam, sds.qx, sds.qy);
     }
-    g.c = scrub(T * sds.sensor_val * val);
-    g.pix = image_pixel(cam, sds.qx, sds.qy);
   }
-  if (!out_dir_valid(b, x.ns, x.ng, wo)) return;
-  float pdf;
-  bsdf_sample_only(b, fr, wo, b0, b1, b2, g.wi, pdf);
-  const F3 bv = bsdf_eval(b, fr, x.ng, kd, wo, g.wi, true) * fabsf(dot(x.ns, g.wi));
-  g.Tn = T * bv / pdf;
-  g.cont = pdf > 0.f && out_dir_valid(b, x.ns, x.ng, g.wi);
-}
-
-// The whole step by one thread (the fused kernels).
-TRN_D bool importance_step(const DeviceScene& s, const CameraDesc& cam, SurfF& x, F3& rdir, F3& T, float b0,
-                           float b1, float b2, F3& contrib, int& pix, Cnt& cnt) {
-  ImportanceGen g;
-  importance_gen(s, cam, x, rdir, T, b0, b1, b2, g, cnt);
-  contrib = F3z();
-  pix = -1;
-  if (g.shadow && !occluded(s, cam_pos(cam), g.sdir, kShadowEps, g.stmax)) { contrib = g.c; pix = g.pix; }
-  if (!g.cont) return false;
+  if (!out_dir_valid(b, x.ns, x.ng, wo)) return false;
+  F3 wi; float pdf;
+  bsdf_sample_only(b, fr, wo, b0, b1, b2, wi, pdf);
+  const F3 bv = bsdf_eval(b, fr, x.ng, kd, wo, wi, true) * fabsf(dot(x.ns, wi));
+  const F3 Tn = T * bv / pdf;
+  if (!(pdf > 0.f) || !out_dir_valid(b, x.ns, x.ng, wi)) return false;
   Hit h;
   cnt.v[kCntClosest]++;
-  if (!trace<false>(s, x.p, g.wi, kShadowEps, kRayMax, h)) return false;
+  if (!trace<false>(s, x.p, wi, kShadowEps, kRayMax, h)) return false;
   x = post_intersect(s, h.tri, h.u, h.v);
-  rdir = g.wi;
-  T = g.Tn;
+  rdir = wi;
+  T = Tn;
   return true;
 }
 
@@ -2207,6 +2179,254 @@ __global__ void __launch_bounds__(256, TRN_MINB) k_pixel_adj(TRN_KPARAMS) {
   flush_cnt(cnt, P.stats);
 }
 
+// ---------------------------------------------------------------------------
+// paths and scatter of the boundary samples that passed their set-up
+// ---------------------------------------------------------------------------
+// One kernel per side runs a round's samples to their ends, one thread per
+// sample, and a lane whose path has ended takes the next sample of the queue at
+// once. Each sample scatters when its path ends, together with the lanes of its
+// warp that end in the same turn.
+//
+// Not as a wavefront like the interior term's paths: a few vertices (a ground
+// plane's, a light's) get millions of 32-bit adds each, and which small ones are
+// lost in the large running sum depends on how many lanes' adds are summed
+// before them and on their order. A scatter of 32 queued samples at a time, all
+// of one bounce before those of the next, moved nearly cancelling components of
+// the 16.8M-sample gradient by 2 % of its RMS (0.1 % between two runs).
+// (16.8M slots of depth 5, as a wavefront and here, in ms: primary 11.2 and
+// 13.6, direct 2.4 and 2.3, indirect 28.6 and 34.6, pixel 16.0 and 23.7.)
+
+// Slot of a sample in its launch, which indexes a caller's sample table.
+TRN_D long long item_gslot(const Params& P, const ViewDesc& V, long long p) {
+  return p + (P.term == TRN_PIXEL_EDGE ? V.begin / 4 : V.begin);
+}
+
+// Warp-uniform: hands every lane that wants one the next index of [0, n);
+// `done` is set for those that come behind the end.
+TRN_D void take_next(unsigned long long* next, unsigned long long n, bool want, unsigned long long& k, bool& done) {
+  const unsigned need = __ballot_sync(0xffffffffu, want);
+  if (!need) return;
+  const int lane = threadIdx.x & 31, leader = __ffs(need) - 1;
+  unsigned long long base = 0;
+  if (lane == leader) base = atomicAdd(next, (unsigned long long)__popc(need));
+  base = __shfl_sync(0xffffffffu, base, leader);
+  if (want) {
+    k = base + __popc(need & ((1u << lane) - 1u));
+    done = k >= n;
+  }
+}
+
+// Primary and pixel terms: detached radiance of the sample, then the scatter.
+__global__ void __launch_bounds__(256, TRN_MINB) k_primary_body(TRN_KPARAMS, unsigned long long* next) {
+  stage_begin();
+  Cnt cnt;
+  const DeviceScene& s = P.s;
+  const PrimaryItem* q = reinterpret_cast<const PrimaryItem*>(P.queue);
+  const unsigned long long n = min(*P.q_count, (unsigned long long)P.q_cap);
+  const int dim0 = P.term == TRN_PIXEL_EDGE ? 1 : 2;
+  bool active = false, done = false;
+  unsigned long long k = 0;
+  const ViewDesc* V = nullptr;
+  SurfF x;
+  F3 T, rdir, L;
+  int b = 0, D = 0;
+  for (;;) {
+    const bool want = !active && !done;
+    take_next(next, n, want, k, done);
+    if (want && !done) {
+      const PrimaryItem& it = q[k];
+      V = P.views + it.view;
+      D = V->D;
+      x = post_intersect(s, it.x_tri, it.x_u, it.x_v);
+      T = F3(it.T0, it.T0, it.T0);
+      rdir = it.rdir;
+      L = scrub(T * emitted(s, x, -rdir));
+      b = 0;
+      active = true;
+    }
+    if (!__any_sync(0xffffffffu, active)) break;
+    if (active) {
+      bool fin = b >= D;
+      if (!fin) {
+        const long long p = q[k].p;
+        const PathSmp S{&P, V->seed, item_gslot(P, *V, p), p + V->slot_off};
+        const int o = dim0 + 5 * b;
+        F3 c;
+        const bool more = radiance_step(s, x, rdir, T, S(o), S(o + 1), S(o + 2), S(o + 3), S(o + 4), c, nullptr, cnt);
+        L = L + c;
+        b++;
+        fin = !more || (T.x == 0.f && T.y == 0.f && T.z == 0.f) || b >= D;
+      }
+      if (fin) {
+        const PrimaryItem& it = q[k];
+        const float W = dot(it.g, L * it.w0);
+        if (W != 0.f && isfinite(W))
+          xdotn_vjp(P, *V, W, cam_pos(V->cam), false, -1, 0.f, 0.f, it.v0, it.v1, it.sedge, it.p0, it.far_tri, it.n,
+                    cnt);
+        active = false;
+      }
+    }
+  }
+  flush_cnt(cnt, P.stats);
+}
+
+// Direct term: importance path and scatter. (Few samples pass the set-up, and
+// they leave their receiver towards one sensor: no lane waits for long.)
+__global__ void __launch_bounds__(256, TRN_MINB) k_direct_body(TRN_KPARAMS) {
+  stage_begin();
+  Cnt cnt;
+  const DirectItem* q = reinterpret_cast<const DirectItem*>(P.queue);
+  const unsigned long long n = min(*P.q_count, (unsigned long long)P.q_cap);
+  for (unsigned long long k = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; k < n;
+       k += (unsigned long long)gridDim.x * blockDim.x) {
+    const DirectItem& it = q[k];
+    const ViewDesc& V = P.views[it.view];
+    const SurfF x = post_intersect(P.s, it.x_tri, it.x_u, it.x_v);
+    direct_body(P, V, item_gslot(P, V, it.p), it.p, x, it.rdir, it.ev0, it.v0, it.v1, it.sedge, it.p0, it.far_tri,
+                it.n, cnt);
+  }
+  flush_cnt(cnt, P.stats);
+}
+
+// Indirect term, a sample whose sensor side reached the image: the set-up's
+// item, how deep its emitter side has to go, the weight of each sensor depth.
+template <int MAXD>
+struct IndirectLit {
+  unsigned item;
+  int jmax;
+  F3 sc[MAXD - 1];
+};
+
+// Sensor side (the steps of indirect_sensor).
+template <int MAXD>
+__global__ void __launch_bounds__(256, TRN_MINB) k_indirect_sensor(TRN_KPARAMS, unsigned long long* next,
+                                                                   IndirectLit<MAXD>* lit, unsigned long long* n_lit) {
+  stage_begin();
+  Cnt cnt;
+  const DeviceScene& s = P.s;
+  const IndirectItem* q = reinterpret_cast<const IndirectItem*>(P.queue);
+  const unsigned long long n = min(*P.q_count, (unsigned long long)P.q_cap);
+  bool active = false, done = false;
+  unsigned long long k = 0;
+  const ViewDesc* V = nullptr;
+  SurfF x;
+  F3 T, rdir;
+  F3 sc[MAXD - 1];
+  int b = 0, D = 0, bmin = 0;
+  for (;;) {
+    const bool want = !active && !done;
+    take_next(next, n, want, k, done);
+    if (want && !done) {
+      const IndirectItem& it = q[k];
+      V = P.views + it.view;
+      D = min(V->D, MAXD);
+      x = post_intersect(s, it.xs_tri, it.xs_u, it.xs_v);
+      rdir = it.rdir;
+      T = F3(1.f, 1.f, 1.f);
+      for (int j = 0; j < D - 1; j++) sc[j] = F3z();
+      bmin = D;
+      b = 0;
+      active = true;
+    }
+    if (!__any_sync(0xffffffffu, active)) break;
+    bool fin = false;
+    if (active) {
+      fin = b >= D - 1;
+      if (!fin) {
+        const long long p = q[k].p();
+        const PathSmp S{&P, V->seed, item_gslot(P, *V, p), p + V->slot_off};
+        const int o = 3 + 5 * (D - 1) + 3 * b;
+        F3 c;
+        int pix;
+        const bool more = importance_step(s, V->cam, x, rdir, T, S(o), S(o + 1), S(o + 2), c, pix, cnt);
+        if (pix >= 0) {
+          sc[b] = g_at(P, *V, pix) * c;
+          if (sc[b].x != 0.f || sc[b].y != 0.f || sc[b].z != 0.f) bmin = min(bmin, b);
+        }
+        b++;
+        fin = !more || b >= D - 1;
+      }
+    }
+    const bool push = fin && bmin < D - 1;
+    const unsigned m = __ballot_sync(0xffffffffu, push);
+    if (m) {
+      const int lane = threadIdx.x & 31, leader = __ffs(m) - 1;
+      unsigned long long base = 0;
+      if (lane == leader) base = atomicAdd(n_lit, (unsigned long long)__popc(m));
+      base = __shfl_sync(0xffffffffu, base, leader);
+      if (push) {
+        IndirectLit<MAXD>& it = lit[base + __popc(m & ((1u << lane) - 1u))];  // at most one per item
+        it.item = (unsigned)k;
+        it.jmax = D - 2 - bmin;
+        for (int j = 0; j < D - 1; j++) it.sc[j] = sc[j];
+      }
+    }
+    if (fin) active = false;
+  }
+  flush_cnt(cnt, P.stats);
+}
+
+// Emitter side of the lit samples (the steps and the additions of
+// indirect_emitter: when the path has ended, the remaining depths pair with its
+// last radiance), then the scatter.
+template <int MAXD>
+__global__ void __launch_bounds__(256, TRN_MINB) k_indirect_emitter(TRN_KPARAMS, unsigned long long* next,
+                                                                    const IndirectLit<MAXD>* lit,
+                                                                    const unsigned long long* n_lit) {
+  stage_begin();
+  Cnt cnt;
+  const DeviceScene& s = P.s;
+  const IndirectItem* q = reinterpret_cast<const IndirectItem*>(P.queue);
+  const unsigned long long n = *n_lit;
+  bool active = false, done = false;
+  unsigned long long k = 0;
+  const ViewDesc* V = nullptr;
+  SurfF x;
+  F3 T, rdir, cur;
+  float W = 0.f;
+  int j = 0;
+  for (;;) {
+    const bool want = !active && !done;
+    take_next(next, n, want, k, done);
+    if (want && !done) {
+      const IndirectItem& it = q[lit[k].item];
+      V = P.views + it.view;
+      x = post_intersect(s, it.xe_tri, it.xe_u, it.xe_v);
+      rdir = -it.rdir;
+      T = F3(1.f, 1.f, 1.f);
+      cur = F3z();
+      W = 0.f;
+      j = 0;
+      active = true;
+    }
+    if (!__any_sync(0xffffffffu, active)) break;
+    if (active) {
+      const IndirectLit<MAXD>& l = lit[k];
+      const IndirectItem& it = q[l.item];
+      const int D = min(V->D, MAXD), jmax = l.jmax;
+      const long long p = it.p();
+      const PathSmp S{&P, V->seed, item_gslot(P, *V, p), p + V->slot_off};
+      const int o = 3 + 5 * j;
+      F3 c;
+      bool alive = radiance_step(s, x, rdir, T, S(o), S(o + 1), S(o + 2), S(o + 3), S(o + 4), c, nullptr, cnt);
+      cur = cur + c;
+      if (T.x == 0.f && T.y == 0.f && T.z == 0.f) alive = false;
+      W += dot(l.sc[D - 2 - j], cur) * it.w0;
+      j++;
+      if (!alive || j > jmax) {
+        for (; j <= jmax; j++) W += dot(l.sc[D - 2 - j], cur) * it.w0;
+        if (W != 0.f && isfinite(W)) {
+          const SurfF xs = post_intersect(s, it.xs_tri, it.xs_u, it.xs_v);
+          xdotn_vjp(P, *V, W, xs.p, true, it.xs_tri, it.xs_u, it.xs_v, it.v0, it.v1, it.sedge, it.p0, it.far_tri,
+                    it.n, cnt);
+        }
+        active = false;
+      }
+    }
+  }
+  flush_cnt(cnt, P.stats);
+}
+
 #include "wavefront.cuh"
 
 // ---------------------------------------------------------------------------
@@ -2342,7 +2562,7 @@ struct trn_viewset {
   // depth; hash samples only)
   void* pc = nullptr;
   size_t pc_bytes = 0;
-  unsigned long long* pc_count = nullptr;  // [2] records, paths ended
+  unsigned long long* pc_count = nullptr;  // records
   long long pc_limit = 0;  // bytes the records may take (0 = off)
   bool pc_valid = false;
   std::vector<char> pc_key;
@@ -2608,22 +2828,27 @@ size_t wave_layout(Wave& W, void** items, void* base, long long cap, int integra
   const bool edge = integrator != TRN_PATH_TRACER;
   *items = take(item_bytes(integrator) * n);
   W.cap = cap;
+  const size_t setup = off;
   W.ro = static_cast<float4*>(take(2 * n * sizeof(float4)));
   W.rd = static_cast<float4*>(take(2 * n * sizeof(float4)));
-  W.hit[0] = static_cast<float4*>(take(n * sizeof(float4)));
+  for (float4*& h : W.hit) h = static_cast<float4*>(take(edge || &h == W.hit ? n * sizeof(float4) : 0));
   W.occ = static_cast<unsigned char*>(take(n));
   W.list[0] = static_cast<unsigned*>(take(n * sizeof(unsigned)));
   W.list[1] = static_cast<unsigned*>(take(n * sizeof(unsigned)));
-  for (float4*& s : W.st) s = static_cast<float4*>(take(n * sizeof(float4)));
-  W.hit[1] = W.st[0];  // of a set-up's second rays, before any path has state
-  W.p = static_cast<long long*>(take(edge ? 0 : n * sizeof(long long)));
-  W.view = static_cast<int*>(take(edge ? 0 : n * sizeof(int)));
-  W.rec = static_cast<unsigned*>(take(n * sizeof(unsigned)));
-  W.L = static_cast<F3*>(take(edge ? 0 : n * sizeof(F3)));
-  W.W = static_cast<float*>(take(edge ? n * sizeof(float) : 0));
-  const bool ind = integrator == TRN_INDIRECT_EDGE;
-  W.list2 = static_cast<unsigned*>(take(ind ? n * sizeof(unsigned) : 0));
-  W.sc = static_cast<float*>(take(ind ? 3 * sizeof(float) * n * (size_t)std::max(depth - 1, 0) : 0));
+  W.W = static_cast<float*>(take(integrator == TRN_DIRECT_EDGE ? n * sizeof(float) : 0));
+  if (!edge) {
+    for (float4*& s : W.st) s = static_cast<float4*>(take(n * sizeof(float4)));
+    W.p = static_cast<long long*>(take(n * sizeof(long long)));
+    W.view = static_cast<int*>(take(n * sizeof(int)));
+    W.rec = static_cast<unsigned*>(take(n * sizeof(unsigned)));
+    W.L = static_cast<F3*>(take(n * sizeof(F3)));
+  }
+  if (integrator == TRN_INDIRECT_EDGE) {  // in the place of the set-up's buffers, which are done with by then
+    const size_t end = off;
+    off = setup;
+    W.lit = take((depth <= 8 ? sizeof(IndirectLit<8>) : sizeof(IndirectLit<kMaxDepth>)) * n);
+    off = std::max(off, end);
+  }
   return off;
 }
 
@@ -2746,7 +2971,7 @@ struct WaveRun {
     launch<k_trace>(std::min((long long)sms() * TRN_TRACE_MINB, need), TRN_TRACE_BLOCK, P.s, W, r0, n, ctr(),
                     W.hit[which], P.err);
   }
-  // bounces of the entries that a start kernel left in list[0]
+  // bounces of the entries that the start kernel left in list[0]
   template <int MODE>
   void bounces(const unsigned long long* n, unsigned long long* n_ray, int depth) {
     for (int b = 0; b < depth; b++) {
@@ -2754,18 +2979,6 @@ struct WaveRun {
       Stage S{n, W.list[b & 1], ctr(), W.list[(b + 1) & 1], ctr(), nullptr, b};
       go<k_wf_shade<MODE>>(P, W, S, R);
       n = S.n_out; n_ray = S.n_ray;
-    }
-  }
-  template <bool SENSOR>
-  void importance(int depth) {
-    Stage S{P.q_count, nullptr, ctr(), W.list[0], ctr(), nullptr, 0};
-    go<k_wi_start<SENSOR>>(P, W, S);
-    const unsigned long long *n = S.n_out, *n_ray = S.n_ray;
-    for (int b = 0; b < depth; b++) {
-      trace(0, n_ray, 0);
-      Stage B{n, W.list[b & 1], ctr(), W.list[(b + 1) & 1], ctr(), nullptr, b};
-      go<k_wi_step<SENSOR>>(P, W, B);
-      n = B.n_out; n_ray = B.n_ray;
     }
   }
   // set-up rays and geometry of a boundary term: items to P.queue
@@ -2814,7 +3027,6 @@ int path_wave(trn_viewset* vs, const Params& P0, const trn_launch* ln, long long
   const size_t wb = wave_layout(r.W, &items, vs->iq, cap, TRN_PATH_TRACER, depth);
   if (MODE == kWfRec) {
     r.R = *cache;
-    r.R.n_end = vs->pc_count + 1;
   }
   if (MODE == kWfReplay) {
     path_soa(r.R, static_cast<char*>(vs->iq) + wb, cap, depth);
@@ -2826,7 +3038,6 @@ int path_wave(trn_viewset* vs, const Params& P0, const trn_launch* ln, long long
     r.W.first = first;
     if (MODE == kWfReplay) {
       r.P.q_count = r.ctr();
-      r.R.n_end = r.ctr();
     }
     unsigned long long* rays = r.ctr();
     r.go<k_wf_camera>(r.P, r.W, n, MODE == kWfReplay, rays);
@@ -3028,6 +3239,15 @@ int order_round(trn_viewset* vs, Params& P, int term, cudaStream_t st) {
   return 0;
 }
 
+// Sensor side, then the emitter side of the samples that it leaves.
+template <int MAXD>
+void indirect_sides(WaveRun& r) {
+  IndirectLit<MAXD>* lit = static_cast<IndirectLit<MAXD>*>(r.W.lit);
+  unsigned long long* n_lit = r.ctr();
+  r.go<k_indirect_sensor<MAXD>>(r.P, r.ctr(), lit, n_lit);
+  r.go<k_indirect_emitter<MAXD>>(r.P, r.ctr(), lit, n_lit);
+}
+
 // A boundary term over all slots, in rounds: run order, set-up, the paths of
 // the samples that passed, scatter.
 template <int TERM>
@@ -3051,22 +3271,12 @@ int edge_wave(trn_viewset* vs, const Params& P0, const trn_launch* ln, long long
     r.P.q_count = r.ctr();
     r.setup<TERM>(first);
     if constexpr (TERM == TRN_DIRECT_EDGE) {
-      r.importance<false>(depth);
-      r.go<k_wi_direct_scatter>(r.P, r.W);
+      r.go<k_direct_body>(r.P);
     } else if constexpr (TERM == TRN_INDIRECT_EDGE) {
-      const int d = std::min(depth, (int)kMaxDepth) - 1;
-      r.importance<true>(d);
-      unsigned long long* n_emit = r.ctr();
-      r.go<k_wi_collect>(r.P, r.W, n_emit);
-      Stage S{n_emit, r.W.list2, r.ctr(), r.W.list[0], r.ctr(), nullptr, 0};
-      r.go<k_wf_start<kWfEmit>>(r.P, r.W, S, r.R);
-      r.bounces<kWfEmit>(S.n_out, S.n_ray, d);
-      r.go<k_wf_emit_scatter>(r.P, r.W, n_emit);
+      if (depth <= 8) indirect_sides<8>(r);
+      else indirect_sides<kMaxDepth>(r);
     } else {
-      Stage S{r.P.q_count, nullptr, r.ctr(), r.W.list[0], r.ctr(), nullptr, 0};
-      r.go<k_wf_start<kWfBody>>(r.P, r.W, S, r.R);
-      r.bounces<kWfBody>(S.n_out, S.n_ray, depth);
-      r.go<k_wf_body_scatter>(r.P, r.W);
+      r.go<k_primary_body>(r.P, r.ctr());
     }
   }
   TRN_CUDA_TRY(cudaGetLastError());
@@ -3118,7 +3328,7 @@ int path_cache_fwd(trn_viewset* vs, Params P, const trn_launch* ln, const trn_re
     vs->pc = nullptr;
     vs->pc_bytes = 0;
     if (cudaMalloc(&vs->pc, bytes) != cudaSuccess ||
-        (!vs->pc_count && cudaMalloc(&vs->pc_count, 2 * sizeof(unsigned long long)) != cudaSuccess)) {
+        (!vs->pc_count && cudaMalloc(&vs->pc_count, sizeof(unsigned long long)) != cudaSuccess)) {
       cudaGetLastError();  // out of memory: render without records
       if (vs->pc) cudaFree(vs->pc);
       vs->pc = nullptr;
@@ -3126,7 +3336,7 @@ int path_cache_fwd(trn_viewset* vs, Params P, const trn_launch* ln, const trn_re
     }
     vs->pc_bytes = bytes;
   }
-  TRN_CUDA_TRY(cudaMemsetAsync(vs->pc_count, 0, 2 * sizeof(unsigned long long), st));
+  TRN_CUDA_TRY(cudaMemsetAsync(vs->pc_count, 0, sizeof(unsigned long long), st));
   P.q_count = vs->pc_count;
   P.q_cap = total;
   path_soa(R, vs->pc, total, vs->max_depth);
@@ -3147,7 +3357,6 @@ int path_cache_grad(trn_viewset* vs, Params P, const trn_launch* ln, const trn_r
   P.q_cap = total;
   PathSoA R;
   path_soa(R, vs->pc, total, vs->max_depth);
-  R.n_end = vs->pc_count + 1;
   int grid, block;
   launch_dims(ln, total, grid, block);
   k_path_reverse<true><<<grid, block, 0, st>>>(P, R);

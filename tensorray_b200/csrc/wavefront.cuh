@@ -1,22 +1,19 @@
-// Wavefront form of the integrators: paths of one round advance together, one
-// bounce per pair of launches. A shading kernel ends the previous bounce
-// with its ray results and decides the next bounce's rays; k_trace runs all of
-// them. Between them only the rays, their results and 64 bytes of path state
-// pass through memory (an L2's worth at a time).
+// Wavefront form of the interior term and of the boundary terms' set-ups: paths
+// of one round advance together, one bounce per pair of launches. A shading
+// kernel ends the previous bounce with its ray results and decides the next
+// bounce's rays; k_trace runs all of them. Between them only the rays, their
+// results and 64 bytes of path state pass through memory (an L2's worth at a
+// time).
 //
 // Why: with one thread per path, traversal and shading of 32 unrelated paths
 // shared a warp, with 6 to 8 of 32 lanes active per instruction. Here a
 // traversal warp refills its free lanes with rays of any path (trace_stream),
 // and a shading warp holds 32 paths at the same bounce. 16.8M samples of depth
-// 5 on 102,400 triangles, one thread per path and here, in ms: image 27.6 and
-// 15.8, primary 14.8 and 11.2, direct 2.8 and 2.4, indirect 37.3 and 28.8,
-// pixel 20.6 and 16.0. k_trace takes 65 % of that.
+// 5 on 102,400 triangles, one thread per path and here: image 27.6 and 15.8 ms.
 //
-// The price is a launch pair per bounce, each as long as its longest ray: at
-// 0.5M samples of depth 12 the image is even (1.92 and 1.93 ms) and the
-// boundary terms are behind (direct 0.64 and 0.94, indirect 3.5 and 3.8, pixel
-// 1.6 and 1.9), less than the interior adjoint's records from the same kernels
-// give back (1.1 and 0.4, primary 2.3 and 1.9). One form serves all sizes.
+// The price is a launch pair per bounce, each as long as its longest ray.
+// (The paths of a boundary term's samples run in one kernel each, behind these
+// set-ups: render.cu says why.)
 //
 // Included by render.cu (uses its parameter block and path functions).
 #pragma once
@@ -28,15 +25,14 @@ struct Wave {
   float4* hit[2];           // [cap] closest-hit results by ray id: tri, u, v, t
   unsigned char* occ;       // [cap] occlusion results by ray id
   unsigned* list[2];        // [cap] active samples of a stage, ping-pong
-  unsigned* list2;          // [cap] samples that go on to the emitter side
   float4* st[4];            // [cap] path state
-  long long* p;             // [cap] view-local sample index (interior term;
-  int* view;                // [cap]  the other terms' items hold theirs)
-  unsigned* rec;            // [cap] record index (recording modes) / sensor depths seen
-  float* W;                 // [cap] weight of the sample's scatter
+  long long* p;             // [cap] view-local sample index
+  int* view;                // [cap]
+  unsigned* rec;            // [cap] record index (recording modes)
   F3* L;                    // [cap] radiance by slot of the round (forward modes)
   long long first;          // first slot of the round (interior term)
-  float* sc;                // [max depth - 1][cap][3] sensor-side weights (indirect term)
+  float* W;                 // [cap] values of the guiding samples
+  void* lit;                // [cap] indirect samples that go on to the emitter side
 };
 
 // ray ids: bit 31 marks an occlusion query
@@ -143,24 +139,11 @@ __global__ void __launch_bounds__(TRN_TRACE_BLOCK, TRN_TRACE_MINB)
 }
 
 // ---------------------------------------------------------------------------
-// radiance paths: interior term (image, records, replay), primary / pixel
-// bodies, indirect emitter side
+// radiance paths of the interior term (image, records, replay)
 // ---------------------------------------------------------------------------
 // kWfFwd: forward image; kWfRec: forward image and path records; kWfReplay:
-// path records for the adjoint; kWfBody: detached radiance of a queued primary
-// or pixel sample; kWfEmit: emitter side of a queued indirect sample.
-enum WfMode { kWfFwd = 0, kWfRec, kWfReplay, kWfBody, kWfEmit };
-
-// first sample dimension of bounce b
-template <int MODE>
-TRN_D int wf_dim(const Params& P, int b) {
-  if (MODE == kWfBody) return (P.term == TRN_PIXEL_EDGE ? 1 : 2) + 5 * b;
-  return (MODE == kWfEmit ? 3 : 2) + 5 * b;
-}
-// launch-global slot of a sample, which indexes a caller's sample table
-TRN_D long long wf_gslot(const Params& P, const ViewDesc& V, long long p) {
-  return p + (P.term == TRN_PIXEL_EDGE ? V.begin / 4 : V.begin);
-}
+// path records for the adjoint.
+enum WfMode { kWfFwd = 0, kWfRec, kWfReplay };
 
 struct WfPath {
   SurfF x;
@@ -175,10 +158,10 @@ TRN_D void wf_advance(const Params& P, const Wave& W, const Stage& S, int b, boo
   RadianceGen g;
   g.shadow = g.cont = false;
   if (go) {
-    const PathSmp smp{&P, V->seed, wf_gslot(P, *V, p), p + V->slot_off};
-    const int o = wf_dim<MODE>(P, b);
+    const PathSmp smp{&P, V->seed, p + V->begin, p + V->slot_off};
+    const int o = 2 + 5 * b;
     BounceRec br;
-    constexpr bool rec = MODE == kWfRec || MODE == kWfReplay;
+    constexpr bool rec = MODE != kWfFwd;
     radiance_gen(P.s, q.x, q.rdir, q.T, smp(o), smp(o + 1), smp(o + 2), smp(o + 3), smp(o + 4), g, rec ? &br : nullptr,
                  cnt);
     W.st[0][i] = make_float4(__int_as_float(q.x.tri), q.x.u, q.x.v, g.pdf);
@@ -196,25 +179,12 @@ TRN_D void wf_advance(const Params& P, const Wave& W, const Stage& S, int b, boo
   if (go) S.out[j] = i | (g.shadow ? kCastShadow : 0u) | (g.cont ? kCastCont : 0u);
 }
 
-// Ends the path of sample i.
+// Ends the path of sample p of view V.
 template <int MODE>
-TRN_D void wf_finish(const Params& P, const Wave& W, unsigned i, const ViewDesc& V, long long p, const F3& L, Cnt& cnt) {
-  if (MODE == kWfFwd || MODE == kWfRec) {
-    cnt.v[kCntPixel]++;
-    W.L[p + V.begin - W.first] = L;
-  } else if (MODE == kWfBody) {
-    const PrimaryItem& it = reinterpret_cast<const PrimaryItem*>(P.queue)[i];
-    W.W[i] = dot(it.g, L * it.w0);
-  }
-}
-
-// Lists the records of the paths that end here (all lanes of the warp call it).
-template <int MODE>
-TRN_D void wf_record_end(const Wave& W, const PathSoA& R, bool ends, unsigned i) {
-  if constexpr (MODE == kWfRec || MODE == kWfReplay) {
-    const unsigned long long j = warp_append(R.n_end, ends);
-    if (ends) R.order[j] = W.rec[i];
-  }
+TRN_D void wf_finish(const Wave& W, const ViewDesc& V, long long p, const F3& L, Cnt& cnt) {
+  if (MODE == kWfReplay) return;
+  cnt.v[kCntPixel]++;
+  W.L[p + V.begin - W.first] = L;
 }
 
 // Camera rays of the round's n slots. For the adjoint (grad), slots whose pixel
@@ -291,73 +261,46 @@ __global__ void __launch_bounds__(256, 3) k_wf_start(TRN_KPARAMS, const __grid_c
     Hit h;
     h.tri = -1;
     int D = 0;
-    if constexpr (MODE <= kWfReplay) {
-      if (in) h = get_hit(W.hit[0], k);
-      in = h.tri >= 0;
-      // a state and, in the recording modes, a record for the path
-      const unsigned long long j = warp_append(S.n_state, in);
-      unsigned long long kr = 0;
-      if (MODE != kWfFwd) {
-        kr = warp_append(P.q_count, in);
-        if (in && kr >= (unsigned long long)P.q_cap) { atomicExch(P.err, 2); in = false; }
-      }
-      if (in) {
-        i = (unsigned)j;
-        const long long slot = W.first + (long long)S.in[k];
-        V = &view_of(P, slot, vhint);
-        p = slot - V->begin;
-        W.p[i] = p;
-        W.view[i] = (int)(V - P.views);
-        D = V->D;
-        const CameraDesc& cam = V->cam;
-        const F3 org = cam_pos(cam);
-        q.x = post_intersect(s, h.tri, h.u, h.v);
-        const float t1 = camera_factor<float>(cam, q.x.p, q.x.ng, 1.f);
-        q.T = F3(t1, t1, t1);
-        q.rdir = normalize(q.x.p - org);
-        const F3 m1 = emitted(s, q.x, -q.rdir);
-        if (MODE == kWfFwd) {
-          q.L = scrub(q.T * m1);
-        } else {
-          W.rec[i] = (unsigned)kr;
-          const F3 m = finite3(q.T * m1) ? m1 : F3z();
-          q.L = q.T * m;
-          R.p(kr) = p; R.view(kr) = (int)(V - P.views);
-          R.g(kr) = MODE == kWfReplay ? g_at(P, *V, (int)(p % ((long long)cam.w * cam.h))) : F3z();
-          R.vr(kr, 1) = {h.tri, h.u, h.v};
-          R.Tk(kr, 1) = q.T;
-          R.Mk(kr, 1) = m;
-          R.K(kr) = 1; R.D(kr) = D; R.nee(kr) = 0u;
-        }
-      }
-    } else if (in) {
-      F3 T0(1.f, 1.f, 1.f);
-      if constexpr (MODE == kWfBody) {
-        i = (unsigned)k;
-        const PrimaryItem& it = reinterpret_cast<const PrimaryItem*>(P.queue)[i];
-        V = P.views + it.view;
-        p = it.p;
-        q.x = post_intersect(s, it.x_tri, it.x_u, it.x_v);
-        q.rdir = it.rdir;
-        T0 = F3(it.T0, it.T0, it.T0);
-        q.L = scrub(T0 * emitted(s, q.x, -q.rdir));
-        D = V->D;
+    if (in) h = get_hit(W.hit[0], k);
+    in = h.tri >= 0;
+    // a state and, in the recording modes, a record for the path
+    const unsigned long long j = warp_append(S.n_state, in);
+    unsigned long long kr = 0;
+    if (MODE != kWfFwd) {
+      kr = warp_append(P.q_count, in);
+      if (in && kr >= (unsigned long long)P.q_cap) { atomicExch(P.err, 2); in = false; }
+    }
+    if (in) {
+      i = (unsigned)j;
+      const long long slot = W.first + (long long)S.in[k];
+      V = &view_of(P, slot, vhint);
+      p = slot - V->begin;
+      W.p[i] = p;
+      W.view[i] = (int)(V - P.views);
+      D = V->D;
+      const CameraDesc& cam = V->cam;
+      const F3 org = cam_pos(cam);
+      q.x = post_intersect(s, h.tri, h.u, h.v);
+      const float t1 = camera_factor<float>(cam, q.x.p, q.x.ng, 1.f);
+      q.T = F3(t1, t1, t1);
+      q.rdir = normalize(q.x.p - org);
+      const F3 m1 = emitted(s, q.x, -q.rdir);
+      if (MODE == kWfFwd) {
+        q.L = scrub(q.T * m1);
       } else {
-        i = S.in[k];
-        const IndirectItem& it = reinterpret_cast<const IndirectItem*>(P.queue)[i];
-        V = P.views + it.view;
-        p = it.p();
-        q.x = post_intersect(s, it.xe_tri, it.xe_u, it.xe_v);
-        q.rdir = -it.rdir;
-        q.L = F3z();
-        W.W[i] = 0.f;
-        D = 1;  // queued only when it pairs with a sensor depth
+        W.rec[i] = (unsigned)kr;
+        const F3 m = finite3(q.T * m1) ? m1 : F3z();
+        q.L = q.T * m;
+        R.p(kr) = p; R.view(kr) = (int)(V - P.views);
+        R.g(kr) = MODE == kWfReplay ? g_at(P, *V, (int)(p % ((long long)cam.w * cam.h))) : F3z();
+        R.vr(kr, 1) = {h.tri, h.u, h.v};
+        R.Tk(kr, 1) = q.T;
+        R.Mk(kr, 1) = m;
+        R.K(kr) = 1; R.D(kr) = D; R.nee(kr) = 0u;
       }
-      q.T = T0;
     }
     const bool go = in && D > 0;
-    if (in && !go) wf_finish<MODE>(P, W, i, *V, p, q.L, cnt);
-    wf_record_end<MODE>(W, R, in && !go, i);
+    if (in && !go) wf_finish<MODE>(W, *V, p, q.L, cnt);
     wf_advance<MODE>(P, W, S, 0, go, i, V, p, q, R, cnt);
   });
   flush_cnt(cnt, P.stats);
@@ -373,7 +316,7 @@ __global__ void __launch_bounds__(256, 3) k_wf_shade(TRN_KPARAMS, const __grid_c
   stage_begin();
   Cnt cnt;
   const DeviceScene& s = P.s;
-  constexpr bool rec = MODE == kWfRec || MODE == kWfReplay;
+  constexpr bool rec = MODE != kWfFwd;
   const int b = S.b, k = b + 1;
   for_each_entry(*S.n, [&](unsigned long long idx, bool in) {
     WfPath q;
@@ -389,18 +332,8 @@ __global__ void __launch_bounds__(256, 3) k_wf_shade(TRN_KPARAMS, const __grid_c
       h.tri = -1;
       if (e & kCastCont) h = get_hit(W.hit[0], idx);
       const float4 a = W.st[0][i], c1 = W.st[1][i], c2 = W.st[2][i], c3 = W.st[3][i];
-      if constexpr (MODE <= kWfReplay) {
-        p = W.p[i];
-        V = P.views + W.view[i];
-      } else if constexpr (MODE == kWfBody) {
-        const PrimaryItem& it = reinterpret_cast<const PrimaryItem*>(P.queue)[i];
-        p = it.p;
-        V = P.views + it.view;
-      } else {
-        const IndirectItem& it = reinterpret_cast<const IndirectItem*>(P.queue)[i];
-        p = it.p();
-        V = P.views + it.view;
-      }
+      p = W.p[i];
+      V = P.views + W.view[i];
       q.rdir = F3(c1.x, c1.y, c1.z);
       q.T = F3(c1.w, c2.x, c2.y);
       q.L = F3(c2.z, c2.w, c3.x);
@@ -410,7 +343,6 @@ __global__ void __launch_bounds__(256, 3) k_wf_shade(TRN_KPARAMS, const __grid_c
       const bool more = radiance_resolve(s, q.x, q.rdir, q.T, nee_ok, F3(c3.y, c3.z, c3.w), a.w, h, c, rec ? &br : nullptr);
       q.L = q.L + c;
       const bool dark = q.T.x == 0.f && q.T.y == 0.f && q.T.z == 0.f;
-      int D = V->D;
       if constexpr (rec) {
         const unsigned kr = W.rec[i];
         // a scrubbed (non-finite) bounce contributes nothing and carries no gradient
@@ -423,225 +355,11 @@ __global__ void __launch_bounds__(256, 3) k_wf_shade(TRN_KPARAMS, const __grid_c
           R.K(kr) = k + 1;
         }
       }
-      go = more && !dark;
-      if constexpr (MODE == kWfEmit) {
-        // the radiance accumulated over b + 1 bounces pairs with sensor depth
-        // D - 2 - b (BoundaryIndirect.cpp:158-175); when the path has ended, the
-        // remaining depths pair with its last radiance
-        const float w0 = reinterpret_cast<const IndirectItem*>(P.queue)[i].w0;
-        const unsigned seen = W.rec[i];
-        D = min(D, kMaxDepth);
-        const int jmax = D - 2 - (int)(seen >> 16);
-        float w = W.W[i];
-        go = go && b < jmax;
-        for (int j = b; j <= (go ? b : jmax); j++) {
-          const int d = D - 2 - j;
-          const float* sc = W.sc + 3 * ((long long)d * W.cap + i);
-          const F3 v = (seen >> d) & 1u ? F3(sc[0], sc[1], sc[2]) : F3z();
-          w += dot(v, q.L) * w0;
-        }
-        W.W[i] = w;
-      } else {
-        go = go && b + 1 < D;
-        if (!go) wf_finish<MODE>(P, W, i, *V, p, q.L, cnt);
-      }
+      go = more && !dark && b + 1 < V->D;
+      if (!go) wf_finish<MODE>(W, *V, p, q.L, cnt);
     }
-    wf_record_end<MODE>(W, R, in && !go, i);
     wf_advance<MODE>(P, W, S, b + 1, go, i, V, p, q, R, cnt);
   });
-  flush_cnt(cnt, P.stats);
-}
-
-// xDotN scatter of the bodies' samples (all of the queue).
-__global__ void __launch_bounds__(256, 3) k_wf_body_scatter(TRN_KPARAMS, const __grid_constant__ Wave W) {
-  stage_begin();
-  Cnt cnt;
-  const PrimaryItem* q = reinterpret_cast<const PrimaryItem*>(P.queue);
-  const unsigned long long n = min(*P.q_count, (unsigned long long)P.q_cap);
-  for (unsigned long long k = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; k < n;
-       k += (unsigned long long)gridDim.x * blockDim.x) {
-    const float w = W.W[k];
-    if (w == 0.f || !isfinite(w)) continue;
-    const PrimaryItem& it = q[k];
-    const ViewDesc& V = P.views[it.view];
-    xdotn_vjp(P, V, w, cam_pos(V.cam), false, -1, 0.f, 0.f, it.v0, it.v1, it.sedge, it.p0, it.far_tri, it.n, cnt);
-  }
-  flush_cnt(cnt, P.stats);
-}
-
-// Scatter of the indirect samples that reached the emitter side (list2).
-__global__ void __launch_bounds__(256, 3) k_wf_emit_scatter(TRN_KPARAMS, const __grid_constant__ Wave W, const unsigned long long* n_emit) {
-  stage_begin();
-  Cnt cnt;
-  const IndirectItem* q = reinterpret_cast<const IndirectItem*>(P.queue);
-  const unsigned long long n = *n_emit;
-  for (unsigned long long k = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; k < n;
-       k += (unsigned long long)gridDim.x * blockDim.x) {
-    const unsigned i = W.list2[k];
-    const float w = W.W[i];
-    if (w == 0.f || !isfinite(w)) continue;
-    const IndirectItem& it = q[i];
-    const SurfF xs = post_intersect(P.s, it.xs_tri, it.xs_u, it.xs_v);
-    xdotn_vjp(P, P.views[it.view], w, xs.p, true, it.xs_tri, it.xs_u, it.xs_v, it.v0, it.v1, it.sedge, it.p0,
-              it.far_tri, it.n, cnt);
-  }
-  flush_cnt(cnt, P.stats);
-}
-
-// ---------------------------------------------------------------------------
-// importance paths: direct body, indirect sensor side
-// ---------------------------------------------------------------------------
-// State: st[0] = contribution of the current depth and its pixel, st[1] =
-// continuation direction and throughput x, st[2] = throughput y, z.
-TRN_D int wi_depths(const ViewDesc& V, bool sensor) { return sensor ? min(V.D, kMaxDepth) - 1 : V.D; }
-
-template <bool SENSOR>
-TRN_D void wi_advance(const Params& P, const Wave& W, const Stage& S, int b, bool go, unsigned i, const ViewDesc* V,
-                      long long p, const SurfF& x, const F3& rdir, const F3& T, Cnt& cnt) {
-  ImportanceGen g;
-  g.shadow = g.cont = false;
-  F3 cpos;
-  if (go) {
-    const PathSmp smp{&P, V->seed, p + V->begin, p + V->slot_off};
-    const int D = wi_depths(*V, SENSOR);
-    const int o = 3 + 3 * b + (SENSOR ? 5 * D : 0);
-    cpos = cam_pos(V->cam);
-    importance_gen(P.s, V->cam, x, rdir, T, smp(o), smp(o + 1), smp(o + 2), g, cnt);
-    // nothing reads the hit behind the last depth
-    g.cont = g.cont && b + 1 < D;
-    if (g.cont) cnt.v[kCntClosest]++;
-    go = g.shadow || g.cont;
-    if (go) {
-      W.st[0][i] = make_float4(g.c.x, g.c.y, g.c.z, __int_as_float(g.pix));
-      W.st[1][i] = make_float4(g.wi.x, g.wi.y, g.wi.z, g.Tn.x);
-      W.st[2][i] = make_float4(g.Tn.y, g.Tn.z, 0.f, 0.f);
-    }
-  }
-  const unsigned long long j = warp_append(S.n_out, go);
-  push_ray(W, S.n_ray, g.shadow, cpos, g.sdir, g.stmax, (unsigned)j | kAnyRay);
-  push_ray(W, S.n_ray, g.cont, x.p, g.wi, kRayMax, (unsigned)j);
-  if (go) S.out[j] = i | (g.shadow ? kCastShadow : 0u) | (g.cont ? kCastCont : 0u);
-}
-
-template <bool SENSOR>
-__global__ void __launch_bounds__(256, 3) k_wi_start(TRN_KPARAMS, const __grid_constant__ Wave W, const __grid_constant__ Stage S) {
-  stage_begin();
-  Cnt cnt;
-  for_each_entry(min(*P.q_count, (unsigned long long)P.q_cap), [&](unsigned long long k, bool in) {
-    const unsigned i = (unsigned)k;
-    SurfF x;
-    F3 rdir;
-    const ViewDesc* V = nullptr;
-    long long p = 0;
-    bool go = false;
-    if (in) {
-      if constexpr (SENSOR) {
-        const IndirectItem& it = reinterpret_cast<const IndirectItem*>(P.queue)[i];
-        V = P.views + it.view; p = it.p(); rdir = it.rdir;
-        x = post_intersect(P.s, it.xs_tri, it.xs_u, it.xs_v);
-        W.rec[i] = 0u;
-      } else {
-        const DirectItem& it = reinterpret_cast<const DirectItem*>(P.queue)[i];
-        V = P.views + it.view; p = it.p; rdir = it.rdir;
-        x = post_intersect(P.s, it.x_tri, it.x_u, it.x_v);
-      }
-      W.W[i] = 0.f;
-      go = wi_depths(*V, SENSOR) > 0;
-    }
-    wi_advance<SENSOR>(P, W, S, 0, go, i, V, p, x, rdir, F3(1.f, 1.f, 1.f), cnt);
-  });
-  flush_cnt(cnt, P.stats);
-}
-
-// Sensor side: W.rec collects the depths whose weight is kept (bits 0-15);
-// a path that ends with a nonzero weight at some depth goes on to the emitter
-// side, with the shallowest such depth in bits 16 and up (BoundaryIndirect.cpp:
-// 158-175 pairs sensor depth b with the radiance over D - 1 - b bounces).
-template <bool SENSOR>
-__global__ void __launch_bounds__(256, 3) k_wi_step(TRN_KPARAMS, const __grid_constant__ Wave W, const __grid_constant__ Stage S) {
-  stage_begin();
-  Cnt cnt;
-  const int b = S.b;
-  for_each_entry(*S.n, [&](unsigned long long idx, bool in) {
-    unsigned i = 0;
-    SurfF x;
-    F3 rdir, T;
-    const ViewDesc* V = nullptr;
-    long long p = 0;
-    bool go = false;
-    if (in) {
-      const unsigned e = __ldcs(S.in + idx);
-      i = e & kEntryMask;
-      if constexpr (SENSOR) {
-        const IndirectItem& it = reinterpret_cast<const IndirectItem*>(P.queue)[i];
-        V = P.views + it.view; p = it.p();
-      } else {
-        const DirectItem& it = reinterpret_cast<const DirectItem*>(P.queue)[i];
-        V = P.views + it.view; p = it.p;
-      }
-      if ((e & kCastShadow) && !W.occ[idx]) {
-        const float4 a = W.st[0][i];
-        const int pix = __float_as_int(a.w);
-        if (pix >= 0) {
-          const F3 c(a.x, a.y, a.z);
-          if constexpr (SENSOR) {
-            const F3 v = g_at(P, *V, pix) * c;
-            float* sc = W.sc + 3 * ((long long)b * W.cap + i);
-            sc[0] = v.x; sc[1] = v.y; sc[2] = v.z;
-            const unsigned seen = W.rec[i];
-            const bool lit = v.x != 0.f || v.y != 0.f || v.z != 0.f;
-            // bits 16 and up hold 1 + the shallowest lit depth until the path ends
-            W.rec[i] = seen | (1u << b) | (lit && !(seen >> 16) ? (unsigned)(b + 1) << 16 : 0u);
-          } else {
-            W.W[i] += dot(g_at(P, *V, pix), reinterpret_cast<const DirectItem*>(P.queue)[i].ev0 * c);
-          }
-        }
-      }
-      if (e & kCastCont) {
-        const Hit h = get_hit(W.hit[0], idx);
-        if (h.tri >= 0) {
-          const float4 c1 = W.st[1][i], c2 = W.st[2][i];
-          x = post_intersect(P.s, h.tri, h.u, h.v);
-          rdir = F3(c1.x, c1.y, c1.z);
-          T = F3(c1.w, c2.x, c2.y);
-          go = true;  // a continuation is cast only before the last depth
-        }
-      }
-    }
-    wi_advance<SENSOR>(P, W, S, b + 1, go, i, V, p, x, rdir, T, cnt);
-  });
-  flush_cnt(cnt, P.stats);
-}
-
-// Samples whose sensor side reached the image: to list2.
-__global__ void __launch_bounds__(256) k_wi_collect(TRN_KPARAMS, const __grid_constant__ Wave W, unsigned long long* n_emit) {
-  stage_begin();
-  for_each_entry(min(*P.q_count, (unsigned long long)P.q_cap), [&](unsigned long long k, bool in) {
-    unsigned seen = 0;
-    if (in) seen = W.rec[k];
-    const bool lit = (seen >> 16) != 0u;
-    const unsigned long long j = warp_append(n_emit, lit);
-    if (lit) {
-      W.list2[j] = (unsigned)k;
-      W.rec[k] = seen - (1u << 16);
-    }
-  });
-}
-
-__global__ void __launch_bounds__(256, 3) k_wi_direct_scatter(TRN_KPARAMS, const __grid_constant__ Wave W) {
-  stage_begin();
-  Cnt cnt;
-  const DirectItem* q = reinterpret_cast<const DirectItem*>(P.queue);
-  const unsigned long long n = min(*P.q_count, (unsigned long long)P.q_cap);
-  for (unsigned long long k = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; k < n;
-       k += (unsigned long long)gridDim.x * blockDim.x) {
-    const float w = W.W[k];
-    if (w == 0.f || !isfinite(w)) continue;
-    const DirectItem& it = q[k];
-    const SurfF x = post_intersect(P.s, it.x_tri, it.x_u, it.x_v);
-    xdotn_vjp(P, P.views[it.view], w, x.p, true, it.x_tri, it.x_u, it.x_v, it.v0, it.v1, it.sedge, it.p0, it.far_tri,
-              it.n, cnt);
-  }
   flush_cnt(cnt, P.stats);
 }
 
