@@ -367,8 +367,23 @@ struct BounceRec {
 
 // One bounce in two halves, so that the wavefront kernels can run the ray
 // queries between them: radiance_gen decides the shadow ray and the
-// continuation ray of a vertex and evaluates the next-event estimate as if the
-// light were visible; radiance_resolve adds what the queries showed.
+// continuation ray of a vertex and evaluates the next-event estimate where
+// `visible` says so; radiance_resolve adds what the queries showed. `visible`
+// is true for a query that comes later; the fused step answers it at once, and a
+// shadowed light is not evaluated (nor kept over the ray's traversal).
+struct Shading {  // of a vertex
+  BsdfDesc b;
+  F3 kd;
+  Frame<float> fr;
+};
+TRN_D Shading shading_at(const DeviceScene& s, const SurfF& x) {
+  Shading m;
+  m.b = s.bsdfs[x.bsdf];
+  long long texel;
+  m.kd = bsdf_albedo(s, m.b, x.tu, x.tv, texel);
+  m.fr = make_frame(x.ns);
+  return m;
+}
 struct RadianceGen {
   F3 nee;       // contribution of the light sample if it is visible
   F3 sdir;      // shadow ray from the vertex: direction and end
@@ -380,13 +395,11 @@ struct RadianceGen {
 };
 
 // rec (may be null) takes the light sample's record.
-TRN_D void radiance_gen(const DeviceScene& s, const SurfF& x, const F3& rdir, const F3& T, float l0, float l1, float b0,
-                        float b1, float b2, RadianceGen& g, BounceRec* rec, Cnt& cnt) {
-  const BsdfDesc b = s.bsdfs[x.bsdf];
+template <class Visible>
+TRN_D void radiance_gen(const DeviceScene& s, const SurfF& x, const Shading& m, const F3& rdir, const F3& T, float l0,
+                        float l1, float b0, float b1, float b2, RadianceGen& g, BounceRec* rec, Cnt& cnt,
+                        Visible&& visible) {
   count_shade(cnt, s, x);
-  long long texel;
-  const F3 kd = bsdf_albedo(s, b, x.tu, x.tv, texel);
-  const Frame<float> fr = make_frame(x.ns);
   const F3 wo = -rdir;
   g.shadow = false;
   LightSample ls;
@@ -402,13 +415,13 @@ TRN_D void radiance_gen(const DeviceScene& s, const SurfF& x, const F3& rdir, co
     const float dotSh = dot(x.ns, wi), dotGeo = dot(x.ng, wi);
     const bool stable = d > kShadowEps && fabsf(dotSh) > kEdgeEps;
     const bool noleak = dotSh * dotGeo > 0.f;
-    if (stable && noleak) {
-      cnt.v[kCntShadow]++;
+    if (stable && noleak) cnt.v[kCntShadow]++;
+    if (stable && noleak && visible(wi, d - kShadowEps)) {
       const F3 Le = dot(-wi, nl) > 0.f ? light_radiance(s, ls.light) : F3z();
       const float G = fabsf(dot(nl, -wi)) / d2;
-      const float bpdf = bsdf_pdf_local(b, fr.to_local(wo), fr.to_local(wi)) * G;
+      const float bpdf = bsdf_pdf_local(m.b, m.fr.to_local(wo), m.fr.to_local(wi)) * G;
       const float mis = ls.pdf * ls.pdf / (ls.pdf * ls.pdf + bpdf * bpdf);
-      const F3 bv = bsdf_eval(b, fr, x.ng, kd, wo, wi, false) * fabsf(dotSh);
+      const F3 bv = bsdf_eval(m.b, m.fr, x.ng, m.kd, wo, wi, false) * fabsf(dotSh);
       for (int c = 0; c < 3; c++) g.nee[c] = T[c] * (bv[c] * 1.f * G * Le[c] / ls.pdf * mis);
       g.sdir = wi; g.stmax = d - kShadowEps; g.shadow = true;
       if (rec) {
@@ -417,8 +430,8 @@ TRN_D void radiance_gen(const DeviceScene& s, const SurfF& x, const F3& rdir, co
     }
   }
   // continuation (BSDF sampling)
-  bsdf_sample_only(b, fr, wo, b0, b1, b2, g.wi, g.pdf);
-  g.cont = g.pdf > 0.f && out_dir_valid(b, x.ns, x.ng, g.wi);
+  bsdf_sample_only(m.b, m.fr, wo, b0, b1, b2, g.wi, g.pdf);
+  g.cont = g.pdf > 0.f && out_dir_valid(m.b, x.ns, x.ng, g.wi);
   if (g.cont) cnt.v[kCntClosest]++;
 }
 
@@ -426,8 +439,9 @@ TRN_D void radiance_gen(const DeviceScene& s, const SurfF& x, const F3& rdir, co
 // 0: none was cast or it missed). Returns the contribution of this bounce
 // (already NaN-scrubbed) in contrib; x/rdir/T move to the next vertex, and the
 // return value says whether it exists.
-TRN_D bool radiance_resolve(const DeviceScene& s, SurfF& x, F3& rdir, F3& T, bool nee_ok, const F3& nee, float pdf,
-                            const Hit& h, F3& contrib, BounceRec* rec) {
+template <class ShadingAt>
+TRN_D bool radiance_resolve(const DeviceScene& s, SurfF& x, ShadingAt&& shading, F3& rdir, F3& T, bool nee_ok,
+                            const F3& nee, float pdf, const Hit& h, F3& contrib, BounceRec* rec) {
   F3 val = F3z();
   if (nee_ok) val = val + nee;
   if (rec) { rec->nee_ok = nee_ok; rec->next_ok = 0; }
@@ -436,17 +450,14 @@ TRN_D bool radiance_resolve(const DeviceScene& s, SurfF& x, F3& rdir, F3& T, boo
     if (rec) rec->scrubbed = !finite3(val);
     return false;
   }
-  const BsdfDesc b = s.bsdfs[x.bsdf];
-  long long texel;
-  const F3 kd = bsdf_albedo(s, b, x.tu, x.tv, texel);
-  const Frame<float> fr = make_frame(x.ns);
+  const Shading m = shading();
   const F3 wo = -rdir;
   const SurfF xn = post_intersect(s, h.tri, h.u, h.v);
   F3 dir = xn.p - x.p;
   const float dist2 = dot(dir, dir);
   dir = dir / sqrtf(dist2);
   const float G = fabsf(dot(xn.ng, -dir)) / dist2;
-  const F3 bv = bsdf_eval(b, fr, x.ng, kd, wo, dir, false) * fabsf(dot(x.ns, dir));
+  const F3 bv = bsdf_eval(m.b, m.fr, x.ng, m.kd, wo, dir, false) * fabsf(dot(x.ns, dir));
   const float prev_pdf = pdf * G;
   F3 Tn;
   for (int c = 0; c < 3; c++) Tn[c] = T[c] * bv[c] * G * 1.f / prev_pdf;
@@ -471,13 +482,14 @@ TRN_D bool radiance_resolve(const DeviceScene& s, SurfF& x, F3& rdir, F3& T, boo
 // The whole bounce by one thread (the fused kernels).
 TRN_D bool radiance_step(const DeviceScene& s, SurfF& x, F3& rdir, F3& T, float l0, float l1, float b0, float b1,
                          float b2, F3& contrib, BounceRec* rec, Cnt& cnt) {
+  const Shading m = shading_at(s, x);
   RadianceGen g;
-  radiance_gen(s, x, rdir, T, l0, l1, b0, b1, b2, g, rec, cnt);
-  const bool nee_ok = g.shadow && !occluded(s, x.p, g.sdir, kShadowEps, g.stmax);
+  radiance_gen(s, x, m, rdir, T, l0, l1, b0, b1, b2, g, rec, cnt,
+               [&](const F3& wi, float end) { return !occluded(s, x.p, wi, kShadowEps, end); });
   Hit h;
   h.tri = -1;
   if (g.cont && !trace<false>(s, x.p, g.wi, kShadowEps, kRayMax, h)) h.tri = -1;
-  return radiance_resolve(s, x, rdir, T, nee_ok, g.nee, g.pdf, h, contrib, rec);
+  return radiance_resolve(s, x, [&] { return m; }, rdir, T, g.shadow, g.nee, g.pdf, h, contrib, rec);
 }
 
 // One shared (non-inlined) copy of the step, with the traversal inlined inside
@@ -2193,8 +2205,11 @@ __global__ void __launch_bounds__(256, TRN_MINB) k_pixel_adj(TRN_KPARAMS) {
 // before them and on their order. A scatter of 32 queued samples at a time, all
 // of one bounce before those of the next, moved nearly cancelling components of
 // the 16.8M-sample gradient by 2 % of its RMS (0.1 % between two runs).
-// (16.8M slots of depth 5, as a wavefront and here, in ms: primary 11.2 and
-// 13.6, direct 2.4 and 2.3, indirect 28.6 and 34.6, pixel 16.0 and 23.7.)
+// And few samples pass: 0.5M slots of depth 12 take 0.69, 3.0 and 1.4 ms for
+// direct, indirect and pixel here, and 0.92, 3.8 and 1.9 with two launches per
+// bounce. The wavefront was ahead for many slots (16.8M of depth 5: primary 11.2
+// and here 11.8, direct 2.4 and 2.2, indirect 28.6 and 30.3, pixel 16.0 and
+// 19.2).
 
 // Slot of a sample in its launch, which indexes a caller's sample table.
 TRN_D long long item_gslot(const Params& P, const ViewDesc& V, long long p) {

@@ -37,22 +37,14 @@ TRN_D Pair fma2(const Pair& x, const Pair& y, const Pair& z) {
   return r;
 }
 
-// A ray as the traversal uses it: the shear of the watertight triangle test
-// (kx, ky, kz, sx, sy, sz) and, for the box slabs, the reciprocal direction
-// with the origin folded in: the distances of an axis' two planes are one
-// packed multiply-add, (lo, hi) * inv + c. c holds -o * inv, moved by
-// |o * inv| 2^-22 away from the box (down for the plane that is entered, up for
-// the one that is left): more than the rounding of o * inv and of its product,
-// so that a box is never missed (see `slab`).
-struct RayPre {
+// The shear of the watertight triangle test.
+struct RayShear {
   F3 o;
-  Pair ix, iy, iz, cx, cy, cz;
   int kx, ky, kz;
   float sx, sy, sz;
 };
 
-TRN_D RayPre ray_setup(const F3& o, const F3& d) {
-  RayPre r;
+TRN_D void ray_shear(RayShear& r, const F3& o, const F3& d) {
   r.o = o;
   float ax = fabsf(d.x), ay = fabsf(d.y), az = fabsf(d.z);
   int kz = 0; float m = ax;
@@ -65,10 +57,35 @@ TRN_D RayPre ray_setup(const F3& o, const F3& d) {
   r.sx = __fdiv_rn(d[kx], d[kz]);
   r.sy = __fdiv_rn(d[ky], d[kz]);
   r.sz = __fdiv_rn(1.f, d[kz]);
-  // reciprocal direction for the box slabs (culling only)
-  auto safe = [](float x) { return fabsf(x) < 1e-20f ? copysignf(1e-20f, x) : x; };
+}
+
+// reciprocal direction for the box slabs (culling only)
+TRN_D float ray_inv(float d) { return 1.f / (fabsf(d) < 1e-20f ? copysignf(1e-20f, d) : d); }
+
+// A ray with its reciprocal direction (one ray per thread).
+struct RayInv : RayShear { F3 inv; };
+
+TRN_D RayInv ray_inverse(const F3& o, const F3& d) {
+  RayInv r;
+  ray_shear(r, o, d);
+  r.inv = F3(ray_inv(d.x), ray_inv(d.y), ray_inv(d.z));
+  return r;
+}
+
+// A ray with the origin folded into the slabs (the stream traversal): the
+// distances of an axis' two planes are one packed multiply-add, (lo, hi) * inv +
+// c. c holds -o * inv, moved by |o * inv| 2^-22 away from the box (down for the
+// plane that is entered, up for the one that is left): more than the rounding of
+// o * inv and of its product, so that a box is never missed (see `slab`).
+struct RayPre : RayShear {
+  Pair ix, iy, iz, cx, cy, cz;
+};
+
+TRN_D RayPre ray_setup(const F3& o, const F3& d) {
+  RayPre r;
+  ray_shear(r, o, d);
   auto axis = [&](float o, float d, Pair& inv, Pair& c) {
-    inv.a = inv.b = 1.f / safe(d);
+    inv.a = inv.b = ray_inv(d);
     const float k = -(o * inv.a), e = fabsf(k) * 2.384185791015625e-7f;  // 2^-22
     c.a = inv.a < 0.f ? k + e : k - e;
     c.b = inv.a < 0.f ? k - e : k + e;
@@ -81,7 +98,7 @@ TRN_D RayPre ray_setup(const F3& o, const F3& d) {
 
 // Woop et al. 2013, section 3 (algorithm of figure 1), with the double
 // precision fallback when an edge function is exactly zero.
-TRN_D bool intersect_tri(const RayPre& r, const F3& p0, const F3& p1, const F3& p2,
+TRN_D bool intersect_tri(const RayShear& r, const F3& p0, const F3& p1, const F3& p2,
                          float tmin, float tmax, float& t_out, float& u_out, float& v_out) {
   F3 A(__fsub_rn(p0.x, r.o.x), __fsub_rn(p0.y, r.o.y), __fsub_rn(p0.z, r.o.z));
   F3 B(__fsub_rn(p1.x, r.o.x), __fsub_rn(p1.y, r.o.y), __fsub_rn(p1.z, r.o.z));
@@ -119,9 +136,9 @@ TRN_D bool intersect_tri(const RayPre& r, const F3& p0, const F3& p1, const F3& 
 
 // ---- box steps ---------------------------------------------------------------
 // What bounds traversal here is instruction issue and the L1's data path (one
-// lane's line per cycle and SM). A node is fetched in two 32-byte loads, a
-// triangle in two; plane distances are one multiply-add each and the slab's
-// extremes three-input min/max.
+// lane's line per cycle and SM). The stream traversal fetches a node in two
+// 32-byte loads and a triangle in two; its plane distances are one multiply-add
+// each and the slab's extremes three-input min/max.
 TRN_D float max3(float a, float b, float c) {
 #if defined(__CUDA_ARCH__) && __CUDA_ARCH__ >= 1000
   float r;
@@ -141,16 +158,9 @@ TRN_D float min3(float a, float b, float c) {
 #endif
 }
 
-// 32 bytes at a 32-byte aligned address, WIDE in one load (the stream
-// traversal; ptxas 12.9 crashes on the wide load in the fused kernels, which
-// spill).
-template <bool WIDE>
+// 32 bytes at a 32-byte aligned address in one load. (Not in the fused kernels:
+// ptxas 12.9 crashes on it where registers are spilled.)
 TRN_D void load8(const void* p, float4& a, float4& b) {
-  if (!WIDE) {
-    a = __ldg(static_cast<const float4*>(p));
-    b = __ldg(static_cast<const float4*>(p) + 1);
-    return;
-  }
 #if defined(__CUDA_ARCH__) && __CUDA_ARCH__ >= 1000
   asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
       : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
@@ -178,12 +188,19 @@ TRN_D bool slab(const RayPre& r, const Pair& bx, const Pair& by, const Pair& bz,
   return tnear <= tf * 1.0000004f;
 }
 
-// Traversal stacks: entries are (child, bits of its box's entry distance).
-struct LocalStack {
-  int2 e[kStackSize];
-  TRN_D void set(int i, int2 v) { e[i] = v; }
-  TRN_D int2 get(int i) const { return e[i]; }
-};
+// The same with an axis at a time and no slack in the ray.
+TRN_D bool slab(const RayInv& r, float lx, float hx, float ly, float hy, float lz, float hz, float tmin, float tmax,
+                float& tnear) {
+  const float x0 = (lx - r.o.x) * r.inv.x, x1 = (hx - r.o.x) * r.inv.x;
+  const float y0 = (ly - r.o.y) * r.inv.y, y1 = (hy - r.o.y) * r.inv.y;
+  const float z0 = (lz - r.o.z) * r.inv.z, z1 = (hz - r.o.z) * r.inv.z;
+  tnear = fmaxf(fmaxf(fminf(x0, x1), fminf(y0, y1)), fmaxf(fminf(z0, z1), tmin));
+  const float tf = fminf(fminf(fmaxf(x0, x1), fmaxf(y0, y1)), fminf(fmaxf(z0, z1), tmax));
+  return tnear <= tf * 1.0000004f;
+}
+
+// Traversal stack of the stream: entries are (child, bits of its box's entry
+// distance).
 // The stream traversal's first entries lie in shared memory: the lanes of a
 // warp stand at different depths, and an access to local memory then takes a
 // pass through the L1 for every depth among them, where here each lane has its
@@ -216,13 +233,13 @@ TRN_D float pop_limit(float best_t) { return best_t + fabsf(best_t) * 4e-7f; }
 // 0) or kTracePop; the farther one goes to the stack as (child, bits of its
 // entry distance). Straight-line code: lanes of a warp differ in which children
 // they hit, and every branch would run once more per warp.
-template <bool WIDE, class Stack>
+template <class Stack>
 TRN_D int visit_node(const DeviceScene& s, const RayPre& r, int node, float tmin, float best_t, Stack& stack, int& sp,
                      int* err) {
   const char* n = reinterpret_cast<const char*>(s.nodes) + ((size_t)(unsigned)node << 6);
   float4 a, b, c, d;
-  load8<WIDE>(n, a, b);
-  load8<WIDE>(n + 32, c, d);
+  load8(n, a, b);
+  load8(n + 32, c, d);
   float t0, t1;
   const bool h0 = slab(r, {a.x, a.y}, {a.z, a.w}, {b.x, b.y}, tmin, best_t, t0);
   const bool h1 = slab(r, {b.z, b.w}, {c.x, c.y}, {c.z, c.w}, tmin, best_t, t1);
@@ -250,11 +267,17 @@ TRN_D void pop_entry(const Stack& stack, int& sp, float limit, int& cur) {
   }
 }
 
+// The triangle of a leaf, read in two loads (WIDE) or three.
 template <bool WIDE>
 TRN_D void leaf_tri(const DeviceScene& s, int leaf, F3& p0, F3& p1, F3& p2, int& tri) {
   const char* q = reinterpret_cast<const char*>(s.tri_verts) + ((size_t)(unsigned)leaf << 6);
   float4 a, b;
-  load8<WIDE>(q, a, b);
+  if (WIDE) {
+    load8(q, a, b);
+  } else {
+    a = __ldg(reinterpret_cast<const float4*>(q));
+    b = __ldg(reinterpret_cast<const float4*>(q) + 1);
+  }
   const float2 c = __ldg(reinterpret_cast<const float2*>(q + 32));
   p0 = F3(a.x, a.y, a.z); tri = __float_as_int(a.w);
   p1 = F3(b.x, b.y, b.z); p2 = F3(b.w, c.x, c.y);
@@ -268,34 +291,55 @@ TRN_D bool ray_is_void(const F3& o, const F3& d) {
          (d.x == 0.f && d.y == 0.f && d.z == 0.f);
 }
 
-// Closest hit (ANY == false) or occlusion (ANY == true). Returns true on hit.
+// Closest hit (ANY == false) or occlusion (ANY == true) of one ray by one
+// thread. Returns true on hit. The stack holds nodes alone and the slab is the
+// plain one: next to the stream traversal's steps this is a shorter chain for a
+// lone ray and half the local memory for a fused kernel (allocation-free terms
+// of 1M samples of depth 12 on 102,400 triangles with the stream's steps and
+// here, in ms: interior 11.0 and 9.8, primary 7.0 and 5.5, indirect 15.0 and
+// 12.5, pixel 4.2 and 3.1).
 template <bool ANY>
 TRN_D bool trace(const DeviceScene& s, const F3& o, const F3& d, float tmin, float tmax, Hit& hit,
                  int* err = nullptr) {
   hit.tri = -1; hit.u = 0.f; hit.v = 0.f; hit.t = -1.f;
   if (s.nt <= 0 || ray_is_void(o, d)) return false;
-  const RayPre r = ray_setup(o, d);
+  const RayInv r = ray_inverse(o, d);
   float best_t = tmax;
   int best_tri = -1;
-  LocalStack stack;
+  int stack[kStackSize];
   int sp = 0, cur = s.nt == 1 ? ~0 : 0;
   // leaves are visited through the loop like inner nodes, so the triangle
   // test is instantiated once per traversal (smaller code)
   for (;;) {
-    while (cur == kTracePop) pop_entry(stack, sp, pop_limit(best_t), cur);
-    if (cur == kTraceDone) break;
-    if (cur >= 0) {
-      cur = visit_node<false>(s, r, cur, tmin, best_t, stack, sp, err);
+    if (cur < 0) {
+      F3 p0, p1, p2; int tri;
+      leaf_tri<false>(s, ~cur, p0, p1, p2, tri);
+      float t, u, v;
+      // best_tri = -1 before the first hit: a hit at exactly the ray's end is none
+      if (intersect_tri(r, p0, p1, p2, tmin, INFINITY, t, u, v) && (t < best_t || (t == best_t && tri < best_tri))) {
+        best_t = t; best_tri = tri; hit.u = u; hit.v = v;
+        if (ANY) break;
+      }
+      if (sp == 0) break;
+      cur = stack[--sp];
       continue;
     }
-    F3 p0, p1, p2; int tri;
-    leaf_tri<false>(s, ~cur, p0, p1, p2, tri);
-    cur = kTracePop;
-    float t, u, v;
-    // best_tri = -1 before the first hit: a hit at exactly the ray's end is none
-    if (intersect_tri(r, p0, p1, p2, tmin, INFINITY, t, u, v) && (t < best_t || (t == best_t && tri < best_tri))) {
-      best_t = t; best_tri = tri; hit.u = u; hit.v = v;
-      if (ANY) break;
+    const BvhNode* n = &s.nodes[cur];
+    const float4 a = __ldg(&n->a), b = __ldg(&n->b), c = __ldg(&n->c);
+    const int4 e = __ldg(&n->d);
+    float t0, t1;
+    const bool h0 = slab(r, a.x, a.y, a.z, a.w, b.x, b.y, tmin, best_t, t0);
+    const bool h1 = slab(r, b.z, b.w, c.x, c.y, c.z, c.w, tmin, best_t, t1);
+    if (h0 && h1) {
+      const bool second = t1 < t0;   // the nearer one is child 1
+      if (sp < kStackSize) stack[sp++] = second ? e.x : e.y;
+      else if (err) atomicExch(err, 1);
+      cur = second ? e.y : e.x;
+    } else if (h0 || h1) {
+      cur = h0 ? e.x : e.y;
+    } else {
+      if (sp == 0) break;
+      cur = stack[--sp];
     }
   }
   if (best_tri < 0) return false;
@@ -381,7 +425,7 @@ TRN_D void trace_stream(const DeviceScene& s, Fetch&& fetch, Load&& load, Store&
         leaf = cur;
         cur = kTracePop;
       }
-      if (cur >= 0 && cur < kTracePop) cur = visit_node<true>(s, r, cur, tmin, best_t, stack, sp, err);
+      if (cur >= 0 && cur < kTracePop) cur = visit_node(s, r, cur, tmin, best_t, stack, sp, err);
     }
     const unsigned leaves = __ballot_sync(0xffffffffu, leaf < 0);
     if (4 * __popc(leaves) < TRN_LEAF_SHARE * (32 - __popc(idle)) &&

@@ -162,8 +162,8 @@ TRN_D void wf_advance(const Params& P, const Wave& W, const Stage& S, int b, boo
     const int o = 2 + 5 * b;
     BounceRec br;
     constexpr bool rec = MODE != kWfFwd;
-    radiance_gen(P.s, q.x, q.rdir, q.T, smp(o), smp(o + 1), smp(o + 2), smp(o + 3), smp(o + 4), g, rec ? &br : nullptr,
-                 cnt);
+    radiance_gen(P.s, q.x, shading_at(P.s, q.x), q.rdir, q.T, smp(o), smp(o + 1), smp(o + 2), smp(o + 3), smp(o + 4), g, rec ? &br : nullptr,
+                 cnt, [](const F3&, float) { return true; });
     W.st[0][i] = make_float4(__int_as_float(q.x.tri), q.x.u, q.x.v, g.pdf);
     W.st[1][i] = make_float4(q.rdir.x, q.rdir.y, q.rdir.z, q.T.x);
     W.st[2][i] = make_float4(q.T.y, q.T.z, q.L.x, q.L.y);
@@ -340,7 +340,7 @@ __global__ void __launch_bounds__(256, 3) k_wf_shade(TRN_KPARAMS, const __grid_c
       q.x = post_intersect(s, __float_as_int(a.x), a.y, a.z);
       F3 c;
       BounceRec br;
-      const bool more = radiance_resolve(s, q.x, q.rdir, q.T, nee_ok, F3(c3.y, c3.z, c3.w), a.w, h, c, rec ? &br : nullptr);
+      const bool more = radiance_resolve(s, q.x, [&] { return shading_at(s, q.x); }, q.rdir, q.T, nee_ok, F3(c3.y, c3.z, c3.w), a.w, h, c, rec ? &br : nullptr);
       q.L = q.L + c;
       const bool dark = q.T.x == 0.f && q.T.y == 0.f && q.T.z == 0.f;
       if constexpr (rec) {
