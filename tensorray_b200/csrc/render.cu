@@ -2496,10 +2496,6 @@ __global__ void k_view_loss(long long npix, const ViewDesc* views, const long lo
 // rays are spread over all warps of the GPU as well, down to one each, since a
 // query is then as long as its longest ray (1,000 rays on 7,000 triangles: 56 us
 // with four per warp, 46 with one).
-// Against one ray per thread (the traversal before), on 102,400 triangles, closest
-// hit: 1,000 rays 123 -> 83 us, 4,099 111 -> 93, 2^20 1.44x as fast. In between
-// one slow ray decides, and a box step takes a lone ray a fifth longer here:
-// 32,000 rays 206 -> 250 us, 300,000 340 -> 323.
 template <bool ANY>
 __global__ void __launch_bounds__(TRN_TRACE_BLOCK, TRN_TRACE_MINB)
     k_query(const __grid_constant__ DeviceScene s, int n, int chunk, const float* org, const float* dir,
@@ -2523,6 +2519,19 @@ __global__ void __launch_bounds__(TRN_TRACE_BLOCK, TRN_TRACE_MINB)
       if (ANY) tri_[i] = tri >= 0 ? 0 : 1;
       else { tri_[i] = tri; u_[i] = u; v_[i] = v; t_[i] = t; }
     }, err);
+}
+
+// The same with one ray per thread, for the batches that query_streams() names.
+template <bool ANY>
+__global__ void __launch_bounds__(128)
+    k_query_one(const __grid_constant__ DeviceScene s, int n, const float* org, const float* dir, const float* tmin,
+                const float* tmax, int* tri, float* u, float* v, float* t, int* err) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  Hit h;
+  const bool hit = trace<ANY>(s, make_f3(org + 3ll * i), make_f3(dir + 3ll * i), tmin[i], tmax[i], h, err);
+  if (ANY) tri[i] = hit ? 0 : 1;
+  else { tri[i] = h.tri; u[i] = h.u; v[i] = h.v; t[i] = h.t; }
 }
 
 }  // namespace trn
@@ -2767,8 +2776,25 @@ void launch_dims(const trn_launch* ln, long long total, int& grid, int& block) {
   grid = (int)std::max<long long>(1, std::min(want, need));
 }
 
-// Rays per tile of a query: down to 4 while all warps that fit the GPU get one,
-// up to 32.
+// Whether a query of n rays runs as a stream. A stream wins where most lanes
+// would idle (few rays: one per warp) and where rays are many (its warps refill).
+// In between, some warps hold several rays from the start and none is refilled
+// for long: a lone long ray decides, and its box step takes a fifth longer in the
+// stream. That holds longer in a large tree, whose longest rays are ten times the
+// mean (324 nodes against 32 on 102,400 triangles; 70 against 20 on 1,284).
+// One ray per thread against the stream, closest hit / occlusion in us:
+//   triangles        16,000 rays         32,000             128,000            300,000            600,000
+//     1,284     48/42 and 39/37     49/44 and 48/45    65/56 and 60/55  123/107 and 102/91  220/183 and 179/156
+//     7,000     84/76 and 80/70     88/81 and 93/87  114/99 and 121/103 205/181 and 177/160 349/285 and 258/231
+//   102,400   121/101 and 122/102 208/195 and 251/242 262/191 and 314/222 318/258 and 322/242 528/432 and 472/456
+//   200,000   136/120 and 131/129 138/125 and 154/133 267/233 and 297/253 343/284 and 428/327 545/440 and 456/357
+bool query_streams(int n, int triangles) {
+  const int lanes = sms() * TRN_TRACE_MINB * TRN_TRACE_BLOCK;
+  return n < lanes / 8 || n >= (triangles > 32768 ? lanes * 5 / 2 : lanes * 3 / 2);
+}
+
+// Rays per tile of a stream: as few as give every warp that fits the GPU one
+// tile, up to 32.
 void query_dims(int n, int& grid, int& chunk) {
   const long long blocks = (long long)sms() * TRN_TRACE_MINB, warps = blocks * (TRN_TRACE_BLOCK / 32);
   chunk = (int)std::min<long long>(32, std::max<long long>(1, (n + warps - 1) / warps));
@@ -3823,9 +3849,13 @@ int trn_intersect(trn_scene* s, int n, const float* org, const float* dir, const
   if (!s || !s->configured) { set_error("trn_intersect: scene not configured"); return -1; }
   if (n <= 0) return 0;
   if (!org || !dir || !tmin || !tmax || !tri || !u || !v || !t) { set_error("trn_intersect: null argument"); return -1; }
-  int grid, chunk;
-  query_dims(n, grid, chunk);
-  k_query<false><<<grid, TRN_TRACE_BLOCK, 0, st>>>(s->view(), n, chunk, org, dir, tmin, tmax, tri, u, v, t, s->err);
+  if (query_streams(n, s->nt)) {
+    int grid, chunk;
+    query_dims(n, grid, chunk);
+    k_query<false><<<grid, TRN_TRACE_BLOCK, 0, st>>>(s->view(), n, chunk, org, dir, tmin, tmax, tri, u, v, t, s->err);
+  } else {
+    k_query_one<false><<<(n + 127) / 128, 128, 0, st>>>(s->view(), n, org, dir, tmin, tmax, tri, u, v, t, s->err);
+  }
   count_launch(1);
   TRN_CUDA_TRY(cudaGetLastError());
   return 0;
@@ -3836,10 +3866,15 @@ int trn_occluded(trn_scene* s, int n, const float* org, const float* dir, const 
   if (!s || !s->configured) { set_error("trn_occluded: scene not configured"); return -1; }
   if (n <= 0) return 0;
   if (!org || !dir || !tmin || !tmax || !vis) { set_error("trn_occluded: null argument"); return -1; }
-  int grid, chunk;
-  query_dims(n, grid, chunk);
-  k_query<true><<<grid, TRN_TRACE_BLOCK, 0, st>>>(s->view(), n, chunk, org, dir, tmin, tmax, vis, nullptr, nullptr,
-                                                  nullptr, s->err);
+  if (query_streams(n, s->nt)) {
+    int grid, chunk;
+    query_dims(n, grid, chunk);
+    k_query<true><<<grid, TRN_TRACE_BLOCK, 0, st>>>(s->view(), n, chunk, org, dir, tmin, tmax, vis, nullptr, nullptr,
+                                                    nullptr, s->err);
+  } else {
+    k_query_one<true><<<(n + 127) / 128, 128, 0, st>>>(s->view(), n, org, dir, tmin, tmax, vis, nullptr, nullptr,
+                                                       nullptr, s->err);
+  }
   count_launch(1);
   TRN_CUDA_TRY(cudaGetLastError());
   return 0;

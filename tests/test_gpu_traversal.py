@@ -80,3 +80,29 @@ def test_rays_without_a_direction_hit_nothing(built_lib):
     args = [x.cuda() for x in (org, d, tmin, tmax)]
     assert bool((scene.intersect(*args)[0] == -1).all())
     assert bool((scene.occluded(*args) == 1).all())
+
+
+def test_queries_of_every_size_agree(built_lib):
+    """A batch's size decides between the two traversals (one ray per thread from
+    1/8 of the GPU's lanes to 3/2 of them, or 5/2 in a large tree): the same rays
+    give the same results in any batch, at both sides of each limit."""
+    lanes = torch.cuda.get_device_properties(0).multi_processor_count * 8 * 128
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    for spec, high in ((scenes.config1_scene(8, 8), lanes * 3 // 2), (scenes.config2_scene(8, 8, tris=40_000), lanes * 5 // 2)):
+        scene = api.Scene(spec)
+        scene.configure()
+        n = high + 1
+        org = torch.randn(n, 3, generator=gen, device="cuda") * 2
+        d = torch.randn(n, 3, generator=gen, device="cuda") - 0.5 * org
+        d /= d.norm(dim=1, keepdim=True)
+        rays = (org, d, torch.full((n,), 1e-2, device="cuda"), torch.full((n,), 1e32, device="cuda"))
+        small = lanes // 8 - 1
+        parts = [[x[i:i + small].contiguous() for x in rays] for i in range(0, n, small)]
+        ref = [torch.cat(x) for x in zip(*(scene.intersect(*p) for p in parts))]
+        vis = torch.cat([scene.occluded(*p) for p in parts])
+        assert 0.1 < float((ref[0] >= 0).float().mean()) < 0.9
+        for k in (lanes // 8 - 1, lanes // 8, high - 1, high, high + 1):
+            part = [x[:k].contiguous() for x in rays]
+            for a, b in zip(scene.intersect(*part), ref):
+                assert torch.equal(a, b[:k])
+            assert torch.equal(scene.occluded(*part), vis[:k])
