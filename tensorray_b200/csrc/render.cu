@@ -2842,6 +2842,9 @@ void launch(K kernel, const trn_launch* ln, long long total, const Params& P, cu
 constexpr long long kRound = 1LL << TRN_ROUND_LOG2;
 constexpr long long kReplayRound = 1LL << TRN_PATH_ROUND_LOG2;
 constexpr int kWaveCounters = 256;
+#ifndef TRN_TAIL_LOG2
+#define TRN_TAIL_LOG2 17
+#endif
 
 // Slots (or paths) per round: the launch's round_log2 when set, never above
 // the default that the buffers are sized for.
@@ -2972,7 +2975,8 @@ struct WaveRun {
   // Launches K over the round: as many blocks as fit the GPU at once (the
   // kernels stride over a count they read on the device), or the shape the
   // caller asked for; fewer when the round is small.
-  template <auto K, class... A>
+  // ALL: the GPU's worth of blocks for any round (for_each_spread).
+  template <auto K, bool ALL = false, class... A>
   void go(A... args) const {
     const int block = ln && ln->block > 0 ? ln->block : 128;
     int per_sm = ln && ln->blocks_per_sm > 0 ? ln->blocks_per_sm : 0;
@@ -2983,7 +2987,8 @@ struct WaveRun {
       }();
       per_sm = std::max(1, fit * 128 / block);
     }
-    launch<K>(std::min<long long>((long long)sms() * per_sm, (W.cap + block - 1) / block), block, args...);
+    const long long most = (long long)sms() * per_sm;
+    launch<K>(ALL ? most : std::min<long long>(most, (W.cap + block - 1) / block), block, args...);
   }
   template <auto K, class... A>
   void launch(long long grid, int block, A... args) const {
@@ -3012,13 +3017,30 @@ struct WaveRun {
     launch<k_trace>(std::min((long long)sms() * TRN_TRACE_MINB, need), TRN_TRACE_BLOCK, P.s, W, r0, n, ctr(),
                     W.hit[which], P.err);
   }
+  // First bounce that the tail kernel runs for a round of n samples. A bounce by
+  // launches is as long as its longest ray twice over; it is worth that while
+  // there are more paths than the GPU holds threads (2^17). About half of the paths
+  // are left after each bounce. Images of depth 12 on 102,400 triangles, us, with a
+  // launch pair per bounce / the tail from 2^16, 2^17 or 2^18 paths on / one thread
+  // per path: 768 samples 440 / 266 / 374, 12,288 781 / 454 / 587, 131,072 1308 /
+  // 877, 865, 879 / 1018, 393,216 1569 / 1232, 1107, 1415 / 1593, 1,048,576 2393 /
+  // 1977, 1881, 2165 / 3253, 4,194,304 5148 / 4879, 4741, 4989 / 9914.
+  static int tail_bounce(long long n) {
+    int b = 1;
+    while ((n >> b) > (1 << TRN_TAIL_LOG2)) b++;
+    return b;
+  }
   // bounces of the entries that the start kernel left in list[0]
   template <int MODE>
-  void bounces(const unsigned long long* n, unsigned long long* n_ray, int depth) {
+  void bounces(const unsigned long long* n, unsigned long long* n_ray, int depth, int tail) {
     for (int b = 0; b < depth; b++) {
       trace(0, n_ray, 0);
       Stage S{n, W.list[b & 1], ctr(), W.list[(b + 1) & 1], ctr(), nullptr, b};
-      go<k_wf_shade<MODE>>(P, W, S, R);
+      if (b + 1 >= tail && b + 1 < depth) {
+        go<k_wf_shade<MODE, true>, true>(P, W, S, R);
+        return;
+      }
+      go<k_wf_shade<MODE, false>>(P, W, S, R);
       n = S.n_out; n_ray = S.n_ray;
     }
   }
@@ -3085,7 +3107,7 @@ int path_wave(trn_viewset* vs, const Params& P0, const trn_launch* ln, long long
     r.trace(0, rays, 0);
     Stage S{rays, r.W.list[1], r.ctr(), r.W.list[0], r.ctr(), r.ctr(), 0};
     r.go<k_wf_start<MODE>>(r.P, r.W, S, r.R);
-    r.bounces<MODE>(S.n_out, S.n_ray, depth);
+    r.bounces<MODE>(S.n_out, S.n_ray, depth, WaveRun::tail_bounce(n));
     if (MODE == kWfReplay) r.go<k_path_reverse<false>>(r.P, r.R);
     else r.go<k_wf_pixels>(r.P, r.W, n);
   }

@@ -89,6 +89,16 @@ TRN_D void for_each_entry(unsigned long long n, F&& body) {
     body(k0 + lane, k0 + lane < n);
 }
 
+// The same with the entries spread over all warps, down to one each, for work
+// that takes every lane another way: few lanes of a warp then wait for each other.
+template <class F>
+TRN_D void for_each_spread(unsigned long long n, F&& body) {
+  const int lane = threadIdx.x & 31;
+  const unsigned long long warps = gridDim.x * (blockDim.x >> 5), w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const unsigned long long own = min(32ull, max(1ull, (n + warps - 1) / warps));
+  for (unsigned long long k0 = w * own; k0 < n; k0 += warps * own) body(k0 + lane, lane < own && k0 + lane < n);
+}
+
 // ---------------------------------------------------------------------------
 // ray queries of a stage: rays [r0, r0 + *n_ray) of the queue
 // ---------------------------------------------------------------------------
@@ -98,7 +108,8 @@ TRN_D void for_each_entry(unsigned long long n, F&& body) {
 
 // Each warp starts on rays of its own and then fetches from `next`; few rays
 // are spread over all warps (a query is as long as its longest ray, and a warp
-// of few rays takes fewer turns).
+// of few rays takes fewer turns). (One ray per thread for batches of 19K to 230K,
+// as for a program's own rays: images of 131,072 samples 130 -> 163 us.)
 __global__ void __launch_bounds__(TRN_TRACE_BLOCK, TRN_TRACE_MINB)
     k_trace(const __grid_constant__ DeviceScene s, const __grid_constant__ Wave W, long long r0, const unsigned long long* n_ray,
             unsigned long long* next, float4* hits, int* err) {
@@ -150,6 +161,25 @@ struct WfPath {
   F3 rdir, T, L;
 };
 
+TRN_D bool is_dark(const F3& T) { return T.x == 0.f && T.y == 0.f && T.z == 0.f; }
+
+// Bounce k's light sample, and what the bounce came to (the vertex q when it
+// goes on), into record kr.
+TRN_D void wf_record_light(const PathSoA& R, unsigned kr, int k, const BounceRec& br) {
+  LRec& l = R.br(kr, k);
+  l.ltri = br.ltri; l.lu = br.lu; l.lv = br.lv; l.lpdf = br.lpdf; l.lmis = br.lmis;
+}
+TRN_D void wf_record(const PathSoA& R, unsigned kr, int k, const BounceRec& br, bool more, const WfPath& q) {
+  // a scrubbed (non-finite) bounce contributes nothing and carries no gradient
+  if (br.nee_ok && !br.scrubbed) R.nee(kr) |= 1u << k;
+  if (!more) return;
+  R.br(kr, k).ppdf = br.prev_pdf;
+  R.vr(kr, k + 1) = {q.x.tri, q.x.u, q.x.v};
+  R.Tk(kr, k + 1) = q.T;
+  R.Mk(kr, k + 1) = (br.scrubbed || br.emis == 0.f) ? F3z() : br.eLe * br.emis;
+  R.K(kr) = k + 1;
+}
+
 // Decides the rays of bounce b for the lanes that go on, appends them and the
 // lanes' list entries, and stores the path state. All lanes of the warp call it.
 template <int MODE>
@@ -168,10 +198,7 @@ TRN_D void wf_advance(const Params& P, const Wave& W, const Stage& S, int b, boo
     W.st[1][i] = make_float4(q.rdir.x, q.rdir.y, q.rdir.z, q.T.x);
     W.st[2][i] = make_float4(q.T.y, q.T.z, q.L.x, q.L.y);
     W.st[3][i] = make_float4(q.L.z, g.nee.x, g.nee.y, g.nee.z);
-    if (rec && g.shadow) {
-      LRec& l = R.br(W.rec[i], b + 1);
-      l.ltri = br.ltri; l.lu = br.lu; l.lv = br.lv; l.lpdf = br.lpdf; l.lmis = br.lmis;
-    }
+    if (rec && g.shadow) wf_record_light(R, W.rec[i], b + 1, br);
   }
   const unsigned long long j = warp_append(S.n_out, go);
   push_ray(W, S.n_ray, g.shadow, q.x.p, g.sdir, g.stmax, (unsigned)j | kAnyRay);
@@ -310,15 +337,19 @@ __global__ void __launch_bounds__(256, 3) k_wf_start(TRN_KPARAMS, const __grid_c
 // next for the paths that go on. Bound by the gathers of the two vertices
 // (latency) and the state traffic; 32 paths of a warp take the same branches
 // but for material and light.
-template <int MODE>
+// TAIL: runs those paths to their ends instead, one thread each, with the fused
+// bounce, for the late bounces of few paths (WaveRun::tail_bounce). Bound by the
+// chain of the longest path: its paths are spread over all warps (12,288 samples
+// of depth 5 on 1,284 triangles: 236 us packed, 163 spread).
+template <int MODE, bool TAIL>
 __global__ void __launch_bounds__(256, 3) k_wf_shade(TRN_KPARAMS, const __grid_constant__ Wave W, const __grid_constant__ Stage S,
                            const __grid_constant__ PathSoA R) {
   stage_begin();
   Cnt cnt;
   const DeviceScene& s = P.s;
   constexpr bool rec = MODE != kWfFwd;
-  const int b = S.b, k = b + 1;
-  for_each_entry(*S.n, [&](unsigned long long idx, bool in) {
+  const int b = S.b;
+  auto each = [&](unsigned long long idx, bool in) {
     WfPath q;
     unsigned i = 0;
     const ViewDesc* V = nullptr;
@@ -342,24 +373,28 @@ __global__ void __launch_bounds__(256, 3) k_wf_shade(TRN_KPARAMS, const __grid_c
       BounceRec br;
       const bool more = radiance_resolve(s, q.x, [&] { return shading_at(s, q.x); }, q.rdir, q.T, nee_ok, F3(c3.y, c3.z, c3.w), a.w, h, c, rec ? &br : nullptr);
       q.L = q.L + c;
-      const bool dark = q.T.x == 0.f && q.T.y == 0.f && q.T.z == 0.f;
-      if constexpr (rec) {
-        const unsigned kr = W.rec[i];
-        // a scrubbed (non-finite) bounce contributes nothing and carries no gradient
-        if (br.nee_ok && !br.scrubbed) R.nee(kr) |= 1u << k;
-        if (more) {
-          R.br(kr, k).ppdf = br.prev_pdf;
-          R.vr(kr, k + 1) = {q.x.tri, q.x.u, q.x.v};
-          R.Tk(kr, k + 1) = q.T;
-          R.Mk(kr, k + 1) = (br.scrubbed || br.emis == 0.f) ? F3z() : br.eLe * br.emis;
-          R.K(kr) = k + 1;
+      if constexpr (rec) wf_record(R, W.rec[i], b + 1, br, more, q);
+      go = more && !is_dark(q.T) && b + 1 < V->D;
+      if constexpr (TAIL) {
+        const PathSmp smp{&P, V->seed, p + V->begin, p + V->slot_off};
+        for (int t = b + 1; go; t++) {
+          const int o = 2 + 5 * t;
+          const bool on = radiance_step(s, q.x, q.rdir, q.T, smp(o), smp(o + 1), smp(o + 2), smp(o + 3), smp(o + 4), c,
+                                        rec ? &br : nullptr, cnt);
+          q.L = q.L + c;
+          if constexpr (rec) {
+            if (br.nee_ok) wf_record_light(R, W.rec[i], t + 1, br);
+            wf_record(R, W.rec[i], t + 1, br, on, q);
+          }
+          go = on && !is_dark(q.T) && t + 1 < V->D;
         }
       }
-      go = more && !dark && b + 1 < V->D;
       if (!go) wf_finish<MODE>(W, *V, p, q.L, cnt);
     }
-    wf_advance<MODE>(P, W, S, b + 1, go, i, V, p, q, R, cnt);
-  });
+    if constexpr (!TAIL) wf_advance<MODE>(P, W, S, b + 1, go, i, V, p, q, R, cnt);
+  };
+  if constexpr (TAIL) for_each_spread(*S.n, each);
+  else for_each_entry(*S.n, each);
   flush_cnt(cnt, P.stats);
 }
 

@@ -86,3 +86,32 @@ def test_capture_without_buffers_and_replay_after_growth(built_lib):
     out.zero_()
     graphs[1].replay()
     torch.testing.assert_close(out, ref, rtol=1e-5, atol=1e-6)
+
+
+@pytest.mark.parametrize("depth", [1, 2, 3, 6, 16])
+def test_late_bounces_give_the_same_in_either_form(built_lib, depth):
+    """The bounces that the tail kernel runs begin earlier in a small round (here
+    at the first) than in a large one (at the fifth of 3.1M samples): a small
+    view's image is the same bit for bit alone and beside a large view, and its
+    gradient but for the order of the adds."""
+    sc = _scene()
+    small = api.Camera((0.5, 1.5, 3.5), (0.0, 0.0, 0.0), (0.0, 1.0, 0.0), 37, 23, 45.0)
+    large = api.Camera((0.0, 0.0, 4.0), (0.0, 0.0, 0.0), (0.0, 1.0, 0.0), 512, 512, 45.0)
+    opts = api.RenderOptions(3, depth, 0, 0, 0, 0, 0)
+    n = small.width * small.height
+    gen = torch.Generator(device="cuda").manual_seed(depth)
+    d1 = torch.rand(n, 3, generator=gen, device=sc.device) - 0.3
+    for cache in (0, 1 << 32):
+        got = []
+        for cams, spps in (([small], [5]), ([small, large], [5, 12])):
+            vs = api.ViewSet(sc, cams, spps, seeds=list(range(len(cams))))
+            vs.set_path_cache(cache)
+            img = vs.render(api.TRN_PATH_TRACER, opts)[:n].clone()
+            d = torch.zeros(vs.npix, 3, device=sc.device)
+            d[:n] = d1
+            vs.render_grad(api.TRN_PATH_TRACER, opts, d)
+            got.append((img, sc.get_grads()["positions"].clone()))
+            sc.clear_grads()
+        assert torch.equal(got[0][0], got[1][0])
+        assert float(got[0][1].abs().sum()) > 0
+        assert rel_l2(got[0][1], got[1][1]) <= 1e-5
