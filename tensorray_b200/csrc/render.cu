@@ -2560,6 +2560,7 @@ struct trn_viewset {
   long long npix = 0;
   std::vector<trn_view> h_views;
   std::vector<long long> h_pbegin;
+  std::vector<long long> h_slots;  // of each view, in the uploaded table
   ViewDesc* views = nullptr;      // device [nviews]
   long long* vbegin = nullptr;    // device [nviews], rewritten per integrator (spp differs)
   long long* pbegin = nullptr;    // device [nviews] first pixel of each view
@@ -2669,6 +2670,7 @@ int upload_views(trn_viewset* vs, const trn_render_options* o, int integrator, i
   ViewDesc* d = vs->h_stage + (size_t)slot * vs->cap;
   long long* begin = vs->h_stage_begin + (size_t)slot * 2 * vs->cap;
   total = 0;
+  vs->h_slots.assign(vs->nviews, 0);
   for (int v = 0; v < vs->nviews; v++) {
     const trn_view& hv = vs->h_views[v];
     const int spp = spp_override >= 0 ? spp_override : hv.spp;
@@ -2696,6 +2698,7 @@ int upload_views(trn_viewset* vs, const trn_render_options* o, int integrator, i
     d[v].pcdf = vs->pcdf ? vs->pcdf + (long long)v * vs->ne : nullptr;
     d[v].pint = vs->pint ? vs->pint + v : nullptr;
     begin[v] = total;
+    vs->h_slots[v] = d[v].n;
     total += d[v].n;
   }
   TRN_CUDA_TRY(cudaMemcpyAsync(vs->views, d, sizeof(ViewDesc) * vs->nviews, cudaMemcpyHostToDevice, st));
@@ -3072,6 +3075,20 @@ WaveRun wave_run(trn_viewset* vs, const Params& P, const trn_launch* ln, long lo
   return r;
 }
 
+// Image of a round of n slots from its radiance.
+void pixel_sums(const WaveRun& r, long long n) {
+  int deep = 0, rest = 0;
+  for (int v = 0; v < r.vs->nviews; v++) {
+    const trn_camera& c = r.vs->h_views[v].camera;
+    (deep_pixels((long long)c.width * c.height, r.vs->h_slots[v]) ? deep : rest)++;
+  }
+  if (rest) r.go<k_wf_pixels>(r.P, r.W, n);
+  if (!deep) return;
+  // 16 blocks of 4 warps per SM over the deep views
+  const int per_view = std::max(1, sms() * 16 / deep);
+  r.launch<k_wf_deep_pixels>((long long)per_view * r.vs->nviews, 128, r.P, r.W, n, per_view);
+}
+
 // Interior term over all slots, in rounds: forward image (kWfFwd), with records
 // into P.queue (kWfRec, records given by `cache`), or replayed records and the
 // reverse sweep of each round (kWfReplay). Returns 1 when there are no buffers
@@ -3109,7 +3126,7 @@ int path_wave(trn_viewset* vs, const Params& P0, const trn_launch* ln, long long
     r.go<k_wf_start<MODE>>(r.P, r.W, S, r.R);
     r.bounces<MODE>(S.n_out, S.n_ray, depth, WaveRun::tail_bounce(n));
     if (MODE == kWfReplay) r.go<k_path_reverse<false>>(r.P, r.R);
-    else r.go<k_wf_pixels>(r.P, r.W, n);
+    else pixel_sums(r, n);
   }
   TRN_CUDA_TRY(cudaGetLastError());
   return 0;

@@ -252,6 +252,10 @@ __global__ void __launch_bounds__(256, 4) k_wf_camera(TRN_KPARAMS, const __grid_
   flush_cnt(cnt, P.stats);
 }
 
+// Whether a view's pixels are summed by a warp each: so few pixels that a thread
+// each leaves most of the GPU idle, and samples enough for a warp.
+TRN_HD bool deep_pixels(long long pixels, long long samples) { return pixels <= 16384 && samples >= 32 * pixels; }
+
 // Adds the round's radiance to the image: one thread per pixel sums its samples
 // of this round in slot order (a view's samples of one pixel lie W * H slots
 // apart). The image does not depend on the order in which paths end.
@@ -264,11 +268,35 @@ __global__ void __launch_bounds__(256) k_wf_pixels(TRN_KPARAMS, const __grid_con
     const ViewDesc& V = view_of(P, slot, vhint);
     const long long WH = (long long)V.cam.w * V.cam.h;
     // the view's first W * H slots of the round stand for its pixels
-    if (slot - max(W.first, V.begin) >= WH) continue;
+    if (slot - max(W.first, V.begin) >= WH || deep_pixels(WH, V.n)) continue;
     const long long last = min(end, V.begin + V.n);
     F3 acc = F3z();
     for (long long q = slot; q < last; q += WH) acc = acc + W.L[q - W.first] * V.inv_spp;
     atomic_add3((V.image ? V.image : P.image + 3 * V.pix_off) + 3 * ((slot - V.begin) % WH), acc);
+  }
+}
+
+// The same for the views with deep pixels, `per_view` blocks each: a warp per
+// pixel, every 32nd sample by a lane, then the lanes in a fixed order. Bound by the
+// chain of a lane's adds (16 x 16 pixels of 65,536 samples of depth 1: the image took 39 ms with a thread
+// per pixel, 9.2 here, 1.2 of them in this kernel).
+__global__ void __launch_bounds__(256) k_wf_deep_pixels(TRN_KPARAMS, const __grid_constant__ Wave W, long long n, int per_view) {
+  stage_begin();
+  const ViewDesc& V = P.views[blockIdx.x / per_view];
+  if (!deep_pixels((long long)V.cam.w * V.cam.h, V.n)) return;
+  const int lane = threadIdx.x & 31;
+  const int WH = V.cam.w * V.cam.h;
+  const long long first = max(W.first, V.begin), last = min(W.first + n, V.begin + V.n);
+  for (int i = blockIdx.x % per_view * (blockDim.x >> 5) + (threadIdx.x >> 5); i < WH; i += per_view * (blockDim.x >> 5)) {
+    F3 acc = F3z();
+#pragma unroll 4
+    for (long long q = first + i + (long long)lane * WH; q < last; q += 32ll * WH)
+      acc = acc + W.L[q - W.first] * V.inv_spp;
+    for (int o = 16; o > 0; o >>= 1)
+      acc = acc + F3(__shfl_xor_sync(0xffffffffu, acc.x, o), __shfl_xor_sync(0xffffffffu, acc.y, o),
+                     __shfl_xor_sync(0xffffffffu, acc.z, o));
+    if (lane == 0 && first + i < last)
+      atomic_add3((V.image ? V.image : P.image + 3 * V.pix_off) + 3 * ((first + i - V.begin) % WH), acc);
   }
 }
 

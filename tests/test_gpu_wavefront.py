@@ -115,3 +115,29 @@ def test_late_bounces_give_the_same_in_either_form(built_lib, depth):
         assert torch.equal(got[0][0], got[1][0])
         assert float(got[0][1].abs().sum()) > 0
         assert rel_l2(got[0][1], got[1][1]) <= 1e-5
+
+
+@pytest.mark.parametrize("w,h,spp,round_log2", [(8, 8, 31, 0), (8, 8, 32, 0), (8, 8, 33, 0), (1, 1, 4099, 0), (5, 3, 7001, 16),
+                                                (128, 128, 33, 0), (129, 128, 33, 0), (8, 6, 3000, 16)])
+def test_pixels_of_many_samples(built_lib, w, h, spp, round_log2):
+    """A warp sums a pixel of 32 samples and more in a view of up to 16,384
+    pixels: against one thread per path, which a capture without round buffers
+    runs, in whole rounds and in some that end inside a pixel's samples, with a
+    view of the other kind beside it, and the same bit for bit in two runs."""
+    sc = _scene()
+    cams = [api.Camera((0.5, 1.5, 3.5), (0.0, 0.0, 0.0), (0.0, 1.0, 0.0), 40, 28, 45.0),
+            api.Camera((0.0, 0.5, 4.0), (0.0, 0.0, 0.0), (0.0, 1.0, 0.0), w, h, 45.0)]
+    opts = api.RenderOptions(3, 3, 0, 0, 0, 0, 0)
+    bare, vs = api.ViewSet(sc, cams, [7, spp]), api.ViewSet(sc, cams, [7, spp])
+    bare.render(api.TRN_PRIMARY_EDGE, opts)              # uploads the view table, allocates none
+    ref = torch.empty(bare.npix, 3, device=sc.device)
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        bare.render(api.TRN_PATH_TRACER, opts, out=ref)
+    ref.zero_()
+    g.replay()
+    launch = api.launch_config(round_log2=round_log2) if round_log2 else None
+    img = vs.render(api.TRN_PATH_TRACER, opts, launch=launch).clone()
+    # spp additions of 32-bit values in another order
+    torch.testing.assert_close(img, ref, rtol=spp * 2 ** -24 + 1e-6, atol=1e-7)
+    assert torch.equal(img, vs.render(api.TRN_PATH_TRACER, opts, launch=launch))
