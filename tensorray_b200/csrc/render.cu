@@ -3349,7 +3349,8 @@ int edge_wave(trn_viewset* vs, const Params& P0, const trn_launch* ln, long long
     if (!ordered && order_round(vs, r.P, TERM, st)) return -1;
     if (r.begin()) return -1;
     r.P.q_count = r.ctr();
-    r.setup<TERM>(first);
+    if (TERM == TRN_DIRECT_EDGE && r.P.total - first <= 1 << 19) r.go<k_setup_direct>(r.P, first);
+    else r.setup<TERM>(first);
     if constexpr (TERM == TRN_DIRECT_EDGE) {
       r.go<k_direct_body>(r.P);
     } else if constexpr (TERM == TRN_INDIRECT_EDGE) {

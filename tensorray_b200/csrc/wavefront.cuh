@@ -516,6 +516,37 @@ __global__ void __launch_bounds__(256, 4) k_setup_rays2(TRN_KPARAMS, const __gri
   flush_cnt(cnt, P.stats);
 }
 
+// Queues the boundary samples of the lanes that have one as the term's items
+// (all lanes of the warp call it).
+template <int TERM>
+TRN_D void queue_item(const Params& P, const EdgeState& st, bool in) {
+  const unsigned long long j = warp_append(P.q_count, in);
+  if (in && j >= (unsigned long long)P.q_cap) { atomicExch(P.err, 2); in = false; }
+  if (!in) return;
+  if constexpr (TERM == TRN_DIRECT_EDGE) {
+    DirectItem& it = reinterpret_cast<DirectItem*>(P.queue)[j];
+    it.p = st.p; it.view = (int)(st.V - P.views);
+    it.x_tri = st.x.tri; it.x_u = st.x.u; it.x_v = st.x.v; it.v0 = st.v0; it.v1 = st.v1; it.far_tri = st.far_tri;
+    it.sedge = st.sedge; it.rdir = st.rdir; it.ev0 = st.T0 * st.w0; it.p0 = st.p0; it.n = st.n;
+  } else if constexpr (TERM == TRN_INDIRECT_EDGE) {
+    IndirectItem& it = reinterpret_cast<IndirectItem*>(P.queue)[j];
+    it.p_lo = (unsigned)st.p; it.p_hi = (int)(st.p >> 32); it.view = (int)(st.V - P.views);
+    it.xe_tri = st.xe.tri; it.xe_u = st.xe.u; it.xe_v = st.xe.v;
+    it.xs_tri = st.x.tri; it.xs_u = st.x.u; it.xs_v = st.x.v;
+    it.v0 = st.v0; it.v1 = st.v1; it.far_tri = st.far_tri; it.w0 = st.w0; it.sedge = st.sedge;
+    it.rdir = st.rdir; it.p0 = st.p0; it.n = st.n;
+  } else {
+    constexpr bool pixel = TERM == TRN_PIXEL_EDGE;
+    PrimaryItem& it = reinterpret_cast<PrimaryItem*>(P.queue)[j];
+    it.p = st.p; it.view = (int)(st.V - P.views);
+    it.x_tri = st.x.tri; it.x_u = st.x.u; it.x_v = st.x.v; it.T0 = st.T0.x; it.w0 = st.w0;
+    it.sedge = pixel ? 0.f : st.sedge;
+    it.v0 = pixel ? -1 : st.v0; it.v1 = pixel ? -1 : st.v1;  // a pixel-edge point is no scene parameter
+    it.far_tri = st.far_tri;
+    it.rdir = st.rdir; it.p0 = st.p0; it.n = st.n; it.g = st.g;
+  }
+}
+
 // Boundary geometry of the samples whose rays allow one, queued as the term's
 // items. n: the rays of the last query (the pixel term has only one).
 template <int TERM>
@@ -562,32 +593,27 @@ __global__ void __launch_bounds__(256, 3) k_setup_finish(TRN_KPARAMS, const __gr
         }
       }
     }
-    const unsigned long long j = warp_append(P.q_count, in);
-    if (in && j >= (unsigned long long)P.q_cap) { atomicExch(P.err, 2); in = false; }
-    if (!in) return;
-    if constexpr (TERM == TRN_DIRECT_EDGE) {
-      DirectItem& it = reinterpret_cast<DirectItem*>(P.queue)[j];
-      it.p = st.p; it.view = (int)(st.V - P.views);
-      it.x_tri = st.x.tri; it.x_u = st.x.u; it.x_v = st.x.v; it.v0 = st.v0; it.v1 = st.v1; it.far_tri = st.far_tri;
-      it.sedge = st.sedge; it.rdir = st.rdir; it.ev0 = st.T0 * st.w0; it.p0 = st.p0; it.n = st.n;
-    } else if constexpr (TERM == TRN_INDIRECT_EDGE) {
-      IndirectItem& it = reinterpret_cast<IndirectItem*>(P.queue)[j];
-      it.p_lo = (unsigned)st.p; it.p_hi = (int)(st.p >> 32); it.view = (int)(st.V - P.views);
-      it.xe_tri = st.xe.tri; it.xe_u = st.xe.u; it.xe_v = st.xe.v;
-      it.xs_tri = st.x.tri; it.xs_u = st.x.u; it.xs_v = st.x.v;
-      it.v0 = st.v0; it.v1 = st.v1; it.far_tri = st.far_tri; it.w0 = st.w0; it.sedge = st.sedge;
-      it.rdir = st.rdir; it.p0 = st.p0; it.n = st.n;
-    } else {
-      constexpr bool pixel = TERM == TRN_PIXEL_EDGE;
-      PrimaryItem& it = reinterpret_cast<PrimaryItem*>(P.queue)[j];
-      it.p = st.p; it.view = (int)(st.V - P.views);
-      it.x_tri = st.x.tri; it.x_u = st.x.u; it.x_v = st.x.v; it.T0 = st.T0.x; it.w0 = st.w0;
-      it.sedge = pixel ? 0.f : st.sedge;
-      it.v0 = pixel ? -1 : st.v0; it.v1 = pixel ? -1 : st.v1;  // a pixel-edge point is no scene parameter
-      it.far_tri = st.far_tri;
-      it.rdir = st.rdir; it.p0 = st.p0; it.n = st.n; it.g = st.g;
-    }
+    queue_item<TERM>(P, st, in);
   });
+}
+
+// The whole direct set-up by one thread per slot, for small rounds: most slots
+// end before their first ray (the edge lies wrong for the light), and the
+// launches between the rays then cost more than the lanes that wait. The term
+// at depth 3 in the wavefront's launches / here, us, on 1,284 and on 102,400
+// triangles: 12,288 slots 204 / 186 and 334 / 323, 393,216 287 / 265 and 499 /
+// 436, 1,048,576 342 / 365 and 577 / 557; 16.8M slots of depth 5 on 102,400
+// triangles 2,200 / 3,430.
+__global__ void __launch_bounds__(256, 4) k_setup_direct(TRN_KPARAMS, long long first) {
+  stage_begin();
+  Cnt cnt;
+  int vhint = 0;
+  for_each_entry((unsigned long long)(P.total - first), [&](unsigned long long k, bool in) {
+    EdgeState st;
+    in = in && direct_setup(P, slot_at(P, first + (long long)k), st, vhint, cnt);
+    queue_item<TRN_DIRECT_EDGE>(P, st, in);
+  });
+  flush_cnt(cnt, P.stats);
 }
 
 // ---------------------------------------------------------------------------

@@ -141,3 +141,20 @@ def test_pixels_of_many_samples(built_lib, w, h, spp, round_log2):
     # spp additions of 32-bit values in another order
     torch.testing.assert_close(img, ref, rtol=spp * 2 ** -24 + 1e-6, atol=1e-7)
     assert torch.equal(img, vs.render(api.TRN_PATH_TRACER, opts, launch=launch))
+
+
+def test_direct_set_up_in_either_form(built_lib):
+    """Rounds of up to 2^19 slots run the direct set-up in one kernel, larger ones
+    as a wavefront: one round of 2^19 + 4,096 slots against the same in rounds of
+    2^16, and one of 2^19."""
+    sc = _scene(64, 64)
+    opts = api.RenderOptions(3, 3, 0, 0, 0, 0, 0)
+    for spp in (128, 129):
+        vs = api.ViewSet(sc, [api.Camera((0.5, 1.5, 3.5), (0.0, 0.0, 0.0), (0.0, 1.0, 0.0), 64, 64, 45.0)], [spp])
+        d = torch.rand(vs.npix, 3, device=sc.device) - 0.3
+        got = []
+        for launch in (None, api.launch_config(round_log2=16)):
+            vs.render_grad(api.TRN_DIRECT_EDGE, opts, d, launch=launch)
+            got.append(sc.get_grads()["positions"].clone())
+        assert float(got[0].abs().sum()) > 0
+        assert rel_l2(got[0], got[1]) <= 1e-5
