@@ -831,6 +831,7 @@ int trn_scene_destroy(trn_scene* s) {
                   s->cluster_box, s->cluster_meet, s->cluster_count};
   for (void* p : ptrs)
     if (p) cudaFree(p);
+  for (void* p : s->aq_kept) cudaFree(p);
   delete s;
   return 0;
 }

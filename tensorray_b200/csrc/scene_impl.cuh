@@ -74,6 +74,10 @@ struct trn_scene {
   float* aq_eval = nullptr;
   int* aq_flag = nullptr;
   int* aq_prefix = nullptr;
+  // a captured launch holds the addresses of the arrays above: a growth then
+  // keeps the old ones until the scene is destroyed
+  bool aq_captured = false;
+  std::vector<void*> aq_kept;
   // acceleration structure
   trn::BvhNode* nodes = nullptr;  // [T-1]
   trn::LeafTri* tri_verts = nullptr;  // [T]

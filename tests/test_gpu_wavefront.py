@@ -158,3 +158,36 @@ def test_direct_set_up_in_either_form(built_lib):
             got.append(sc.get_grads()["positions"].clone())
         assert float(got[0].abs().sum()) > 0
         assert rel_l2(got[0], got[1]) <= 1e-5
+
+
+@pytest.mark.parametrize("term,guided", [(t, False) for t in TERMS] + [(api.TRN_DIRECT_EDGE, True)])
+def test_captured_gradients_replay_after_growth(built_lib, term, guided):
+    """A captured gradient call holds the set's round and sort buffers, and a
+    guided one the scene's tree: it still replays after a larger call grew them."""
+    sc = _scene()
+
+    def options(size):
+        o = api.RenderOptions(3, 3, 0, 0, 0, 0, 0)
+        o.g_direct, o.g_direct_depth, o.g_direct_max_size, o.g_direct_spp = guided, 1, size, 4
+        return o
+
+    vs = _views(sc)
+    d = torch.rand(vs.npix, 3, device=sc.device) - 0.3
+    sc.clear_grads()
+    vs.render_grad(term, options(3000), d)               # allocates what this call needs
+    ref = sc.get_grads()["positions"].clone()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        vs.render_grad(term, options(3000), d)
+        got = sc.get_grads()["positions"]
+    vs.reserve(8)
+    large = _views(sc, 3, (90, 90, 90))
+    for s in (vs, large):
+        for t in TERMS:
+            s.render_grad(t, options(90_000), d)
+    junk = [torch.full((1 << 22,), float("nan"), device=sc.device) for _ in range(64)]  # over memory given back
+    sc.clear_grads()
+    g.replay()
+    del junk
+    assert float(ref.abs().sum()) > 0
+    assert rel_l2(got, ref) <= 1e-5
