@@ -208,9 +208,32 @@ __global__ void k_morton(int nt, const float* pos, const int* idx, const unsigne
 constexpr int kClusters = 16;
 constexpr int kClusterR = 4;
 
+// Height of the tree (inner nodes on the longest way to a leaf): a traversal's
+// stack holds an entry per inner node above it at most. Chains of merges could
+// make it 16 levels per level of the radix tree (nested boxes, equal boxes), so a
+// cluster may only merge below a height that leaves one level for each possible
+// ancestor of its radix node and four for the root's last 16 clusters. Pairs of
+// neighbours always fit: a child's bound is at least one lower than its parent's.
+constexpr int kTreeHeight = kStackSize - 1;
+constexpr int kRootLevels = 4;
+static_assert((1 << kRootLevels) == kClusters, "a pass of pairs halves the root's clusters");
+static_assert(62 + kRootLevels < kTreeHeight, "every level of the radix tree can have its level");
+
+// Possible ancestors of the radix node over the sorted keys [left, right]: the
+// bits that its keys share beyond those that all keys share (an index below n
+// has no branch in its leading zeros).
+__device__ __forceinline__ int radix_ancestors(int n, const unsigned long long* keys, int left, int right) {
+  auto shared_bits = [&](int a, int b) {
+    const int p = __clzll(keys[a] ^ keys[b]);
+    return p >= 32 ? p - __clz(n - 1) : p;
+  };
+  return shared_bits(left, right) - shared_bits(0, n - 1);
+}
+
 struct Cluster {
   float lo[3], hi[3];
-  int id;  // >= 0 inner node, < 0 ~leaf
+  int id;      // >= 0 inner node, < 0 ~leaf
+  int height;
 };
 
 // Cluster boxes in memory: leaf i at slot i, inner node k at slot n + k.
@@ -256,10 +279,11 @@ __device__ __forceinline__ float shfl_area(const Cluster& c, int src) {
 }
 
 // Merges the clusters of the children [left, split) and [split, right] until at
-// most `limit` are left, and stores those from `left` on. Called by the whole
-// warp with the same arguments.
-__device__ __forceinline__ void cluster_merge(int n, int left, int split, int right, int limit, int* cid, float* cbox,
-                                              BvhNode* nodes, int* parent, int* counter, int* perm) {
+// most `limit` are left, and stores those from `left` on. top: the greatest height
+// of a cluster that a merge of neighbours makes. Called by the whole warp with the
+// same arguments.
+__device__ __forceinline__ void cluster_merge(int n, int left, int split, int right, int limit, int top, int* cid,
+                                              float* cbox, BvhNode* nodes, int* parent, int* counter, int* perm) {
   const int lane = threadIdx.x & 31;
   // a child of more than kClusters leaves has left at most kClusters clusters;
   // the entries behind them are marked
@@ -274,7 +298,9 @@ __device__ __forceinline__ void cluster_merge(int n, int left, int split, int ri
   int count = __popc(have);
   const int src = lane < nl ? lane : 16 + lane - nl;
   c.id = __shfl_sync(0xffffffffu, c.id, src & 31);
+  c.height = 0;
   if (lane < count) {
+    if (c.id >= 0) c.height = __ldcg(&nodes[c.id].d.z);
     const float* b = cbox + 6 * cluster_slot(c.id, n);
 #pragma unroll
     for (int k = 0; k < 3; k++) { c.lo[k] = __ldcg(b + k); c.hi[k] = __ldcg(b + 3 + k); }
@@ -282,26 +308,39 @@ __device__ __forceinline__ void cluster_merge(int n, int left, int split, int ri
     for (int k = 0; k < 3; k++) { c.lo[k] = 0.f; c.hi[k] = 0.f; }
   }
   while (count > limit) {
-    // nearest neighbour within the window; ties go to the smaller position,
-    // which keeps at least one mutual pair
+    // nearest neighbour within the window, of the clusters that may still merge;
+    // ties go to the smaller position, which keeps at least one mutual pair
+    const unsigned open = __ballot_sync(0xffffffffu, lane < count && c.height < top);
     float best = INFINITY;
-    int nn = 0;
+    int nn = lane;
 #pragma unroll
     for (int r = -kClusterR; r <= kClusterR; r++) {
       if (r == 0) continue;
       const int j = lane + r;
       // (a NaN or an infinite area counts as the largest)
       const float a = fminf(shfl_area(c, j & 31), 3.402823466e+38f);
-      if (j >= 0 && j < count && a < best) { best = a; nn = j; }
+      if (j >= 0 && j < 32 && (open >> j & open >> lane & 1u) && a < best) { best = a; nn = j; }
     }
-    const bool mutual = __shfl_sync(0xffffffffu, nn, nn) == lane && lane < count;
+    bool mutual = __shfl_sync(0xffffffffu, nn, nn) == lane && nn != lane;
+    if (!__any_sync(0xffffffffu, mutual)) {
+      // none: pairs by position, of the clusters that may still merge. (With at
+      // most one of them left there are no more than kClusters clusters, as each of
+      // the others holds two: only the root goes on then, and pairs them all.)
+      const unsigned all = count < 32 ? (1u << count) - 1u : 0xffffffffu;
+      const unsigned pairs = count > kClusters && __popc(open) > 1 ? open : all;
+      const int rank = __popc(pairs & ((1u << lane) - 1u));
+      const int partner = rank & 1 ? 31 - __clz(pairs & ((1u << lane) - 1u)) : __ffs(pairs & ~((2u << lane) - 1u)) - 1;
+      mutual = (pairs >> lane & 1u) && partner >= 0;
+      nn = mutual ? partner : lane;
+    }
     const bool merges = mutual && lane < nn;
     const unsigned mm = __ballot_sync(0xffffffffu, merges);
     int first = 0;
     if (lane == 0) first = atomicAdd(counter, __popc(mm));
     first = __shfl_sync(0xffffffffu, first, 0);
-    const int other = __shfl_sync(0xffffffffu, c.id, nn);
+    const int other = __shfl_sync(0xffffffffu, c.id, nn), other_height = __shfl_sync(0xffffffffu, c.height, nn);
     Cluster u = c, o;
+    if (merges) u.height = max(c.height, other_height) + 1;
 #pragma unroll
     for (int k = 0; k < 3; k++) {
       const float l = __shfl_sync(0xffffffffu, c.lo[k], nn), h = __shfl_sync(0xffffffffu, c.hi[k], nn);
@@ -313,7 +352,7 @@ __device__ __forceinline__ void cluster_merge(int n, int left, int split, int ri
       nodes[u.id].a = make_float4(c.lo[0], c.hi[0], c.lo[1], c.hi[1]);
       nodes[u.id].b = make_float4(c.lo[2], c.hi[2], o.lo[0], o.hi[0]);
       nodes[u.id].c = make_float4(o.lo[1], o.hi[1], o.lo[2], o.hi[2]);
-      nodes[u.id].d = make_int4(c.id, other, 0, 0);
+      nodes[u.id].d = make_int4(c.id, other, u.height, 0);
       parent[c.id < 0 ? n - 1 + ~c.id : c.id] = u.id;
       parent[other < 0 ? n - 1 + ~other : other] = u.id;
       float* b = cbox + 6 * cluster_slot(u.id, n);
@@ -329,6 +368,7 @@ __device__ __forceinline__ void cluster_merge(int n, int left, int split, int ri
     const int from = lane < count ? perm[lane] : lane;
     __syncwarp();
     c.id = __shfl_sync(0xffffffffu, u.id, from);
+    c.height = __shfl_sync(0xffffffffu, u.height, from);
 #pragma unroll
     for (int k = 0; k < 3; k++) {
       c.lo[k] = __shfl_sync(0xffffffffu, u.lo[k], from);
@@ -369,7 +409,8 @@ __global__ void __launch_bounds__(128) k_cluster(int n, const unsigned long long
       todo &= todo - 1;
       const int l = __shfl_sync(0xffffffffu, left, k), sp = __shfl_sync(0xffffffffu, split, k),
                 r = __shfl_sync(0xffffffffu, right, k);
-      cluster_merge(n, l, sp, r, r - l + 1 == n ? 1 : kClusters, cid, cbox, nodes, parent, counter,
+      cluster_merge(n, l, sp, r, r - l + 1 == n ? 1 : kClusters,
+                    kTreeHeight - kRootLevels - radix_ancestors(n, keys, l, r), cid, cbox, nodes, parent, counter,
                     perm[threadIdx.x >> 5]);
       __threadfence();
       __syncwarp();  // all lanes' writes before the one lane that arrives at the parent

@@ -33,12 +33,16 @@ struct TexDesc {
   long long offset;  // texel offset into the texel array (RGB triples)
 };
 
+// Entries of a traversal's stack: one per inner node above a node at most, and one
+// to spare. The build bounds the tree's height by it.
+constexpr int kStackSize = 72;
+
 struct alignas(64) BvhNode {
   // child boxes as (lo, hi) per axis, children (>= 0 node, < 0 ~leaf)
   float4 a;  // l0x h0x l0y h0y
   float4 b;  // l0z h0z l1x h1x
   float4 c;  // l1y h1y l1z h1z
-  int4 d;    // c0 c1 - -
+  int4 d;    // c0 c1, height of the subtree (the build's), -
 };
 
 // A leaf's triangle, two sectors: 40 bytes used.

@@ -171,7 +171,6 @@ TRN_D void load8(const void* p, float4& a, float4& b) {
 #endif
 }
 
-constexpr int kStackSize = 72;          // one entry per level at most, and one to spare
 // traversal states beside the node to visit next (>= 0 inner, < 0 leaf)
 constexpr int kTraceDone = 0x7fffffff;  // nothing left
 constexpr int kTracePop = 0x7ffffffe;   // the stack's next entry
@@ -249,7 +248,7 @@ TRN_D int visit_node(const DeviceScene& s, const RayPre& r, int node, float tmin
   if (both) {
     stack.set(sp, make_int2(second ? c0 : c1, __float_as_int(second ? t0 : t1)));
     sp++;
-    if (sp >= kStackSize) {
+    if (sp >= kStackSize) {  // (the build's bound on the height excludes it)
       sp = kStackSize - 1;
       if (err) atomicExch(err, 1);
     }
@@ -332,7 +331,7 @@ TRN_D bool trace(const DeviceScene& s, const F3& o, const F3& d, float tmin, flo
     const bool h1 = slab(r, b.z, b.w, c.x, c.y, c.z, c.w, tmin, best_t, t1);
     if (h0 && h1) {
       const bool second = t1 < t0;   // the nearer one is child 1
-      if (sp < kStackSize) stack[sp++] = second ? e.x : e.y;
+      if (sp < kStackSize) stack[sp++] = second ? e.x : e.y;  // (the build's bound on the height excludes the rest)
       else if (err) atomicExch(err, 1);
       cur = second ? e.y : e.x;
     } else if (h0 || h1) {

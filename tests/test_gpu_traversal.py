@@ -106,3 +106,36 @@ def test_queries_of_every_size_agree(built_lib):
             for a, b in zip(scene.intersect(*part), ref):
                 assert torch.equal(a, b[:k])
             assert torch.equal(scene.occluded(*part), vis[:k])
+
+
+@pytest.mark.parametrize("kind,n", [("nested", 100), ("nested", 512), ("nested", 3000), ("equal", 3000)])
+def test_trees_of_nested_boxes_have_a_bounded_height(built_lib, kind, n):
+    """Triangles around one centre, from which a ray meets the boxes of all of
+    them at once: merged nearest first they made one chain (95 levels for 512, 127
+    for 2,048), above the traversal's 72 stack entries, and triangles were missed.
+    (The sizes of 100 stay a chain.) Equal boxes tie and chain likewise."""
+    rng = np.random.default_rng(n)
+    tri = np.array([[1.0, -0.5, -0.5], [-0.5, 1.0, -0.5], [-0.5, -0.5, 1.0]])
+    size = np.geomspace(1, 8, n) if kind == "nested" else np.ones(n)
+    P = (size[:, None, None] * tri).reshape(-1, 3)
+    F = np.arange(3 * n).reshape(n, 3)
+    scene = _scene(P, F)
+    pos = torch.as_tensor(P.astype(np.float32)).reshape(n, 3, 3)
+    org = 0.02 * rng.normal(size=(600, 3))
+    d = rng.normal(size=(600, 3))
+    d[::2] = -tri[0] + 0.2 * d[::2]
+    d /= np.linalg.norm(d, axis=1, keepdims=True)
+    f = lambda x: torch.as_tensor(np.ascontiguousarray(x, np.float32))
+    rays = f(org), f(d), torch.full((600,), 1e-4), torch.full((600,), 20.0)
+    ref = O.intersect_brute(pos[:, 0], pos[:, 1], pos[:, 2], *rays)
+    hit = ref[0] >= 0
+    assert int(hit.sum()) > 100
+    for refit in (False, True):
+        scene.configure(refit=refit)
+        for k in (7, 600):
+            part = [x[:k] for x in rays]
+            got = [x.cpu() for x in scene.intersect(*(x.cuda() for x in part))]
+            assert torch.equal(got[0].long(), ref[0][:k])
+            for a, b in zip(got[1:], ref[1:]):
+                assert torch.equal(a[hit[:k]], b[:k][hit[:k]])
+            assert torch.equal(scene.occluded(*(x.cuda() for x in part)).cpu(), (~hit[:k]).int())
