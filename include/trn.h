@@ -189,7 +189,10 @@ long long trn_mesh_edges(int num_triangles, const int* indices, int* out, long l
 
 /* Scene lifetime. Replaces Scene::Configure (Scene.cpp:522-533): create
  * uploads the description; configure runs Primitive::Configure, face/vertex
- * normals, light distribution, secondary edge list and the BVH build. */
+ * normals, light distribution, secondary edge list and the BVH build. configure
+ * waits for the stream up to the triangles' bounds, and fails when those are not
+ * finite (positions NaN, or so large that the box's area overflows); inside a
+ * stream capture it neither waits nor checks. */
 int trn_scene_create(const trn_scene_desc* desc, trn_scene** out);
 int trn_scene_configure(trn_scene* scene, cudaStream_t stream);
 int trn_scene_destroy(trn_scene* scene);

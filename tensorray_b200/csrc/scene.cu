@@ -113,24 +113,41 @@ __device__ __forceinline__ float unordered(unsigned int u) {
 }
 
 __global__ void k_bounds_init(unsigned int* b) {
-  if (threadIdx.x < 3) { b[threadIdx.x] = 0xffffffffu; b[3 + threadIdx.x] = 0u; }
+  if (threadIdx.x < 12) b[threadIdx.x] = threadIdx.x / 3 % 2 == 0 ? 0xffffffffu : 0u;
 }
-__global__ void k_bounds(int nt, const float* pos, const int* idx, unsigned int* b) {
+// Bounds of the triangles' centroids (b[0..5]) and of their vertices (b[6..11];
+// a coordinate that is a number at none of a triangle's vertices is left out).
+__global__ void __launch_bounds__(256) k_bounds(int nt, const float* pos, const int* idx, unsigned int* b) {
   int f = blockIdx.x * blockDim.x + threadIdx.x;
-  F3 c(0.f, 0.f, 0.f);
-  bool ok = f < nt;
+  F3 c(0.f, 0.f, 0.f), l(0.f, 0.f, 0.f), h(0.f, 0.f, 0.f);
+  const bool ok = f < nt;
   if (ok) {
     const F3 p0 = make_f3(pos + 3 * idx[3 * f]), p1 = make_f3(pos + 3 * idx[3 * f + 1]),
              p2 = make_f3(pos + 3 * idx[3 * f + 2]);
     c = (p0 + p1 + p2) * (1.f / 3.f);
-  }
-  for (int k = 0; k < 3; k++) {
-    unsigned int lo = ok ? ordered(c[k]) : 0xffffffffu, hi = ok ? ordered(c[k]) : 0u;
-    for (int o = 16; o > 0; o >>= 1) {
-      lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, o));
-      hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+    for (int k = 0; k < 3; k++) {
+      l[k] = fminf(fminf(p0[k], p1[k]), p2[k]);
+      h[k] = fmaxf(fmaxf(p0[k], p1[k]), p2[k]);
     }
-    if ((threadIdx.x & 31) == 0) { atomicMin(&b[k], lo); atomicMax(&b[3 + k], hi); }
+  }
+  // one atomic per block and bound: they all meet in the same twelve words
+  __shared__ unsigned part[12][8];
+  auto bound = [&](int at, bool in, float low, float high) {
+    const unsigned lo = __reduce_min_sync(0xffffffffu, in ? ordered(low) : 0xffffffffu);
+    const unsigned hi = __reduce_max_sync(0xffffffffu, in ? ordered(high) : 0u);
+    if ((threadIdx.x & 31) == 0) { part[at][threadIdx.x >> 5] = lo; part[at + 3][threadIdx.x >> 5] = hi; }
+  };
+  for (int k = 0; k < 3; k++) {
+    bound(k, ok, c[k], c[k]);
+    bound(6 + k, ok && l[k] <= h[k], l[k], h[k]);
+  }
+  __syncthreads();
+  if (threadIdx.x < 12) {
+    const bool low = threadIdx.x / 3 % 2 == 0;
+    unsigned x = part[threadIdx.x][0];
+    for (int w = 1; w < 8; w++) x = low ? min(x, part[threadIdx.x][w]) : max(x, part[threadIdx.x][w]);
+    if (low) atomicMin(&b[threadIdx.x], x);
+    else atomicMax(&b[threadIdx.x], x);
   }
 }
 
@@ -145,10 +162,16 @@ __device__ __forceinline__ unsigned int expand_bits(unsigned int v) {
 #ifndef TRN_LARGE_SPLIT
 #define TRN_LARGE_SPLIT 1
 #endif
+// Also says whether the scene can have a tree of boxes: its box's area is finite.
 __global__ void k_morton(int nt, const float* pos, const int* idx, const unsigned int* b,
-                         unsigned long long* keys) {
+                         unsigned long long* keys, int* boundless) {
   int f = blockIdx.x * blockDim.x + threadIdx.x;
   if (f >= nt) return;
+  if (f == 0) {
+    float e[3];
+    for (int k = 0; k < 3; k++) e[k] = unordered(b[9 + k]) - unordered(b[6 + k]);
+    *boundless = !(e[0] * e[1] + e[1] * e[2] + e[2] * e[0] < 3.402823466e+38f);
+  }
   const F3 p0 = make_f3(pos + 3 * idx[3 * f]), p1 = make_f3(pos + 3 * idx[3 * f + 1]),
            p2 = make_f3(pos + 3 * idx[3 * f + 2]);
   const F3 c = (p0 + p1 + p2) * (1.f / 3.f);
@@ -828,7 +851,7 @@ int trn_scene_create(const trn_scene_desc* d, trn_scene** out) {
       dev_alloc_copy(&s->flags, (const int*)nullptr, std::max(1, nt - 1)) ||
       dev_alloc_copy(&s->keys, (const unsigned long long*)nullptr, (size_t)nt) ||
       dev_alloc_copy(&s->keys_alt, (const unsigned long long*)nullptr, (size_t)nt) ||
-      dev_alloc_copy(&s->bounds, (const float*)nullptr, 6) ||
+      dev_alloc_copy(&s->bounds, (const float*)nullptr, 12) ||
       dev_alloc_copy(&s->g_pos, (const float*)nullptr, 3 * (size_t)nv) ||
       dev_alloc_copy(&s->g_vnormal, (const float*)nullptr, 3 * (size_t)nv) ||
       dev_alloc_copy(&s->g_texels, (const float*)nullptr, std::max<size_t>(3, 3 * (size_t)ntexel)) ||
@@ -853,6 +876,11 @@ int trn_scene_create(const trn_scene_desc* d, trn_scene** out) {
       dev_alloc_copy(&s->cluster_meet, (const int*)nullptr, (size_t)nt) ||
       dev_alloc_copy(&s->cluster_count, (const int*)nullptr, 1))
     return fail();
+  if (cudaHostAlloc(&s->boundless, sizeof(int), cudaHostAllocMapped) != cudaSuccess ||
+      cudaEventCreateWithFlags(&s->bounds_done, cudaEventDisableTiming) != cudaSuccess) {
+    set_error("trn_scene_create: out of memory");
+    return fail();
+  }
   *out = s;
   return 0;
 }
@@ -873,6 +901,8 @@ int trn_scene_destroy(trn_scene* s) {
   for (void* p : ptrs)
     if (p) cudaFree(p);
   for (void* p : s->aq_kept) cudaFree(p);
+  if (s->boundless) cudaFreeHost(s->boundless);
+  if (s->bounds_done) cudaEventDestroy(s->bounds_done);
   delete s;
   return 0;
 }
@@ -901,6 +931,11 @@ int configure_geometry(trn_scene* s, cudaStream_t st) {
   }
   return 0;
 }
+
+bool stream_captures(cudaStream_t st) {
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  return cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone;
+}
 }  // namespace
 
 extern "C" {
@@ -912,7 +947,10 @@ int trn_scene_configure(trn_scene* s, cudaStream_t st) {
   // BVH
   k_bounds_init<<<1, 32, 0, st>>>((unsigned int*)s->bounds);
   k_bounds<<<nblk(nt), 256, 0, st>>>(nt, s->pos, s->idx, (unsigned int*)s->bounds);
-  k_morton<<<nblk(nt), 256, 0, st>>>(nt, s->pos, s->idx, (const unsigned int*)s->bounds, s->keys);
+  k_morton<<<nblk(nt), 256, 0, st>>>(nt, s->pos, s->idx, (const unsigned int*)s->bounds, s->keys, s->boundless);
+  // (a captured build cannot wait: it is not checked)
+  const bool check = nt > 1 && !stream_captures(st);
+  if (check) TRN_CUDA_TRY(cudaEventRecord(s->bounds_done, st));
   count_launch(4);  // bounds init, bounds, morton, and the radix sort counted as one
   size_t bytes = s->sort_tmp_bytes;
   if (cub::DeviceRadixSort::SortKeys(s->sort_tmp, bytes, s->keys, s->keys_alt, nt, 32, 63, st) != cudaSuccess) {
@@ -925,6 +963,15 @@ int trn_scene_configure(trn_scene* s, cudaStream_t st) {
     k_cluster<<<nblk(nt, 128), 128, 0, st>>>(nt, s->keys_alt, s->cluster_id, s->cluster_box, s->cluster_meet, s->nodes,
                                              s->parent, s->cluster_count);
     count_launch(2);
+    // The answer is waited for when all of the build is under way; the GPU is
+    // busy with it for longer than the host takes to go on.
+    if (check) {
+      TRN_CUDA_TRY(cudaEventSynchronize(s->bounds_done));
+      if (*static_cast<volatile int*>(s->boundless)) {
+        set_error("trn_scene_configure: the triangles' bounding box is not finite (positions NaN or above 1e19)");
+        return -1;
+      }
+    }
   } else {
     k_refit<<<1, 1, 0, st>>>(nt, s->keys_alt, s->pos, s->idx, s->nodes, s->parent, s->flags, s->tri_verts);
     count_launch(1);

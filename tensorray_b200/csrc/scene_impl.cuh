@@ -93,7 +93,9 @@ struct trn_scene {
   float* cluster_box = nullptr;   // [2T][6]
   int* cluster_meet = nullptr;    // [T]
   int* cluster_count = nullptr;   // [1]
-  float* bounds = nullptr;        // [6]
+  float* bounds = nullptr;        // [12] of the centroids, of the vertices
+  int* boundless = nullptr;       // (host, mapped) the last build's vertices have no finite box
+  cudaEvent_t bounds_done = nullptr;
   // ---- gradients (device) ------------------------------------------------------
   float* g_pos = nullptr;         // [V][3] dL/d(world position)
   float* g_vnormal = nullptr;     // [V][3] dL/d(vertex normal)

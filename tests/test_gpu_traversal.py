@@ -139,3 +139,35 @@ def test_trees_of_nested_boxes_have_a_bounded_height(built_lib, kind, n):
             for a, b in zip(got[1:], ref[1:]):
                 assert torch.equal(a[hit[:k]], b[:k][hit[:k]])
             assert torch.equal(scene.occluded(*(x.cuda() for x in part)).cpu(), (~hit[:k]).int())
+
+
+def test_positions_without_a_finite_box_are_refused(built_lib):
+    """No tree over triangles whose common box's area overflows, or that have no
+    number in some coordinate; single ones of either kind are left alone, and the
+    scene works again with other positions."""
+    rng = np.random.default_rng(1)
+    P, F = _mesh("soup", 50, rng)
+    scene = _scene(P, F)
+    scene.configure()
+    good = scene._raw_positions.clone()
+    rays = [x.cuda() for x in _rays(200, rng)]
+    ref = [x.clone() for x in scene.intersect(*rays)]
+    for value, part in ((3e19, slice(0, 1)), (float("nan"), slice(None)), (float("inf"), slice(7, 8))):
+        bad = good.clone()
+        bad[part, :2] = value
+        scene.set_vertex_positions(bad)
+        with pytest.raises(RuntimeError, match="finite"):
+            scene.configure()
+        scene.set_vertex_positions(good)
+        scene.configure()
+        for a, b in zip(scene.intersect(*rays), ref):
+            assert torch.equal(a, b)
+    far = good.clone()
+    far[0] = 1e18
+    few = good.clone()
+    few[:3] = float("nan")   # one triangle
+    for ok in (far, few):
+        scene.set_vertex_positions(ok)
+        scene.configure()
+    one = _scene(P[:3] * 1e25, F[:1])
+    one.configure()
