@@ -1060,6 +1060,8 @@ struct PathSoA {
   VRec* vr_;
   LRec* br_;
   F3 *Tk_, *Mk_;
+  unsigned* order;            // [cap] the records in the order their paths ended
+  unsigned long long* n_end;  // paths ended so far (nullptr: their order is not kept)
   TRN_D long long& p(long long i) const { return p_[i]; }
   TRN_D int& view(long long i) const { return view_[i]; }
   TRN_D int& K(long long i) const { return K_[i]; }
@@ -1089,6 +1091,8 @@ inline size_t path_soa(PathSoA& a, void* base, long long cap, int depth) {
   a.br_ = reinterpret_cast<LRec*>(take(sizeof(LRec) * n * std::max(depth, 1)));
   a.Tk_ = reinterpret_cast<F3*>(take(sizeof(F3) * n * v));
   a.Mk_ = reinterpret_cast<F3*>(take(sizeof(F3) * n * v));
+  a.order = reinterpret_cast<unsigned*>(take(sizeof(unsigned) * n));
+  a.n_end = nullptr;
   return off;
 }
 
@@ -1105,16 +1109,20 @@ struct PathRef {
   struct M { const PathSoA& a; long long i; TRN_D const F3& operator[](int k) const { return a.Mk(i, k); } } Mk;
 };
 
-// Reverse sweep over the records, in their own order (the paths' slots, but for
-// the order in which warps start). The order matters to the sums: a few vertices
-// get millions of 32-bit adds, and small ones are lost in a large sum. In the
-// order in which paths ended a warp's sweeps have the same length, and the sweep
-// takes half the time (16.8M paths of depth 5: 11.8 ms, in this order 23.7), but
-// the lanes that add together are others, and the position gradient moves by
-// 6e-5, where two runs differ by 1.5e-5. Bound by instruction fetch: the sweep is
-// one long body of inlined scatters, and the few warps that fit its registers do
-// not hide the misses. (Its six scatters in a loop, or one shared function, take
-// 5 to 10 times as long: lanes then enter them one group at a time.)
+// Reverse sweep over the records, in the order in which their paths ended (up to
+// kEndOrder paths) or in their own, that of the paths' slots but for the order in
+// which warps start. Paths that ended together have the same length, and so have
+// their sweeps: 1M paths of depth 3 on 1,284 triangles 0.59 ms, in record order
+// 0.94. But the order matters to the sums. A few vertices get millions of 32-bit
+// adds, small ones are lost in a large sum, and paths of another length beside it
+// make the lanes' adds others. 16.8M paths of depth 5 move the position gradient by
+// 6e-5 in ending order, where two runs differ by 1.5e-5; 4M by 7e-6 (two runs 6e-6),
+// 1M by no more than the means of four runs differ (2e-6). Bound by instruction
+// fetch: the sweep is one long body of inlined scatters, and the few warps that fit
+// its registers do not hide the misses. (Its six scatters in a loop, or one shared
+// function, take 5 to 10 times as long: lanes then enter them one group at a time.)
+constexpr long long kEndOrder = 1 << 20;
+
 // CACHED: the records come from the recording forward render and carry no
 // dL/dI yet; each path reads its pixel's now and is skipped when that is zero,
 // as the replaying form skips it.
@@ -1125,7 +1133,7 @@ __global__ void __launch_bounds__(256, TRN_MINB_REVERSE) k_path_reverse(TRN_KPAR
   const unsigned long long n = min(*P.q_count, (unsigned long long)P.q_cap);
   for (unsigned long long k = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; k < n;
        k += (unsigned long long)gridDim.x * blockDim.x) {
-    const long long i = (long long)k;
+    const long long i = R.n_end ? (long long)__ldcs(R.order + k) : (long long)k;
     const int view = R.view(i);
     F3 g;
     if (CACHED) {
@@ -2588,7 +2596,7 @@ struct trn_viewset {
   // depth; hash samples only)
   void* pc = nullptr;
   size_t pc_bytes = 0;
-  unsigned long long* pc_count = nullptr;  // records
+  unsigned long long* pc_count = nullptr;  // [2] records, paths ended
   long long pc_limit = 0;  // bytes the records may take (0 = off)
   bool pc_valid = false;
   std::vector<char> pc_key;
@@ -3112,6 +3120,7 @@ int path_wave(trn_viewset* vs, const Params& P0, const trn_launch* ln, long long
   const size_t wb = wave_layout(r.W, &items, vs->iq, cap, TRN_PATH_TRACER, depth);
   if (MODE == kWfRec) {
     r.R = *cache;
+    if (total <= kEndOrder) r.R.n_end = vs->pc_count + 1;
   }
   if (MODE == kWfReplay) {
     path_soa(r.R, static_cast<char*>(vs->iq) + wb, cap, depth);
@@ -3123,6 +3132,7 @@ int path_wave(trn_viewset* vs, const Params& P0, const trn_launch* ln, long long
     r.W.first = first;
     if (MODE == kWfReplay) {
       r.P.q_count = r.ctr();
+      if (total <= kEndOrder) r.R.n_end = r.ctr();
     }
     unsigned long long* rays = r.ctr();
     r.go<k_wf_camera>(r.P, r.W, n, MODE == kWfReplay, rays);
@@ -3419,7 +3429,7 @@ int path_cache_fwd(trn_viewset* vs, Params P, const trn_launch* ln, const trn_re
     vs->pc = nullptr;
     vs->pc_bytes = 0;
     if (cudaMalloc(&vs->pc, bytes) != cudaSuccess ||
-        (!vs->pc_count && cudaMalloc(&vs->pc_count, sizeof(unsigned long long)) != cudaSuccess)) {
+        (!vs->pc_count && cudaMalloc(&vs->pc_count, 2 * sizeof(unsigned long long)) != cudaSuccess)) {
       cudaGetLastError();  // out of memory: render without records
       if (vs->pc) cudaFree(vs->pc);
       vs->pc = nullptr;
@@ -3427,7 +3437,7 @@ int path_cache_fwd(trn_viewset* vs, Params P, const trn_launch* ln, const trn_re
     }
     vs->pc_bytes = bytes;
   }
-  TRN_CUDA_TRY(cudaMemsetAsync(vs->pc_count, 0, sizeof(unsigned long long), st));
+  TRN_CUDA_TRY(cudaMemsetAsync(vs->pc_count, 0, 2 * sizeof(unsigned long long), st));
   P.q_count = vs->pc_count;
   P.q_cap = total;
   path_soa(R, vs->pc, total, vs->max_depth);
@@ -3448,6 +3458,7 @@ int path_cache_grad(trn_viewset* vs, Params P, const trn_launch* ln, const trn_r
   P.q_cap = total;
   PathSoA R;
   path_soa(R, vs->pc, total, vs->max_depth);
+  if (total <= kEndOrder) R.n_end = vs->pc_count + 1;
   int grid, block;
   launch_dims(ln, total, grid, block);
   k_path_reverse<true><<<grid, block, 0, st>>>(P, R);

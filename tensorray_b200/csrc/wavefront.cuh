@@ -214,6 +214,16 @@ TRN_D void wf_finish(const Wave& W, const ViewDesc& V, long long p, const F3& L,
   W.L[p + V.begin - W.first] = L;
 }
 
+// Lists the records of the paths that end here (all lanes of the warp call it).
+template <int MODE>
+TRN_D void wf_record_end(const Wave& W, const PathSoA& R, bool ends, unsigned i) {
+  if constexpr (MODE != kWfFwd) {
+    if (!R.n_end) return;
+    const unsigned long long j = warp_append(R.n_end, ends);
+    if (ends) R.order[j] = W.rec[i];
+  }
+}
+
 // Camera rays of the round's n slots. For the adjoint (grad), slots whose pixel
 // has a zero dL/dI are left out (they carry no gradient); for an image, the
 // radiance of slots that end without a path is zero.
@@ -356,6 +366,7 @@ __global__ void __launch_bounds__(256, 3) k_wf_start(TRN_KPARAMS, const __grid_c
     }
     const bool go = in && D > 0;
     if (in && !go) wf_finish<MODE>(W, *V, p, q.L, cnt);
+    wf_record_end<MODE>(W, R, in && !go, i);
     wf_advance<MODE>(P, W, S, 0, go, i, V, p, q, R, cnt);
   });
   flush_cnt(cnt, P.stats);
@@ -419,6 +430,7 @@ __global__ void __launch_bounds__(256, 3) k_wf_shade(TRN_KPARAMS, const __grid_c
       }
       if (!go) wf_finish<MODE>(W, *V, p, q.L, cnt);
     }
+    wf_record_end<MODE>(W, R, in && !go, i);
     if constexpr (!TAIL) wf_advance<MODE>(P, W, S, b + 1, go, i, V, p, q, R, cnt);
   };
   if constexpr (TAIL) for_each_spread(*S.n, each);
