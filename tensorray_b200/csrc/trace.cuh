@@ -403,8 +403,9 @@ TRN_D void trace_stream(const DeviceScene& s, Fetch&& fetch, Load&& load, Store&
       if (!more) break;
       int lim;
       const int base = fetch(__popc(idle), lim, more);
-      if (free_ && base + __popc(idle & lt) < lim) {
-        id = base + __popc(idle & lt);
+      const int rank = __popc(idle & lt);
+      if (free_ && rank < lim - base) {  // (base + rank may not fit an int)
+        id = base + rank;
         F3 o, d;
         load(id, o, d, tmin, best_t, any);
         best_tri = -1; bu = bv = 0.f;
