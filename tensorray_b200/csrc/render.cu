@@ -3353,6 +3353,7 @@ void indirect_sides(WaveRun& r) {
 template <int TERM>
 int edge_wave(trn_viewset* vs, const Params& P0, const trn_launch* ln, long long total, cudaStream_t st) {
   const int depth = vs->max_depth;
+  if (TERM == TRN_INDIRECT_EDGE && depth < 2) return 0;  // a sensor and an emitter side take a bounce each
   const long long cap = std::min(total, round_cap(ln, kRound));
   WaveRun r = wave_run(vs, P0, ln, cap, st);
   void* items;
