@@ -307,13 +307,11 @@ def run_single(a):
         "interior_fwd": path_kernels,
         "interior_adj": (["k_path_reverse<true> (over the forward's path records)"] if not a.no_path_cache
                          else path_kernels[:-1] + ["k_path_reverse<false>"]),
-        "primary": ["k_edge_keys", "cub radix sort", "k_setup_*", "k_trace", "k_wf_start", "k_wf_shade",
-                    "k_wf_body_scatter"],
-        "direct": ["k_edge_keys", "cub radix sort", "k_setup_*", "k_trace", "k_wi_start", "k_wi_step",
-                   "k_wi_direct_scatter"],
-        "indirect": ["k_edge_keys", "cub radix sort", "k_setup_*", "k_trace", "k_wi_*", "k_wf_start", "k_wf_shade",
-                     "k_wf_emit_scatter"],
-        "pixel": ["k_setup_*", "k_trace", "k_wf_start", "k_wf_shade", "k_wf_body_scatter"],
+        "primary": ["k_edge_keys", "cub radix sort", "k_setup_*", "k_trace", "k_primary_body"],
+        "direct": ["k_edge_keys", "cub radix sort", "k_setup_*", "k_trace", "k_direct_body"],
+        "indirect": ["k_edge_keys", "cub radix sort", "k_setup_*", "k_trace", "k_indirect_sensor",
+                     "k_indirect_emitter"],
+        "pixel": ["k_setup_*", "k_trace", "k_primary_body"],
     }
     units_per_step = a.res * a.res * a.spp * 5
     V0 = scene._raw_positions.clone()

@@ -226,10 +226,12 @@ int trn_occluded(trn_scene* scene, int n, const float* org, const float* dir, co
                  const float* tmax, int* out_visible, cudaStream_t stream);
 
 /* Single-view calls (trn_render_fwd / trn_render_grad) reuse one view table
- * held by the scene: the first such call allocates it, later calls neither
- * allocate nor synchronise the stream. Calls on one scene must therefore be
- * ordered on one stream (as the reference's single default stream orders
- * them); use view sets for concurrent rendering.
+ * held by the scene, which the first such call allocates, and its round
+ * buffers (see trn_viewset_reserve), which grow when a call has more samples
+ * than any before it: that call frees them, allocates larger ones and waits
+ * for the stream. Other calls neither allocate nor wait. Calls on one scene
+ * must therefore be ordered on one stream (as the reference's single default
+ * stream orders them); use view sets for concurrent rendering.
  *
  * Forward render of one integrator (Integrator::RenderC, Integrator.h:96-104,
  * PathTracer.h:60-68). image_out [W*H*3] is overwritten. Only
@@ -254,8 +256,9 @@ int trn_render_grad(trn_scene* scene, const trn_camera* camera, const trn_render
  * the library until the process exits), and the call does not synchronise
  * the stream.
  * - Speed: it runs each term as one fused kernel (no wavefront, no edge-sorted
- *   set-up order, since those need scratch that grows with the launch), which
- *   is slower per term than trn_render_grad but for a few 100K samples.
+ *   set-up order, since those need scratch that grows with the launch). That is
+ *   1.1 to 3 times as slow per term as trn_render_grad from about 0.4M samples
+ *   on (the direct term: as fast), and can be faster for a few 10K.
  * - Limit: for TRN_PRIMARY_EDGE the scene may have at most 1048576 edges;
  *   larger scenes are rejected with an error.
  * - A guided direct term with g_direct_depth > 0 needs the refined tree's
@@ -292,11 +295,17 @@ int trn_viewset_update(trn_viewset* views, int nviews, const trn_view* view_arra
 int trn_viewset_num_pixels(const trn_viewset* views, long long* npix);
 /* Allocate the set's round buffers now: the wavefront's (one full round of any
  * term at up to max_bounces) and those of the edge-sorted run order of the
- * boundary set-up. Without it the first call of each term allocates them, and a larger batch later grows
- * them (each growth synchronises the stream and frees the old buffer). For a
- * serving loop, or before capturing render calls into a CUDA graph. No
+ * boundary set-up. Without it the first call of each term allocates them, and
+ * a larger batch later grows them (each growth synchronises the stream and
+ * frees the old buffer). For a serving loop, or before capturing render calls
+ * into a CUDA graph: a gradient call without its buffers fails inside a
+ * capture, and an image is then captured in the slower form that needs none
+ * (one thread per path), as it is rendered when there is no memory for them.
+ * Buffers that a captured call holds are kept, when they grow, until the set
+ * is destroyed; its views must not be updated while the capture is in use. No
  * counterpart in the reference (its tensor library allocates per call).
- * About 6 GB for max_bounces <= 8 (rounds of 16M boundary samples). */
+ * 3.7 GB for max_bounces <= 8 (rounds of 16M samples), of which a set that
+ * only renders images takes up to 3 GB. */
 int trn_viewset_reserve(trn_viewset* views, int max_bounces, cudaStream_t stream);
 /* Path cache. A forward render of TRN_PATH_TRACER can keep the record of
  * every path it traced (hit points, light samples, throughputs: about 620

@@ -1,11 +1,13 @@
 // Integrator kernels: the interior path tracer (forward and replaying
 // adjoint) and the primary / direct / indirect / pixel boundary terms.
 //
-// One thread owns one sample slot (one path) end to end. Where the reference
-// builds a tensor expression per stage and compacts surviving rays between
-// stages (Integrator.cpp:178-303, Ray.cpp:65-116), a path here keeps its
-// state in registers and simply stops; the per-slot sample layout replaces
-// the reference's per-call RandomFloat tensors (see SampleSource).
+// The reference builds a tensor expression per stage and compacts surviving rays
+// between stages (Integrator.cpp:178-303, Ray.cpp:65-116). Here the interior
+// paths and the boundary set-ups run as a wavefront of a few kernels per bounce
+// (wavefront.cuh); the paths of boundary samples, the late bounces of few paths and
+// the calls that may not allocate run one path per thread, which keeps its state
+// in registers and simply stops. The per-slot sample layout replaces the
+// reference's per-call RandomFloat tensors (see SampleSource).
 #include <algorithm>
 #include <atomic>
 #include <cstring>
@@ -152,7 +154,8 @@ TRN_D void atomic_add3(float* a, const F3& g) {
 // plain per-element atomicAdd of IndexedWriteKernel (TensorKernels.cuh:177-209),
 // which serialises when many paths hit the same few vertices (quads, lights).
 // (Summing in shared memory instead serialised such groups as well: a float
-// atomicAdd on shared memory is a compare-and-swap loop.)
+// atomicAdd on shared memory is a compare-and-swap loop.) The rounds are those of
+// E. Westphal, "Voting and Shuffling to Optimize Atomic Operations" (2015).
 TRN_D void agg_add3(float* base, long long idx, const F3& g) {
   const unsigned active = __activemask();
   const int lane = threadIdx.x & 31;
@@ -862,9 +865,8 @@ struct AdjState {
 };
 
 // Interior adjoint set-up: the camera ray of the slot (paths whose pixel has a
-// zero dL/dI carry no gradient and are skipped; with need_g false, as in the
-// recording forward render, no path is skipped and st.g is zero).
-TRN_D bool path_adj_setup(const Params& P, long long gslot, AdjState& st, int& vhint, Cnt& cnt, bool need_g = true) {
+// zero dL/dI carry no gradient and are skipped).
+TRN_D bool path_adj_setup(const Params& P, long long gslot, AdjState& st, int& vhint, Cnt& cnt) {
   const DeviceScene& s = P.s;
   const ViewDesc& V = view_of(P, gslot, vhint);
   const long long p = gslot - V.begin;
@@ -872,9 +874,9 @@ TRN_D bool path_adj_setup(const Params& P, long long gslot, AdjState& st, int& v
   const PathSmp S{&P, V.seed, gslot, p + V.slot_off};
   const int W = cam.w, WH = cam.w * cam.h;
   const int pix = (int)(p % WH);
-  if (need_g) cnt.v[kCntPixel]++;
-  const F3 g = need_g ? g_at(P, V, pix) : F3z();
-  if (need_g && g.x == 0.f && g.y == 0.f && g.z == 0.f) return false;
+  cnt.v[kCntPixel]++;
+  const F3 g = g_at(P, V, pix);
+  if (g.x == 0.f && g.y == 0.f && g.z == 0.f) return false;
   const F3 dir = camera_ray_dir(cam, pix % W, pix / W, S(0), S(1));
   cnt.v[kCntClosest]++;
   if (!trace<false>(s, cam_pos(cam), dir, kShadowEps, kRayMax, st.h, P.err)) return false;
@@ -2583,7 +2585,7 @@ struct trn_viewset {
   unsigned long long* iq_count = nullptr;
   // A captured launch holds the addresses of iq and sq: from then on a growth
   // keeps the old buffer until the set is destroyed (one per capture and growth
-  // at most; none is above a full round, 3.3 GB and 0.5 GB at depth <= 8).
+  // at most; none is above a full round, 3.4 GB and 0.3 GB at depth <= 8).
   bool iq_captured = false, sq_captured = false;
   std::vector<void*> kept;
   // run order of the split set-up rounds: keys and values double-buffered for
@@ -2845,10 +2847,10 @@ void launch(K kernel, const trn_launch* ln, long long total, const Params& P, cu
 
 // Slots per round of the boundary terms and the image, and paths per round of
 // the replaying adjoint. Larger rounds give each edge more samples per sort and
-// the terms fewer kernel tails, at up to 341 bytes per slot (indirect term,
-// depth 8): 2^24 against 2^23 slots, indirect 30.4 -> 28.2 ms, direct 3.2 ->
-// 2.4, primary 12.1 -> 11.2 (16.8M samples on 102,400 triangles). The replay
-// keeps 2^22 (0.7 kB of records and state per path at depth 8).
+// the terms fewer kernel tails, at up to 205 bytes per slot (direct term; an image
+// 181): 16.8M samples of depth 5 on 102,400 triangles, image 16.8 ms in rounds of
+// 2^22, 15.3 of 2^23, 14.6 of 2^24. The replay keeps 2^22, where it takes as long as
+// with 2^24 (0.74 kB of records and state per path at depth 8).
 #ifndef TRN_ROUND_LOG2
 #define TRN_ROUND_LOG2 24
 #endif
@@ -2951,7 +2953,7 @@ int ensure_queue(trn_viewset* vs, size_t need, size_t most, cudaStream_t st) {
     return 0;
   }
   if (cap) {
-    set_error("boundary term: its queue must be allocated before stream capture (run it once first)");
+    set_error("round buffers must be allocated before stream capture (run the call once first, or reserve them)");
     return 1;
   }
   TRN_CUDA_TRY(cudaStreamSynchronize(st));
@@ -2965,13 +2967,13 @@ int ensure_queue(trn_viewset* vs, size_t need, size_t most, cudaStream_t st) {
     if (cudaMalloc(&vs->iq, bytes) != cudaSuccess) {
       cudaGetLastError();
       vs->iq = nullptr;
-      set_error("boundary term: out of memory for its queue");
+      set_error("out of memory for the round buffers");
       return 1;
     }
     vs->iq_bytes = bytes;
   }
   if (!vs->iq_count && cudaMalloc(&vs->iq_count, kWaveCounters * sizeof(unsigned long long)) != cudaSuccess) {
-    set_error("boundary term: out of memory");
+    set_error("out of memory for the round counters");
     return -1;
   }
   return 0;
@@ -3076,7 +3078,7 @@ struct WaveRun {
   }
 };
 
-WaveRun wave_run(trn_viewset* vs, const Params& P, const trn_launch* ln, long long cap, cudaStream_t st) {
+WaveRun wave_run(trn_viewset* vs, const Params& P, const trn_launch* ln, cudaStream_t st) {
   WaveRun r;
   std::memset(&r.W, 0, sizeof(r.W));
   std::memset(&r.R, 0, sizeof(r.R));
@@ -3115,7 +3117,7 @@ int path_wave(trn_viewset* vs, const Params& P0, const trn_launch* ln, long long
   const size_t most = MODE == kWfReplay ? full_queue_bytes(depth <= 8) : path_round_bytes(kRound, depth, false);
   const int rc = ensure_queue(vs, path_round_bytes(cap, depth, MODE == kWfReplay), most, st);
   if (rc) return rc;
-  WaveRun r = wave_run(vs, P0, ln, cap, st);
+  WaveRun r = wave_run(vs, P0, ln, st);
   void* items;
   const size_t wb = wave_layout(r.W, &items, vs->iq, cap, TRN_PATH_TRACER, depth);
   if (MODE == kWfRec) {
@@ -3155,7 +3157,7 @@ int guide_wave(trn_viewset* vs, const Params& P, const trn_launch* ln, const Gui
                float* value, float* poly, cudaStream_t st) {
   const long long leaves = std::min(limit, std::max(1LL, round_cap(ln, kRound) / tree.per));
   const long long cap = leaves * tree.per;
-  WaveRun r = wave_run(vs, P, ln, cap, st);
+  WaveRun r = wave_run(vs, P, ln, st);
   void* items;
   const int rc = ensure_queue(vs, wave_layout(r.W, &items, nullptr, cap, TRN_DIRECT_EDGE, vs->max_depth),
                               full_queue_bytes(vs->max_depth <= 8), st);
@@ -3355,7 +3357,7 @@ int edge_wave(trn_viewset* vs, const Params& P0, const trn_launch* ln, long long
   const int depth = vs->max_depth;
   if (TERM == TRN_INDIRECT_EDGE && depth < 2) return 0;  // a sensor and an emitter side take a bounce each
   const long long cap = std::min(total, round_cap(ln, kRound));
-  WaveRun r = wave_run(vs, P0, ln, cap, st);
+  WaveRun r = wave_run(vs, P0, ln, st);
   void* items;
   if (ensure_queue(vs, wave_layout(r.W, &items, nullptr, cap, TERM, depth), full_queue_bytes(depth <= 8), st))
     return -1;
@@ -3416,7 +3418,7 @@ std::vector<char> path_key(const trn_viewset* vs, const trn_render_options* o, i
 // Recording forward render of the interior term into the view set's path
 // cache. Returns 1 when the cache is not used (off, a sample table, stream
 // capture, above the limit, or no memory for it): the caller then renders
-// with k_path_fwd.
+// without records.
 int path_cache_fwd(trn_viewset* vs, Params P, const trn_launch* ln, const trn_render_options* o, int spp_override,
                    long long total, cudaStream_t st) {
   vs->pc_valid = false;
@@ -3584,8 +3586,9 @@ int upload_pbegin(trn_viewset* vs, cudaStream_t st) {
 
 // The scene's cached one-view set, re-pointed at `cam`: the first call
 // allocates it, later calls only restage the view table (a pinned slot of
-// the set's staging ring), so single-view calls neither allocate nor
-// synchronise the stream.
+// the set's staging ring). A call for more samples than any before it grows the
+// set's round buffers (ensure_queue), which waits for the stream; others neither
+// allocate nor wait.
 int single_view(trn_scene* s, const trn_camera* cam, trn_viewset** out) {
   if (!cam) { set_error("null camera"); return -1; }
   trn_view v;
@@ -3735,9 +3738,9 @@ int trn_render_grad(trn_scene* s, const trn_camera* cam, const trn_render_option
 // ---------------------------------------------------------------------------
 // Allocation-free single-view gradient.
 //
-// trn_render_grad allocates device memory (the scene's one-view table, work
-// counter and silhouette-edge distribution) on a scene's first single-view
-// call. Callers that may not allocate (a host that forbids cudaMalloc
+// trn_render_grad allocates device memory: the scene's one-view table, work
+// counter and silhouette-edge distribution on a scene's first single-view call,
+// and round buffers whenever a call has more samples than those before. Callers that may not allocate (a host that forbids cudaMalloc
 // between set-up and teardown, a caching allocator that must not be bypassed,
 // a real-time loop that cannot afford the implicit synchronisation of
 // cudaFree) use trn_render_grad_noalloc instead: all of its scratch lives in

@@ -101,12 +101,12 @@ struct trn_scene {
   float* g_vnormal = nullptr;     // [V][3] dL/d(vertex normal)
   float* g_texels = nullptr;      // [ntexel][3]
   float* g_translation = nullptr; // [M][3]
-  int* err = nullptr;             // device error word
+  int* err = nullptr;             // device error word: checks that the sizes of the buffers and the tree's height exclude
   unsigned long long* stats = nullptr;  // [16] work counters of the integrator kernels
   bool stats_on = false;
   float h_light_integral = 0.f;
   bool configured = false;
-  bool built = false;             // an LBVH topology exists (refit possible)
+  bool built = false;             // a BVH topology exists (refit possible)
   bool grads_finalized = true;
   // bumped by every change of parameters or geometry: path records of an
   // older version are not reused

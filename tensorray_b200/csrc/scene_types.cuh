@@ -12,7 +12,7 @@
 //   bsdf_id    [T]    i32  material per triangle (mSbtIndexBuffer)
 //   emitter_id [T]    i32  area-light id or -1 (mEmitterIDBuffer)
 //   tri_verts  [T]    LeafTri  leaf-ordered triangles for traversal
-//   nodes      [T-1]  BvhNode  binary LBVH, child boxes stored in the parent
+//   nodes      [T-1]  BvhNode  binary BVH, child boxes stored in the parent
 #pragma once
 #include "common.cuh"
 

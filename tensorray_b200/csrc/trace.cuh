@@ -1,4 +1,4 @@
-// Ray queries against the project LBVH: closest hit and occlusion.
+// Ray queries against the project's BVH: closest hit and occlusion.
 //
 // Replaces the OptiX ray-query seam RayIntersectOptix (LibTensorRay/Renderer/
 // Optix.cpp:252-305) and its programs (ptx.cu:61-113). Hit semantics:

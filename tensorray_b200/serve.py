@@ -39,9 +39,9 @@ PHASE_FWD, PHASE_GRAD, PHASE_FINISH, PHASE_DONE = 0, 1, 2, 3
 ALL_TERMS = (TRN_PATH_TRACER, TRN_PRIMARY_EDGE, TRN_DIRECT_EDGE, TRN_INDIRECT_EDGE, TRN_PIXEL_EDGE)
 
 # Device bytes a view set holds for the wavefront's round buffers (one round: 16M
-# samples, at most 341 bytes each at depth <= 8) and for the boundary set-up's
+# samples, at most 205 bytes each at depth <= 8) and for the boundary set-up's
 # run order (16 bytes per slot plus the sort's temporary storage).
-VIEWSET_QUEUE_BYTES = 6_000_000_000
+VIEWSET_QUEUE_BYTES = 4_000_000_000
 
 
 @dataclass
