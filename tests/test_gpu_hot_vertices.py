@@ -40,5 +40,5 @@ def test_sums_of_hot_vertices_keep_their_values(built_lib):
         total += sc.get_grads()["positions"][-8:].double().cpu()
     ref = torch.tensor(HOT, dtype=torch.float64)
     scale = ref.abs().clamp_min(RMS)
-    # single runs lie within 0.3 % of the values; the changes above lie at 0.9 %
-    assert float(((total / runs - ref).abs() / scale).max()) < 4e-3
+    # the mean of four runs lies within 0.1 % of the values, the changes above at 0.9 %
+    assert float(((total / runs - ref).abs() / scale).max()) < 3e-3
