@@ -40,8 +40,10 @@ ALL_TERMS = (TRN_PATH_TRACER, TRN_PRIMARY_EDGE, TRN_DIRECT_EDGE, TRN_INDIRECT_ED
 
 # Device bytes a view set holds for the wavefront's round buffers (one round: 16M
 # samples, at most 205 bytes each at depth <= 8) and for the boundary set-up's
-# run order (16 bytes per slot plus the sort's temporary storage).
+# run order (16 bytes per slot plus the sort's temporary storage): 3.7 GB, and 5.4
+# GB when it is reserved for deeper paths.
 VIEWSET_QUEUE_BYTES = 4_000_000_000
+VIEWSET_QUEUE_BYTES_DEEP = 5_600_000_000
 
 
 @dataclass
@@ -91,7 +93,7 @@ class Server:
         # created (deeper requests still run; their first batch grows them)
         self.max_depth = int(max_depth)
         # the view set of every scene holds one round of buffers
-        self.reserve = len(scenes) * VIEWSET_QUEUE_BYTES
+        self.reserve = len(scenes) * (VIEWSET_QUEUE_BYTES if self.max_depth <= 8 else VIEWSET_QUEUE_BYTES_DEEP)
         self.budget = int(hbm_budget_bytes) - self.reserve
         self.chunk_spp = chunk_spp
         self.iter_samples = int(iter_samples)
