@@ -2214,12 +2214,12 @@ __global__ void __launch_bounds__(256, TRN_MINB) k_pixel_adj(TRN_KPARAMS) {
 // lost in the large running sum depends on how many lanes' adds are summed
 // before them and on their order. A scatter of 32 queued samples at a time, all
 // of one bounce before those of the next, moved nearly cancelling components of
-// the 16.8M-sample gradient by 2 % of its RMS (0.1 % between two runs).
+// the 16.8M-sample gradient by 1 to 2 % of its RMS (0.1 % between two runs).
 // And few samples pass: 0.5M slots of depth 12 take 0.69, 3.0 and 1.4 ms for
 // direct, indirect and pixel here, and 0.92, 3.8 and 1.9 with two launches per
 // bounce. The wavefront was ahead for many slots (16.8M of depth 5: primary 11.2
-// and here 11.8, direct 2.4 and 2.2, indirect 28.6 and 30.3, pixel 16.0 and
-// 19.2).
+// and here 11.8, direct 2.4 and 2.2, indirect 28.6 and 30.4, pixel 16.0 and
+// 18.7).
 
 // Slot of a sample in its launch, which indexes a caller's sample table.
 TRN_D long long item_gslot(const Params& P, const ViewDesc& V, long long p) {

@@ -11,7 +11,8 @@
 // and a shading warp holds 32 paths at the same bounce. 16.8M samples of depth
 // 5 on 102,400 triangles, one thread per path and here: image 27.6 and 15.8 ms.
 //
-// The price is a launch pair per bounce, each as long as its longest ray.
+// The price is a launch pair per bounce, each as long as its longest ray: the
+// late bounces of few paths run in one kernel instead (WaveRun::tail_bounce).
 // (The paths of a boundary term's samples run in one kernel each, behind these
 // set-ups: render.cu says why.)
 //
@@ -24,7 +25,7 @@ struct Wave {
   float4 *ro, *rd;          // [2 cap] rays: origin + id bits, direction + end
   float4* hit[2];           // [cap] closest-hit results by ray id: tri, u, v, t
   unsigned char* occ;       // [cap] occlusion results by ray id
-  unsigned* list[2];        // [cap] active samples of a stage, ping-pong
+  unsigned* list[2];        // [cap] active samples of a stage, ping-pong; a set-up's samples by ray id
   float4* st[4];            // [cap] path state
   long long* p;             // [cap] view-local sample index
   int* view;                // [cap]
